@@ -36,7 +36,7 @@ def run(cmd):
 
 
 def build():
-    if not os.path.isdir(REF):
+    if not os.path.isfile(os.path.join(REF, "layer.cu")):
         print("reference sources not present; keeping prebuilt oracle/_ref if any")
         return False
     os.makedirs(OUT, exist_ok=True)
