@@ -841,7 +841,7 @@ int Network::readTensor(int l, int kind, float* dst_h, size_t count) {
     }
     NET_TRY(synchronize());
     const void* src = kind == VDNN_TENSOR_WEIGHT ? layer[l]->FilterData() : layer[l]->BiasData();
-    NET_CU(cudaMemcpy(dst_h, src, count * sizeof(float), cudaMemcpyDeviceToHost));
+    NET_CU(hostCopy.to_host(dst_h, src, count * sizeof(float), device));
     return VDNN_OK;
 }
 
@@ -851,7 +851,7 @@ int Network::writeTensor(int l, int kind, const float* src_h, size_t count) {
     if (ctx.dry_run) return VDNN_ERR_STATE;
     NET_TRY(synchronize());
     void* dst = kind == VDNN_TENSOR_WEIGHT ? layer[l]->FilterData() : layer[l]->BiasData();
-    NET_CU(cudaMemcpy(dst, src_h, count * sizeof(float), cudaMemcpyHostToDevice));
+    NET_CU(hostCopy.to_device(dst, src_h, count * sizeof(float), device));
     return VDNN_OK;
 }
 

@@ -7,6 +7,7 @@
 #include <string>
 #include <vector>
 
+#include "host_copy.h"
 #include "layer.h"
 
 class Network {
@@ -130,6 +131,7 @@ private:
     bool                externalInput;
     bool                forwardDone;
     uint64_t            stepCounter;
+    vdnn::HostCopy      hostCopy;              // readTensor / writeTensor
     float*              stage_h;               // pinned staging for generated input / labels
     double*             loss_h;
     cudaEvent_t         ev_fwd_t0, ev_fwd_t1;  // timing events around the forward pass (eager offload budget)
