@@ -328,23 +328,35 @@ __global__ void __launch_bounds__(256) bwd_bias_narrow_kernel(int n, int k, int 
 }
 
 // ---------------------------------------------------------------- max pooling
-__global__ void __launch_bounds__(kThreads) maxpool_fwd_generic(int planes, int h, int w, int P, int Q, int wh, int ww,
+// One thread per output; the flat index is taken apart with multiplications (a 64-bit division per output was a third of the
+// time of this kernel).  WIN > 0: square window of that size, unrolled, so its loads are in flight together; 0: any window.
+// Bound by L1 (a stride-2 row touches every line twice): 64 x 96 x 55 x 55, 3 x 3 / 2: 44.3 us before, 17 now.
+template <int WIN>
+__global__ void __launch_bounds__(kThreads) maxpool_fwd_generic(uint32_t total, int h, int w, FastDiv div_p, FastDiv div_q, int wh, int ww,
                                                                 int sh, int sw, const float* __restrict__ x,
                                                                 float* __restrict__ y) {
-    const size_t total = static_cast<size_t>(planes) * P * Q;
-    const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
-    for (size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total; idx += stride) {
-        const int q = static_cast<int>(idx % Q);
-        const size_t t = idx / Q;
-        const int p = static_cast<int>(t % P);
-        const size_t plane = t / P;
-        const float* xp = x + plane * h * w + static_cast<size_t>(p * sh) * w + q * sw;
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += stride) {
+        uint32_t t, q, plane, p;
+        div_q.divmod(idx, t, q);
+        div_p.divmod(t, plane, p);
+        const float* xp = x + static_cast<size_t>(plane) * h * w + static_cast<size_t>(p * sh) * w + q * sw;
         float m = -INFINITY;
-        for (int i = 0; i < wh; ++i)
-            for (int j = 0; j < ww; ++j) {
-                const float v = xp[i * w + j];
-                if (v > m) m = v;
-            }
+        if (WIN > 0) {
+            float v[WIN > 0 ? WIN * WIN : 1];
+#pragma unroll
+            for (int i = 0; i < WIN; ++i)
+#pragma unroll
+                for (int j = 0; j < WIN; ++j) v[i * WIN + j] = __ldg(xp + i * w + j);
+#pragma unroll
+            for (int i = 0; i < WIN * WIN; ++i) if (v[i] > m) m = v[i];
+        } else {
+            for (int i = 0; i < wh; ++i)
+                for (int j = 0; j < ww; ++j) {
+                    const float v = xp[i * w + j];
+                    if (v > m) m = v;
+                }
+        }
         y[idx] = m;
     }
 }
@@ -367,42 +379,113 @@ __global__ void __launch_bounds__(kThreads) maxpool_fwd_2x2(size_t pairs, int w,
     }
 }
 
-// Gather form: one thread per input element; for each window that contains it, recompute the
-// window's first maximum and take dy if this element is it.  No atomics, no pre-zeroing.
-__global__ void __launch_bounds__(kThreads) maxpool_bwd_generic(int planes, int h, int w, int P, int Q, int wh, int ww,
-                                                                int sh, int sw, const float* __restrict__ dy,
-                                                                const float* __restrict__ x, float* __restrict__ dx) {
-    const size_t total = static_cast<size_t>(planes) * h * w;
-    const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
-    for (size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total; idx += stride) {
-        const int iw = static_cast<int>(idx % w);
-        const size_t t = idx / w;
-        const int ih = static_cast<int>(t % h);
-        const size_t plane = t / h;
-        const float* xp = x + plane * h * w;
-        const float* dyp = dy + plane * P * Q;
-        int p_lo = ih - wh + 1 <= 0 ? 0 : (ih - wh + 1 + sh - 1) / sh;
-        int p_hi = ih / sh; if (p_hi > P - 1) p_hi = P - 1;
-        int q_lo = iw - ww + 1 <= 0 ? 0 : (iw - ww + 1 + sw - 1) / sw;
-        int q_hi = iw / sw; if (q_hi > Q - 1) q_hi = Q - 1;
-        float g = 0.0f;
-        for (int p = p_lo; p <= p_hi; ++p)
-            for (int q = q_lo; q <= q_hi; ++q) {
-                float m = -INFINITY;
-                int bi = 0, bj = 0;
-                for (int i = 0; i < wh; ++i)
-                    for (int j = 0; j < ww; ++j) {
-                        const float v = xp[static_cast<size_t>(p * sh + i) * w + q * sw + j];
-                        if (v > m) { m = v; bi = i; bj = j; }
-                    }
-                if (p * sh + bi == ih && q * sw + bj == iw) g += dyp[static_cast<size_t>(p) * Q + q];
+// Any window.  A block takes a band of dx rows of one plane: the x rows that the band's windows cover go to shared memory,
+// one thread per window finds the window's first maximum there and leaves its place and dy, and one thread per input
+// element (or 2 x 2 of them) adds up the few windows around it that point to it, in scan order.  x and dy are read and dx is written once,
+// in full rows, with no atomics and no pre-zeroed dx; the sums come out the same every time.
+// Before: overlapping windows zeroed dx and added with atomics (64 x 96 x 55 x 55, 3 x 3 / 2: 13.6 + 51.1 us, now 36),
+// others searched every window again for each of its elements (64 x 512 x 14 x 14, 2 x 2 / 2: 18 us, now 13).
+// WIN, STRIDE > 0: square window and stride known at compile time.
+template <int WIN, int STRIDE>
+__global__ void __launch_bounds__(kThreads) maxpool_bwd_band(int bands, int band_rows, int h, FastDiv div_w, FastDiv div_hw, int P, FastDiv div_q, int wh_, int ww_,
+                                                             int sh_, int sw_, const float* __restrict__ dy,
+                                                             const float* __restrict__ x, float* __restrict__ dx) {
+    extern __shared__ float smem[];
+    const int wh = WIN > 0 ? WIN : wh_, ww = WIN > 0 ? WIN : ww_, sh = STRIDE > 0 ? STRIDE : sh_, sw = STRIDE > 0 ? STRIDE : sw_;
+    const int w = div_w.d, Q = div_q.d;
+    const unsigned plane = blockIdx.x / bands, band = blockIdx.x - plane * bands;
+    const int r0 = band * band_rows, r1 = min(h, r0 + band_rows);
+    // windows that reach rows r0 .. r1 - 1, and the rows they cover
+    const int p0 = r0 < wh ? 0 : (r0 - wh) / sh + 1, p1 = min(P, (r1 - 1) / sh + 1);
+    const int np = max(0, p1 - p0);
+    const int x0 = p0 * sh, xrows = np > 0 ? (np - 1) * sh + wh : 0;
+    const float* xp = x + static_cast<size_t>(plane) * h * w;
+    const float* dyp = dy + static_cast<size_t>(plane) * P * Q;
+    float* dxp = dx + static_cast<size_t>(plane) * h * w;
+    float* xs = smem;                                           // [xrows][w]
+    const int rows_max = band_rows / sh + (wh + sh - 1) / sh + 1;        // windows rows of any band
+    float2* win = reinterpret_cast<float2*>(xs + (((rows_max - 1) * sh + wh) * w + 1) / 2 * 2);    // [np][Q] dy, place of the maximum
+    // dy first: its loads are in flight together with those of x
+#pragma unroll 2
+    for (int i = threadIdx.x; i < np * Q; i += kThreads) win[i].x = __ldg(dyp + p0 * Q + i);
+#pragma unroll 8
+    for (int i = threadIdx.x; i < xrows * w; i += kThreads) xs[i] = __ldg(xp + x0 * w + i);
+    __syncthreads();
+    for (int i = threadIdx.x; i < np * Q; i += blockDim.x) {
+        uint32_t p, q;
+        div_q.divmod(i, p, q);
+        const int o = p * sh * w + q * sw;
+        float m = -INFINITY;
+        int best = 0;                                           // position inside the window: row * ww + column
+#pragma unroll
+        for (int a = 0; a < (WIN > 0 ? WIN : wh); ++a)
+#pragma unroll
+            for (int b = 0; b < (WIN > 0 ? WIN : ww); ++b) {
+                const float v = xs[o + a * w + b];
+                if (v > m) { m = v; best = a * ww + b; }
             }
-        dx[idx] = g;
+        win[i].y = __int_as_float(best);
+    }
+    __syncthreads();
+    if (STRIDE == 2 && WIN <= 3) {
+        // a thread takes the 2 x 2 inputs below and right of a window origin (bands begin on even rows): every place of
+        // the (up to four) windows around them is known, so one read of a window serves all of its inputs
+        const int half_w = (w + 1) / 2, items = (r1 - r0 + 1) / 2 * half_w;
+        for (int i = threadIdx.x; i < items; i += blockDim.x) {
+            uint32_t a, b;
+            div_hw.divmod(i, a, b);
+            const int p = r0 / 2 + static_cast<int>(a), q = static_cast<int>(b);
+            auto window = [&](int pp, int qq, float* g) -> int {
+                if (pp < p0 || pp >= p1 || qq < 0 || qq >= Q) return -1;
+                const float2 v = win[(pp - p0) * Q + qq];
+                *g = v.x;
+                return __float_as_int(v.y);
+            };
+            float g11 = 0.f, g = 0.f, o00 = 0.f, o01 = 0.f, o10 = 0.f, o11 = 0.f;
+            if (WIN == 3) {
+                int k = window(p - 1, q - 1, &g);
+                if (k == 8) o00 += g;
+                k = window(p - 1, q, &g);
+                if (k == 6) o00 += g;
+                if (k == 7) o01 += g;
+                k = window(p, q - 1, &g);
+                if (k == 2) o00 += g;
+                if (k == 5) o10 += g;
+            }
+            const int k = window(p, q, &g11);
+            if (k == 0) o00 += g11;
+            if (k == 1) o01 += g11;
+            if (k == WIN) o10 += g11;
+            if (k == WIN + 1) o11 += g11;
+            const int ih = 2 * p, iw = 2 * q;
+            float* o = dxp + static_cast<size_t>(ih) * w + iw;
+            o[0] = o00;
+            if (iw + 1 < w) o[1] = o01;
+            if (ih + 1 < r1) {
+                o[w] = o10;
+                if (iw + 1 < w) o[w + 1] = o11;
+            }
+        }
+        return;
+    }
+    for (int i = threadIdx.x; i < (r1 - r0) * w; i += blockDim.x) {
+        uint32_t row, col;
+        div_w.divmod(i, row, col);
+        const int iw = col, ih = r0 + row;
+        const int pl = max(p0, ih < wh ? 0 : (ih - wh) / sh + 1), ph = min(p1 - 1, ih / sh);
+        const int ql = iw < ww ? 0 : (iw - ww) / sw + 1, qh = min(Q - 1, iw / sw);
+        float g = 0.0f;
+        for (int p = pl; p <= ph; ++p)
+            for (int q = ql; q <= qh; ++q) {
+                const float2 v = win[(p - p0) * Q + q];
+                if (__float_as_int(v.y) == (ih - p * sh) * ww + iw - q * sw) g += v.x;
+            }
+        dxp[r0 * w + i] = g;
     }
 }
 
-// Overlapping windows (AlexNet's 3x3 / stride 2): one thread per window finds its first maximum once and adds dy
-// there; dx is zeroed beforehand.  An input element collects at most four contributions, in arbitrary order.
+// Windows too large for a band in shared memory: one thread per window finds its first maximum and adds dy there; dx is
+// zeroed beforehand.  An input element's contributions are added in arbitrary order.
 __global__ void __launch_bounds__(kThreads) maxpool_bwd_scatter(int planes, int h, int w, int P, int Q, int wh, int ww,
                                                                 int sh, int sw, const float* __restrict__ dy,
                                                                 const float* __restrict__ x, float* __restrict__ dx) {
@@ -641,44 +724,79 @@ __global__ void __launch_bounds__(kThreads) lrn_bwd_kernel(int n, int c, int hw,
     }
 }
 
-// Window of 5 (the AlexNet setting): one pass over the channels per position.  Channel j's scale s_j and
-// t_j = dy_j * y_j / s_j are produced once and kept in a five-entry shift register; channel i = j - 2 is finished
-// as soon as t_{i+2} exists:  dx_i = dy_i * s_i^-beta - 2*alpha*beta/n * x_i * sum_{|j-i|<=2} t_j.
-__global__ void __launch_bounds__(kThreads) lrn_bwd_win5_kernel(int n, int c, int hw, float alpha_over_n, float beta, float k,
-                                                                const float* __restrict__ x, const float* __restrict__ y,
-                                                                const float* __restrict__ dy, float* __restrict__ dx) {
-    const size_t total = static_cast<size_t>(n) * hw;
-    const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
-    for (size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total; idx += stride) {
-        const size_t in = idx / hw;
-        const size_t base = in * c * hw + (idx - in * hw);
-        float t[5] = {0.f, 0.f, 0.f, 0.f, 0.f};     // t[4] newest (channel j), t[0] = channel j - 4
-        float sc[3] = {k, k, k};                     // scales of channels j-2 (sc[0]), j-1, j
-        float xq[5] = {0.f, 0.f, 0.f, 0.f, 0.f};     // x of channels j-2 .. j+2, for the sliding sum of squares
-        // prime x window for j = 0: channels 0..2 at xq[2..4]
-        for (int m = 0; m < 3; ++m) xq[2 + m] = m < c ? x[base + static_cast<size_t>(m) * hw] : 0.0f;
-        for (int j = 0; j < c + 2; ++j) {
-            if (j < c) {
-                const float ss = xq[0] * xq[0] + xq[1] * xq[1] + xq[2] * xq[2] + xq[3] * xq[3] + xq[4] * xq[4];
-                const float sj = fmaf(alpha_over_n, ss, k);
-                const size_t o = base + static_cast<size_t>(j) * hw;
-                t[0] = t[1]; t[1] = t[2]; t[2] = t[3]; t[3] = t[4];
-                t[4] = dy[o] * y[o] / sj;
-                sc[0] = sc[1]; sc[1] = sc[2]; sc[2] = sj;
-            } else {
-                t[0] = t[1]; t[1] = t[2]; t[2] = t[3]; t[3] = t[4]; t[4] = 0.0f;
-                sc[0] = sc[1]; sc[1] = sc[2];
-            }
-            const int i = j - 2;
-            if (i >= 0) {
-                // x_i sits at xq[0] (the window is centred on j = i + 2)
-                const size_t o = base + static_cast<size_t>(i) * hw;
-                dx[o] = dy[o] * powf(sc[0], -beta) - 2.0f * alpha_over_n * beta * xq[0] * (t[0] + t[1] + t[2] + t[3] + t[4]);
-            }
-            // slide the x window to be centred on j + 1
-            xq[0] = xq[1]; xq[1] = xq[2]; xq[2] = xq[3]; xq[3] = xq[4];
-            xq[4] = (j + 3 < c) ? x[base + static_cast<size_t>(j + 3) * hw] : 0.0f;
-        }
+// s^-beta and, where asked for, 1 / s, for the scale s >= k > 0 of a position.  beta = 0.75 (AlexNet's, and the default of
+// the callers) takes two square roots instead of powf: r = s^-1/2, s^-3/4 = r * sqrt(r), 1 / s = r * r, each within a few
+// units in the last place like powf itself.
+template <bool BETA34>
+__device__ __forceinline__ float lrn_pow(float s, float beta, float* inv_s) {
+    if (BETA34) {
+        const float r = rsqrtf(s);
+        if (inv_s) *inv_s = r * r;
+        return r * sqrtf(r);
+    }
+    if (inv_s) *inv_s = 1.0f / s;
+    return powf(s, -beta);
+}
+
+// Window of 5 (the AlexNet setting).  Bound by memory: forward reads x and writes y, backward reads x and dy and writes dx.
+// A thread takes LRN_CH channels of one position; their x (with two neighbours on either side, for backward four) is loaded
+// at once, so the loads of a thread are in flight together and there are c / LRN_CH times as many threads as positions;
+// adjacent chunks of a block of positions sit in one block, so the overlap is read from L1.  One thread per position,
+// walking all channels with one load in flight and a powf per channel, took 128.9 us forward and 272.5 backward for
+// 64 x 96 x 55 x 55 (1.15 and 1.09 TB/s); now 31 and 49.
+constexpr int LRN_CH = 16, LRN_POS = 64, LRN_CHUNKS = 4;
+template <bool BETA34>
+__global__ void __launch_bounds__(LRN_POS * LRN_CHUNKS) lrn_fwd_win5_kernel(int c, int hw, float alpha_over_n, float beta, float k,
+                                                                            const float* __restrict__ x, float* __restrict__ y) {
+    const int pos = blockIdx.x * LRN_POS + threadIdx.x, c0 = (blockIdx.y * LRN_CHUNKS + threadIdx.y) * LRN_CH;
+    if (pos >= hw || c0 >= c) return;
+    const size_t base = static_cast<size_t>(blockIdx.z) * c * hw + pos;
+    float v[LRN_CH + 4];
+#pragma unroll
+    for (int j = 0; j < LRN_CH + 4; ++j) {
+        const int ch = c0 + j - 2;
+        v[j] = ch >= 0 && ch < c ? __ldg(x + base + static_cast<size_t>(ch) * hw) : 0.0f;
+    }
+#pragma unroll
+    for (int j = 0; j < LRN_CH; ++j) {
+        if (c0 + j >= c) break;
+        const float ss = (v[j] * v[j] + v[j + 1] * v[j + 1]) + (v[j + 2] * v[j + 2] + v[j + 3] * v[j + 3]) + v[j + 4] * v[j + 4];
+        y[base + static_cast<size_t>(c0 + j) * hw] = v[j + 2] * lrn_pow<BETA34>(fmaf(alpha_over_n, ss, k), beta, nullptr);
+    }
+}
+
+// dx_i = dy_i * s_i^-beta - 2*alpha*beta/n * x_i * sum_{|j-i|<=2} t_j with t_j = dy_j * y_j / s_j.  y_j = x_j * s_j^-beta is
+// formed again from x, which is read anyway: one tensor less to read.
+template <bool BETA34>
+__global__ void __launch_bounds__(LRN_POS * LRN_CHUNKS) lrn_bwd_win5_kernel(int c, int hw, float alpha_over_n, float beta, float k,
+                                                                            const float* __restrict__ x, const float* __restrict__ dy,
+                                                                            float* __restrict__ dx) {
+    const int pos = blockIdx.x * LRN_POS + threadIdx.x, c0 = (blockIdx.y * LRN_CHUNKS + threadIdx.y) * LRN_CH;
+    if (pos >= hw || c0 >= c) return;
+    const size_t base = static_cast<size_t>(blockIdx.z) * c * hw + pos;
+    float v[LRN_CH + 8], g[LRN_CH + 4];
+#pragma unroll
+    for (int j = 0; j < LRN_CH + 8; ++j) {
+        const int ch = c0 + j - 4;
+        v[j] = ch >= 0 && ch < c ? __ldg(x + base + static_cast<size_t>(ch) * hw) : 0.0f;
+    }
+#pragma unroll
+    for (int j = 0; j < LRN_CH + 4; ++j) {
+        const int ch = c0 + j - 2;
+        g[j] = ch >= 0 && ch < c ? __ldg(dy + base + static_cast<size_t>(ch) * hw) : 0.0f;
+    }
+    const float f = 2.0f * alpha_over_n * beta;
+    float t[5] = {0.f, 0.f, 0.f, 0.f, 0.f}, pw[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < LRN_CH + 4; ++j) {                      // channel c0 + j - 2: x at v[j + 2], dy at g[j]
+        const float ss = (v[j] * v[j] + v[j + 1] * v[j + 1]) + (v[j + 2] * v[j + 2] + v[j + 3] * v[j + 3]) + v[j + 4] * v[j + 4];
+        float inv;
+        pw[0] = pw[1]; pw[1] = pw[2];
+        pw[2] = lrn_pow<BETA34>(fmaf(alpha_over_n, ss, k), beta, &inv);
+        t[0] = t[1]; t[1] = t[2]; t[2] = t[3]; t[3] = t[4];
+        t[4] = g[j] * (v[j + 2] * pw[2]) * inv;                 // 0 outside the tensor: dy is
+        if (j >= 4 && c0 + j - 4 < c)                           // channel i = c0 + j - 4
+            dx[base + static_cast<size_t>(c0 + j - 4) * hw] = g[j - 2] * pw[0] - f * v[j] * (((t[0] + t[1]) + (t[2] + t[3])) + t[4]);
     }
 }
 
@@ -851,12 +969,24 @@ int vdnn_maxpool_fwd(int n, int c, int h, int w, int win_h, int win_w, int strid
     if (pool_fast_2x2(h, w, win_h, win_w, stride_h, stride_w, x, y, nullptr)) {
         const size_t pairs = static_cast<size_t>(planes) * P * (Q / 2);
         maxpool_fwd_2x2<<<stream_grid(pairs, 1), kThreads, 0, as_stream(stream)>>>(pairs, w, Q / 2, x, y);
-    } else {
-        const size_t total = static_cast<size_t>(planes) * P * Q;
-        maxpool_fwd_generic<<<stream_grid(total, 1), kThreads, 0, as_stream(stream)>>>(planes, h, w, P, Q, win_h, win_w,
-                                                                                       stride_h, stride_w, x, y);
+        VDNN_LAUNCHED();
+        return VDNN_OK;
     }
-    VDNN_LAUNCHED();
+    const size_t out_plane = static_cast<size_t>(P) * Q, in_plane = static_cast<size_t>(h) * w;
+    const int per_launch = images_per_launch(planes, out_plane);          // 32-bit indexes inside a launch
+    if (per_launch < 1) return VDNN_ERR_UNSUPPORTED;
+    const FastDiv dp(P), dq(Q);
+    for (int p0 = 0; p0 < planes; p0 += per_launch) {
+        const uint32_t total = static_cast<uint32_t>((planes - p0 < per_launch ? planes - p0 : per_launch) * out_plane);
+        const float* xs = x + p0 * in_plane;
+        float* ys = y + p0 * out_plane;
+        const int grid = stream_grid(total, 1);
+        const int win = win_h == win_w ? win_h : 0;
+        if (win == 2) maxpool_fwd_generic<2><<<grid, kThreads, 0, as_stream(stream)>>>(total, h, w, dp, dq, 2, 2, stride_h, stride_w, xs, ys);
+        else if (win == 3) maxpool_fwd_generic<3><<<grid, kThreads, 0, as_stream(stream)>>>(total, h, w, dp, dq, 3, 3, stride_h, stride_w, xs, ys);
+        else maxpool_fwd_generic<0><<<grid, kThreads, 0, as_stream(stream)>>>(total, h, w, dp, dq, win_h, win_w, stride_h, stride_w, xs, ys);
+        VDNN_LAUNCHED();
+    }
     return VDNN_OK;
 }
 
@@ -870,14 +1000,32 @@ int vdnn_maxpool_bwd(int n, int c, int h, int w, int win_h, int win_w, int strid
     if (pool_fast_2x2(h, w, win_h, win_w, stride_h, stride_w, x, dx, dy)) {
         const size_t pairs = static_cast<size_t>(planes) * P * (Q / 2);
         maxpool_bwd_2x2<<<stream_grid(pairs, 1), kThreads, 0, as_stream(stream)>>>(pairs, w, Q / 2, dy, x, dx);
-    } else if (win_h > stride_h || win_w > stride_w) {
+        VDNN_LAUNCHED();
+        return VDNN_OK;
+    }
+    // rows of a band: about 16 KB of shared memory, so that a full set of blocks stays resident, but at least two rows
+    auto smem_of = [&](int rows) {
+        const size_t np = rows / stride_h + (win_h + stride_h - 1) / stride_h + 1;
+        return ((((np - 1) * stride_h + win_h) * w + 1) / 2 * 2 + 2 * np * Q) * sizeof(float);
+    };
+    int band = h;
+    while (band > 2 && smem_of(band) > 16 * 1024) band = (band + 1) / 2;
+    if (band < h) band = (band + 1) / 2 * 2;                             // bands begin on even rows
+    const size_t smem = smem_of(band);
+    const long long blocks = static_cast<long long>(planes) * ceil_div(h, band);
+    // a window so large that not even one row's share fits is outside what any network here has
+    if (smem <= 200 * 1024 && blocks <= 0x7fffffffLL) {
+        const int bands = ceil_div(h, band);
+        auto kern = maxpool_bwd_band<0, 0>;
+        if (win_h == win_w && stride_h == stride_w && stride_h == 2 && win_h == 3) kern = maxpool_bwd_band<3, 2>;
+        else if (win_h == win_w && stride_h == stride_w && stride_h == 2 && win_h == 2) kern = maxpool_bwd_band<2, 2>;
+        if (smem > 48 * 1024) VDNN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        kern<<<static_cast<unsigned>(blocks), kThreads, smem, as_stream(stream)>>>(bands, band, h, FastDiv(w), FastDiv((w + 1) / 2), P, FastDiv(Q), win_h, win_w, stride_h, stride_w,
+                                                                                  dy, x, dx);
+    } else {
         VDNN_CUDA(cudaMemsetAsync(dx, 0, static_cast<size_t>(planes) * h * w * sizeof(float), as_stream(stream)));
         const size_t total = static_cast<size_t>(planes) * P * Q;
         maxpool_bwd_scatter<<<stream_grid(total, 1), kThreads, 0, as_stream(stream)>>>(planes, h, w, P, Q, win_h, win_w,
-                                                                                       stride_h, stride_w, dy, x, dx);
-    } else {
-        const size_t total = static_cast<size_t>(planes) * h * w;
-        maxpool_bwd_generic<<<stream_grid(total, 1), kThreads, 0, as_stream(stream)>>>(planes, h, w, P, Q, win_h, win_w,
                                                                                        stride_h, stride_w, dy, x, dx);
     }
     VDNN_LAUNCHED();
@@ -920,25 +1068,47 @@ int vdnn_loss(int rows, int cols, const float* y, const float* label, double* ou
     return VDNN_OK;
 }
 
+// The chunked kernels of the 5-wide window: grid.z carries the images (longer batches go in several launches).
+static dim3 lrn_grid(int c, int hw) { return dim3(ceil_div(hw, LRN_POS), ceil_div(c, LRN_CH * LRN_CHUNKS), 1); }
+static bool lrn_chunked(int c, int win) { return win == 5 && ceil_div(c, LRN_CH * LRN_CHUNKS) <= 65535; }
+
 int vdnn_lrn_fwd(int n, int c, int hw, int win, float alpha, float beta, float k, const float* x, float* y,
                  void* stream) {
     if (!x || !y || n <= 0 || c <= 0 || hw <= 0 || win <= 0 || win % 2 == 0) return VDNN_ERR_BAD_ARG;
-    lrn_fwd_kernel<<<stream_grid(static_cast<size_t>(n) * hw, 1), kThreads, 0, as_stream(stream)>>>(
-        n, c, hw, win, alpha / win, beta, k, x, y);
-    VDNN_LAUNCHED();
+    if (!lrn_chunked(c, win)) {
+        lrn_fwd_kernel<<<stream_grid(static_cast<size_t>(n) * hw, 1), kThreads, 0, as_stream(stream)>>>(
+            n, c, hw, win, alpha / win, beta, k, x, y);
+        VDNN_LAUNCHED();
+        return VDNN_OK;
+    }
+    dim3 grid = lrn_grid(c, hw);
+    for (int n0 = 0; n0 < n; n0 += 65535) {
+        grid.z = n - n0 < 65535 ? n - n0 : 65535;
+        const size_t off = static_cast<size_t>(n0) * c * hw;
+        auto kern = beta == 0.75f ? lrn_fwd_win5_kernel<true> : lrn_fwd_win5_kernel<false>;
+        kern<<<grid, dim3(LRN_POS, LRN_CHUNKS), 0, as_stream(stream)>>>(c, hw, alpha / win, beta, k, x + off, y + off);
+        VDNN_LAUNCHED();
+    }
     return VDNN_OK;
 }
 
 int vdnn_lrn_bwd(int n, int c, int hw, int win, float alpha, float beta, float k, const float* x, const float* y,
                  const float* dy, float* dx, void* stream) {
     if (!x || !y || !dy || !dx || n <= 0 || c <= 0 || hw <= 0 || win <= 0 || win % 2 == 0) return VDNN_ERR_BAD_ARG;
-    if (win == 5)
-        lrn_bwd_win5_kernel<<<stream_grid(static_cast<size_t>(n) * hw, 1), kThreads, 0, as_stream(stream)>>>(
-            n, c, hw, alpha / win, beta, k, x, y, dy, dx);
-    else
+    if (!lrn_chunked(c, win)) {
         lrn_bwd_kernel<<<stream_grid(static_cast<size_t>(n) * hw, 1), kThreads, 0, as_stream(stream)>>>(
             n, c, hw, win, alpha / win, beta, k, x, y, dy, dx);
-    VDNN_LAUNCHED();
+        VDNN_LAUNCHED();
+        return VDNN_OK;
+    }
+    dim3 grid = lrn_grid(c, hw);
+    for (int n0 = 0; n0 < n; n0 += 65535) {
+        grid.z = n - n0 < 65535 ? n - n0 : 65535;
+        const size_t off = static_cast<size_t>(n0) * c * hw;
+        auto kern = beta == 0.75f ? lrn_bwd_win5_kernel<true> : lrn_bwd_win5_kernel<false>;
+        kern<<<grid, dim3(LRN_POS, LRN_CHUNKS), 0, as_stream(stream)>>>(c, hw, alpha / win, beta, k, x + off, dy + off, dx + off);
+        VDNN_LAUNCHED();
+    }
     return VDNN_OK;
 }
 
