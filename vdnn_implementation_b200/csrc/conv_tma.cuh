@@ -28,9 +28,7 @@
 // No load carries a cluster multicast qualifier, and every tensor map covers this GPU's own workspace only.
 #pragma once
 
-#include <cuda.h>
-
-#include "gemm_tc.cuh"
+#include "tensor_map.cuh"
 
 namespace vdnn {
 namespace tma {
@@ -41,8 +39,7 @@ using tc::BM;
 
 constexpr int DRAIN_WARPS = 16;
 constexpr int THREADS = (DRAIN_WARPS + 2) * 32;      // + the TMA warp and the MMA warp
-constexpr int BOX_PIXELS = 32, BOXES = BM / BOX_PIXELS;
-constexpr int BOX_BYTES = BOX_PIXELS * BK * 4;       // 4 KB: four swizzle atoms
+constexpr int BOXES = BM / BOX_PIXELS;
 constexpr int TR_PIX = 128;                          // pixels per block of the image transform passes
 
 template <int BN> struct Config {
@@ -341,11 +338,6 @@ __device__ __forceinline__ uint64_t make_desc_at(uint32_t saddr) {
     return tc::make_desc(saddr) | (static_cast<uint64_t>((saddr >> 7) & 7u) << 49);
 }
 
-__device__ __forceinline__ void tma_load_rows(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int row) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(row) : "memory");
-}
-
 template <int BN, int MH>
 __global__ void __launch_bounds__(THREADS, StripConfig<BN, MH>::CTAS_PER_SM)
 strip_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo, const StripParams p) {
@@ -463,7 +455,8 @@ strip_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__
         }
     } else if (warp == DRAIN_WARPS) {
         // ------------------------------------------------------------------ TMA producer: strips and weight tiles
-        if (lane == 0) {
+        const bool elected = tc::elect_one();
+        {
             const char* b_col = p.b_tiles + static_cast<size_t>(blockIdx.y) * p.kblocks_total * Cfg::B_STAGE_BYTES;
             unsigned i = 0, gcount = 0;                     // running k-block and strip counts (ring positions)
             bool ok = true;
@@ -481,28 +474,35 @@ strip_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__
                                           (p.inner == 1 ? p.row0 + p.row_step * s_first : 0);
                     const uint32_t abar = tc::smem_u32(&a_full[sa]);
                     const uint32_t ast = tc::smem_u32(tiles + sa * Cfg::A_STAGE_BYTES);
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(abar), "r"(MH * 2u * strip_bytes) : "memory");
+                    if (elected) {
+                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(abar), "r"(MH * 2u * strip_bytes) : "memory");
 #pragma unroll
-                    for (int h = 0; h < MH; ++h) {      // one strip pair (hi, lo) per 128-row half of the tile
-                        tma_load_rows(ast + h * 2 * STRIP_HALF_BYTES, &map_hi, abar, cb * BK, static_cast<int>(row) + h * BM);
-                        tma_load_rows(ast + h * 2 * STRIP_HALF_BYTES + STRIP_HALF_BYTES, &map_lo, abar, cb * BK, static_cast<int>(row) + h * BM);
+                        for (int h = 0; h < MH; ++h) {      // one strip pair (hi, lo) per 128-row half of the tile
+                            tma_load_rows(ast + h * 2 * STRIP_HALF_BYTES, &map_hi, abar, cb * BK, static_cast<int>(row) + h * BM);
+                            tma_load_rows(ast + h * 2 * STRIP_HALF_BYTES + STRIP_HALF_BYTES, &map_lo, abar, cb * BK, static_cast<int>(row) + h * BM);
+                        }
                     }
+                    __syncwarp();
                     for (int sx = 0; sx < p.inner; ++sx, ++i) {
                         const int sb = i % SB;
                         if (!tc::mbar_wait(tc::smem_u32(&b_empty[sb]), ((i / SB) & 1u) ^ 1u)) { ok = false; break; }
                         const int kb = (r * p.S + s_first + sx) * p.cblocks + cb;
                         const uint32_t bbar = tc::smem_u32(&b_full[sb]);
-                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bbar), "r"(Cfg::B_STAGE_BYTES) : "memory");
-                        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                                     ::"r"(tc::smem_u32(b_ring + sb * Cfg::B_STAGE_BYTES)), "l"(b_col + static_cast<size_t>(kb) * Cfg::B_STAGE_BYTES),
-                                       "r"(Cfg::B_STAGE_BYTES), "r"(bbar) : "memory");
+                        if (elected) {
+                            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bbar), "r"(Cfg::B_STAGE_BYTES) : "memory");
+                            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                                         ::"r"(tc::smem_u32(b_ring + sb * Cfg::B_STAGE_BYTES)), "l"(b_col + static_cast<size_t>(kb) * Cfg::B_STAGE_BYTES),
+                                           "r"(Cfg::B_STAGE_BYTES), "r"(bbar) : "memory");
+                        }
+                        __syncwarp();
                     }
                 }
             }
             if (!ok) atomicCAS(&tc::g_tc_error, 0, 101);
         }
-    } else if (lane == 0) {
-        // ------------------------------------------------------------------ MMA issuer
+    } else {
+        // ------------------------------------------------------------------ MMA issuer (tc::elect_one)
+        const bool elected = tc::elect_one();
         unsigned i = 0, gcount = 0, pair = 0;
         bool ok = true;
         for (long long tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
@@ -523,6 +523,7 @@ strip_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__
                     const uint32_t b_hi = tc::smem_u32(b_ring + sb * Cfg::B_STAGE_BYTES);
                     const uint32_t b_lo = b_hi + Cfg::B_TILE_BYTES;
                     const uint64_t dbh = tc::make_desc(b_hi), dbl = tc::make_desc(b_lo);
+                    if (elected) {
 #pragma unroll
                     for (int h = 0; h < MH; ++h) {      // the row halves share the weight operand
                         const uint32_t d_tmem = tmem_base + static_cast<uint32_t>((b * MH + h) * Cfg::ACC_COLS);
@@ -536,7 +537,10 @@ strip_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__
                     }
                     tc::mma_commit(tc::smem_u32(&b_empty[sb]));
                     if (sx == p.inner - 1) tc::mma_commit(tc::smem_u32(&a_empty[sa]));
-                    if (!first_of_pair || kb_in_tile == nkb - 1) { tc::mma_commit(tc::smem_u32(&acc_ready[b])); ++pair; }
+                    if (!first_of_pair || kb_in_tile == nkb - 1) tc::mma_commit(tc::smem_u32(&acc_ready[b]));
+                    }
+                    __syncwarp();
+                    if (!first_of_pair || kb_in_tile == nkb - 1) ++pair;
                 }
             }
         }
@@ -647,22 +651,6 @@ struct WgradParams {
     int mode;
     size_t partial_stride;
 };
-
-// Shared-memory descriptor of an MN-major tf32 operand made of 32-wide strips.  32-bit operands can only be read
-// MN-major in the "128-byte swizzle with 32-byte atoms" layout: rows of 128 bytes (one pixel, 32 channels) whose
-// 32-byte quarters are XORed with the row number modulo 4, the pattern repeating every 4 rows (512 bytes); the TMA
-// unit writes exactly that with CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B.  One MMA takes 8 pixels = two such groups, 512
-// bytes apart (stride dimension); strips of 32 rows / columns (one TMA box each) follow each other at BOX_BYTES
-// (leading dimension).  Descriptor version 1, layout type 1.
-__device__ __forceinline__ uint64_t make_desc_mn(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);
-    d |= static_cast<uint64_t>(BOX_BYTES >> 4) << 16;
-    d |= static_cast<uint64_t>(512 >> 4) << 32;
-    d |= static_cast<uint64_t>(1) << 46;
-    d |= static_cast<uint64_t>(1) << 61;
-    return d;
-}
 
 // MH = 128-row halves of a tile (MH * four row groups).  A tile's dy slice (BN * 256 bytes per k block) is fetched once
 // for all its rows, and the SM's ingest rate is what bounds the narrow tiles: with 128 or 64 filters a CTA takes two
@@ -817,7 +805,8 @@ wgrad_kernel(const __grid_constant__ CUtensorMap x_hi, const __grid_constant__ C
                 }
             }
         }
-    } else if (lane == 0) {
+    } else {
+        const bool elected = tc::elect_one();
         for (int i = 0; i < nkb; ++i) {
             const int s = i % S, pair = i >> 1, b = pair & 1;
             const uint32_t phase = static_cast<uint32_t>(i / S) & 1u;
@@ -832,6 +821,7 @@ wgrad_kernel(const __grid_constant__ CUtensorMap x_hi, const __grid_constant__ C
             const uint32_t b_hi = a0 + Cfg::A_BYTES;
             const uint32_t b_lo = b_hi + Cfg::B_TILE_BYTES;
             const uint64_t dbh = make_desc_mn(b_hi), dbl = make_desc_mn(b_lo);
+            if (elected) {
 #pragma unroll
             for (int h = 0; h < MH; ++h) {      // the row halves share the dy slice
                 const uint32_t a_hi = a0 + h * 2 * A_TILE_BYTES, a_lo = a_hi + A_TILE_BYTES;
@@ -841,6 +831,8 @@ wgrad_kernel(const __grid_constant__ CUtensorMap x_hi, const __grid_constant__ C
             }
             tc::mma_commit(tc::smem_u32(&bars[S + s]));
             if ((i & 1) || i == nkb - 1) tc::mma_commit(tc::smem_u32(&bars[2 * S + b]));
+            }
+            __syncwarp();
         }
     }
 
@@ -910,22 +902,6 @@ __global__ void __launch_bounds__(256) nchw_to_split_nhwc_kernel(const float* __
             if (lane == 0) atomicAdd(sums + c0 + warp * 4 + j, scale * v);
         }
     }
-}
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-// cuTensorMapEncodeTiled from the driver the runtime is bound to (the library links no libcuda stub).
-inline EncodeTiledFn encode_tiled() {
-    static EncodeTiledFn fn = []() -> EncodeTiledFn {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
-            return nullptr;
-        return reinterpret_cast<EncodeTiledFn>(f);
-    }();
-    return fn;
 }
 
 // Tensor map over a channels-last image [n][h][w][c] (fp32, dense) with boxes of 32 channels x bw x bh pixels of one

@@ -224,8 +224,9 @@ strip_pair_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_const
             }
             if (!ok) atomicCAS(&tc::g_tc_error, 0, 101);
         }
-    } else if (lane == 0 && leader) {
-        // ------------------------------------------------------------------ MMA issuer of the pair
+    } else if (leader) {
+        // ------------------------------------------------------------------ MMA issuer of the pair (tc::elect_one)
+        const bool elected = tc::elect_one();
         unsigned i = 0, gcount = 0, pair = 0;
         bool ok = true;
         for (long long tile = pair_id; tile < num_tiles && ok; tile += num_pairs) {
@@ -244,11 +245,16 @@ strip_pair_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_const
                     const uint32_t a_lo = a_hi + STRIP_HALF_BYTES;
                     const uint32_t b_hi = tc::smem_u32(b_ring + sb * Cfg::B_STAGE_BYTES);
                     const uint32_t b_lo = b_hi + Cfg::B_TILE_BYTES;
-                    mma_block_3xtf32_2cta<2>(tmem_base + static_cast<uint32_t>(b * BNP), tc::make_desc(a_hi), tc::make_desc(a_lo),
-                                             tc::make_desc(b_hi), tc::make_desc(b_lo), first_of_pair, Cfg::IDESC);
-                    mma_commit_both(tc::smem_u32(&b_empty[sb]));
-                    if (sx == p.S - 1) mma_commit_both(tc::smem_u32(&a_empty[sa]));
-                    if (!first_of_pair || kb_in_tile == nkb - 1) { mma_commit_both(tc::smem_u32(&acc_ready[b])); ++pair; }
+                    const uint64_t dah = tc::make_desc(a_hi), dal = tc::make_desc(a_lo), dbh = tc::make_desc(b_hi), dbl = tc::make_desc(b_lo);
+                    const bool last_of_pair = !first_of_pair || kb_in_tile == nkb - 1;
+                    if (elected) {
+                        mma_block_3xtf32_2cta<2>(tmem_base + static_cast<uint32_t>(b * BNP), dah, dal, dbh, dbl, first_of_pair, Cfg::IDESC);
+                        mma_commit_both(tc::smem_u32(&b_empty[sb]));
+                        if (sx == p.S - 1) mma_commit_both(tc::smem_u32(&a_empty[sa]));
+                        if (last_of_pair) mma_commit_both(tc::smem_u32(&acc_ready[b]));
+                    }
+                    __syncwarp();
+                    if (last_of_pair) ++pair;
                 }
             }
         }
@@ -507,7 +513,8 @@ wgrad_pair_kernel(const __grid_constant__ CUtensorMap x_hi, const __grid_constan
                 }
             }
         }
-    } else if (lane == 0 && leader) {
+    } else if (leader) {
+        const bool elected = tc::elect_one();
         for (int i = 0; i < nkb; ++i) {
             const int s = i % S, pair = i >> 1, b = pair & 1;
             const uint32_t phase = static_cast<uint32_t>(i / S) & 1u;
@@ -522,10 +529,13 @@ wgrad_pair_kernel(const __grid_constant__ CUtensorMap x_hi, const __grid_constan
             const uint32_t b_hi = a_hi + 2 * A_TILE_BYTES;
             const uint32_t b_lo = b_hi + WCfg::B_TILE_BYTES;
             // one k slice = 8 pixels = 1024 bytes further into every strip
-            mma_block_3xtf32_2cta<1024 / 16>(tmem_base + static_cast<uint32_t>(b * BNP), make_desc_mn(a_hi), make_desc_mn(a_lo),
-                                             make_desc_mn(b_hi), make_desc_mn(b_lo), !(i & 1), WCfg::IDESC_MN);
-            mma_commit_both(tc::smem_u32(&empty[s]));
-            if ((i & 1) || i == nkb - 1) mma_commit_both(tc::smem_u32(&acc_ready[b]));
+            const uint64_t dah = make_desc_mn(a_hi), dal = make_desc_mn(a_lo), dbh = make_desc_mn(b_hi), dbl = make_desc_mn(b_lo);
+            if (elected) {
+                mma_block_3xtf32_2cta<1024 / 16>(tmem_base + static_cast<uint32_t>(b * BNP), dah, dal, dbh, dbl, !(i & 1), WCfg::IDESC_MN);
+                mma_commit_both(tc::smem_u32(&empty[s]));
+                if ((i & 1) || i == nkb - 1) mma_commit_both(tc::smem_u32(&acc_ready[b]));
+            }
+            __syncwarp();
         }
     }
 

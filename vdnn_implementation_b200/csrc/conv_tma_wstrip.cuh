@@ -176,7 +176,8 @@ wgrad_strip_kernel(const __grid_constant__ CUtensorMap x_hi, const __grid_consta
                 }
             }
         }
-    } else if (lane == 0) {
+    } else {
+        const bool elected = tc::elect_one();
         for (int i = 0; i < nkb; ++i) {
             const int s = i % S, pair = i >> 1, b = pair & 1;
             const uint32_t phase = static_cast<uint32_t>(i / S) & 1u;
@@ -190,6 +191,7 @@ wgrad_strip_kernel(const __grid_constant__ CUtensorMap x_hi, const __grid_consta
             const uint32_t b_hi = a0 + Cfg::A_BYTES;
             const uint32_t b_lo = b_hi + Cfg::B_TILE_BYTES;
             const uint64_t dbh = make_desc_mn(b_hi), dbl = make_desc_mn(b_lo);
+            if (elected) {
             for (int h = 0; h < my_tiles; ++h) {        // the tiles share the dy slice
                 const uint32_t a_hi = a0 + h * 2 * WSTRIP_A_HALF, a_lo = a_hi + WSTRIP_A_HALF;
                 // the four 32-row groups of the tile start one position (128 bytes) apart: taps s = 0 .. 3; one k slice =
@@ -199,6 +201,8 @@ wgrad_strip_kernel(const __grid_constant__ CUtensorMap x_hi, const __grid_consta
             }
             tc::mma_commit(tc::smem_u32(&empty[s]));
             if ((i & 1) || i == nkb - 1) tc::mma_commit(tc::smem_u32(&acc_ready[b]));
+            }
+            __syncwarp();
         }
     }
 

@@ -33,6 +33,7 @@ static_assert(PRODUCERS == 256 || PRODUCERS == 512, "producer mappings are writt
 constexpr int A_TILE_BYTES = BM * BK * 4;              // 16 KB, one per hi / lo
 constexpr unsigned long long SPIN_CYCLES = 4000000000ull;   // ~2 s at 1.9 GHz
 constexpr unsigned SPIN_TRIES = 1u << 26;
+constexpr unsigned SUSPEND_NS = 20000;      // a waiting warp may sleep this long in one try: polls take issue slots from its neighbours
 
 // 0 = healthy; otherwise 100 + role of the first wait that expired (1 producer, 2 mma, 3 epilogue, 4 the self-test).
 __device__ int g_tc_error = 0;
@@ -64,8 +65,8 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 // Bounded wait for the phase with the given parity.  Returns false when the limit expired.
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity), "r"(SUSPEND_NS) : "memory");
     return ok != 0;
 }
 __device__ __forceinline__ bool mbar_wait_for(uint32_t bar, uint32_t parity, unsigned long long cycles, unsigned tries) {
@@ -129,6 +130,15 @@ __device__ __forceinline__ void mma_block_3xtf32(uint32_t d_tmem, uint64_t dah, 
         mma_tf32_acc(d_tmem, dah, dbh, idesc);
     }
 }
+// One lane of a converged warp (the same one every time).  An issuing warp walks its loop with all lanes and lets this one
+// issue: loop counters, addresses and descriptors then stay in uniform registers.  With `if (lane == 0)` around the loop
+// the compiler has to move every descriptor from vector to uniform registers in front of each MMA: an MMA took 117 clocks
+// instead of 45 beside busy warps (dense kernel, 64 columns, 25088 -> 4096: 151 us, with this 111).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e != 0;
+}
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -156,6 +166,14 @@ __device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
 __device__ __forceinline__ void split_tf32_safe(float x, float& hi, float& lo) {
     hi = __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u);
     lo = (__float_as_uint(hi) & 0x7F800000u) == 0x7F800000u ? 0.0f : x - hi;
+}
+
+// Two values at once: the subtraction as one packed instruction (rounding and results as split_tf32).
+__device__ __forceinline__ void split_tf32_x2(float x0, float x1, float& h0, float& h1, float& l0, float& l1) {
+    h0 = __uint_as_float((__float_as_uint(x0) + 0x1000u) & 0xFFFFE000u);
+    h1 = __uint_as_float((__float_as_uint(x1) + 0x1000u) & 0xFFFFE000u);
+    asm("{\n\t.reg .b64 x, h, m, l;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 h, {%4, %5};\n\tmov.b64 m, {%6, %6};\n\t"
+        "fma.rn.f32x2 l, h, m, x;\n\tmov.b64 {%0, %1}, l;\n\t}" : "=f"(l0), "=f"(l1) : "f"(x0), "f"(x1), "f"(h0), "f"(h1), "f"(-1.0f));
 }
 
 // Gathers a ROWS x 32 operand tile into registers and stores its hi / lo images.
@@ -341,8 +359,9 @@ gemm_kernel(const OpA opa, const OpB opb, const Epilogue epi, int M, int N, int 
                 if (n < N) epi.store(roff, n, acc[j], blockIdx.z);
             }
         }
-    } else if (lane == 0) {
-        // ------------------------------------------------------------------ MMA issuer
+    } else {
+        // ------------------------------------------------------------------ MMA issuer (see elect_one)
+        const bool elected = elect_one();
         for (int i = 0; i < nkb; ++i) {
             const int s = i % S;
             const uint32_t phase = static_cast<uint32_t>(i / S) & 1u;
@@ -354,10 +373,14 @@ gemm_kernel(const OpA opa, const OpB opb, const Epilogue epi, int M, int N, int 
             const uint32_t b_lo = b_hi + Cfg::B_TILE_BYTES;
             // two consecutive k blocks share an accumulator buffer (a chain of 24 MMAs), then the other buffer is used
             const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(((i >> 1) & 1) * BN);
-            mma_block_3xtf32(d_tmem, make_desc(a_hi), make_desc(a_lo), make_desc(b_hi), make_desc(b_lo), Cfg::IDESC, !(i & 1));
-            mma_commit(smem_u32(&bars[S + s]));             // stage s may be overwritten once these finish
-            if ((i & 1) || i == nkb - 1)
-                mma_commit(smem_u32(&bars[2 * S + ((i >> 1) & 1)]));   // and this pair's sums may be collected
+            const uint64_t dah = make_desc(a_hi), dal = make_desc(a_lo), dbh = make_desc(b_hi), dbl = make_desc(b_lo);
+            if (elected) {
+                mma_block_3xtf32(d_tmem, dah, dal, dbh, dbl, Cfg::IDESC, !(i & 1));
+                mma_commit(smem_u32(&bars[S + s]));             // stage s may be overwritten once these finish
+                if ((i & 1) || i == nkb - 1)
+                    mma_commit(smem_u32(&bars[2 * S + ((i >> 1) & 1)]));   // and this pair's sums may be collected
+            }
+            __syncwarp();
         }
     }
 
