@@ -1,0 +1,39 @@
+"""SGEMM on operands that tensor copies can fetch (16-byte aligned columns), which run on the kernel with A in tensor memory:
+all orientations at tile edges, against the CPU oracle."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def dev(a):
+    return torch.from_numpy(np.ascontiguousarray(a, np.float32)).cuda()
+
+
+# m, n, k: one block; ragged in every dimension (column tiles of 32, 64 and 128); several tiles; a reduction long enough to split
+SIZES = [(4, 4, 4), (128, 32, 32), (132, 36, 40), (260, 68, 100), (12, 132, 36), (384, 256, 64), (516, 20, 2052), (1000, 60, 4100)]
+
+
+@pytest.mark.parametrize("algo", [0, 1])
+@pytest.mark.parametrize("trans", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("size", SIZES)
+def test_sgemm_aligned(vdnn, oracle, size, trans, algo):
+    (m, n, k), (ta, tb), ops = size, trans, vdnn.ops
+    rng = np.random.default_rng(m + 3 * n + 7 * k + 2 * ta + tb)
+    lda, ldb = (k if ta else m) + 4, ((n if tb else k) + 3) // 4 * 4
+    A = rng.standard_normal(lda * (m if ta else k), dtype=np.float32)
+    B = rng.standard_normal(ldb * (k if tb else n), dtype=np.float32)
+    for ldc, alpha, beta in [(m, 1.0, 0.0), (m, -0.5, 1.0), (m + 3, 0.5, 2.0)]:
+        C0 = rng.standard_normal(ldc * n, dtype=np.float32)
+        C = dev(C0)
+        need = ops.sgemm_workspace_bytes(algo, m, n, k)
+        ws = torch.empty(max(need, 4) // 4, device="cuda")
+        ops.sgemm(ta, tb, m, n, k, alpha, dev(A), lda, dev(B), ldb, beta, C, ldc, algo_mode=algo, workspace=ws, workspace_bytes=need)
+        want = oracle.sgemm(ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C0, ldc).reshape(n, ldc)
+        got = C.cpu().numpy().reshape(n, ldc)
+        assert rel_err(got[:, :m], want[:, :m]) < 1e-5
+        assert np.array_equal(got[:, m:], C0.reshape(n, ldc)[:, m:])
+    assert ops.engine_status() == 0

@@ -8,6 +8,7 @@
 #include "common.cuh"
 #include "gemm_ffma.cuh"
 #include "gemm_tc.cuh"
+#include "gemm_dense.cuh"
 #include "conv_tma.cuh"
 
 namespace vdnn {
@@ -383,6 +384,21 @@ int run_engine(const OpA& a, const OpB& b, const Epilogue& epi, int M, int N, in
     return ffma::launch<OpA, OpB, AKC, BKC>(a, b, epi, M, N, K, splits, k_chunk, stream);
 }
 
+// Zero-workspace split reductions: out = beta * out first, then every split adds alpha * its part atomically.
+int scale_output(float* out, float beta, int M, int N, size_t dense_elems, int ld_rows, cudaStream_t stream) {
+    if (beta == 1.0f) return VDNN_OK;
+    if (dense_elems > 0 && beta == 0.0f) {
+        VDNN_CUDA(cudaMemsetAsync(out, 0, dense_elems * sizeof(float), stream));
+    } else if (dense_elems > 0) {
+        scale_dense_kernel<<<stream_blocks(dense_elems), 256, 0, stream>>>(dense_elems, beta, out);
+        VDNN_LAUNCHED();
+    } else {
+        scale_matrix_kernel<<<dim3(ceil_div(M, 256), N < 65535 ? N : 65535), 256, 0, stream>>>(M, N, ld_rows, beta, out);
+        VDNN_LAUNCHED();
+    }
+    return VDNN_OK;
+}
+
 // `epi` arrives configured for a direct store (out, alpha, beta, bias, addressing).
 // dense_elems > 0 says the output is one dense block of that many floats (needed for PARTIAL).
 template <class OpA, class OpB, bool AKC, bool BKC>
@@ -405,22 +421,36 @@ int contract(const OpA& a, const OpB& b, Epilogue epi, int M, int N, int K, size
         if (st != VDNN_OK) return st;
         return reduce_partials(dense_elems, plan.splits, epi.alpha, epi.beta, static_cast<const float*>(ws), epi.out, stream);
     }
-    // zero-workspace path: out = beta * out, then every split adds alpha * partial atomically
-    if (epi.beta != 1.0f) {
-        if (dense_elems > 0) {
-            if (epi.beta == 0.0f) VDNN_CUDA(cudaMemsetAsync(epi.out, 0, dense_elems * sizeof(float), stream));
-            else {
-                scale_dense_kernel<<<stream_blocks(dense_elems), 256, 0, stream>>>(dense_elems, epi.beta, epi.out);
-                VDNN_LAUNCHED();
-            }
-        } else {
-            dim3 grid(ceil_div(M, 256), N < 65535 ? N : 65535);
-            scale_matrix_kernel<<<grid, 256, 0, stream>>>(M, N, ld_rows, epi.beta, epi.out);
-            VDNN_LAUNCHED();
-        }
-    }
+    const int st = scale_output(epi.out, epi.beta, M, N, dense_elems, ld_rows, stream);
+    if (st != VDNN_OK) return st;
     epi.mode = EPI_ATOMIC;
     return run_engine<OpA, OpB, AKC, BKC>(a, b, epi, M, N, K, plan.splits, plan.k_chunk, stream, b_tiles);
+}
+
+// SGEMM on the dense kernel (gemm_dense.cuh) with the split handling of contract().
+int sgemm_dense(int transa, int transb, int m, int n, int k, float alpha, const float* A, int lda, const float* B, int ldb, float beta,
+                float* C, int ldc, int algo_mode, void* ws, size_t ws_bytes, cudaStream_t stream) {
+    const dense::Plan plan = dense::make_plan(m, n, k);
+    const size_t dense_elems = ldc == m ? static_cast<size_t>(m) * n : 0;
+    dense::Params p{};
+    p.M = m; p.N = n; p.kblocks = ceil_div(k, 32); p.splits = plan.splits; p.kb_chunk = plan.kb_chunk;
+    p.out = C; p.ldc = ldc; p.alpha = alpha; p.beta = beta; p.mode = EPI_DIRECT;
+    const bool partials = plan.splits > 1 && algo_mode == VDNN_ALGO_PERF_OPT && dense_elems > 0;
+    if (partials) {
+        if (!ws || ws_bytes < plan.splits * dense_elems * sizeof(float)) return VDNN_ERR_WORKSPACE;
+        p.out = static_cast<float*>(ws); p.mode = EPI_PARTIAL; p.partial_stride = dense_elems; p.alpha = 1.0f; p.beta = 0.0f;
+    } else if (plan.splits > 1) {
+        const int st = scale_output(C, beta, m, n, dense_elems, ldc, stream);
+        if (st != VDNN_OK) return st;
+        p.mode = EPI_ATOMIC;
+    }
+    int st;
+    if (transa && !transb) st = dense::launch<true, true>(A, lda, B, ldb, p, k, stream);
+    else if (!transa && !transb) st = dense::launch<false, true>(A, lda, B, ldb, p, k, stream);
+    else if (!transa && transb) st = dense::launch<false, false>(A, lda, B, ldb, p, k, stream);
+    else st = dense::launch<true, false>(A, lda, B, ldb, p, k, stream);
+    if (st != VDNN_OK || !partials) return st;
+    return reduce_partials(dense_elems, plan.splits, alpha, beta, static_cast<const float*>(ws), C, stream);
 }
 
 // The TMA-fed contraction with the split handling of contract(): `ws` holds the images, then the per-split partials.
@@ -1193,8 +1223,10 @@ int vdnn_conv_bwd_filter_static(const vdnn_conv_desc* d, float alpha, const floa
 
 size_t vdnn_sgemm_workspace_bytes(int algo_mode, int m, int n, int k) {
     if (algo_mode != VDNN_ALGO_PERF_OPT || m <= 0 || n <= 0 || k <= 0) return 0;
-    const SplitPlan plan = plan_split(m, n, k);
-    return plan.splits > 1 ? static_cast<size_t>(plan.splits) * m * n * sizeof(float) : 0;
+    // which kernel runs depends on the operands' alignment, which is not known yet: room for the splits of either
+    const int gather = plan_split(m, n, k).splits, dense = dense::make_plan(m, n, k).splits;
+    const int splits = gather > dense ? gather : dense;
+    return splits > 1 ? static_cast<size_t>(splits) * m * n * sizeof(float) : 0;
 }
 
 int vdnn_sgemm(int transa, int transb, int m, int n, int k, float alpha, const float* A, int lda, const float* B,
@@ -1213,6 +1245,9 @@ int vdnn_sgemm(int transa, int transb, int m, int n, int k, float alpha, const f
     e.row_div = FastDiv(1u << 30); e.row_hi = 0; e.row_lo = 1; e.col_stride = ldc;
     const size_t dense = (ldc == m) ? static_cast<size_t>(m) * n : 0;
     cudaStream_t s = as_stream(stream);
+    // operands that tensor copies can fetch run on the dense kernel, the others on the gather-fed one
+    if (g_engine != VDNN_ENGINE_FFMA && dense::supported(A, lda, B, ldb))
+        return sgemm_dense(transa, transb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, algo_mode, workspace, workspace_bytes, s);
     if (transa && !transb) return contract<SplitDense, SplitDense, true, true>(a, b, e, m, n, k, dense, ldc, algo_mode, workspace, workspace_bytes, s);
     if (!transa && !transb) return contract<SplitDense, SplitDense, false, true>(a, b, e, m, n, k, dense, ldc, algo_mode, workspace, workspace_bytes, s);
     if (!transa && transb) return contract<SplitDense, SplitDense, false, false>(a, b, e, m, n, k, dense, ldc, algo_mode, workspace, workspace_bytes, s);

@@ -1,0 +1,469 @@
+// Dense fp32-accurate GEMM on tcgen05 with the A operand in tensor memory: C(m x n, column-major) = alpha op(A) op(B) + beta C.
+//
+// This is what the fully connected layers run on: one operand is a weight matrix of hundreds of megabytes, the other a batch
+// of at most a few hundred rows, so the call is bound by streaming the weights -- if enough bytes are in flight and the
+// shared memory is not the bottleneck first.  The gather-fed kernel (gemm_tc.cuh) had one k block in flight per SM and moved
+// every operand element through registers and twice (hi, lo) through shared memory.  Here
+//   * one thread fetches raw fp32 tiles of both operands with tensor copies into a ring of 4 .. 7 stages (96 .. 170 KB in
+//     flight per SM);
+//   * eight warps split them into tf32 hi / lo: the A tile goes from shared memory through registers into TENSOR MEMORY
+//     (tcgen05.st; lane = row, column = k), where tcgen05.mma reads it without touching shared memory, whatever its
+//     orientation in memory was; the B tile is split in place (hi over the raw values, lo beside it);
+//   * one thread issues the 3xTF32 MMAs, eight warps add finished accumulators into fp32 registers and store.
+// Shared-memory traffic per 128 x 64 x 32 block is 704 clocks' worth instead of 1344 with A staged as hi / lo tiles, just
+// under what HBM delivers (16 KB of weights in 712 clocks).
+// Measured (batch 64, 25088 -> 4096, B200): see vdnn_sgemm.
+#pragma once
+
+#include "gemm_tc.cuh"
+#include "tensor_map.cuh"
+
+namespace vdnn {
+namespace dense {
+
+using tc::BK;
+using tc::BM;
+
+constexpr int DRAIN_WARPS = 8;
+constexpr int SPLIT_GROUP = 4 * 32;                                  // threads that split one stage: a row of A each
+
+// STAGED: C goes out through shared memory (short reductions, see tile_n), which costs stages.
+template <int BN, bool STAGED> struct Config {
+    static_assert(!STAGED || BN <= 64, "no room for C tiles beside 128-column stages");
+    static constexpr int A_BYTES = BM * BK * 4;
+    static constexpr int B_BYTES = BN * BK * 4;                      // hi (over the raw tile); lo follows
+    static constexpr int STAGE_BYTES = A_BYTES + 2 * B_BYTES;
+    // Splitting a stage takes its group about 1700 clocks from barrier to barrier, 500 of issue: three groups in turn keep up
+    // with the memory; with 128 columns (registers for the wider accumulators, twice the MMA time per stage) two do.
+    static constexpr int GROUPS = BN == 128 ? 2 : 3;
+    static constexpr int TMA_WARP = DRAIN_WARPS + 4 * GROUPS, MMA_WARP = TMA_WARP + 1;
+    static constexpr int THREADS = (MMA_WARP + 1) * 32;
+    // MERGED: the lo tile of B follows the hi tile, so one MMA of 2 * BN columns forms a_hi * [b_hi | b_lo] and a second one
+    // adds a_lo * b_hi: an MMA of up to 64 columns costs 45 clocks whatever its width, one of 128 columns 64.  The drain adds
+    // the halves of the accumulator.
+    static constexpr bool MERGED = BN <= 64;
+    static constexpr int ACC_COLS = MERGED ? 2 * BN : BN;
+    // two accumulators, then slots of 64 columns (32 hi, 32 lo) of A fill the 512 columns of tensor memory
+    static constexpr int STAGES = BN == 128 ? 4 : (BN == 64 && STAGED ? 5 : 7);
+    static constexpr int A_COL = 2 * ACC_COLS;
+    static constexpr int A_SLOTS = (512 - A_COL) / (2 * BK) < STAGES ? (512 - A_COL) / (2 * BK) : STAGES;
+    static constexpr int C_TILES = STAGED ? 2 : 0;                   // finished tiles, column by column
+    static constexpr int C_BYTES = BM * BN * 4;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + C_TILES * C_BYTES + 1024 + 256;
+    __host__ __device__ static constexpr uint32_t idesc(int cols) {
+        return (1u << 4) | (2u << 7) | (2u << 10) | (static_cast<uint32_t>(cols >> 3) << 17) | (static_cast<uint32_t>(BM >> 4) << 24);
+    }
+};
+
+struct Params {
+    int M, N, tiles_m, tiles_n, kblocks, splits, kb_chunk;           // k blocks of 32; a split walks kb_chunk of them
+    long long units;                                                 // tiles_m * tiles_n * splits
+    float* out;                                                      // element (i, j) at out[j * ldc + i]
+    long long ldc;
+    float alpha, beta;
+    int mode;                                                        // EPI_DIRECT, EPI_ATOMIC, EPI_PARTIAL
+    size_t partial_stride;
+};
+
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const float (&v)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+                 ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]),
+                   "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15]) : "memory");
+}
+// Two groups of 16 columns, `apart` columns from each other, with one wait for both.
+__device__ __forceinline__ void tmem_ld16_2(uint32_t taddr, int apart, float (&v)[16], float (&w)[16]) {
+    uint32_t r[16], q[16];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%32];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%33];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7]), "=&r"(r[8]),
+                   "=&r"(r[9]), "=&r"(r[10]), "=&r"(r[11]), "=&r"(r[12]), "=&r"(r[13]), "=&r"(r[14]), "=&r"(r[15]), "=&r"(q[0]), "=&r"(q[1]),
+                   "=&r"(q[2]), "=&r"(q[3]), "=&r"(q[4]), "=&r"(q[5]), "=&r"(q[6]), "=&r"(q[7]), "=&r"(q[8]), "=&r"(q[9]), "=&r"(q[10]),
+                   "=&r"(q[11]), "=&r"(q[12]), "=&r"(q[13]), "=&r"(q[14]), "=&r"(q[15])
+                 : "r"(taddr), "r"(taddr + static_cast<uint32_t>(apart)) : "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) { v[i] = __uint_as_float(r[i]); w[i] = __uint_as_float(q[i]); }
+}
+__device__ __forceinline__ void drain_sync() {
+    __syncwarp();
+    asm volatile("bar.sync 1, %0;" ::"n"(DRAIN_WARPS * 32) : "memory");
+}
+// D += A * B with A in tensor memory.
+__device__ __forceinline__ void mma_tf32_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
+                 ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+// One 32-wide k block of the 3xTF32 product; A hi at tmem_a, lo 32 columns further; STEP as in tc::mma_block_3xtf32.
+template <int STEP, bool MERGED>
+__device__ __forceinline__ void mma_block_ta(uint32_t d_tmem, uint32_t tmem_a, uint64_t dbh, uint64_t dbl, uint32_t idesc, uint32_t idesc_wide,
+                                             bool fresh) {
+#pragma unroll
+    for (int ks = 0; ks < BK / 8; ++ks) {
+        const uint32_t acc = (fresh && ks == 0) ? 0u : 1u;
+        if (MERGED) {
+            mma_tf32_ta(d_tmem, tmem_a + ks * 8, dbh + ks * STEP, idesc_wide, acc);
+            mma_tf32_ta(d_tmem, tmem_a + BK + ks * 8, dbh + ks * STEP, idesc, 1u);
+        } else {
+            mma_tf32_ta(d_tmem, tmem_a + BK + ks * 8, dbh + ks * STEP, idesc, acc);
+            mma_tf32_ta(d_tmem, tmem_a + ks * 8, dbl + ks * STEP, idesc, 1u);
+            mma_tf32_ta(d_tmem, tmem_a + ks * 8, dbh + ks * STEP, idesc, 1u);
+        }
+    }
+}
+
+// AK / BKM: the operand is contiguous along k (its tile has a 128-byte row of 32 k per m or n), else along m / n.
+//   A, AK   box 32 k x 128 rows, 128-byte swizzle;   !AK  box 128 m x 32 k, no swizzle (rows of 512 bytes)
+//   B, BKM  box 32 k x BN rows, 128-byte swizzle;    !BKM BN / 32 boxes of 32 n x 32 k, 32-byte-atom swizzle (MN-major MMA)
+// Elements outside the matrices read as zero.
+template <bool AK, bool BKM, int BN, bool STAGED>
+__global__ void __launch_bounds__(Config<BN, STAGED>::THREADS, 1)
+gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Params p) {
+    typedef Config<BN, STAGED> Cfg;
+    constexpr int S = Cfg::STAGES;
+    constexpr uint32_t B_MN = BKM ? 0u : 1u << 16;
+    constexpr uint32_t IDESC = Cfg::idesc(BN) | B_MN, IDESC_WIDE = Cfg::idesc(Cfg::MERGED ? 2 * BN : BN) | B_MN;
+    constexpr int TMA_WARP = Cfg::TMA_WARP, MMA_WARP = Cfg::MMA_WARP;
+    extern __shared__ char smem_raw[];
+    char* tiles = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+    float* c_tile = reinterpret_cast<float*>(tiles + S * Cfg::STAGE_BYTES);
+    uint64_t* raw_full = reinterpret_cast<uint64_t*>(tiles + S * Cfg::STAGE_BYTES + Cfg::C_TILES * Cfg::C_BYTES);      // [S] tensor copies have landed
+    uint64_t* split_full = raw_full + S;    // [S] both operands are split
+    uint64_t* empty = split_full + S;       // [S] the MMAs have read the stage
+    uint64_t* acc_ready = empty + S;        // [2]
+    uint64_t* acc_free = acc_ready + 2;     // [2]
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + 2);
+
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    if (t == 0) {
+        for (int s = 0; s < S; ++s) {
+            tc::mbar_init(tc::smem_u32(&raw_full[s]), 1);
+            tc::mbar_init(tc::smem_u32(&split_full[s]), SPLIT_GROUP);
+            tc::mbar_init(tc::smem_u32(&empty[s]), 1);
+        }
+        for (int b = 0; b < 2; ++b) { tc::mbar_init(tc::smem_u32(&acc_ready[b]), 1); tc::mbar_init(tc::smem_u32(&acc_free[b]), DRAIN_WARPS); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == MMA_WARP) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::smem_u32(tmem_slot)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = *tmem_slot;
+
+    // Every role walks the same units: row tile fastest, then split, then column tile.  The CTAs then work side by side along
+    // the contiguous direction of C: with column tiles fastest, a filter gradient (25088 x 4096) was written in pieces of 512
+    // bytes all over its 411 MB.
+    auto unit_of = [&](long long u, int* m0, int* n0, int* split, int* kb0, int* nkb) {
+        const int mt = static_cast<int>(u % p.tiles_m);
+        const long long v = u / p.tiles_m;
+        *split = static_cast<int>(v % p.splits);
+        *m0 = mt * BM;
+        *n0 = static_cast<int>(v / p.splits) * BN;
+        *kb0 = *split * p.kb_chunk;
+        *nkb = min(p.kblocks, *kb0 + p.kb_chunk) - *kb0;
+    };
+    int m0, n0, split, kb0, nkb;
+
+    if (warp < DRAIN_WARPS) {
+        // ------------------------------------------------------------------ accumulator drain + epilogue
+        constexpr int NACC = BN / 2;
+        const int col_beg = (warp >> 2) * NACC;
+        const uint32_t tmem_mine = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + static_cast<uint32_t>(col_beg);
+        unsigned pair = 0;
+        bool alive = true;
+        // Tiles go out through shared memory where C's alignment allows: a warp then moves whole 512-byte columns, 16 bytes a
+        // lane, and with beta the old values of the NEXT unit's tile are under way while this one is summed.  With one 4-byte
+        // load and store per lane and column the weight step of a 25088 x 4096 layer took 490 us (822 MB), the plain product
+        // 220 (411 MB).  Thread (warp, lane) fetches and stores the same elements: columns warp * COLS .., rows 4 * lane ..
+        constexpr int COLS = BN / DRAIN_WARPS;
+        const bool old_c = STAGED && p.beta != 0.0f;
+        auto fetch_old = [&](long long u, int buf) {
+            unit_of(u, &m0, &n0, &split, &kb0, &nkb);
+            const int m = m0 + lane * 4, n = n0 + warp * COLS;
+            const int bytes = max(0, min(16, (p.M - m) * 4));
+            const float* q = p.out + (bytes > 0 ? static_cast<long long>(n) * p.ldc + m : 0);
+            uint32_t dst = tc::smem_u32(c_tile + buf * (Cfg::C_BYTES / 4) + warp * COLS * BM + lane * 4);
+#pragma unroll
+            for (int j = 0; j < COLS; ++j, dst += BM * 4) {
+                const bool in = n + j < p.N && bytes > 0;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(in ? q : p.out), "r"(in ? bytes : 0) : "memory");
+                q += p.ldc;
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        int buf = 0;
+        if (old_c && blockIdx.x < p.units) fetch_old(blockIdx.x, 0);
+        // (a warp whose wait expired waits no more, but walks the units to the end: it owes the others its part of drain_sync)
+        for (long long u = blockIdx.x; u < p.units; u += gridDim.x, buf ^= 1) {
+            const bool more = u + gridDim.x < p.units;
+            if (old_c && more) fetch_old(u + gridDim.x, buf ^ 1);
+            unit_of(u, &m0, &n0, &split, &kb0, &nkb);
+            float acc[NACC];
+#pragma unroll
+            for (int j = 0; j < NACC; ++j) acc[j] = 0.0f;
+            for (int i = 0; i < nkb && alive; i += 2, ++pair) {
+                const int b = pair & 1;
+                bool ok = tc::mbar_wait(tc::smem_u32(&acc_ready[b]), (pair >> 1) & 1u);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) { atomicCAS(&tc::g_tc_error, 0, 103); alive = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                for (int c = 0; c < NACC; c += 16) {
+                    float v[16];
+                    if (Cfg::MERGED) {
+                        float w[16];
+                        tmem_ld16_2(tmem_mine + static_cast<uint32_t>(b * Cfg::ACC_COLS + c), BN, v, w);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) acc[c + j] += v[j] + w[j];
+                    } else {
+                        tc::tmem_ld16(tmem_mine + static_cast<uint32_t>(b * Cfg::ACC_COLS + c), v);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) acc[c + j] += v[j];
+                    }
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(tc::smem_u32(&acc_free[b]));
+            }
+            if (STAGED) {
+                float* tile = c_tile + buf * (Cfg::C_BYTES / 4);
+                float* c = tile + col_beg * BM + (warp & 3) * 32 + lane;
+                if (old_c) {
+                    if (more) asm volatile("cp.async.wait_group 1;" ::: "memory");
+                    else asm volatile("cp.async.wait_group 0;" ::: "memory");
+                    drain_sync();
+#pragma unroll
+                    for (int j = 0; j < NACC; ++j) c[j * BM] = fmaf(p.beta, c[j * BM], p.alpha * acc[j]);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < NACC; ++j) c[j * BM] = p.alpha * acc[j];     // last read two units ago, a barrier before this
+                }
+                drain_sync();
+                const int m = m0 + lane * 4, n = n0 + warp * COLS;
+                if (!alive || m >= p.M) continue;
+                float* o = p.out + static_cast<long long>(n) * p.ldc + m + (p.mode == EPI_PARTIAL ? split * p.partial_stride : 0);
+                const float* src = tile + warp * COLS * BM + lane * 4;
+#pragma unroll
+                for (int j = 0; j < COLS; ++j, o += p.ldc) {
+                    if (n + j >= p.N) break;
+                    const float4 v = *reinterpret_cast<const float4*>(src + j * BM);
+                    if (m + 4 <= p.M) {
+                        *reinterpret_cast<float4*>(o) = v;
+                    } else {                                        // the last one to three rows of a ragged matrix
+                        o[0] = v.x;
+                        if (m + 1 < p.M) o[1] = v.y;
+                        if (m + 2 < p.M) o[2] = v.z;
+                    }
+                }
+                continue;
+            }
+            // parts of a split reduction, and a C of odd alignment
+            const int m = m0 + (warp & 3) * 32 + lane;
+            if (!alive || m >= p.M) continue;
+            float* o = p.out + static_cast<long long>(n0 + col_beg) * p.ldc + m;
+            if (p.mode == EPI_PARTIAL) o += static_cast<size_t>(split) * p.partial_stride;
+            const int cols = p.N - n0 - col_beg;                    // of this thread's NACC
+#pragma unroll
+            for (int j = 0; j < NACC; ++j) {
+                if (j < cols) {
+                    const float v = p.alpha * acc[j];
+                    if (p.mode == EPI_ATOMIC) atomicAdd(o, v);
+                    else *o = p.beta != 0.0f ? fmaf(p.beta, *o, v) : v;
+                }
+                o += p.ldc;
+            }
+        }
+    } else if (warp < TMA_WARP) {
+        // ------------------------------------------------------------------ split: group g takes every second stage
+        const int g = (warp - DRAIN_WARPS) >> 2, row = (warp & 3) * 32 + lane;
+        const uint32_t tmem_lane = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + Cfg::A_COL;
+        unsigned i = 0;
+        bool alive = true;
+        for (long long u = blockIdx.x; u < p.units && alive; u += gridDim.x) {
+            unit_of(u, &m0, &n0, &split, &kb0, &nkb);
+            for (int kb = 0; kb < nkb; ++kb, ++i) {
+                if (i % Cfg::GROUPS != static_cast<unsigned>(g)) continue;
+                const int s = i % S;
+                bool ok = tc::mbar_wait(tc::smem_u32(&raw_full[s]), (i / S) & 1u);
+                // the slot of tensor memory is free once the MMAs of k block i - A_SLOTS have read it (with as many slots as
+                // stages, the copies into this stage waited for that)
+                if (Cfg::A_SLOTS < S && i >= Cfg::A_SLOTS) {
+                    const unsigned j = i - Cfg::A_SLOTS;
+                    ok = ok && tc::mbar_wait(tc::smem_u32(&empty[j % S]), (j / S) & 1u);
+                }
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) { atomicCAS(&tc::g_tc_error, 0, 101); alive = false; break; }
+                char* st = tiles + s * Cfg::STAGE_BYTES;
+                const uint32_t slot = tmem_lane + (i % Cfg::A_SLOTS) * (2 * BK);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    float hi[16], lo[16];
+                    if (AK) {
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            const float4 v = *reinterpret_cast<const float4*>(st + row * 128 + (((half * 4 + c) ^ (row & 7)) << 4));
+                            tc::split_tf32_x2(v.x, v.y, hi[4 * c], hi[4 * c + 1], lo[4 * c], lo[4 * c + 1]);
+                            tc::split_tf32_x2(v.z, v.w, hi[4 * c + 2], hi[4 * c + 3], lo[4 * c + 2], lo[4 * c + 3]);
+                        }
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 16; k += 2) {
+                            const char* q = st + (half * 16 + k) * (BM * 4) + row * 4;
+                            tc::split_tf32_x2(*reinterpret_cast<const float*>(q), *reinterpret_cast<const float*>(q + BM * 4), hi[k], hi[k + 1], lo[k],
+                                              lo[k + 1]);
+                        }
+                    }
+                    tmem_st16(slot + half * 16, hi);
+                    tmem_st16(slot + BK + half * 16, lo);
+                }
+                float4* b_raw = reinterpret_cast<float4*>(st + Cfg::A_BYTES);
+                float4* b_lo = reinterpret_cast<float4*>(st + Cfg::A_BYTES + Cfg::B_BYTES);
+#pragma unroll
+                for (int j = 0; j < BN * BK / 4 / SPLIT_GROUP; ++j) {
+                    const int e = j * SPLIT_GROUP + row;
+                    const float4 v = b_raw[e];
+                    float4 h, l;
+                    tc::split_tf32_x2(v.x, v.y, h.x, h.y, l.x, l.y);
+                    tc::split_tf32_x2(v.z, v.w, h.z, h.w, l.z, l.w);
+                    b_raw[e] = h;
+                    b_lo[e] = l;
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                tc::mbar_arrive(tc::smem_u32(&split_full[s]));
+            }
+        }
+    } else if (warp == TMA_WARP) {
+        // ------------------------------------------------------------------ tensor copies
+        if (lane == 0) {
+            unsigned i = 0;
+            bool ok = true;
+            for (long long u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
+                unit_of(u, &m0, &n0, &split, &kb0, &nkb);
+                for (int kb = 0; kb < nkb; ++kb, ++i) {
+                    const int s = i % S;
+                    if (!tc::mbar_wait(tc::smem_u32(&empty[s]), ((i / S) & 1u) ^ 1u)) { ok = false; break; }
+                    const uint32_t bar = tc::smem_u32(&raw_full[s]);
+                    const uint32_t st = tc::smem_u32(tiles + s * Cfg::STAGE_BYTES);
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(Cfg::A_BYTES + Cfg::B_BYTES) : "memory");
+                    const int k0 = (kb0 + kb) * BK;
+                    tma::tma_load_rows(st, &map_a, bar, AK ? k0 : m0, AK ? m0 : k0);
+                    if (BKM) {
+                        tma::tma_load_rows(st + Cfg::A_BYTES, &map_b, bar, k0, n0);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < BN / 32; ++j) tma::tma_load_rows(st + Cfg::A_BYTES + j * (32 * BK * 4), &map_b, bar, n0 + j * 32, k0);
+                    }
+                }
+            }
+            if (!ok) atomicCAS(&tc::g_tc_error, 0, 101);
+        }
+    } else {
+        // ------------------------------------------------------------------ MMA issuer: the whole warp walks the loop (so that
+        // addresses and descriptors stay in uniform registers), one elected lane issues
+        const bool elected = tc::elect_one();
+        unsigned i = 0, pair = 0;
+        bool ok = true;
+        for (long long u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
+            unit_of(u, &m0, &n0, &split, &kb0, &nkb);
+            for (int kb = 0; kb < nkb; ++kb, ++i) {
+                const int s = i % S, b = pair & 1;
+                const bool fresh = !(kb & 1);
+                // hand-overs `pair` and `pair - 2` share an accumulator: the drain warps must have emptied it
+                if (fresh && pair >= 2 && !tc::mbar_wait(tc::smem_u32(&acc_free[b]), ((pair >> 1) - 1) & 1u)) { ok = false; break; }
+                if (!tc::mbar_wait(tc::smem_u32(&split_full[s]), (i / S) & 1u)) { ok = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t b_hi = tc::smem_u32(tiles + s * Cfg::STAGE_BYTES) + Cfg::A_BYTES, b_lo = b_hi + Cfg::B_BYTES;
+                const uint32_t a = tmem_base + Cfg::A_COL + (i % Cfg::A_SLOTS) * (2 * BK), d = tmem_base + static_cast<uint32_t>(b * Cfg::ACC_COLS);
+                const uint64_t dbh = BKM ? tc::make_desc(b_hi) : tma::make_desc_mn(b_hi), dbl = BKM ? tc::make_desc(b_lo) : tma::make_desc_mn(b_lo);
+                const bool last = !fresh || kb == nkb - 1;
+                if (elected) {
+                    mma_block_ta<BKM ? 2 : 1024 / 16, Cfg::MERGED>(d, a, dbh, dbl, IDESC, IDESC_WIDE, fresh);
+                    tc::mma_commit(tc::smem_u32(&empty[s]));
+                    if (last) tc::mma_commit(tc::smem_u32(&acc_ready[b]));
+                }
+                __syncwarp();
+                if (last) ++pair;
+            }
+        }
+        if (!ok) atomicCAS(&tc::g_tc_error, 0, 102);
+    }
+
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == MMA_WARP) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
+    }
+}
+
+struct Plan { int splits, kb_chunk; };
+
+// Columns of a tile.  A short reduction spends its time on C, not on the product: there 64-column tiles, which leave room
+// for two C tiles in shared memory, are the faster ones at any width.
+inline bool short_reduction(int K) { return K <= 256; }
+inline int tile_n(int N, int K) { return N <= 32 ? 32 : (N <= 64 || short_reduction(K) ? 64 : 128); }
+
+// Split of the reduction.  CTAs are persistent, one per SM: a wave of units costs its k blocks plus about three for the
+// hand-over between units; the split with the shortest sum of waves wins.  Each split adds the whole output once more
+// (atomics, or partial sums and their reduction): worth about one k block per 64 KB and SM.
+inline Plan make_plan(int M, int N, int K) {
+    const int bn = tile_n(N, K), kblocks = ceil_div(K, BK), sms = sm_count();
+    const long long tiles = static_cast<long long>(ceil_div(M, BM)) * ceil_div(N, bn);
+    const double out_cost = static_cast<double>(M) * N * 4.0 / (65536.0 * sms);
+    Plan best{1, kblocks};
+    double best_cost = -1.0;
+    for (int s = 1; s <= 32 && (s == 1 || kblocks / s >= 4); ++s) {
+        const int chunk = ceil_div(kblocks, s), splits = ceil_div(kblocks, chunk);
+        const long long waves = ceil_div<long long>(tiles * splits, sms);
+        const double cost = static_cast<double>(waves) * (chunk + 3) + (splits > 1 ? (splits + 1) * out_cost : 0.0);
+        if (best_cost < 0.0 || cost < best_cost) { best_cost = cost; best = Plan{splits, chunk}; }
+    }
+    return best;
+}
+
+// What the tensor copies need: 16-byte aligned matrices whose columns are a multiple of 16 bytes apart.
+inline bool supported(const float* A, int lda, const float* B, int ldb) {
+    return ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 15u) == 0 && lda % 4 == 0 && ldb % 4 == 0;
+}
+
+template <bool AK, bool BKM, int BN, bool STAGED>
+int launch_bn(const float* A, int lda, const float* B, int ldb, Params p, int K, cudaStream_t stream) {
+    typedef Config<BN, STAGED> Cfg;
+    int dev = 0;
+    VDNN_CUDA(cudaGetDevice(&dev));
+    auto kern = gemm_kernel<AK, BKM, BN, STAGED>;
+    if (VDNN_ONCE_PER_DEVICE(dev))
+        VDNN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
+    CUtensorMap ma, mb;
+    int st = AK ? tma::make_matrix_map(&ma, A, K, p.M, lda, BK, BM, CU_TENSOR_MAP_SWIZZLE_128B)
+                : tma::make_matrix_map(&ma, A, p.M, K, lda, BM, BK, CU_TENSOR_MAP_SWIZZLE_NONE);
+    if (st != VDNN_OK) return st;
+    st = BKM ? tma::make_matrix_map(&mb, B, K, p.N, ldb, BK, BN, CU_TENSOR_MAP_SWIZZLE_128B)
+             : tma::make_matrix_map(&mb, B, p.N, K, ldb, 32, BK, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B);
+    if (st != VDNN_OK) return st;
+    p.tiles_m = ceil_div(p.M, BM); p.tiles_n = ceil_div(p.N, BN);
+    p.units = static_cast<long long>(p.tiles_m) * p.tiles_n * p.splits;
+    const int grid = static_cast<int>(p.units < sm_count() ? p.units : sm_count());
+    kern<<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(ma, mb, p);
+    VDNN_LAUNCHED();
+    return VDNN_OK;
+}
+
+template <bool AK, bool BKM>
+int launch(const float* A, int lda, const float* B, int ldb, const Params& p, int K, cudaStream_t stream) {
+    const int bn = tile_n(p.N, K);
+    const bool staged = short_reduction(K) && p.mode != EPI_ATOMIC && p.ldc % 4 == 0 && p.partial_stride % 4 == 0 &&
+                        (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0;
+    if (bn == 32) return staged ? launch_bn<AK, BKM, 32, true>(A, lda, B, ldb, p, K, stream) : launch_bn<AK, BKM, 32, false>(A, lda, B, ldb, p, K, stream);
+    if (bn == 64) return staged ? launch_bn<AK, BKM, 64, true>(A, lda, B, ldb, p, K, stream) : launch_bn<AK, BKM, 64, false>(A, lda, B, ldb, p, K, stream);
+    return launch_bn<AK, BKM, 128, false>(A, lda, B, ldb, p, K, stream);
+}
+
+}  // namespace dense
+}  // namespace vdnn
