@@ -37,3 +37,29 @@ def test_sgemm_aligned(vdnn, oracle, size, trans, algo):
         assert rel_err(got[:, :m], want[:, :m]) < 1e-5
         assert np.array_equal(got[:, m:], C0.reshape(n, ldc)[:, m:])
     assert ops.engine_status() == 0
+
+
+@pytest.mark.parametrize("n", [8, 64, 128])
+def test_sgemm_long_reduction(vdnn, n):
+    """One row tile per SM and a reduction of many times the stage ring: the operand stages are reused over and over while
+    the copies are what everything waits for."""
+    m, k, ops = 148 * 128, 4096, vdnn.ops
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    A, B = torch.randn(m, k, device="cuda", generator=gen), torch.randn(n, k, device="cuda", generator=gen)
+    C = torch.empty(n, m, device="cuda")
+    want = B.double() @ A.double().t()
+    for _ in range(3):
+        ops.sgemm(1, 0, m, n, k, 1.0, A, k, B, k, 0.0, C, m)
+        assert float((C.double() - want).abs().max() / want.abs().max()) < 1e-5
+
+
+def test_weight_step_in_place(vdnn):
+    """C += alpha * A B^T with many tiles per CTA: old tiles are fetched one ahead through two buffers."""
+    m, n, k, ops = 5000, 2000, 68, vdnn.ops
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    A, B, C = (torch.randn(*s, device="cuda", generator=gen) for s in ((k, m), (k, n), (n, m)))
+    want = C.double()
+    for _ in range(3):
+        want = want - 0.5 * (B.double().t() @ A.double())
+        ops.sgemm(0, 1, m, n, k, -0.5, A, m, B, n, 1.0, C, m)
+    assert float((C.double() - want).abs().max() / want.abs().max()) < 1e-5

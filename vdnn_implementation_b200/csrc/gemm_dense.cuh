@@ -70,6 +70,17 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float (&v)[16]) 
                  ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]),
                    "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15]) : "memory");
 }
+// A finished 128 x BN tile from shared memory to the (m, column, split) box of C, and the old values of such a box to shared
+// memory.  Rows and columns outside the matrix are clipped.
+__device__ __forceinline__ void tma_tile_out(const CUtensorMap* map, uint32_t src, int m, int n, int split) {
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
+                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(m), "r"(n), "r"(split) : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void tma_tile_in(uint32_t dst, const CUtensorMap* map, uint32_t bar, int m, int n, int split) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(m), "r"(n), "r"(split) : "memory");
+}
 // Two groups of 16 columns, `apart` columns from each other, with one wait for both.
 __device__ __forceinline__ void tmem_ld16_2(uint32_t taddr, int apart, float (&v)[16], float (&w)[16]) {
     uint32_t r[16], q[16];
@@ -118,7 +129,8 @@ __device__ __forceinline__ void mma_block_ta(uint32_t d_tmem, uint32_t tmem_a, u
 // Elements outside the matrices read as zero.
 template <bool AK, bool BKM, int BN, bool STAGED>
 __global__ void __launch_bounds__(Config<BN, STAGED>::THREADS, 1)
-gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Params p) {
+gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_c,
+            const Params p) {
     typedef Config<BN, STAGED> Cfg;
     constexpr int S = Cfg::STAGES;
     constexpr uint32_t B_MN = BKM ? 0u : 1u << 16;
@@ -132,7 +144,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     uint64_t* empty = split_full + S;       // [S] the MMAs have read the stage
     uint64_t* acc_ready = empty + S;        // [2]
     uint64_t* acc_free = acc_ready + 2;     // [2]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + 2);
+    uint64_t* c_full = acc_free + 2;        // [2] the old values of a C tile
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(c_full + 2);
 
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     if (t == 0) {
@@ -141,7 +154,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             tc::mbar_init(tc::smem_u32(&split_full[s]), SPLIT_GROUP);
             tc::mbar_init(tc::smem_u32(&empty[s]), 1);
         }
-        for (int b = 0; b < 2; ++b) { tc::mbar_init(tc::smem_u32(&acc_ready[b]), 1); tc::mbar_init(tc::smem_u32(&acc_free[b]), DRAIN_WARPS); }
+        for (int b = 0; b < 2; ++b) { tc::mbar_init(tc::smem_u32(&acc_ready[b]), 1); tc::mbar_init(tc::smem_u32(&acc_free[b]), DRAIN_WARPS); tc::mbar_init(tc::smem_u32(&c_full[b]), 1); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == MMA_WARP) {
@@ -174,32 +187,24 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         const uint32_t tmem_mine = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + static_cast<uint32_t>(col_beg);
         unsigned pair = 0;
         bool alive = true;
-        // Tiles go out through shared memory where C's alignment allows: a warp then moves whole 512-byte columns, 16 bytes a
-        // lane, and with beta the old values of the NEXT unit's tile are under way while this one is summed.  With one 4-byte
-        // load and store per lane and column the weight step of a 25088 x 4096 layer took 490 us (822 MB), the plain product
-        // 220 (411 MB).  Thread (warp, lane) fetches and stores the same elements: columns warp * COLS .., rows 4 * lane ..
-        constexpr int COLS = BN / DRAIN_WARPS;
+        // STAGED: tiles go out, and with beta the old values of the NEXT unit's tile come in while this one is summed, by tensor
+        // copies through two tiles of shared memory.  With one 4-byte load and store per lane and column the weight step of a
+        // 25088 x 4096 layer took 490 us (822 MB), the plain product 220 (411 MB).
         const bool old_c = STAGED && p.beta != 0.0f;
         auto fetch_old = [&](long long u, int buf) {
             unit_of(u, &m0, &n0, &split, &kb0, &nkb);
-            const int m = m0 + lane * 4, n = n0 + warp * COLS;
-            const int bytes = max(0, min(16, (p.M - m) * 4));
-            const float* q = p.out + (bytes > 0 ? static_cast<long long>(n) * p.ldc + m : 0);
-            uint32_t dst = tc::smem_u32(c_tile + buf * (Cfg::C_BYTES / 4) + warp * COLS * BM + lane * 4);
-#pragma unroll
-            for (int j = 0; j < COLS; ++j, dst += BM * 4) {
-                const bool in = n + j < p.N && bytes > 0;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(in ? q : p.out), "r"(in ? bytes : 0) : "memory");
-                q += p.ldc;
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc::smem_u32(&c_full[buf])), "r"(Cfg::C_BYTES) : "memory");
+            tma_tile_in(tc::smem_u32(c_tile + buf * (Cfg::C_BYTES / 4)), &map_c, tc::smem_u32(&c_full[buf]), m0, n0, 0);
         };
-        int buf = 0;
-        if (old_c && blockIdx.x < p.units) fetch_old(blockIdx.x, 0);
+        unsigned unit = 0;
+        if (old_c && t == 0 && blockIdx.x < p.units) fetch_old(blockIdx.x, 0);
         // (a warp whose wait expired waits no more, but walks the units to the end: it owes the others its part of drain_sync)
-        for (long long u = blockIdx.x; u < p.units; u += gridDim.x, buf ^= 1) {
-            const bool more = u + gridDim.x < p.units;
-            if (old_c && more) fetch_old(u + gridDim.x, buf ^ 1);
+        for (long long u = blockIdx.x; u < p.units; u += gridDim.x, ++unit) {
+            const int buf = unit & 1;
+            if (old_c && alive && t == 0 && u + gridDim.x < p.units) {
+                asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");      // the last unit's tile has left its buffer
+                fetch_old(u + gridDim.x, buf ^ 1);
+            }
             unit_of(u, &m0, &n0, &split, &kb0, &nkb);
             float acc[NACC];
 #pragma unroll
@@ -229,35 +234,22 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 if (lane == 0) tc::mbar_arrive(tc::smem_u32(&acc_free[b]));
             }
             if (STAGED) {
-                float* tile = c_tile + buf * (Cfg::C_BYTES / 4);
-                float* c = tile + col_beg * BM + (warp & 3) * 32 + lane;
+                float* c = c_tile + buf * (Cfg::C_BYTES / 4) + col_beg * BM + (warp & 3) * 32 + lane;
                 if (old_c) {
-                    if (more) asm volatile("cp.async.wait_group 1;" ::: "memory");
-                    else asm volatile("cp.async.wait_group 0;" ::: "memory");
-                    drain_sync();
+                    bool ok = !alive || tc::mbar_wait(tc::smem_u32(&c_full[buf]), (unit >> 1) & 1u);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) { atomicCAS(&tc::g_tc_error, 0, 103); alive = false; }
 #pragma unroll
                     for (int j = 0; j < NACC; ++j) c[j * BM] = fmaf(p.beta, c[j * BM], p.alpha * acc[j]);
                 } else {
+                    if (t == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");      // the tile before the last has left
+                    drain_sync();
 #pragma unroll
-                    for (int j = 0; j < NACC; ++j) c[j * BM] = p.alpha * acc[j];     // last read two units ago, a barrier before this
+                    for (int j = 0; j < NACC; ++j) c[j * BM] = p.alpha * acc[j];
                 }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 drain_sync();
-                const int m = m0 + lane * 4, n = n0 + warp * COLS;
-                if (!alive || m >= p.M) continue;
-                float* o = p.out + static_cast<long long>(n) * p.ldc + m + (p.mode == EPI_PARTIAL ? split * p.partial_stride : 0);
-                const float* src = tile + warp * COLS * BM + lane * 4;
-#pragma unroll
-                for (int j = 0; j < COLS; ++j, o += p.ldc) {
-                    if (n + j >= p.N) break;
-                    const float4 v = *reinterpret_cast<const float4*>(src + j * BM);
-                    if (m + 4 <= p.M) {
-                        *reinterpret_cast<float4*>(o) = v;
-                    } else {                                        // the last one to three rows of a ragged matrix
-                        o[0] = v.x;
-                        if (m + 1 < p.M) o[1] = v.y;
-                        if (m + 2 < p.M) o[2] = v.z;
-                    }
-                }
+                if (t == 0 && alive) tma_tile_out(&map_c, tc::smem_u32(c_tile + buf * (Cfg::C_BYTES / 4)), m0, n0, p.mode == EPI_PARTIAL ? split : 0);
                 continue;
             }
             // parts of a split reduction, and a C of odd alignment
@@ -276,6 +268,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 o += p.ldc;
             }
         }
+        if (STAGED && t == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     } else if (warp < TMA_WARP) {
         // ------------------------------------------------------------------ split: group g takes every second stage
         const int g = (warp - DRAIN_WARPS) >> 2, row = (warp & 3) * 32 + lane;
@@ -287,13 +280,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             for (int kb = 0; kb < nkb; ++kb, ++i) {
                 if (i % Cfg::GROUPS != static_cast<unsigned>(g)) continue;
                 const int s = i % S;
-                bool ok = tc::mbar_wait(tc::smem_u32(&raw_full[s]), (i / S) & 1u);
-                // the slot of tensor memory is free once the MMAs of k block i - A_SLOTS have read it (with as many slots as
-                // stages, the copies into this stage waited for that)
-                if (Cfg::A_SLOTS < S && i >= Cfg::A_SLOTS) {
+                // The slot of tensor memory is free once the MMAs of k block i - A_SLOTS have read it.  This wait comes first:
+                // it also proves that the stage's last copies (k block i - S, another group's) have landed.  A parity wait
+                // tells a phase from its neighbours only; one that could be two phases ahead of its barrier passes at once.
+                bool ok = true;
+                if (i >= Cfg::A_SLOTS) {
                     const unsigned j = i - Cfg::A_SLOTS;
-                    ok = ok && tc::mbar_wait(tc::smem_u32(&empty[j % S]), (j / S) & 1u);
+                    ok = tc::mbar_wait(tc::smem_u32(&empty[j % S]), (j / S) & 1u);
                 }
+                ok = ok && tc::mbar_wait(tc::smem_u32(&raw_full[s]), (i / S) & 1u);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) { atomicCAS(&tc::g_tc_error, 0, 101); alive = false; break; }
                 char* st = tiles + s * Cfg::STAGE_BYTES;
@@ -447,10 +442,16 @@ int launch_bn(const float* A, int lda, const float* B, int ldb, Params p, int K,
     st = BKM ? tma::make_matrix_map(&mb, B, K, p.N, ldb, BK, BN, CU_TENSOR_MAP_SWIZZLE_128B)
              : tma::make_matrix_map(&mb, B, p.N, K, ldb, 32, BK, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B);
     if (st != VDNN_OK) return st;
+    CUtensorMap mc = ma;                                             // used by staged launches only
+    if (STAGED) {
+        const size_t stride = p.mode == EPI_PARTIAL ? p.partial_stride : static_cast<size_t>(p.ldc) * p.N;
+        st = tma::make_tile_out_map(&mc, p.out, p.M, p.N, p.mode == EPI_PARTIAL ? p.splits : 1, p.ldc, stride, BM, BN);
+        if (st != VDNN_OK) return st;
+    }
     p.tiles_m = ceil_div(p.M, BM); p.tiles_n = ceil_div(p.N, BN);
     p.units = static_cast<long long>(p.tiles_m) * p.tiles_n * p.splits;
     const int grid = static_cast<int>(p.units < sm_count() ? p.units : sm_count());
-    kern<<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(ma, mb, p);
+    kern<<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(ma, mb, mc, p);
     VDNN_LAUNCHED();
     return VDNN_OK;
 }
