@@ -10,6 +10,7 @@
 #include "gemm_tc.cuh"
 #include "gemm_dense.cuh"
 #include "conv_tma.cuh"
+#include "dgrad_window.cuh"
 
 namespace vdnn {
 namespace {
@@ -1018,6 +1019,10 @@ int vdnn_conv_bwd_data(const vdnn_conv_desc* d, int algo_mode, float alpha, cons
     if (is_full_extent(d))      // dX[n][j] = sum_k W[k][j] dY[n][k]   (the FC data-gradient product, layer.cu:725-733)
         return vdnn_sgemm(0, 0, d->c * rs, d->n, d->k, alpha, w, d->c * rs, dy, d->k, beta, dx, d->c * rs, algo_mode, workspace,
                           workspace_bytes, stream);
+    if (d->c <= SMALL_C_MAX) {
+        const int st = window::launch(d, P, Q, alpha, beta, w, dy, dx, as_stream(stream));
+        if (st != VDNN_ERR_UNSUPPORTED) return st;
+    }
     if (d->c <= SMALL_C_MAX && d->stride_h == d->stride_w && d->r <= 3 * d->stride_h && d->s <= 3 * d->stride_w) {
         const bool narrow = (d->w - 1 + d->pad_w) / d->stride_w + 1 <= 64;      // class coordinates fit a 64-wide tile
         cudaStream_t cs = as_stream(stream);
