@@ -39,18 +39,22 @@ def test_sgemm_aligned(vdnn, oracle, size, trans, algo):
     assert ops.engine_status() == 0
 
 
+@pytest.mark.parametrize("rows", [148 * 128, 148 * 128 + 1000])
 @pytest.mark.parametrize("n", [8, 64, 128])
-def test_sgemm_long_reduction(vdnn, n):
+def test_sgemm_long_reduction(vdnn, n, rows):
     """One row tile per SM and a reduction of many times the stage ring: the operand stages are reused over and over while
-    the copies are what everything waits for."""
-    m, k, ops = 148 * 128, 4096, vdnn.ops
+    the copies are what everything waits for.  With rows left over, their tiles are split in a second launch.  The sum of the
+    parts has a fixed order: every run gives the same bits."""
+    m, k, ops = rows, 4096, vdnn.ops
     gen = torch.Generator(device="cuda").manual_seed(n)
     A, B = torch.randn(m, k, device="cuda", generator=gen), torch.randn(n, k, device="cuda", generator=gen)
     C = torch.empty(n, m, device="cuda")
-    want = B.double() @ A.double().t()
+    want, first = B.double() @ A.double().t(), None
     for _ in range(3):
         ops.sgemm(1, 0, m, n, k, 1.0, A, k, B, k, 0.0, C, m)
         assert float((C.double() - want).abs().max() / want.abs().max()) < 1e-5
+        first = C.clone() if first is None else first
+        assert torch.equal(C, first)
 
 
 def test_weight_step_in_place(vdnn):

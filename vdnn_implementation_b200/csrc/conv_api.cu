@@ -428,30 +428,15 @@ int contract(const OpA& a, const OpB& b, Epilogue epi, int M, int N, int K, size
     return run_engine<OpA, OpB, AKC, BKC>(a, b, epi, M, N, K, plan.splits, plan.k_chunk, stream, b_tiles);
 }
 
-// SGEMM on the dense kernel (gemm_dense.cuh) with the split handling of contract().
+// SGEMM on the dense kernel (gemm_dense.cuh), which needs no workspace in either mode.
 int sgemm_dense(int transa, int transb, int m, int n, int k, float alpha, const float* A, int lda, const float* B, int ldb, float beta,
-                float* C, int ldc, int algo_mode, void* ws, size_t ws_bytes, cudaStream_t stream) {
-    const dense::Plan plan = dense::make_plan(m, n, k);
-    const size_t dense_elems = ldc == m ? static_cast<size_t>(m) * n : 0;
+                float* C, int ldc, cudaStream_t stream) {
     dense::Params p{};
-    p.M = m; p.N = n; p.kblocks = ceil_div(k, 32); p.splits = plan.splits; p.kb_chunk = plan.kb_chunk;
-    p.out = C; p.ldc = ldc; p.alpha = alpha; p.beta = beta; p.mode = EPI_DIRECT;
-    const bool partials = plan.splits > 1 && algo_mode == VDNN_ALGO_PERF_OPT && dense_elems > 0;
-    if (partials) {
-        if (!ws || ws_bytes < plan.splits * dense_elems * sizeof(float)) return VDNN_ERR_WORKSPACE;
-        p.out = static_cast<float*>(ws); p.mode = EPI_PARTIAL; p.partial_stride = dense_elems; p.alpha = 1.0f; p.beta = 0.0f;
-    } else if (plan.splits > 1) {
-        const int st = scale_output(C, beta, m, n, dense_elems, ldc, stream);
-        if (st != VDNN_OK) return st;
-        p.mode = EPI_ATOMIC;
-    }
-    int st;
-    if (transa && !transb) st = dense::launch<true, true>(A, lda, B, ldb, p, k, stream);
-    else if (!transa && !transb) st = dense::launch<false, true>(A, lda, B, ldb, p, k, stream);
-    else if (!transa && transb) st = dense::launch<false, false>(A, lda, B, ldb, p, k, stream);
-    else st = dense::launch<true, false>(A, lda, B, ldb, p, k, stream);
-    if (st != VDNN_OK || !partials) return st;
-    return reduce_partials(dense_elems, plan.splits, alpha, beta, static_cast<const float*>(ws), C, stream);
+    p.M = m; p.N = n; p.out = C; p.ldc = ldc; p.alpha = alpha; p.beta = beta;
+    if (transa && !transb) return dense::launch<true, true>(A, lda, B, ldb, p, k, stream);
+    if (!transa && !transb) return dense::launch<false, true>(A, lda, B, ldb, p, k, stream);
+    if (!transa && transb) return dense::launch<false, false>(A, lda, B, ldb, p, k, stream);
+    return dense::launch<true, false>(A, lda, B, ldb, p, k, stream);
 }
 
 // The TMA-fed contraction with the split handling of contract(): `ws` holds the images, then the per-split partials.
@@ -1228,9 +1213,7 @@ int vdnn_conv_bwd_filter_static(const vdnn_conv_desc* d, float alpha, const floa
 
 size_t vdnn_sgemm_workspace_bytes(int algo_mode, int m, int n, int k) {
     if (algo_mode != VDNN_ALGO_PERF_OPT || m <= 0 || n <= 0 || k <= 0) return 0;
-    // which kernel runs depends on the operands' alignment, which is not known yet: room for the splits of either
-    const int gather = plan_split(m, n, k).splits, dense = dense::make_plan(m, n, k).splits;
-    const int splits = gather > dense ? gather : dense;
+    const int splits = plan_split(m, n, k).splits;
     return splits > 1 ? static_cast<size_t>(splits) * m * n * sizeof(float) : 0;
 }
 
@@ -1252,7 +1235,7 @@ int vdnn_sgemm(int transa, int transb, int m, int n, int k, float alpha, const f
     cudaStream_t s = as_stream(stream);
     // operands that tensor copies can fetch run on the dense kernel, the others on the gather-fed one
     if (g_engine != VDNN_ENGINE_FFMA && dense::supported(A, lda, B, ldb))
-        return sgemm_dense(transa, transb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, algo_mode, workspace, workspace_bytes, s);
+        return sgemm_dense(transa, transb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, s);
     if (transa && !transb) return contract<SplitDense, SplitDense, true, true>(a, b, e, m, n, k, dense, ldc, algo_mode, workspace, workspace_bytes, s);
     if (!transa && !transb) return contract<SplitDense, SplitDense, false, true>(a, b, e, m, n, k, dense, ldc, algo_mode, workspace, workspace_bytes, s);
     if (!transa && transb) return contract<SplitDense, SplitDense, false, false>(a, b, e, m, n, k, dense, ldc, algo_mode, workspace, workspace_bytes, s);

@@ -12,8 +12,11 @@
 //   * one thread issues the 3xTF32 MMAs, eight warps add finished accumulators into fp32 registers and store.
 // Shared-memory traffic per 128 x 64 x 32 block is 704 clocks' worth instead of 1344 with A staged as hi / lo tiles, just
 // under what HBM delivers (16 KB of weights in 712 clocks).
-// Measured (batch 64, 25088 -> 4096, B200): see vdnn_sgemm.
+// Measured (batch 64, 25088 -> 4096, flushed L2, B200; 411 MB of weights = 63 us at copy rate), gather-fed kernel before ->
+// now: output 200 -> 106 us, data gradient 258 -> 114, filter gradient 311 -> 143, weight step in place 882 -> 191.
 #pragma once
+
+#include <atomic>
 
 #include "gemm_tc.cuh"
 #include "tensor_map.cuh"
@@ -56,13 +59,11 @@ template <int BN, bool STAGED> struct Config {
 };
 
 struct Params {
-    int M, N, tiles_m, tiles_n, kblocks, splits, kb_chunk;           // k blocks of 32; a split walks kb_chunk of them
-    long long units;                                                 // tiles_m * tiles_n * splits
+    int M, N, tiles_m, kblocks, splits, kb_chunk;                    // k blocks of 32; a split walks kb_chunk of them
+    long long tile0, units;                                          // first tile of the launch; its tiles * splits
     float* out;                                                      // element (i, j) at out[j * ldc + i]
     long long ldc;
     float alpha, beta;
-    int mode;                                                        // EPI_DIRECT, EPI_ATOMIC, EPI_PARTIAL
-    size_t partial_stride;
 };
 
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float (&v)[16]) {
@@ -70,16 +71,22 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float (&v)[16]) 
                  ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]),
                    "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15]) : "memory");
 }
-// A finished 128 x BN tile from shared memory to the (m, column, split) box of C, and the old values of such a box to shared
-// memory.  Rows and columns outside the matrix are clipped.
-__device__ __forceinline__ void tma_tile_out(const CUtensorMap* map, uint32_t src, int m, int n, int split) {
-    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
-                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(m), "r"(n), "r"(split) : "memory");
+// A finished 128 x BN tile from shared memory to its box of C, and the old values of such a box to shared memory.  Rows and
+// columns outside the matrix are clipped.
+__device__ __forceinline__ void tma_tile_out(const CUtensorMap* map, uint32_t src, int m, int n) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];"
+                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(m), "r"(n) : "memory");
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
-__device__ __forceinline__ void tma_tile_in(uint32_t dst, const CUtensorMap* map, uint32_t bar, int m, int n, int split) {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(m), "r"(n), "r"(split) : "memory");
+__device__ __forceinline__ float4 ld_cluster4(uint32_t addr, uint32_t rank) {
+    uint32_t a;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 // Two groups of 16 columns, `apart` columns from each other, with one wait for both.
 __device__ __forceinline__ void tmem_ld16_2(uint32_t taddr, int apart, float (&v)[16], float (&w)[16]) {
@@ -166,19 +173,17 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
 
-    // Every role walks the same units: row tile fastest, then split, then column tile.  The CTAs then work side by side along
-    // the contiguous direction of C: with column tiles fastest, a filter gradient (25088 x 4096) was written in pieces of 512
-    // bytes all over its 411 MB.
-    auto unit_of = [&](long long u, int* m0, int* n0, int* split, int* kb0, int* nkb) {
-        const int mt = static_cast<int>(u % p.tiles_m);
-        const long long v = u / p.tiles_m;
-        *split = static_cast<int>(v % p.splits);
-        *m0 = mt * BM;
-        *n0 = static_cast<int>(v / p.splits) * BN;
-        *kb0 = *split * p.kb_chunk;
+    // Every role walks the same units: the splits of a tile side by side (they are one cluster), row tile before column tile.
+    // The CTAs then work side by side along the contiguous direction of C: with column tiles fastest, a filter gradient
+    // (25088 x 4096) was written in pieces of 512 bytes all over its 411 MB.
+    auto unit_of = [&](long long u, int* m0, int* n0, int* kb0, int* nkb) {
+        const long long tile = p.tile0 + u / p.splits;
+        *m0 = static_cast<int>(tile % p.tiles_m) * BM;
+        *n0 = static_cast<int>(tile / p.tiles_m) * BN;
+        *kb0 = static_cast<int>(u % p.splits) * p.kb_chunk;
         *nkb = min(p.kblocks, *kb0 + p.kb_chunk) - *kb0;
     };
-    int m0, n0, split, kb0, nkb;
+    int m0, n0, kb0, nkb;
 
     if (warp < DRAIN_WARPS) {
         // ------------------------------------------------------------------ accumulator drain + epilogue
@@ -192,9 +197,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         // 25088 x 4096 layer took 490 us (822 MB), the plain product 220 (411 MB).
         const bool old_c = STAGED && p.beta != 0.0f;
         auto fetch_old = [&](long long u, int buf) {
-            unit_of(u, &m0, &n0, &split, &kb0, &nkb);
+            unit_of(u, &m0, &n0, &kb0, &nkb);
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc::smem_u32(&c_full[buf])), "r"(Cfg::C_BYTES) : "memory");
-            tma_tile_in(tc::smem_u32(c_tile + buf * (Cfg::C_BYTES / 4)), &map_c, tc::smem_u32(&c_full[buf]), m0, n0, 0);
+            tma::tma_load_rows(tc::smem_u32(c_tile + buf * (Cfg::C_BYTES / 4)), &map_c, tc::smem_u32(&c_full[buf]), m0, n0);
         };
         unsigned unit = 0;
         if (old_c && t == 0 && blockIdx.x < p.units) fetch_old(blockIdx.x, 0);
@@ -205,7 +210,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");      // the last unit's tile has left its buffer
                 fetch_old(u + gridDim.x, buf ^ 1);
             }
-            unit_of(u, &m0, &n0, &split, &kb0, &nkb);
+            unit_of(u, &m0, &n0, &kb0, &nkb);
             float acc[NACC];
 #pragma unroll
             for (int j = 0; j < NACC; ++j) acc[j] = 0.0f;
@@ -249,21 +254,26 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 drain_sync();
-                if (t == 0 && alive) tma_tile_out(&map_c, tc::smem_u32(c_tile + buf * (Cfg::C_BYTES / 4)), m0, n0, p.mode == EPI_PARTIAL ? split : 0);
+                if (t == 0 && alive) tma_tile_out(&map_c, tc::smem_u32(c_tile + buf * (Cfg::C_BYTES / 4)), m0, n0);
                 continue;
             }
-            // parts of a split reduction, and a C of odd alignment
+            if (p.splits > 1) {
+                // the part goes to shared memory: this CTA's only unit, so the operand stages are done with
+                float* c = reinterpret_cast<float*>(tiles) + col_beg * BM + (warp & 3) * 32 + lane;
+#pragma unroll
+                for (int j = 0; j < NACC; ++j) c[j * BM] = acc[j];
+                continue;
+            }
+            // long reductions, and a C of odd alignment
             const int m = m0 + (warp & 3) * 32 + lane;
             if (!alive || m >= p.M) continue;
             float* o = p.out + static_cast<long long>(n0 + col_beg) * p.ldc + m;
-            if (p.mode == EPI_PARTIAL) o += static_cast<size_t>(split) * p.partial_stride;
             const int cols = p.N - n0 - col_beg;                    // of this thread's NACC
 #pragma unroll
             for (int j = 0; j < NACC; ++j) {
                 if (j < cols) {
                     const float v = p.alpha * acc[j];
-                    if (p.mode == EPI_ATOMIC) atomicAdd(o, v);
-                    else *o = p.beta != 0.0f ? fmaf(p.beta, *o, v) : v;
+                    *o = p.beta != 0.0f ? fmaf(p.beta, *o, v) : v;
                 }
                 o += p.ldc;
             }
@@ -276,7 +286,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         unsigned i = 0;
         bool alive = true;
         for (long long u = blockIdx.x; u < p.units && alive; u += gridDim.x) {
-            unit_of(u, &m0, &n0, &split, &kb0, &nkb);
+            unit_of(u, &m0, &n0, &kb0, &nkb);
             for (int kb = 0; kb < nkb; ++kb, ++i) {
                 if (i % Cfg::GROUPS != static_cast<unsigned>(g)) continue;
                 const int s = i % S;
@@ -339,7 +349,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             unsigned i = 0;
             bool ok = true;
             for (long long u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
-                unit_of(u, &m0, &n0, &split, &kb0, &nkb);
+                unit_of(u, &m0, &n0, &kb0, &nkb);
                 for (int kb = 0; kb < nkb; ++kb, ++i) {
                     const int s = i % S;
                     if (!tc::mbar_wait(tc::smem_u32(&empty[s]), ((i / S) & 1u) ^ 1u)) { ok = false; break; }
@@ -365,7 +375,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         unsigned i = 0, pair = 0;
         bool ok = true;
         for (long long u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
-            unit_of(u, &m0, &n0, &split, &kb0, &nkb);
+            unit_of(u, &m0, &n0, &kb0, &nkb);
             for (int kb = 0; kb < nkb; ++kb, ++i) {
                 const int s = i % S, b = pair & 1;
                 const bool fresh = !(kb & 1);
@@ -389,6 +399,43 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         if (!ok) atomicCAS(&tc::g_tc_error, 0, 102);
     }
 
+    if (!STAGED && p.splits > 1) {
+        // The CTAs of a cluster hold the parts of one tile; each adds a share of it, part 0 first, through distributed shared
+        // memory.  (Adding parts to C with atomics cost a pass that scaled C, read and wrote C once per split, and left the
+        // order of the sum to chance.)
+        __syncwarp();
+        cluster_sync();
+        unit_of(blockIdx.x, &m0, &n0, &kb0, &nkb);
+        constexpr int QUADS = BN * BM / 4;
+        const int share = (QUADS + p.splits - 1) / p.splits, rank = static_cast<int>(blockIdx.x % static_cast<unsigned>(p.splits));
+        const int end = min(QUADS, (rank + 1) * share);
+        const bool vec = ((reinterpret_cast<uintptr_t>(p.out) & 15u) == 0) && p.ldc % 4 == 0;
+        for (int e = rank * share + t; e < end; e += Cfg::THREADS) {
+            const int m = m0 + (e % (BM / 4)) * 4, n = n0 + e / (BM / 4);
+            if (m >= p.M || n >= p.N) continue;
+            const uint32_t a = tc::smem_u32(tiles) + static_cast<uint32_t>(e) * 16u;
+            float4 v = ld_cluster4(a, 0);
+            for (int r = 1; r < p.splits; ++r) {
+                const float4 w = ld_cluster4(a, static_cast<uint32_t>(r));
+                v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
+            }
+            float* o = p.out + static_cast<long long>(n) * p.ldc + m;
+            v.x *= p.alpha; v.y *= p.alpha; v.z *= p.alpha; v.w *= p.alpha;
+            if (vec && m + 4 <= p.M) {
+                if (p.beta != 0.0f) {
+                    const float4 c = *reinterpret_cast<const float4*>(o);
+                    v.x = fmaf(p.beta, c.x, v.x); v.y = fmaf(p.beta, c.y, v.y); v.z = fmaf(p.beta, c.z, v.z); v.w = fmaf(p.beta, c.w, v.w);
+                }
+                *reinterpret_cast<float4*>(o) = v;
+            } else {
+                const float part[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (m + q < p.M) o[q] = p.beta != 0.0f ? fmaf(p.beta, o[q], part[q]) : part[q];
+            }
+        }
+        cluster_sync();                                              // nobody leaves while its part is being read
+    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == MMA_WARP) {
@@ -397,27 +444,26 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     }
 }
 
-struct Plan { int splits, kb_chunk; };
-
 // Columns of a tile.  A short reduction spends its time on C, not on the product: there 64-column tiles, which leave room
 // for two C tiles in shared memory, are the faster ones at any width.
 inline bool short_reduction(int K) { return K <= 256; }
 inline int tile_n(int N, int K) { return N <= 32 ? 32 : (N <= 64 || short_reduction(K) ? 64 : 128); }
 
-// Split of the reduction.  CTAs are persistent, one per SM: a wave of units costs its k blocks plus about three for the
-// hand-over between units; the split with the shortest sum of waves wins.  Each split adds the whole output once more
-// (atomics, or partial sums and their reduction): worth about one k block per 64 KB and SM.
-inline Plan make_plan(int M, int N, int K) {
-    const int bn = tile_n(N, K), kblocks = ceil_div(K, BK), sms = sm_count();
-    const long long tiles = static_cast<long long>(ceil_div(M, BM)) * ceil_div(N, bn);
-    const double out_cost = static_cast<double>(M) * N * 4.0 / (65536.0 * sms);
-    Plan best{1, kblocks};
-    double best_cost = -1.0;
-    for (int s = 1; s <= 32 && (s == 1 || kblocks / s >= 4); ++s) {
-        const int chunk = ceil_div(kblocks, s), splits = ceil_div(kblocks, chunk);
-        const long long waves = ceil_div<long long>(tiles * splits, sms);
-        const double cost = static_cast<double>(waves) * (chunk + 3) + (splits > 1 ? (splits + 1) * out_cost : 0.0);
-        if (best_cost < 0.0 || cost < best_cost) { best_cost = cost; best = Plan{splits, chunk}; }
+constexpr int MAX_SPLITS = 8;                                        // CTAs of a portable cluster
+
+// Split of the reduction for the last, partly filled wave of tiles (`rest` of them), the `splits` CTAs of a tile in one
+// cluster.  A wave costs its k blocks plus about three for its start, three more for the sum over the cluster, and eight
+// (3 us) where it needs a launch of its own after the full waves.  resident(s): clusters of s CTAs that run at once.
+template <class Resident> inline int plan_splits(long long rest, int kblocks, bool own_launch, Resident resident) {
+    int best = 1;
+    double best_cost = kblocks + 3.0;
+    for (int s = 2; s <= MAX_SPLITS && kblocks / s >= 2; ++s) {
+        const int chunk = ceil_div(kblocks, s);
+        if (ceil_div(kblocks, chunk) != s) continue;
+        const int r = resident(s);
+        if (r < 1) continue;
+        const double cost = static_cast<double>(ceil_div<long long>(rest, r)) * (chunk + 6.0) + (own_launch ? 8.0 : 0.0);
+        if (cost < best_cost) { best_cost = cost; best = s; }
     }
     return best;
 }
@@ -425,6 +471,14 @@ inline Plan make_plan(int M, int N, int K) {
 // What the tensor copies need: 16-byte aligned matrices whose columns are a multiple of 16 bytes apart.
 inline bool supported(const float* A, int lda, const float* B, int ldb) {
     return ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 15u) == 0 && lda % 4 == 0 && ldb % 4 == 0;
+}
+
+inline void cluster_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int ctas, int threads, int smem) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(ctas); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg->blockDim = dim3(threads);
+    cfg->dynamicSmemBytes = smem;
+    cfg->attrs = attr; cfg->numAttrs = 1;
 }
 
 template <bool AK, bool BKM, int BN, bool STAGED>
@@ -444,23 +498,48 @@ int launch_bn(const float* A, int lda, const float* B, int ldb, Params p, int K,
     if (st != VDNN_OK) return st;
     CUtensorMap mc = ma;                                             // used by staged launches only
     if (STAGED) {
-        const size_t stride = p.mode == EPI_PARTIAL ? p.partial_stride : static_cast<size_t>(p.ldc) * p.N;
-        st = tma::make_tile_out_map(&mc, p.out, p.M, p.N, p.mode == EPI_PARTIAL ? p.splits : 1, p.ldc, stride, BM, BN);
+        st = tma::make_matrix_map(&mc, p.out, p.M, p.N, p.ldc, BM, BN, CU_TENSOR_MAP_SWIZZLE_NONE);
         if (st != VDNN_OK) return st;
     }
-    p.tiles_m = ceil_div(p.M, BM); p.tiles_n = ceil_div(p.N, BN);
-    p.units = static_cast<long long>(p.tiles_m) * p.tiles_n * p.splits;
-    const int grid = static_cast<int>(p.units < sm_count() ? p.units : sm_count());
-    kern<<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(ma, mb, mc, p);
-    VDNN_LAUNCHED();
-    return VDNN_OK;
+    p.tiles_m = ceil_div(p.M, BM); p.kblocks = ceil_div(K, BK);
+    const long long tiles = static_cast<long long>(p.tiles_m) * ceil_div(p.N, BN);
+    const int sms = sm_count();
+    auto run = [&](long long tile0, long long count, int splits) {
+        p.tile0 = tile0; p.units = count * splits; p.splits = splits; p.kb_chunk = ceil_div(p.kblocks, splits);
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        cluster_config(&cfg, attr, splits, Cfg::THREADS, Cfg::SMEM_BYTES);
+        cfg.stream = stream;
+        cfg.gridDim = dim3(static_cast<unsigned>(splits > 1 || p.units < sms ? p.units : sms));
+        VDNN_CUDA(cudaLaunchKernelEx(&cfg, kern, ma, mb, mc, p));
+        VDNN_LAUNCHED();
+        return static_cast<int>(VDNN_OK);
+    };
+    auto resident = [&](int s) {
+        // a property of kernel and device: asked for once
+        static std::atomic<int> known[64][MAX_SPLITS + 1];
+        int n = dev < 64 ? known[dev][s].load(std::memory_order_relaxed) : 0;
+        if (n == 0) {
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute attr[1];
+            cluster_config(&cfg, attr, s, Cfg::THREADS, Cfg::SMEM_BYTES);
+            cfg.gridDim = dim3(static_cast<unsigned>(sms / s * s));
+            if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) { (void)cudaGetLastError(); n = -1; }
+            if (dev < 64) known[dev][s].store(n, std::memory_order_relaxed);
+        }
+        return n;
+    };
+    const long long rest = tiles % sms, full = tiles - rest;
+    const int splits = STAGED || rest == 0 ? 1 : plan_splits(rest, p.kblocks, full > 0, resident);
+    if (splits == 1) return run(0, tiles, 1);
+    st = full > 0 ? run(0, full, 1) : VDNN_OK;
+    return st != VDNN_OK ? st : run(full, rest, splits);
 }
 
 template <bool AK, bool BKM>
 int launch(const float* A, int lda, const float* B, int ldb, const Params& p, int K, cudaStream_t stream) {
     const int bn = tile_n(p.N, K);
-    const bool staged = short_reduction(K) && p.mode != EPI_ATOMIC && p.ldc % 4 == 0 && p.partial_stride % 4 == 0 &&
-                        (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0;
+    const bool staged = short_reduction(K) && p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0;
     if (bn == 32) return staged ? launch_bn<AK, BKM, 32, true>(A, lda, B, ldb, p, K, stream) : launch_bn<AK, BKM, 32, false>(A, lda, B, ldb, p, K, stream);
     if (bn == 64) return staged ? launch_bn<AK, BKM, 64, true>(A, lda, B, ldb, p, K, stream) : launch_bn<AK, BKM, 64, false>(A, lda, B, ldb, p, K, stream);
     return launch_bn<AK, BKM, 128, false>(A, lda, B, ldb, p, K, stream);

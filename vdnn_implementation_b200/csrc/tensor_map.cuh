@@ -63,20 +63,5 @@ inline int make_matrix_map(CUtensorMap* map, const float* base, size_t cols, siz
     return r == CUDA_SUCCESS ? VDNN_OK : VDNN_ERR_CUDA;
 }
 
-// fp32 planes of `cols` columns of `rows` contiguous elements, col_pitch elements apart, the planes plane_pitch apart, with
-// boxes of box_rows x box_cols elements of one plane (unswizzled): where finished tiles go.
-inline int make_tile_out_map(CUtensorMap* map, float* base, size_t rows, size_t cols, size_t planes, size_t col_pitch, size_t plane_pitch,
-                             int box_rows, int box_cols) {
-    EncodeTiledFn enc = encode_tiled();
-    if (!enc) return VDNN_ERR_UNSUPPORTED;
-    const cuuint64_t dims[3] = {rows, cols, planes};
-    const cuuint64_t strides[2] = {col_pitch * sizeof(float), plane_pitch * sizeof(float)};
-    const cuuint32_t box[3] = {static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(box_cols), 1u};
-    const cuuint32_t elem[3] = {1u, 1u, 1u};
-    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? VDNN_OK : VDNN_ERR_CUDA;
-}
-
 }  // namespace tma
 }  // namespace vdnn
