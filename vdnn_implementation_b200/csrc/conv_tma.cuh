@@ -28,6 +28,8 @@
 // No load carries a cluster multicast qualifier, and every tensor map covers this GPU's own workspace only.
 #pragma once
 
+#include <atomic>
+
 #include "tensor_map.cuh"
 
 namespace vdnn {

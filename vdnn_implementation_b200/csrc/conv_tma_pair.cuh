@@ -340,8 +340,13 @@ int strip_pair_launch(const Problem& q, const float* src, char* images, const ch
     cfg.stream = stream;
     cfg.attrs = attr; cfg.numAttrs = 1;
     cfg.gridDim = dim3(2 * (sm_count() / 2) * Cfg::CTAS_PER_SM, 1, 1);
-    int resident = 0;
-    if (cudaOccupancyMaxActiveClusters(&resident, kern, &cfg) != cudaSuccess || resident < 1) { (void)cudaGetLastError(); return VDNN_ERR_UNSUPPORTED; }
+    // a property of kernel and device: asked for once
+    static std::atomic<int> resident_on[64];
+    int resident = dev < 64 ? resident_on[dev].load(std::memory_order_relaxed) : 0;
+    if (resident == 0) {
+        if (cudaOccupancyMaxActiveClusters(&resident, kern, &cfg) != cudaSuccess || resident < 1) { (void)cudaGetLastError(); return VDNN_ERR_UNSUPPORTED; }
+        if (dev < 64) resident_on[dev].store(resident, std::memory_order_relaxed);
+    }
     const long long tiles = ceil_div<long long>(p.total_pos, 2 * BM);
     long long pairs = resident / (static_cast<long long>(ny) * splits);
     if (pairs < 1) pairs = 1;

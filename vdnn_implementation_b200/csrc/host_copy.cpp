@@ -5,19 +5,24 @@
 #include <string.h>
 
 #include <atomic>
-#include <functional>
 #include <system_error>
-#include <thread>
 
 namespace vdnn {
 
 namespace {
 constexpr size_t kChunk = 2u << 20;         // a huge page of the host
-constexpr size_t kDirect = 256u << 10;      // below this one cudaMemcpy is the faster way
+// Up to these sizes this thread alone is the faster way.  A write takes longer to be worth it: its source has been touched.
+constexpr size_t kDirectRead = 512u << 10, kDirectWrite = 2u << 20;
 constexpr unsigned kMaxWorkers = 8;
 }  // namespace
 
 HostCopy::~HostCopy() {
+    {
+        std::lock_guard<std::mutex> lock(mu_);
+        stop_ = true;
+    }
+    wake_.notify_all();
+    for (std::thread& t : threads_) t.join();
     for (Worker& w : workers_) {
         for (int i = 0; i < 2; ++i) {
             if (w.pinned[i]) cudaFreeHost(w.pinned[i]);
@@ -41,15 +46,42 @@ cudaError_t HostCopy::make_workers(size_t want) {
     return cudaSuccess;
 }
 
+void HostCopy::serve(size_t index) {
+    unsigned long long seen = 0;
+    std::unique_lock<std::mutex> lock(mu_);
+    for (;;) {
+        wake_.wait(lock, [&] { return stop_ || round_ != seen; });
+        if (stop_) return;
+        seen = round_;
+        if (index >= wanted_) continue;
+        lock.unlock();
+        job_(workers_[index]);
+        lock.lock();
+        if (--busy_ == 0) done_.notify_one();
+    }
+}
+
 cudaError_t HostCopy::run(void* host, void* dev, size_t bytes, int device, bool to_host) {
-    if (bytes <= kDirect)
-        return to_host ? cudaMemcpy(host, dev, bytes, cudaMemcpyDeviceToHost) : cudaMemcpy(dev, host, bytes, cudaMemcpyHostToDevice);
+    if (!to_host && bytes <= kDirectWrite) return cudaMemcpy(dev, host, bytes, cudaMemcpyHostToDevice);
+    if (to_host && bytes <= kDirectRead) {
+        // through pinned memory: the driver's way into pageable memory takes 5 us longer
+        const cudaError_t made = make_workers(1);
+        if (made != cudaSuccess) return made;
+        const Worker& w = workers_[0];
+        cudaError_t e = cudaMemcpyAsync(w.pinned[0], dev, bytes, cudaMemcpyDeviceToHost, w.stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(w.stream);
+        if (e == cudaSuccess) memcpy(host, w.pinned[0], bytes);
+        return e;
+    }
     char* const h = static_cast<char*>(host);
     char* const d = static_cast<char*>(dev);
     // chunk 0 ends at the first 2 MB boundary of the host address
     size_t head = kChunk - (reinterpret_cast<uintptr_t>(h) & (kChunk - 1));
     if (head > bytes) head = bytes;
-    const size_t chunks = 1 + (bytes - head + kChunk - 1) / kChunk;
+    // below a few chunks the page faults of the destination are what takes long: smaller pieces for more threads
+    const size_t piece = bytes >= 8 * kChunk ? kChunk : kChunk / 4;
+    if (piece < kChunk && head > piece) head = piece;
+    const size_t chunks = 1 + (bytes - head + piece - 1) / piece;
     unsigned cores = std::thread::hardware_concurrency();
     size_t workers = cores > 2 ? cores / 2 : 1;
     if (workers > kMaxWorkers) workers = kMaxWorkers;
@@ -60,8 +92,8 @@ cudaError_t HostCopy::run(void* host, void* dev, size_t bytes, int device, bool 
     std::atomic<size_t> next(0);
     std::atomic<int> failed(static_cast<int>(cudaSuccess));
     auto span = [&](size_t c, size_t* off, size_t* len) {
-        *off = c == 0 ? 0 : head + (c - 1) * kChunk;
-        const size_t end = c == 0 ? head : *off + kChunk;
+        *off = c == 0 ? 0 : head + (c - 1) * piece;
+        const size_t end = c == 0 ? head : *off + piece;
         *len = (end < bytes ? end : bytes) - *off;
     };
     auto work = [&](const Worker& w) {
@@ -99,14 +131,26 @@ cudaError_t HostCopy::run(void* host, void* dev, size_t bytes, int device, bool 
         if (err == cudaSuccess) err = last;
         if (err != cudaSuccess) failed.store(static_cast<int>(err));
     };
-    std::vector<std::thread> threads;
-    try {
-        for (size_t i = 1; i < workers; ++i) threads.emplace_back(work, std::cref(workers_[i]));
-    } catch (const std::system_error&) {
-        // the threads that could be started, or this one alone, take all chunks
+    {
+        std::lock_guard<std::mutex> lock(mu_);
+        try {
+            while (threads_.size() + 1 < workers) { const size_t index = threads_.size() + 1; threads_.emplace_back([this, index] { serve(index); }); }
+        } catch (const std::system_error&) {
+            // the threads that could be started, or this one alone, take all chunks
+        }
+        if (workers > threads_.size() + 1) workers = threads_.size() + 1;
+        job_ = work;
+        wanted_ = workers;
+        busy_ = workers - 1;
+        ++round_;
     }
+    if (workers > 1) wake_.notify_all();
     work(workers_[0]);
-    for (std::thread& t : threads) t.join();
+    {
+        std::unique_lock<std::mutex> lock(mu_);
+        done_.wait(lock, [&] { return busy_ == 0; });
+        job_ = nullptr;
+    }
     return static_cast<cudaError_t>(failed.load());
 }
 

@@ -6,6 +6,10 @@
 
 #include <cuda_runtime.h>
 
+#include <condition_variable>
+#include <functional>
+#include <mutex>
+#include <thread>
 #include <vector>
 
 namespace vdnn {
@@ -15,11 +19,11 @@ namespace vdnn {
 // link carries.  Here each worker thread owns two pinned buffers and a stream and takes the next chunk of the tensor that
 // nobody has taken yet: the copy engine fills one of its buffers while the thread moves the other to its destination.
 // Chunks begin on 2 MB boundaries of the HOST address, so no two threads fault in the same huge page.
-// The buffers (workers x 2 x 2 MB) are made at the first large copy, kept for the object's life and released with it;
-// one copy runs at a time (the caller is a Network, whose calls are not concurrent).
+// The buffers (workers x 2 x 2 MB) and the threads, which sleep between copies, are made at the first large copy, kept for the
+// object's life and released with it; one copy runs at a time (the caller is a Network, whose calls are not concurrent).
 class HostCopy {
 public:
-    HostCopy() : device_(0) {}
+    HostCopy() : round_(0), wanted_(0), busy_(0), stop_(false) {}
     ~HostCopy();
     // The caller has synchronised whatever produces the source.  Returns a cudaError_t.
     cudaError_t to_host(void* dst_h, const void* src, size_t bytes, int device) { return run(dst_h, const_cast<void*>(src), bytes, device, true); }
@@ -31,8 +35,16 @@ private:
     HostCopy& operator=(const HostCopy&);
     cudaError_t run(void* host, void* dev, size_t bytes, int device, bool to_host);
     cudaError_t make_workers(size_t want);
+    void serve(size_t index);
     std::vector<Worker> workers_;
-    int device_;
+    // threads_[i] takes part in round n for worker i + 1 when job_ wants it to (i + 1 < wanted_)
+    std::vector<std::thread> threads_;
+    std::mutex mu_;
+    std::condition_variable wake_, done_;
+    std::function<void(const Worker&)> job_;
+    unsigned long long round_;
+    size_t wanted_, busy_;
+    bool stop_;
 };
 
 }  // namespace vdnn

@@ -40,7 +40,7 @@ struct Pool {
 };
 Pool g_pool;
 
-void drop_finished_fences_locked();
+void drop_finished_fences_locked(const cudaStream_t* consumers, int n);
 
 size_t round_up(size_t n) { return (n + kGranularity - 1) / kGranularity * kGranularity; }
 
@@ -185,13 +185,29 @@ cnmemStatus_t free_locked(void* ptr, size_t* off_out, size_t* len_out) {
     return CNMEM_STATUS_SUCCESS;
 }
 
-void drop_finished_fences_locked() {
+// Drops fences that have been passed.  The fences of a stream finish in the order they were recorded, which is their order
+// here: behind the first unfinished one of a stream none of its others needs a query.  Those of a stream that will use the
+// new block itself neither rank nor are waited for, and are left alone until there are many.  (Querying every fence at every
+// allocation was most of the host's time in a step of a small network: dozens of fences times some fifty allocations.)
+void drop_finished_fences_locked(const cudaStream_t* consumers, int n) {
+    constexpr size_t kMany = 64;
+    constexpr int kStreams = 8;             // streams whose first unfinished fence is remembered; further ones are all queried
+    cudaStream_t waiting[kStreams];
+    int num_waiting = 0;
+    if (n == 1 && g_pool.fences.size() < kMany)
+        waiting[num_waiting++] = consumers[0];
     size_t keep = 0;
     for (size_t i = 0; i < g_pool.fences.size(); ++i) {
-        if (cudaEventQuery(g_pool.fences[i].event) == cudaErrorNotReady) g_pool.fences[keep++] = g_pool.fences[i];
-        else g_pool.spare_events.push_back(g_pool.fences[i].event);
+        const Fence f = g_pool.fences[i];
+        bool pending = is_consumer(f.stream, waiting, num_waiting);
+        if (!pending && cudaEventQuery(f.event) == cudaErrorNotReady) {
+            pending = true;
+            if (num_waiting < kStreams) waiting[num_waiting++] = f.stream;
+        }
+        if (pending) g_pool.fences[keep++] = f;
+        else g_pool.spare_events.push_back(f.event);
     }
-    (void)cudaGetLastError();
+    if (num_waiting) (void)cudaGetLastError();
     g_pool.fences.resize(keep);
 }
 
@@ -323,7 +339,7 @@ cnmemStatus_t vdnnPoolMallocFor(void** ptr, size_t size, const cudaStream_t* str
 cnmemStatus_t vdnnPoolMallocKindFor(void** ptr, size_t size, const cudaStream_t* streams, int numStreams, int transient) {
     std::lock_guard<std::recursive_mutex> lock(g_pool.mu);
     size_t off = 0, len = 0;
-    if (!g_pool.is_virtual && g_pool.ready) drop_finished_fences_locked();
+    if (!g_pool.is_virtual && g_pool.ready) drop_finished_fences_locked(streams, numStreams);
     cnmemStatus_t st = alloc_locked(ptr, size, &off, &len, streams, g_pool.is_virtual ? 0 : numStreams, transient != 0);
     if (st != CNMEM_STATUS_SUCCESS || size == 0) return st;
     if (!g_pool.holds.empty()) {
