@@ -1,0 +1,32 @@
+"""Data gradients of stride-1 layers without workspace on enough pixels for a kernel that never splits the reduction: boxes that
+cross images, column tiles of 96 and 128 with columns to spare, filter counts that fill neither a chunk nor a 16-byte copy,
+padding on one axis, maps wider than a box; and one size below the rule's limit."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def dev(a):
+    return torch.from_numpy(np.ascontiguousarray(a, np.float32)).cuda()
+
+
+@pytest.mark.parametrize("n,c,h,w,k,r,s,pad", [
+    (64, 70, 13, 17, 7, 5, 5, (2, 2)), (39, 230, 13, 17, 33, 3, 3, (1, 1)), (1, 96, 73, 250, 8, 3, 3, (0, 1)), (14, 190, 7, 128, 5, 7, 5, (3, 2)),
+    (1400, 90, 4, 3, 1, 3, 3, (1, 1)), (10, 70, 13, 17, 7, 3, 3, (1, 1))])
+def test_dgrad_unsplit(vdnn, oracle, n, c, h, w, k, r, s, pad):
+    ops, rng = vdnn.ops, np.random.default_rng(h * w + r)
+    d = ops.conv_desc(n, c, h, w, k, r, s, pad, (1, 1))
+    P, Q = ops.conv_out_dims(d)
+    wt = rng.standard_normal((k, c, r, s), dtype=np.float32)
+    dy = rng.standard_normal((n, k, P, Q), dtype=np.float32)
+    dx0 = rng.standard_normal((n, c, h, w), dtype=np.float32)
+    plain = oracle.conv_bwd_data(wt, dy, dx0.shape, pad, (1, 1))
+    for alpha, beta in ((1.0, 0.0), (0.5, 2.0)):
+        dx = dev(dx0)
+        ops.conv_bwd_data(d, dev(wt), dev(dy), dx, alpha=alpha, beta=beta)
+        assert rel_err(dx.cpu().numpy(), alpha * plain + beta * dx0) < 1e-5
+    assert ops.engine_status() == 0

@@ -10,6 +10,7 @@
 #include "gemm_tc.cuh"
 #include "gemm_dense.cuh"
 #include "conv_tma.cuh"
+#include "conv_halo.cuh"
 #include "dgrad_window.cuh"
 
 namespace vdnn {
@@ -437,6 +438,26 @@ int sgemm_dense(int transa, int transb, int m, int n, int k, float alpha, const 
     if (!transa && !transb) return dense::launch<false, true>(A, lda, B, ldb, p, k, stream);
     if (!transa && transb) return dense::launch<false, false>(A, lda, B, ldb, p, k, stream);
     return dense::launch<true, false>(A, lda, B, ldb, p, k, stream);
+}
+
+// Data gradient of a stride-1 convolution on the halo kernel (conv_halo.cuh), or VDNN_ERR_UNSUPPORTED where the gather-fed one
+// is the better: where no box of the problem fits shared memory; on few columns, which leave the tensor cores waiting for
+// operands on either; on small filters, whose elements it does not use often enough; and where too little of its work is useful
+// (columns and pixels that fill up tiles, tiles that fill up waves: it does not split the reduction).  The limit depends on
+// the filter, as the gather reads dy once per tap: measured at shares of 0.64 .. 0.70 of 3x3 filters 1.06 .. 1.14 times its
+// time, at 0.76 0.78 and 0.95, at 0.82 .. 0.88 0.62 .. 0.97; of 5x5 filters at 0.59 0.56, at 0.82 0.60.
+int dgrad_halo(const vdnn_conv_desc* d, int P, int Q, const float* dy, const float* w, float alpha, float beta, float* dx, cudaStream_t stream) {
+    // dx[h][w] = sum over taps of dy[h + pad - r][w + pad - s]: the taps walked from the last to the first
+    const halo::Problem q{d->n, d->k, P, Q, d->c, d->h, d->w, d->r, d->s, d->pad_h - (d->r - 1), d->pad_w - (d->s - 1)};
+    halo::Params p{};
+    const int bn = halo::tile_n(q.n_cols);
+    if (bn == 0 || d->r * d->s < 9) return VDNN_ERR_UNSUPPORTED;
+    const double useful = static_cast<double>(d->n) * d->h * d->w * d->c / (static_cast<double>(halo::BM) * bn * sm_count()), least = d->r * d->s > 9 ? 0.5 : 0.75;
+    // (too little for a single wave: known without a plan, which costs some microseconds)
+    if (useful < least || !halo::plan(q, bn, &p) || useful < least * static_cast<double>(ceil_div<long long>(p.units, sm_count()))) return VDNN_ERR_UNSUPPORTED;
+    halo::complete(q, dy, w, &p);
+    p.out = dx; p.alpha = alpha; p.beta = beta;
+    return halo::launch(bn, p, stream);
 }
 
 // The TMA-fed contraction with the split handling of contract(): `ws` holds the images, then the per-split partials.
@@ -1032,6 +1053,11 @@ int vdnn_conv_bwd_data(const vdnn_conv_desc* d, int algo_mode, float alpha, cons
             d->n, d->c, d->h, d->w, d->k, d->r, d->s, P, Q, d->pad_h, d->pad_w, d->stride_h, d->stride_w, alpha, beta, w, dy, dx);
         VDNN_LAUNCHED();
         return VDNN_OK;
+    }
+    if (g_engine != VDNN_ENGINE_FFMA && d->stride_h == 1 && d->stride_w == 1 &&
+        (algo_mode == VDNN_ALGO_MEMORY_OPT || g_no_tma || !tma_shape(d, VDNN_CONV_BWD_DATA))) {
+        const int st = dgrad_halo(d, P, Q, dy, w, alpha, beta, dx, as_stream(stream));
+        if (st != VDNN_ERR_UNSUPPORTED) return st;
     }
     DyGather A;
     A.dy = dy; A.K = d->k; A.P = P; A.Q = Q; A.R = d->r; A.S = d->s;
