@@ -379,19 +379,138 @@ __global__ void __launch_bounds__(kThreads) maxpool_fwd_2x2(size_t pairs, int w,
     }
 }
 
+// Windows of 2 x 2 or 3 x 3 at stride 2.  A lane owns two columns of dx (a window's first two) and walks down a band of
+// window rows: it finds each window's first maximum in registers -- the last row of a 3 x 3 window is the first of the next --
+// and hands place and dy to its right neighbour by shuffle, so that no shared memory and no barrier is involved and four
+// windows' loads are in flight.  The columns of all planes form one list: small planes share a warp; of a 3 x 3 warp's 32
+// columns the first is there for its neighbour only.  Sums are in scan order, the same every time.
+// With the windows in shared memory (two barriers, three times the instructions) 64 x 96 x 55 x 55, 3 x 3, took 78 us (now 49,
+// 3.4 TB/s), 128 x 256 x 13 x 13 57 (23), 64 x 512 x 14 x 14, 2 x 2, 57 (21).
+template <int WIN>
+__global__ void __launch_bounds__(kThreads, 4) maxpool_bwd_columns(int total, int h, int w, FastDiv div_items, int P, int Q, int band_rows, bool pairs,
+                                                                   const float* __restrict__ dy, const float* __restrict__ x, float* __restrict__ dx) {
+    constexpr int NEW = WIN == 3 ? 31 : 32, UNROLL = 4;
+    const int lane = threadIdx.x & 31;
+    const long long first = (static_cast<long long>(blockIdx.x) * (kThreads / 32) + (threadIdx.x >> 5)) * NEW;
+    if (first >= total) return;                                  // a whole warp
+    const long long item = first + lane - (WIN == 3 ? 1 : 0);
+    const bool valid = item >= 0 && item < total, out = valid && (WIN == 2 || lane > 0);
+    uint32_t plane = 0, q = 0;
+    if (valid) div_items.divmod(static_cast<uint32_t>(item), plane, q);
+    const bool has = valid && static_cast<int>(q) < Q;           // there is a window in these columns
+    const float* xp = x + static_cast<size_t>(plane) * h * w + 2 * q;
+    const float* gp = dy + static_cast<size_t>(plane) * P * Q + q;
+    float* op = dx + static_cast<size_t>(plane) * h * w + 2 * q;
+    const bool second = 2 * static_cast<int>(q) + 1 < w;
+    const int rows = (h + 1) / 2, p_beg = blockIdx.y * band_rows, p_end = min(rows, p_beg + band_rows);
+
+    auto row_max = [](const float* v, float* m, int* b) {
+        *m = -INFINITY; *b = 0;
+#pragma unroll
+        for (int j = 0; j < WIN; ++j) if (v[j] > *m) { *m = v[j]; *b = j; }
+    };
+    float carry_m = -INFINITY, up_g = 0.0f, up_left_g = 0.0f;    // the window above, and the one to its left
+    int carry_b = 0, up_k = -1, up_left_k = -1;
+    if (WIN == 3) {
+        // the window above the band, whose last row begins the band
+        if (has && p_beg > 0 && p_beg - 1 < P) {
+            const float* r = xp + static_cast<size_t>(2 * p_beg - 2) * w;
+            float v[3][3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                for (int b = 0; b < 3; ++b) v[a][b] = __ldg(r + a * w + b);
+            up_g = __ldg(gp + static_cast<size_t>(p_beg - 1) * Q);
+            float m, mm;
+            int b;
+            row_max(v[0], &m, &up_k);
+            row_max(v[1], &mm, &b);
+            if (mm > m) { m = mm; up_k = 3 + b; }
+            row_max(v[2], &carry_m, &carry_b);
+            if (carry_m > m) up_k = 6 + carry_b;
+        } else if (has && p_beg == 0) {
+            const float v[3] = {__ldg(xp), __ldg(xp + 1), __ldg(xp + 2)};
+            row_max(v, &carry_m, &carry_b);
+        }
+        up_left_k = __shfl_up_sync(0xffffffffu, up_k, 1);
+        up_left_g = __shfl_up_sync(0xffffffffu, up_g, 1);
+        if (q == 0) up_left_k = -1;
+    }
+    for (int p0 = p_beg; p0 < p_end; p0 += UNROLL) {
+        float v[UNROLL][2][WIN], g[UNROLL];                      // rows 2 p + 1, 2 p + 2 (3 x 3) or 2 p, 2 p + 1 of window row p
+#pragma unroll
+        for (int u = 0; u < UNROLL; ++u) {
+            const int p = p0 + u;
+            const bool live = has && p < P && p < p_end;
+            const float* r = xp + static_cast<size_t>(2 * p + (WIN == 3 ? 1 : 0)) * w;
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+#pragma unroll
+                for (int b = 0; b < WIN; ++b) v[u][a][b] = live ? __ldg(r + a * w + b) : 0.0f;
+            g[u] = live ? __ldg(gp + static_cast<size_t>(p) * Q) : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < UNROLL; ++u) {
+            const int p = p0 + u;
+            if (p >= p_end) break;
+            float m, mm;
+            int k, b;
+            if (WIN == 3) {
+                m = carry_m; k = carry_b;
+                row_max(v[u][0], &mm, &b);
+                if (mm > m) { m = mm; k = 3 + b; }
+                row_max(v[u][1], &carry_m, &carry_b);
+                if (carry_m > m) k = 6 + carry_b;
+            } else {
+                row_max(v[u][0], &m, &k);
+                row_max(v[u][1], &mm, &b);
+                if (mm > m) k = 2 + b;
+            }
+            if (!has || p >= P) k = -1;
+            float o00 = 0.0f, o01 = 0.0f, o10 = 0.0f, o11 = 0.0f;
+            if (WIN == 3) {
+                int left_k = __shfl_up_sync(0xffffffffu, k, 1);
+                const float left_g = __shfl_up_sync(0xffffffffu, g[u], 1);
+                if (q == 0) left_k = -1;
+                if (up_left_k == 8) o00 += up_left_g;
+                if (up_k == 6) o00 += up_g;
+                if (up_k == 7) o01 += up_g;
+                if (left_k == 2) o00 += left_g;
+                if (left_k == 5) o10 += left_g;
+                up_k = k; up_g = g[u];
+                up_left_k = left_k; up_left_g = left_g;
+            }
+            if (k == 0) o00 += g[u];
+            if (k == 1) o01 += g[u];
+            if (k == WIN) o10 += g[u];
+            if (k == WIN + 1) o11 += g[u];
+            if (out) {
+                float* o = op + static_cast<size_t>(2 * p) * w;
+                const bool below = 2 * p + 1 < h;
+                if (pairs) {
+                    *reinterpret_cast<float2*>(o) = make_float2(o00, o01);
+                    if (below) *reinterpret_cast<float2*>(o + w) = make_float2(o10, o11);
+                } else {
+                    o[0] = o00;
+                    if (second) o[1] = o01;
+                    if (below) {
+                        o[w] = o10;
+                        if (second) o[w + 1] = o11;
+                    }
+                }
+            }
+        }
+    }
+}
+
 // Any window.  A block takes a band of dx rows of one plane: the x rows that the band's windows cover go to shared memory,
 // one thread per window finds the window's first maximum there and leaves its place and dy, and one thread per input
-// element (or 2 x 2 of them) adds up the few windows around it that point to it, in scan order.  x and dy are read and dx is written once,
-// in full rows, with no atomics and no pre-zeroed dx; the sums come out the same every time.
-// Before: overlapping windows zeroed dx and added with atomics (64 x 96 x 55 x 55, 3 x 3 / 2: 13.6 + 51.1 us, now 36),
-// others searched every window again for each of its elements (64 x 512 x 14 x 14, 2 x 2 / 2: 18 us, now 13).
-// WIN, STRIDE > 0: square window and stride known at compile time.
-template <int WIN, int STRIDE>
-__global__ void __launch_bounds__(kThreads) maxpool_bwd_band(int bands, int band_rows, int h, FastDiv div_w, FastDiv div_hw, int P, FastDiv div_q, int wh_, int ww_,
-                                                             int sh_, int sw_, const float* __restrict__ dy,
+// element adds up the few windows around it that point to it, in scan order.  x and dy are read and dx is written once, in full
+// rows, with no atomics and no pre-zeroed dx; the sums come out the same every time.
+__global__ void __launch_bounds__(kThreads) maxpool_bwd_band(int bands, int band_rows, int h, FastDiv div_w, int P, FastDiv div_q, int wh, int ww,
+                                                             int sh, int sw, const float* __restrict__ dy,
                                                              const float* __restrict__ x, float* __restrict__ dx) {
     extern __shared__ float smem[];
-    const int wh = WIN > 0 ? WIN : wh_, ww = WIN > 0 ? WIN : ww_, sh = STRIDE > 0 ? STRIDE : sh_, sw = STRIDE > 0 ? STRIDE : sw_;
     const int w = div_w.d, Q = div_q.d;
     const unsigned plane = blockIdx.x / bands, band = blockIdx.x - plane * bands;
     const int r0 = band * band_rows, r1 = min(h, r0 + band_rows);
@@ -417,57 +536,14 @@ __global__ void __launch_bounds__(kThreads) maxpool_bwd_band(int bands, int band
         const int o = p * sh * w + q * sw;
         float m = -INFINITY;
         int best = 0;                                           // position inside the window: row * ww + column
-#pragma unroll
-        for (int a = 0; a < (WIN > 0 ? WIN : wh); ++a)
-#pragma unroll
-            for (int b = 0; b < (WIN > 0 ? WIN : ww); ++b) {
+        for (int a = 0; a < wh; ++a)
+            for (int b = 0; b < ww; ++b) {
                 const float v = xs[o + a * w + b];
                 if (v > m) { m = v; best = a * ww + b; }
             }
         win[i].y = __int_as_float(best);
     }
     __syncthreads();
-    if (STRIDE == 2 && WIN <= 3) {
-        // a thread takes the 2 x 2 inputs below and right of a window origin (bands begin on even rows): every place of
-        // the (up to four) windows around them is known, so one read of a window serves all of its inputs
-        const int half_w = (w + 1) / 2, items = (r1 - r0 + 1) / 2 * half_w;
-        for (int i = threadIdx.x; i < items; i += blockDim.x) {
-            uint32_t a, b;
-            div_hw.divmod(i, a, b);
-            const int p = r0 / 2 + static_cast<int>(a), q = static_cast<int>(b);
-            auto window = [&](int pp, int qq, float* g) -> int {
-                if (pp < p0 || pp >= p1 || qq < 0 || qq >= Q) return -1;
-                const float2 v = win[(pp - p0) * Q + qq];
-                *g = v.x;
-                return __float_as_int(v.y);
-            };
-            float g11 = 0.f, g = 0.f, o00 = 0.f, o01 = 0.f, o10 = 0.f, o11 = 0.f;
-            if (WIN == 3) {
-                int k = window(p - 1, q - 1, &g);
-                if (k == 8) o00 += g;
-                k = window(p - 1, q, &g);
-                if (k == 6) o00 += g;
-                if (k == 7) o01 += g;
-                k = window(p, q - 1, &g);
-                if (k == 2) o00 += g;
-                if (k == 5) o10 += g;
-            }
-            const int k = window(p, q, &g11);
-            if (k == 0) o00 += g11;
-            if (k == 1) o01 += g11;
-            if (k == WIN) o10 += g11;
-            if (k == WIN + 1) o11 += g11;
-            const int ih = 2 * p, iw = 2 * q;
-            float* o = dxp + static_cast<size_t>(ih) * w + iw;
-            o[0] = o00;
-            if (iw + 1 < w) o[1] = o01;
-            if (ih + 1 < r1) {
-                o[w] = o10;
-                if (iw + 1 < w) o[w + 1] = o11;
-            }
-        }
-        return;
-    }
     for (int i = threadIdx.x; i < (r1 - r0) * w; i += blockDim.x) {
         uint32_t row, col;
         div_w.divmod(i, row, col);
@@ -1003,6 +1079,19 @@ int vdnn_maxpool_bwd(int n, int c, int h, int w, int win_h, int win_w, int strid
         VDNN_LAUNCHED();
         return VDNN_OK;
     }
+    const int items = (w + 1) / 2, window_rows = (h + 1) / 2;
+    if (win_h == win_w && (win_h == 2 || win_h == 3) && stride_h == 2 && stride_w == 2 && static_cast<long long>(planes) * items < 0x7fffffffLL) {
+        const int total = planes * items, per_block = (kThreads / 32) * (win_h == 3 ? 31 : 32), blocks = ceil_div(total, per_block);
+        // bands of window rows: three waves of blocks, but not less than four rows, of which a band reads one twice
+        const int want = ceil_div(3 * 4 * sm_count(), blocks), most = window_rows / 4 > 1 ? window_rows / 4 : 1;
+        const int band = ceil_div(window_rows, want < most ? want : most);
+        const bool pairs = w % 2 == 0 && (reinterpret_cast<uintptr_t>(dx) & 7u) == 0;
+        const dim3 grid(blocks, ceil_div(window_rows, band));
+        if (win_h == 3) maxpool_bwd_columns<3><<<grid, kThreads, 0, as_stream(stream)>>>(total, h, w, FastDiv(items), P, Q, band, pairs, dy, x, dx);
+        else maxpool_bwd_columns<2><<<grid, kThreads, 0, as_stream(stream)>>>(total, h, w, FastDiv(items), P, Q, band, pairs, dy, x, dx);
+        VDNN_LAUNCHED();
+        return VDNN_OK;
+    }
     // rows of a band: about 16 KB of shared memory, so that a full set of blocks stays resident, but at least two rows
     auto smem_of = [&](int rows) {
         const size_t np = rows / stride_h + (win_h + stride_h - 1) / stride_h + 1;
@@ -1010,17 +1099,13 @@ int vdnn_maxpool_bwd(int n, int c, int h, int w, int win_h, int win_w, int strid
     };
     int band = h;
     while (band > 2 && smem_of(band) > 16 * 1024) band = (band + 1) / 2;
-    if (band < h) band = (band + 1) / 2 * 2;                             // bands begin on even rows
     const size_t smem = smem_of(band);
     const long long blocks = static_cast<long long>(planes) * ceil_div(h, band);
     // a window so large that not even one row's share fits is outside what any network here has
     if (smem <= 200 * 1024 && blocks <= 0x7fffffffLL) {
         const int bands = ceil_div(h, band);
-        auto kern = maxpool_bwd_band<0, 0>;
-        if (win_h == win_w && stride_h == stride_w && stride_h == 2 && win_h == 3) kern = maxpool_bwd_band<3, 2>;
-        else if (win_h == win_w && stride_h == stride_w && stride_h == 2 && win_h == 2) kern = maxpool_bwd_band<2, 2>;
-        if (smem > 48 * 1024) VDNN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-        kern<<<static_cast<unsigned>(blocks), kThreads, smem, as_stream(stream)>>>(bands, band, h, FastDiv(w), FastDiv((w + 1) / 2), P, FastDiv(Q), win_h, win_w, stride_h, stride_w,
+        if (smem > 48 * 1024) VDNN_CUDA(cudaFuncSetAttribute(maxpool_bwd_band, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        maxpool_bwd_band<<<static_cast<unsigned>(blocks), kThreads, smem, as_stream(stream)>>>(bands, band, h, FastDiv(w), P, FastDiv(Q), win_h, win_w, stride_h, stride_w,
                                                                                   dy, x, dx);
     } else {
         VDNN_CUDA(cudaMemsetAsync(dx, 0, static_cast<size_t>(planes) * h * w * sizeof(float), as_stream(stream)));
