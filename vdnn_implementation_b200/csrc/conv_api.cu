@@ -71,6 +71,8 @@ template <int VEC>
 __global__ void __launch_bounds__(256) reduce_partials_kernel(size_t n, int splits, int lanes, float alpha, float beta,
                                                               const float* __restrict__ partial, float* __restrict__ out) {
     __shared__ float part[256 * VEC];
+    tc::follow_up();
+    tc::after_predecessor();
     const int per_block = 256 / lanes, g = threadIdx.x % per_block, l = threadIdx.x / per_block;
     const size_t i = (static_cast<size_t>(blockIdx.x) * per_block + g) * VEC;
     float acc[VEC];
@@ -115,8 +117,8 @@ int reduce_partials(size_t n, int splits, float alpha, float beta, const float* 
     while (lanes < 32 && 4 * lanes <= splits && ceil_div<size_t>(groups * lanes, 256) < static_cast<size_t>(2 * sm_count())) lanes *= 2;
     const size_t blocks = ceil_div<size_t>(groups * lanes, 256);
     if (blocks > 0x7fffffffu) return VDNN_ERR_UNSUPPORTED;
-    if (vec) reduce_partials_kernel<4><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(n, splits, lanes, alpha, beta, partial, out);
-    else reduce_partials_kernel<1><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(n, splits, lanes, alpha, beta, partial, out);
+    if (vec) VDNN_CUDA(tc::launch_early(reduce_partials_kernel<4>, dim3(static_cast<unsigned>(blocks)), 256, 0, stream, n, splits, lanes, alpha, beta, partial, out));
+    else VDNN_CUDA(tc::launch_early(reduce_partials_kernel<1>, dim3(static_cast<unsigned>(blocks)), 256, 0, stream, n, splits, lanes, alpha, beta, partial, out));
     VDNN_LAUNCHED();
     return VDNN_OK;
 }
