@@ -63,6 +63,7 @@ void HostCopy::serve(size_t index) {
 
 cudaError_t HostCopy::run(void* host, void* dev, size_t bytes, int device, bool to_host) {
     if (!to_host && bytes <= kDirectWrite) return cudaMemcpy(dev, host, bytes, cudaMemcpyHostToDevice);
+    std::lock_guard<std::mutex> turn(turn_);
     if (to_host && bytes <= kDirectRead) {
         // through pinned memory: the driver's way into pageable memory takes 5 us longer
         const cudaError_t made = make_workers(1);

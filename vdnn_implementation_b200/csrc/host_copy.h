@@ -20,7 +20,8 @@ namespace vdnn {
 // nobody has taken yet: the copy engine fills one of its buffers while the thread moves the other to its destination.
 // Chunks begin on 2 MB boundaries of the HOST address, so no two threads fault in the same huge page.
 // The buffers (workers x 2 x 2 MB) and the threads, which sleep between copies, are made at the first large copy, kept for the
-// object's life and released with it; one copy runs at a time (the caller is a Network, whose calls are not concurrent).
+// object's life and released with it.  Host threads may call at once, as they may cudaMemcpy: the buffers serve one copy at a
+// time, the others wait for it.
 class HostCopy {
 public:
     HostCopy() : round_(0), wanted_(0), busy_(0), stop_(false) {}
@@ -36,6 +37,7 @@ private:
     cudaError_t run(void* host, void* dev, size_t bytes, int device, bool to_host);
     cudaError_t make_workers(size_t want);
     void serve(size_t index);
+    std::mutex turn_;                   // held for a copy that uses the members below
     std::vector<Worker> workers_;
     // threads_[i] takes part in round n for worker i + 1 when job_ wants it to (i + 1 < wanted_)
     std::vector<std::thread> threads_;
