@@ -1,5 +1,5 @@
 // Runs csrc/host_copy.cpp on a CUDA runtime made of host memory: streams that do their copies only when somebody waits for
-// them, and allocations that can be made to fail.  One check per run, named by the argument; exit code 0 if it holds.
+// them, and allocations that can be made to fail.  One check per run, named by the first argument; exit code 0 if it holds.
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
@@ -104,10 +104,30 @@ int concurrent() {
     return bad == 0 ? 0 : 1;
 }
 
+// Pinned memory or streams run out: before the first worker, in the middle of the second, or after it.  Copies go on with what
+// there is, nothing half-made is kept, and what comes free later is used.
+int scarce(int pinned, int streams) {
+    {
+        vdnn::HostCopy copy;
+        g_pinned_left = pinned;
+        g_streams_left = streams;
+        for (unsigned i = 0; i < 2; ++i)
+            if (!round_trip(copy, 300u << 10, i) || !round_trip(copy, (9u << 20) + 5, i + 2)) return 1;
+        if (g_pinned_live % 2 != 0 || g_pinned_live > pinned) return 3;                 // two buffers to a worker
+        if ((pinned < 2 || streams < 1) && g_plain_copies == 0) return 4;
+        g_pinned_left = g_streams_left = 1 << 20;
+        const int before = g_pinned_live;
+        if (!round_trip(copy, (9u << 20) + 5, 7)) return 1;
+        if (g_pinned_live < 2 || g_pinned_live < before) return 5;
+    }
+    return g_pinned_live == 0 ? 0 : 6;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "concurrent") return concurrent();
+    if (what == "scarce" && argc == 4) return scarce(atoi(argv[2]), atoi(argv[3]));
     return 2;
 }

@@ -15,8 +15,13 @@ def check(tmp_path_factory):
     binary = str(tmp_path_factory.mktemp("host_copy") / "check")
     subprocess.run(["g++", "-std=c++17", "-O1", "-I", CUDA_INCLUDE, "-I", CSRC, os.path.join(HERE, "host_copy_check.cpp"),
                     os.path.join(CSRC, "host_copy.cpp"), "-o", binary, "-lpthread"], check=True)
-    return lambda what: subprocess.run([binary, what], timeout=120).returncode
+    return lambda *what: subprocess.run([binary] + [str(w) for w in what], timeout=120).returncode
 
 
 def test_concurrent_copies_keep_their_bytes_apart(check):
     assert check("concurrent") == 0
+
+
+@pytest.mark.parametrize("pinned,streams", [(0, 99), (1, 99), (2, 99), (3, 99), (99, 0), (99, 1)])
+def test_copies_go_on_when_pinned_memory_or_streams_run_out(check, pinned, streams):
+    assert check("scarce", pinned, streams) == 0

@@ -5,7 +5,7 @@
 #include <string.h>
 
 #include <atomic>
-#include <system_error>
+#include <exception>
 
 namespace vdnn {
 
@@ -13,7 +13,6 @@ namespace {
 constexpr size_t kChunk = 2u << 20;         // a huge page of the host
 // Up to these sizes this thread alone is the faster way.  A write takes longer to be worth it: its source has been touched.
 constexpr size_t kDirectRead = 512u << 10, kDirectWrite = 2u << 20;
-constexpr unsigned kMaxWorkers = 8;
 }  // namespace
 
 HostCopy::~HostCopy() {
@@ -23,27 +22,37 @@ HostCopy::~HostCopy() {
     }
     wake_.notify_all();
     for (std::thread& t : threads_) t.join();
-    for (Worker& w : workers_) {
-        for (int i = 0; i < 2; ++i) {
-            if (w.pinned[i]) cudaFreeHost(w.pinned[i]);
-            if (w.done[i]) cudaEventDestroy(w.done[i]);
-        }
-        if (w.stream) cudaStreamDestroy(w.stream);
-    }
+    for (size_t i = 0; i < made_; ++i) release(&workers_[i]);
 }
 
-cudaError_t HostCopy::make_workers(size_t want) {
-    while (workers_.size() < want) {
-        Worker w = {};
-        cudaError_t e = cudaStreamCreateWithFlags(&w.stream, cudaStreamNonBlocking);
-        for (int i = 0; i < 2 && e == cudaSuccess; ++i) {
-            e = cudaEventCreateWithFlags(&w.done[i], cudaEventDisableTiming);
-            if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void**>(&w.pinned[i]), kChunk, cudaHostAllocDefault);
-        }
-        workers_.push_back(w);              // a half-made worker is released with the rest
-        if (e != cudaSuccess) return e;
+void HostCopy::release(Worker* w) {
+    for (int i = 0; i < 2; ++i) {
+        if (w->pinned[i]) cudaFreeHost(w->pinned[i]);
+        if (w->done[i]) cudaEventDestroy(w->done[i]);
     }
-    return cudaSuccess;
+    if (w->stream) cudaStreamDestroy(w->stream);
+    *w = Worker();
+}
+
+cudaError_t HostCopy::make(Worker* w) {
+    cudaError_t e = cudaStreamCreateWithFlags(&w->stream, cudaStreamNonBlocking);
+    for (int i = 0; i < 2 && e == cudaSuccess; ++i) {
+        e = cudaEventCreateWithFlags(&w->done[i], cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void**>(&w->pinned[i]), kChunk, cudaHostAllocDefault);
+    }
+    return e;
+}
+
+size_t HostCopy::make_workers(size_t want) {
+    while (made_ < want) {
+        if (make(&workers_[made_]) != cudaSuccess) {
+            release(&workers_[made_]);
+            (void)cudaGetLastError();
+            break;
+        }
+        ++made_;
+    }
+    return made_ < want ? made_ : want;
 }
 
 void HostCopy::serve(size_t index) {
@@ -64,10 +73,8 @@ void HostCopy::serve(size_t index) {
 cudaError_t HostCopy::run(void* host, void* dev, size_t bytes, int device, bool to_host) {
     if (!to_host && bytes <= kDirectWrite) return cudaMemcpy(dev, host, bytes, cudaMemcpyHostToDevice);
     std::lock_guard<std::mutex> turn(turn_);
-    if (to_host && bytes <= kDirectRead) {
+    if (to_host && bytes <= kDirectRead && make_workers(1) == 1) {
         // through pinned memory: the driver's way into pageable memory takes 5 us longer
-        const cudaError_t made = make_workers(1);
-        if (made != cudaSuccess) return made;
         const Worker& w = workers_[0];
         cudaError_t e = cudaMemcpyAsync(w.pinned[0], dev, bytes, cudaMemcpyDeviceToHost, w.stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(w.stream);
@@ -87,8 +94,8 @@ cudaError_t HostCopy::run(void* host, void* dev, size_t bytes, int device, bool 
     size_t workers = cores > 2 ? cores / 2 : 1;
     if (workers > kMaxWorkers) workers = kMaxWorkers;
     if (workers > chunks) workers = chunks;
-    cudaError_t e = make_workers(workers);
-    if (e != cudaSuccess) return e;
+    workers = make_workers(workers);
+    if (workers == 0) return cudaMemcpy(to_host ? host : dev, to_host ? dev : host, bytes, to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice);
 
     std::atomic<size_t> next(0);
     std::atomic<int> failed(static_cast<int>(cudaSuccess));
@@ -135,12 +142,13 @@ cudaError_t HostCopy::run(void* host, void* dev, size_t bytes, int device, bool 
     {
         std::lock_guard<std::mutex> lock(mu_);
         try {
+            job_ = work;
             while (threads_.size() + 1 < workers) { const size_t index = threads_.size() + 1; threads_.emplace_back([this, index] { serve(index); }); }
-        } catch (const std::system_error&) {
+        } catch (const std::exception&) {
             // the threads that could be started, or this one alone, take all chunks
         }
+        if (!job_) workers = 1;
         if (workers > threads_.size() + 1) workers = threads_.size() + 1;
-        job_ = work;
         wanted_ = workers;
         busy_ = workers - 1;
         ++round_;

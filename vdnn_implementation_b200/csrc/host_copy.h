@@ -20,11 +20,12 @@ namespace vdnn {
 // nobody has taken yet: the copy engine fills one of its buffers while the thread moves the other to its destination.
 // Chunks begin on 2 MB boundaries of the HOST address, so no two threads fault in the same huge page.
 // The buffers (workers x 2 x 2 MB) and the threads, which sleep between copies, are made at the first large copy, kept for the
-// object's life and released with it.  Host threads may call at once, as they may cudaMemcpy: the buffers serve one copy at a
+// object's life and released with it.  Where pinned memory, streams or threads run out, the workers that could be had do the
+// copy, and cudaMemcpy does it where there is none; the next copy asks for the missing ones again.  Host threads may call at once, as they may cudaMemcpy: the buffers serve one copy at a
 // time, the others wait for it.
 class HostCopy {
 public:
-    HostCopy() : round_(0), wanted_(0), busy_(0), stop_(false) {}
+    HostCopy() : workers_(), made_(0), round_(0), wanted_(0), busy_(0), stop_(false) {}
     ~HostCopy();
     // The caller has synchronised whatever produces the source.  Returns a cudaError_t.
     cudaError_t to_host(void* dst_h, const void* src, size_t bytes, int device) { return run(dst_h, const_cast<void*>(src), bytes, device, true); }
@@ -32,13 +33,17 @@ public:
 
 private:
     struct Worker { cudaStream_t stream; cudaEvent_t done[2]; char* pinned[2]; };
+    static constexpr size_t kMaxWorkers = 8;
+    static cudaError_t make(Worker* w);
+    static void release(Worker* w);
     HostCopy(const HostCopy&);
     HostCopy& operator=(const HostCopy&);
     cudaError_t run(void* host, void* dev, size_t bytes, int device, bool to_host);
-    cudaError_t make_workers(size_t want);
+    size_t make_workers(size_t want);                   // returns how many of them there are
     void serve(size_t index);
     std::mutex turn_;                   // held for a copy that uses the members below
-    std::vector<Worker> workers_;
+    Worker workers_[kMaxWorkers];
+    size_t made_;
     // threads_[i] takes part in round n for worker i + 1 when job_ wants it to (i + 1 < wanted_)
     std::vector<std::thread> threads_;
     std::mutex mu_;
