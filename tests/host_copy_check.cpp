@@ -14,7 +14,9 @@
 #include "host_copy.h"
 
 namespace {
+thread_local int t_device = 0;
 struct FakeStream {
+    const int device = t_device;
     std::mutex mu;
     std::vector<std::function<void()>> ops;
     size_t done = 0;
@@ -27,7 +29,8 @@ struct FakeStream {
     }
 };
 struct FakeEvent { FakeStream* stream = nullptr; size_t upto = 0; };
-std::atomic<int> g_pinned_left(1 << 20), g_streams_left(1 << 20), g_pinned_live(0), g_plain_copies(0);
+std::atomic<int> g_pinned_left(1 << 20), g_streams_left(1 << 20), g_pinned_live(0), g_plain_copies(0), g_away(0);
+int g_home = 0;                          // the device whose memory is copied
 }  // namespace
 
 extern "C" {
@@ -55,6 +58,7 @@ cudaError_t cudaEventSynchronize(cudaEvent_t e) {
 cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t n, cudaMemcpyKind, cudaStream_t s) {
     if (!dst || !src) return cudaErrorInvalidValue;
     FakeStream* st = reinterpret_cast<FakeStream*>(s);
+    if (st->device != g_home) ++g_away;
     std::lock_guard<std::mutex> lock(st->mu);
     st->ops.push_back([=] { memcpy(dst, src, n); });
     return cudaSuccess;
@@ -67,7 +71,6 @@ cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
     return cudaSuccess;
 }
 cudaError_t cudaFreeHost(void* p) { --g_pinned_live; free(p); return cudaSuccess; }
-thread_local int t_device = 0;
 cudaError_t cudaSetDevice(int d) { t_device = d; return cudaSuccess; }
 cudaError_t cudaGetDevice(int* d) { *d = t_device; return cudaSuccess; }
 cudaError_t cudaGetLastError(void) { return cudaSuccess; }
@@ -86,8 +89,8 @@ std::vector<unsigned char> pattern(size_t n, unsigned seed) {
 bool round_trip(vdnn::HostCopy& copy, size_t bytes, unsigned seed) {
     const std::vector<unsigned char> want = pattern(bytes, seed);
     std::vector<unsigned char> got(bytes, 0), there(bytes, 0);
-    if (copy.to_host(got.data(), want.data(), bytes, 0) != cudaSuccess || got != want) return false;
-    return copy.to_device(there.data(), want.data(), bytes, 0) == cudaSuccess && there == want;
+    if (copy.to_host(got.data(), want.data(), bytes, g_home) != cudaSuccess || got != want) return false;
+    return copy.to_device(there.data(), want.data(), bytes, g_home) == cudaSuccess && there == want;
 }
 
 // Several threads use one object at once: small copies, which share a staging buffer, and large ones, which share the threads.
@@ -123,11 +126,27 @@ int scarce(int pinned, int streams) {
     return g_pinned_live == 0 ? 0 : 6;
 }
 
+// A thread whose current device is another one reads and writes: its device stays as it was, and the work is done on the
+// memory's own device, whichever copy comes first.
+int device() {
+    g_home = 3;
+    t_device = 1;
+    for (int first = 0; first < 2; ++first) {
+        vdnn::HostCopy copy;
+        for (unsigned i = 0; i < 2; ++i) {
+            if (!round_trip(copy, static_cast<int>(i) == first ? 300u << 10 : 9u << 20, i)) return 1;
+            if (t_device != 1) return 3;
+        }
+    }
+    return g_away == 0 ? 0 : 4;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "concurrent") return concurrent();
+    if (what == "device") return device();
     if (what == "scarce" && argc == 4) return scarce(atoi(argv[2]), atoi(argv[3]));
     return 2;
 }

@@ -25,3 +25,7 @@ def test_concurrent_copies_keep_their_bytes_apart(check):
 @pytest.mark.parametrize("pinned,streams", [(0, 99), (1, 99), (2, 99), (3, 99), (99, 0), (99, 1)])
 def test_copies_go_on_when_pinned_memory_or_streams_run_out(check, pinned, streams):
     assert check("scarce", pinned, streams) == 0
+
+
+def test_the_current_device_of_the_caller_stays(check):
+    assert check("device") == 0

@@ -13,6 +13,19 @@ namespace {
 constexpr size_t kChunk = 2u << 20;         // a huge page of the host
 // Up to these sizes this thread alone is the faster way.  A write takes longer to be worth it: its source has been touched.
 constexpr size_t kDirectRead = 512u << 10, kDirectWrite = 2u << 20;
+
+// Makes a device current for as long as it lives; the thread gets its own device back.
+struct OnDevice {
+    int before;
+    bool changed;
+    cudaError_t status;
+    explicit OnDevice(int device) : before(device), changed(false), status(cudaGetDevice(&before)) {
+        if (status != cudaSuccess || before == device) return;
+        status = cudaSetDevice(device);
+        changed = status == cudaSuccess;
+    }
+    ~OnDevice() { if (changed) cudaSetDevice(before); }
+};
 }  // namespace
 
 HostCopy::~HostCopy() {
@@ -73,6 +86,8 @@ void HostCopy::serve(size_t index) {
 cudaError_t HostCopy::run(void* host, void* dev, size_t bytes, int device, bool to_host) {
     if (!to_host && bytes <= kDirectWrite) return cudaMemcpy(dev, host, bytes, cudaMemcpyHostToDevice);
     std::lock_guard<std::mutex> turn(turn_);
+    const OnDevice on(device);          // streams, events and staging buffers belong to the device of the memory
+    if (on.status != cudaSuccess) return on.status;
     if (to_host && bytes <= kDirectRead && make_workers(1) == 1) {
         // through pinned memory: the driver's way into pageable memory takes 5 us longer
         const Worker& w = workers_[0];
