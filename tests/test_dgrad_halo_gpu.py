@@ -30,3 +30,23 @@ def test_dgrad_unsplit(vdnn, oracle, n, c, h, w, k, r, s, pad):
         ops.conv_bwd_data(d, dev(wt), dev(dy), dx, alpha=alpha, beta=beta)
         assert rel_err(dx.cpu().numpy(), alpha * plain + beta * dx0) < 1e-5
     assert ops.engine_status() == 0
+
+
+@pytest.mark.parametrize("n,c,h,w,k,r", [(64, 70, 13, 17, 7, 5), (40, 230, 14, 17, 33, 3), (1, 96, 73, 250, 8, 3)])
+def test_perf_opt_dgrad_off_blocks_of_32_runs_on_packed_weights(vdnn, oracle, n, c, h, w, k, r):
+    """With workspace these run on the contraction that reads packed weights: right in the bytes that are reported, refused
+    below them (too little workspace is an error, not a change of algorithm)."""
+    ops, rng = vdnn.ops, np.random.default_rng(h * w + r)
+    d = ops.conv_desc(n, c, h, w, k, r, r, (r // 2,) * 2, (1, 1))
+    wt = rng.standard_normal((k, c, r, r), dtype=np.float32)
+    dy = rng.standard_normal((n, k, h, w), dtype=np.float32)
+    need = ops.conv_workspace_bytes(1, 1, d)
+    assert need > 0
+    ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+    dx = torch.empty(n, c, h, w, device="cuda")
+    ops.conv_bwd_data(d, dev(wt), dev(dy), dx, algo_mode=1, workspace=ws, workspace_bytes=need)
+    assert rel_err(dx.cpu().numpy(), oracle.conv_bwd_data(wt, dy, (n, c, h, w), (r // 2,) * 2, (1, 1))) < 1e-5
+    with pytest.raises(vdnn.VdnnError) as e:
+        ops.conv_bwd_data(d, dev(wt), dev(dy), dx, algo_mode=1, workspace=ws, workspace_bytes=need - 4)
+    assert e.value.status == -3
+    assert ops.engine_status() == 0

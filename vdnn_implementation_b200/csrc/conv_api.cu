@@ -1056,8 +1056,11 @@ int vdnn_conv_bwd_data(const vdnn_conv_desc* d, int algo_mode, float alpha, cons
         VDNN_LAUNCHED();
         return VDNN_OK;
     }
-    if (g_engine != VDNN_ENGINE_FFMA && d->stride_h == 1 && d->stride_w == 1 &&
-        (algo_mode == VDNN_ALGO_MEMORY_OPT || g_no_tma || !tma_shape(d, VDNN_CONV_BWD_DATA))) {
+    // Without workspace only: the gather-fed kernel with packed weights (PERF_OPT, channels or sizes that the TMA-fed kernels do
+    // not take) is faster than the halo kernel on every shape measured -- 1.07 .. 2.0 times as fast at 3x3 (250 <- 500 channels,
+    // 64 images of 28 x 28: 771 against 1565 us; 512 <- 256, 84 x 87: 121 against 209), 1.07 .. 2.5 at 5x5, 1.4 .. 3.0 at 7x7
+    // and 9x9.
+    if (algo_mode == VDNN_ALGO_MEMORY_OPT && g_engine != VDNN_ENGINE_FFMA && d->stride_h == 1 && d->stride_w == 1) {
         const int st = dgrad_halo(d, P, Q, dy, w, alpha, beta, dx, as_stream(stream));
         if (st != VDNN_ERR_UNSUPPORTED) return st;
     }
