@@ -50,3 +50,12 @@ def test_perf_opt_dgrad_off_blocks_of_32_runs_on_packed_weights(vdnn, oracle, n,
         ops.conv_bwd_data(d, dev(wt), dev(dy), dx, algo_mode=1, workspace=ws, workspace_bytes=need - 4)
     assert e.value.status == -3
     assert ops.engine_status() == 0
+
+
+# Both sides of the choice between the halo kernel and the gather without workspace: one wave of tiles and a little more than
+# one, columns that fill the gather's tiles badly and well, rows wider than a box, boxes over many small images, few filters.
+@pytest.mark.parametrize("n,c,h,w,k,r,s,pad", [
+    (1, 300, 31, 250, 20, 3, 3, (1, 1)), (700, 300, 4, 3, 24, 3, 3, (1, 1)), (24, 300, 14, 17, 40, 3, 3, (0, 1)), (25, 300, 14, 17, 40, 3, 3, (1, 1)),
+    (48, 256, 14, 14, 16, 3, 3, (1, 1)), (3, 96, 40, 250, 24, 3, 5, (1, 2)), (3, 130, 20, 21, 9, 5, 5, (2, 1)), (10, 70, 13, 17, 7, 3, 3, (1, 1))])
+def test_dgrad_either_side_of_the_choice(vdnn, oracle, n, c, h, w, k, r, s, pad):
+    test_dgrad_unsplit(vdnn, oracle, n, c, h, w, k, r, s, pad)

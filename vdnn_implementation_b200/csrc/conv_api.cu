@@ -5,6 +5,8 @@
 // into the output (MEMORY_OPT: no workspace) or through per-split partial tiles in the caller's
 // workspace followed by a fixed-order reduction (PERF_OPT: deterministic).
 #include <cuda_pipeline.h>
+#include <math.h>
+
 #include "common.cuh"
 #include "gemm_ffma.cuh"
 #include "gemm_tc.cuh"
@@ -443,20 +445,31 @@ int sgemm_dense(int transa, int transb, int m, int n, int k, float alpha, const 
 }
 
 // Data gradient of a stride-1 convolution on the halo kernel (conv_halo.cuh), or VDNN_ERR_UNSUPPORTED where the gather-fed one
-// is the better: where no box of the problem fits shared memory; on few columns, which leave the tensor cores waiting for
-// operands on either; on small filters, whose elements it does not use often enough; and where too little of its work is useful
-// (columns and pixels that fill up tiles, tiles that fill up waves: it does not split the reduction).  The limit depends on
-// the filter, as the gather reads dy once per tap: measured at shares of 0.64 .. 0.70 of 3x3 filters 1.06 .. 1.14 times its
-// time, at 0.76 0.78 and 0.95, at 0.82 .. 0.88 0.62 .. 0.97; of 5x5 filters at 0.59 0.56, at 0.82 0.60.
+// is the better without workspace: where no box of the problem fits shared memory, on few columns (which leave the tensor cores
+// waiting for operands on either), on small filters (whose elements it does not use often enough), and where its waves of
+// tiles cost more.  A wave is one tile on every SM.  Fitted to 568 shapes (B200, flushed L2; 65 .. 512 columns, reductions over
+// 4 .. 512 filters, maps of 3 x 4 .. 180 x 180), in us: a wave of the halo kernel takes 1.55 per 32 elements of the reduction
+// with 9 taps, 1.25 from 25 taps on, and 2 besides, its start 5; a wave of the gather takes 1.4 and 1.95 on 128 columns (it
+// reads dy once per tap), 2.7 and 4.2 on 256, and 5 per 128 columns besides, but it splits the reduction where a wave is not
+// full.  Time lost against the better kernel of each shape, on average and at worst: 3x3 0.5 and 11 %, more taps 0.1 and 7 %,
+// calls of 10 .. 30 us 0.9 and 30 %.  Going by the share of useful work in the tiles lost 2.6 and 39 %, 1.5 and 59 % (first two).
 int dgrad_halo(const vdnn_conv_desc* d, int P, int Q, const float* dy, const float* w, float alpha, float beta, float* dx, cudaStream_t stream) {
     // dx[h][w] = sum over taps of dy[h + pad - r][w + pad - s]: the taps walked from the last to the first
     const halo::Problem q{d->n, d->k, P, Q, d->c, d->h, d->w, d->r, d->s, d->pad_h - (d->r - 1), d->pad_w - (d->s - 1)};
     halo::Params p{};
-    const int bn = halo::tile_n(q.n_cols);
-    if (bn == 0 || d->r * d->s < 9) return VDNN_ERR_UNSUPPORTED;
-    const double useful = static_cast<double>(d->n) * d->h * d->w * d->c / (static_cast<double>(halo::BM) * bn * sm_count()), least = d->r * d->s > 9 ? 0.5 : 0.75;
-    // (too little for a single wave: known without a plan, which costs some microseconds)
-    if (useful < least || !halo::plan(q, bn, &p) || useful < least * static_cast<double>(ceil_div<long long>(p.units, sm_count()))) return VDNN_ERR_UNSUPPORTED;
+    const int bn = halo::tile_n(q.n_cols), taps = d->r * d->s;
+    if (bn == 0 || taps < 9) return VDNN_ERR_UNSUPPORTED;
+    const int M = d->n * d->h * d->w, K = d->k * taps, sms = sm_count();
+    const double more = (min(taps, 25) - 9) / 16.0;
+    const SplitPlan split = plan_split(M, d->c, K);
+    const int columns = tc::tile_n(d->c) / 128;
+    const double gather_wave = (columns == 2 ? 2.7 + 1.5 * more : 1.4 + 0.55 * more) * (split.k_chunk / 32) + 5.0 * columns;
+    const long long gather_tiles = static_cast<long long>(ceil_div(M, halo::BM)) * ceil_div(d->c, 128 * columns) * split.splits;
+    const double gather = static_cast<double>(ceil_div<long long>(gather_tiles, sms)) * gather_wave;
+    auto slower = [&](long long waves) { return static_cast<double>(waves) * ((1.55 - 0.3 * more) * (K / 32.0) + 2.0) + 5.0 > gather; };
+    // the fewest waves that its tiles can make: known without a plan, which costs some microseconds
+    const double full = static_cast<double>(M) * d->c / (static_cast<double>(halo::BM) * bn * sms);
+    if (slower(static_cast<long long>(ceil(full))) || !halo::plan(q, bn, &p) || slower(ceil_div<long long>(p.units, sms))) return VDNN_ERR_UNSUPPORTED;
     halo::complete(q, dy, w, &p);
     p.out = dx; p.alpha = alpha; p.beta = beta;
     return halo::launch(bn, p, stream);
