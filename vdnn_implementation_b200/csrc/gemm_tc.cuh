@@ -49,6 +49,10 @@ template <int BN, bool PAIRED = false> struct Config {
     static constexpr int STAGES = BN == 256 ? 2 : (BN == 128 ? 3 : (PAIRED ? 2 : 4));
     static constexpr int CTAS_PER_SM = PAIRED ? 2 : 1;
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment*/ + 256 /*barriers*/;
+    // Shared memory of a CTA that shall have an SM to itself.  A grid of no more CTAs than SMs gains nothing from sharing, and
+    // started early, beside the last CTAs of its predecessor, its CTAs were put two to an SM with other SMs idle: 72 tiles of 128
+    // images of 192 x 15 x 17 -> 32, 3 x 3 / 2, without workspace 82 us after a finished predecessor, 124 so, 80 with an SM each.
+    static constexpr int ALONE_BYTES = SMEM_BYTES > 120 * 1024 ? SMEM_BYTES : 120 * 1024;
     // instruction descriptor: D = F32, A = B = TF32, both K-major, N = BN, M = 128
     static constexpr uint32_t IDESC = (1u << 4) | (2u << 7) | (2u << 10) | (static_cast<uint32_t>(BN >> 3) << 17) |
                                       (static_cast<uint32_t>(BM >> 4) << 24);
@@ -485,7 +489,7 @@ int launch_bn(const OpA& a, const OpB& b, const Epilogue& epi, int M, int N, int
     VDNN_CUDA(cudaGetDevice(&dev));
     auto kern = gemm_kernel<OpA, OpB, AKC, BKC, BN, BBULK>;
     if (VDNN_ONCE_PER_DEVICE(dev))
-        VDNN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
+        VDNN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::ALONE_BYTES));
     dim3 grid(ceil_div(M, BM), ceil_div(N, BN), splits);
     if (grid.y > 65535u || grid.z > 65535u) return VDNN_ERR_UNSUPPORTED;
     const int kblocks = ceil_div(K, BK);
@@ -497,7 +501,8 @@ int launch_bn(const OpA& a, const OpB& b, const Epilogue& epi, int M, int N, int
         VDNN_CUDA((launch_early(pack_b_tiles_kernel<OpB, BN, BKC>, dim3(static_cast<unsigned>(blocks)), 256, 0, stream, b, N, K, static_cast<int>(grid.y), kblocks, b_tiles)));
         VDNN_LAUNCHED();
     }
-    VDNN_CUDA(launch_early(kern, grid, THREADS, Cfg::SMEM_BYTES, stream, a, b, epi, M, N, K, k_chunk, b_tiles, kblocks));
+    const bool alone = static_cast<long long>(grid.x) * grid.y * grid.z <= sm_count();
+    VDNN_CUDA(launch_early(kern, grid, THREADS, alone ? Cfg::ALONE_BYTES : Cfg::SMEM_BYTES, stream, a, b, epi, M, N, K, k_chunk, b_tiles, kblocks));
     VDNN_LAUNCHED();
     return VDNN_OK;
 }
