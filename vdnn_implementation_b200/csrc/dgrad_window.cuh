@@ -14,6 +14,8 @@
 // columns of the window (624).
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace vdnn {
@@ -22,7 +24,7 @@ namespace window {
 template <int R, int ST, int TI, int CC> struct Shape {
     static constexpr int U = (R + ST - 1) / ST, ROWS = TI + U - 1;
     static constexpr int PER_K = (R * R * CC + 3) / 4 * 4;           // floats of a filter in shared memory
-    static constexpr int THREADS = TI * ST * ST * CC > 64 ? 384 : 256;
+    static constexpr int THREADS = TI == 1 ? 128 : (TI * ST * ST * CC > 64 ? 384 : 256);
     // 3 x 3 / 1: little code per filter, so the next filter's window can be under way meanwhile, and warps that lie inside the
     // image take a loop without tests.
     static constexpr bool LIGHT = ST == 1 && R == 3;
@@ -198,17 +200,65 @@ int launch_shape(const vdnn_conv_desc* d, int P, int Q, float alpha, float beta,
     return VDNN_OK;
 }
 
-// VDNN_ERR_UNSUPPORTED for the filters that have no instance here.
+// Rows of a thread: the more, the fewer weights are read per sum, as far as the registers (sums; 3 x 3 / 1 also keeps the next
+// window) and the code of a filter go.  Measured at 64 filters and twice 128 registers of sums, 5 x 5 / 3 took 90 us where this
+// takes 66, 7 x 7 / 3 139 and 98, 3 x 3 / 1 with four channels 86 and 49.
+constexpr int rows_each(int r, int st, int cc) {
+    int ti = 8;
+    while (ti > 2 && (ti * st * st * cc > 96 || ti * r * r * cc > 1024 || (r == 3 && st == 1 && ti * cc > 24))) ti /= 2;
+    return ti;
+}
+
+// What a thread does takes the same time however few of them there are (11 x 11 / 4: 2.4 us per filter, 5 x 5 / 1 1.6), so
+// below half a block for each SM strides 1 and 2 take one row per thread: 5 x 5 / 1, 64 filters, four images of 64 x 64:
+// 98 -> 44 us, 7 x 7 / 2 160 -> 109.  At strides 3 and 4 that gains little (11 x 11 / 4 229 -> 195); there the phases go to
+// threads of their own below a seventh of a block for each SM (other kernels: 11 x 11 / 4, 96 filters, four images of 128 x 128
+// 119 against 229 us, 16 images 252 against 225).
+template <int R, int ST, int CC>
+int launch_filter(const vdnn_conv_desc* d, int P, int Q, float alpha, float beta, const float* w, const float* dy, float* dx, cudaStream_t stream) {
+    constexpr int TI = rows_each(R, ST, CC);
+    const long long positions = static_cast<long long>(d->n) * ceil_div((d->h - 1 + d->pad_h) / ST + 1, TI) * ((d->w - 1 + d->pad_w) / ST + 1);
+    const long long blocks = positions / Shape<R, ST, TI, CC>::THREADS;
+    if constexpr (ST <= 2) {
+        if (2 * blocks < sm_count()) return launch_shape<R, ST, 1, CC>(d, P, Q, alpha, beta, w, dy, dx, stream);
+    } else {
+        if (7 * blocks < sm_count()) return VDNN_ERR_UNSUPPORTED;
+    }
+    return launch_shape<R, ST, TI, CC>(d, P, Q, alpha, beta, w, dy, dx, stream);
+}
+
+template <int R>
+int launch_side(const vdnn_conv_desc* d, int P, int Q, float alpha, float beta, const float* w, const float* dy, float* dx, cudaStream_t stream) {
+    auto run = [&](auto st) {
+        constexpr int ST = decltype(st)::value;
+        if constexpr (ST > R) return static_cast<int>(VDNN_ERR_UNSUPPORTED);
+        else return d->c <= 3 ? launch_filter<R, ST, 3>(d, P, Q, alpha, beta, w, dy, dx, stream)
+                              : launch_filter<R, ST, 4>(d, P, Q, alpha, beta, w, dy, dx, stream);
+    };
+    switch (d->stride_h) {
+    case 1: return run(std::integral_constant<int, 1>());
+    case 2: return run(std::integral_constant<int, 2>());
+    case 3: return run(std::integral_constant<int, 3>());
+    case 4: return run(std::integral_constant<int, 4>());
+    default: return VDNN_ERR_UNSUPPORTED;
+    }
+}
+
+// Square filters of an odd side up to 11 at the same stride, up to 4 and to their side, both ways.  Against the kernels that take
+// the others (64 filters, 16 images, output 112 x 112 at stride 1 and 2): 3x3/1 59 and 76 us, 5x5/1 106 and 262, 7x7/1 160 and
+// 494, 9x9/1 293 and 809, 11x11/1 422 and 1412, 3x3/2 80 and 123, 5x5/2 131 and 191, 7x7/2 164 and 553, 9x9/2 248 and 1020,
+// 11x11/2 336 and 1421; 224 x 224 images at stride 3: 51 .. 205 and 68 .. 678; at stride 4: 66 .. 158 and 111 .. 225.
+// VDNN_ERR_UNSUPPORTED for all others.
 inline int launch(const vdnn_conv_desc* d, int P, int Q, float alpha, float beta, const float* w, const float* dy, float* dx, cudaStream_t stream) {
     if (d->r != d->s || d->stride_h != d->stride_w || d->pad_h != d->pad_w || d->c > 4) return VDNN_ERR_UNSUPPORTED;
-    if (d->r == 11 && d->stride_h == 4 && d->c <= 3) return launch_shape<11, 4, 2, 3>(d, P, Q, alpha, beta, w, dy, dx, stream);
-    if (d->r == 3 && d->stride_h == 1)
-        return d->c <= 3 ? launch_shape<3, 1, 8, 3>(d, P, Q, alpha, beta, w, dy, dx, stream) : launch_shape<3, 1, 8, 4>(d, P, Q, alpha, beta, w, dy, dx, stream);
-    if (d->r == 5 && d->stride_h == 1)
-        return d->c <= 3 ? launch_shape<5, 1, 8, 3>(d, P, Q, alpha, beta, w, dy, dx, stream) : launch_shape<5, 1, 8, 4>(d, P, Q, alpha, beta, w, dy, dx, stream);
-    if (d->r == 7 && d->stride_h == 2)
-        return d->c <= 3 ? launch_shape<7, 2, 4, 3>(d, P, Q, alpha, beta, w, dy, dx, stream) : launch_shape<7, 2, 4, 4>(d, P, Q, alpha, beta, w, dy, dx, stream);
-    return VDNN_ERR_UNSUPPORTED;
+    switch (d->r) {
+    case 3: return launch_side<3>(d, P, Q, alpha, beta, w, dy, dx, stream);
+    case 5: return launch_side<5>(d, P, Q, alpha, beta, w, dy, dx, stream);
+    case 7: return launch_side<7>(d, P, Q, alpha, beta, w, dy, dx, stream);
+    case 9: return launch_side<9>(d, P, Q, alpha, beta, w, dy, dx, stream);
+    case 11: return launch_side<11>(d, P, Q, alpha, beta, w, dy, dx, stream);
+    default: return VDNN_ERR_UNSUPPORTED;
+    }
 }
 
 }  // namespace window
