@@ -93,7 +93,8 @@ int vdnn_pool_out_dims(int h, int w, int win_h, int win_w, int stride_h, int str
 
 /* cudnnGetConvolution{Forward,BackwardData,BackwardFilter}WorkspaceSize (layer.cu:268-294)
  * together with the algorithm choice of find{MemOpt,PerfOpt}*Algo (layer.cu:1013-1089):
- * 0 for VDNN_ALGO_MEMORY_OPT, the split-K scratch of the PERF_OPT kernel otherwise. */
+ * 0 for VDNN_ALGO_MEMORY_OPT; otherwise what the PERF_OPT kernel that takes the shape reads or writes beside the tensors
+ * (operand images, packed weights, split-K parts), 0 where it needs none. */
 size_t vdnn_conv_workspace_bytes(int op, int algo_mode, const vdnn_conv_desc* d);
 
 /* cudnnConvolutionForward (layer.cu:560-569): y = alpha * (x corr w) + beta * y.
@@ -152,8 +153,9 @@ int vdnn_conv_bwd_shares_dy(const vdnn_conv_desc* d, int algo_mode);
  * buffer to pass as `workspace`.  The entry point calls no cudaMalloc / cudaFree and no routine
  * that allocates.
  *   - Shapes whose partial sums exceed the array (vdnn_conv_workspace_bytes(VDNN_CONV_BWD_FILTER,
- *     VDNN_ALGO_PERF_OPT, d) > VDNN_STATIC_SCRATCH_BYTES) are refused with VDNN_ERR_SCRATCH_LIMIT;
- *     nothing is launched.
+ *     VDNN_ALGO_PERF_OPT, d) > VDNN_STATIC_SCRATCH_BYTES, for a filter of full extent
+ *     vdnn_sgemm_workspace_bytes of its product) are refused with VDNN_ERR_SCRATCH_LIMIT; nothing is
+ *     launched.
  *   - The first call on a device looks up the array's device address (once per device, with that
  *     device current).  Make that first call before any stream capture begins.
  *   - All calls on a device share the one array, which keeps whatever the last call left in it.
@@ -164,7 +166,9 @@ int vdnn_conv_bwd_filter_static(const vdnn_conv_desc* d, float alpha, const floa
                                 float beta, float* dw, void* stream);
 
 /* cublasSgemm (layer.cu:677-685, 697-705, 725-733, 736-744, 752-760): column-major
- * C(m x n) = alpha * op(A) * op(B) + beta * C, transa/transb: 0 = N, 1 = T. */
+ * C(m x n) = alpha * op(A) * op(B) + beta * C, transa/transb: 0 = N, 1 = T.
+ * The workspace is enough for operands of any address and leading dimension.  Operands on 16-byte boundaries whose leading
+ * dimensions are multiples of four floats use none of it. */
 size_t vdnn_sgemm_workspace_bytes(int algo_mode, int m, int n, int k);
 int vdnn_sgemm(int transa, int transb, int m, int n, int k, float alpha, const float* A, int lda,
                const float* B, int ldb, float beta, float* C, int ldc,

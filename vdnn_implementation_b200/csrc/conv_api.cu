@@ -7,6 +7,8 @@
 #include <cuda_pipeline.h>
 #include <math.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "gemm_ffma.cuh"
 #include "gemm_tc.cuh"
@@ -278,6 +280,7 @@ __global__ void __launch_bounds__(TW) dgrad_small_c_phase_kernel(int C, int H, i
     }
 }
 
+// Without tensors (dx null) it only answers whether it would launch.
 template <int TW, int CC>
 int launch_dgrad_small_c_phase(const vdnn_conv_desc* d, int P, int Q, float alpha, float beta, const float* w, const float* dy,
                                float* dx, cudaStream_t stream) {
@@ -286,6 +289,7 @@ int launch_dgrad_small_c_phase(const vdnn_conv_desc* d, int P, int Q, float alph
                         static_cast<size_t>(S1_KC) * (S1_TH + 2) * (TW + 2) * sizeof(float);
     const long long slices = static_cast<long long>(d->n) * st * st;
     if (smem > 96 * 1024 || slices > 65535) return VDNN_ERR_UNSUPPORTED;
+    if (!dx) return VDNN_OK;
     auto kern = dgrad_small_c_phase_kernel<TW, CC>;
     int dev = 0;
     VDNN_CUDA(cudaGetDevice(&dev));
@@ -298,6 +302,39 @@ int launch_dgrad_small_c_phase(const vdnn_conv_desc* d, int P, int Q, float alph
     VDNN_LAUNCHED();
     return VDNN_OK;
 }
+
+// Data gradient of a first layer (at most four input channels), or VDNN_ERR_UNSUPPORTED where only the contraction can take
+// it.  None of these kernels uses workspace.  Without tensors (dx null) it only answers whether one of them would run.
+int dgrad_few_channels(const vdnn_conv_desc* d, int P, int Q, float alpha, const float* w, const float* dy, float beta, float* dx,
+                       cudaStream_t stream) {
+    if (d->c > SMALL_C_MAX) return VDNN_ERR_UNSUPPORTED;
+    int st = window::launch(d, P, Q, alpha, beta, w, dy, dx, stream);
+    if (st != VDNN_ERR_UNSUPPORTED) return st;
+    if (d->stride_h == d->stride_w && d->r <= 3 * d->stride_h && d->s <= 3 * d->stride_w) {
+        const bool narrow = (d->w - 1 + d->pad_w) / d->stride_w + 1 <= 64;      // class coordinates fit a 64-wide tile
+        if (d->c == 3) st = narrow ? launch_dgrad_small_c_phase<64, 3>(d, P, Q, alpha, beta, w, dy, dx, stream)
+                                   : launch_dgrad_small_c_phase<128, 3>(d, P, Q, alpha, beta, w, dy, dx, stream);
+        else st = narrow ? launch_dgrad_small_c_phase<64, 4>(d, P, Q, alpha, beta, w, dy, dx, stream)
+                         : launch_dgrad_small_c_phase<128, 4>(d, P, Q, alpha, beta, w, dy, dx, stream);
+        if (st != VDNN_ERR_UNSUPPORTED) return st;
+    }
+    const size_t small_smem = static_cast<size_t>(d->k) * d->c * d->r * d->s * sizeof(float);
+    if (small_smem > SMALL_C_SMEM_MAX) return VDNN_ERR_UNSUPPORTED;
+    if (!dx) return VDNN_OK;
+    int dev = 0;
+    VDNN_CUDA(cudaGetDevice(&dev));
+    if (VDNN_ONCE_PER_DEVICE(dev))
+        VDNN_CUDA(cudaFuncSetAttribute(dgrad_small_c_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SMALL_C_SMEM_MAX)));
+    const long long total = static_cast<long long>(d->n) * d->h * d->w;
+    long long blocks = (total + 255) / 256;
+    const long long cap = static_cast<long long>(sm_count()) * (small_smem > 100 * 1024 ? 1 : 2) * 2;
+    if (blocks > cap) blocks = cap;
+    dgrad_small_c_kernel<<<static_cast<int>(blocks), 256, small_smem, stream>>>(
+        d->n, d->c, d->h, d->w, d->k, d->r, d->s, P, Q, d->pad_h, d->pad_w, d->stride_h, d->stride_w, alpha, beta, w, dy, dx);
+    VDNN_LAUNCHED();
+    return VDNN_OK;
+}
+
 
 // A convolution whose filter covers the whole (unpadded) input produces one output pixel per image: it is a fully
 // connected layer, y[n][k] = sum_j w[k][j] x[n][j] with j running over (c, r, s) -- both operands contiguous in j.
@@ -406,18 +443,20 @@ int scale_output(float* out, float beta, int M, int N, size_t dense_elems, int l
 }
 
 // `epi` arrives configured for a direct store (out, alpha, beta, bias, addressing).
-// dense_elems > 0 says the output is one dense block of that many floats (needed for PARTIAL).
+// dense_elems > 0 says the output is one dense block of that many floats (needed for PARTIAL).  parts_optional: without room
+// for the parts in `ws` the reduction runs unsplit; else that is an error.
 template <class OpA, class OpB, bool AKC, bool BKC>
 int contract(const OpA& a, const OpB& b, Epilogue epi, int M, int N, int K, size_t dense_elems, int ld_rows,
-             int algo_mode, void* ws, size_t ws_bytes, cudaStream_t stream, char* b_tiles = nullptr) {
+             int algo_mode, void* ws, size_t ws_bytes, cudaStream_t stream, char* b_tiles = nullptr, bool parts_optional = false) {
     SplitPlan plan = plan_split(M, N, K);
-    if (epi.bias) { plan.splits = 1; plan.k_chunk = ceil_div(K, 32) * 32; }
+    const size_t need = static_cast<size_t>(plan.splits) * dense_elems * sizeof(float);
+    const bool whole = parts_optional && algo_mode == VDNN_ALGO_PERF_OPT && (!ws || ws_bytes < need);
+    if (epi.bias || whole) { plan.splits = 1; plan.k_chunk = ceil_div(K, 32) * 32; }
     if (plan.splits == 1) {
         epi.mode = EPI_DIRECT;
         return run_engine<OpA, OpB, AKC, BKC>(a, b, epi, M, N, K, 1, plan.k_chunk, stream, b_tiles);
     }
     if (algo_mode == VDNN_ALGO_PERF_OPT && dense_elems > 0) {
-        const size_t need = static_cast<size_t>(plan.splits) * dense_elems * sizeof(float);
         if (!ws || ws_bytes < need) return VDNN_ERR_WORKSPACE;
         Epilogue part = epi;
         part.mode = EPI_PARTIAL;
@@ -888,6 +927,41 @@ XGather make_xgather(const vdnn_conv_desc* d, const float* x, int P, int Q) {
     return g;
 }
 
+// vdnn_sgemm; parts_optional as in contract().
+int sgemm(int transa, int transb, int m, int n, int k, float alpha, const float* A, int lda, const float* B, int ldb, float beta, float* C,
+          int ldc, int algo_mode, void* workspace, size_t workspace_bytes, cudaStream_t s, bool parts_optional) {
+    if (!A || !B || !C || m <= 0 || n <= 0 || k <= 0 || ldc < m) return VDNN_ERR_BAD_ARG;
+    if (lda < (transa ? k : m) || ldb < (transb ? n : k)) return VDNN_ERR_BAD_ARG;
+    const long long lim = 0x7fffffffLL;
+    if (1LL * lda * (transa ? m : k) >= lim || 1LL * ldb * (transb ? k : n) >= lim || 1LL * ldc * n >= lim)
+        return VDNN_ERR_UNSUPPORTED;
+    // A'(i, kk) = op(A)[i][kk], B'(j, kk) = op(B)[kk][j]
+    SplitDense a = transa ? make_dense(A, m, k, lda, 1) : make_dense(A, m, k, 1, lda);
+    SplitDense b = transb ? make_dense(B, n, k, 1, ldb) : make_dense(B, n, k, ldb, 1);
+    Epilogue e{};
+    e.out = C; e.bias = nullptr; e.alpha = alpha; e.beta = beta;
+    e.row_div = FastDiv(1u << 30); e.row_hi = 0; e.row_lo = 1; e.col_stride = ldc;
+    const size_t dense = (ldc == m) ? static_cast<size_t>(m) * n : 0;
+    // operands that tensor copies can fetch run on the dense kernel, the others on the gather-fed one
+    if (g_engine != VDNN_ENGINE_FFMA && dense::supported(A, lda, B, ldb))
+        return sgemm_dense(transa, transb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, s);
+    auto run = [&](auto a_along_k, auto b_along_k) {
+        return contract<SplitDense, SplitDense, decltype(a_along_k)::value, decltype(b_along_k)::value>(a, b, e, m, n, k, dense, ldc, algo_mode, workspace,
+                                                                                                        workspace_bytes, s, nullptr, parts_optional);
+    };
+    const std::true_type yes{};
+    const std::false_type no{};
+    if (transa) return transb ? run(yes, no) : run(yes, yes);
+    return transb ? run(no, no) : run(no, yes);
+}
+
+// A convolution of full extent is a dense product with rows of C * R * S and K floats.  Where these are whole 16 bytes, tensors
+// that begin on 16-byte boundaries run on the dense kernel, and no workspace is reported.  Other tensors of such a shape, which
+// the gather-fed kernel takes, run unsplit in that.
+bool full_extent_dense(const vdnn_conv_desc* d, int op) {
+    return g_engine != VDNN_ENGINE_FFMA && d->c * d->r * d->s % 4 == 0 && (op == VDNN_CONV_FWD || d->k % 4 == 0);
+}
+
 }  // namespace
 }  // namespace vdnn
 
@@ -966,6 +1040,7 @@ size_t vdnn_conv_workspace_bytes(int op, int algo_mode, const vdnn_conv_desc* d)
         return own;
     }
     if (is_full_extent(d)) {        // runs as the corresponding FC product
+        if (full_extent_dense(d, op)) return 0;
         switch (op) {
         case VDNN_CONV_FWD: return vdnn_sgemm_workspace_bytes(algo_mode, d->k, d->n, crs);
         case VDNN_CONV_BWD_DATA: return vdnn_sgemm_workspace_bytes(algo_mode, crs, d->n, d->k);
@@ -973,6 +1048,9 @@ size_t vdnn_conv_workspace_bytes(int op, int algo_mode, const vdnn_conv_desc* d)
         default: return 0;
         }
     }
+    // layers of few input channels: kernels without workspace
+    if (op == VDNN_CONV_FWD && g_engine != VDNN_ENGINE_FFMA && wgrad_small_c_shape(d, Q)) return 0;
+    if (op == VDNN_CONV_BWD_DATA && fits_int32(d, P, Q) && dgrad_few_channels(d, P, Q, 1.0f, nullptr, nullptr, 0.0f, nullptr, nullptr) == VDNN_OK) return 0;
     switch (op) {
     case VDNN_CONV_FWD: M = d->n * P * Q; N = d->k; K = crs; out = static_cast<size_t>(M) * N; break;
     case VDNN_CONV_BWD_DATA: M = d->n * d->h * d->w; N = d->c; K = d->k * d->r * d->s; out = static_cast<size_t>(M) * N; break;
@@ -995,13 +1073,17 @@ int vdnn_conv_fwd(const vdnn_conv_desc* d, int algo_mode, float alpha, const flo
     if (!fits_int32(d, P, Q)) return VDNN_ERR_UNSUPPORTED;
     const int crs = d->c * d->r * d->s, pq = P * Q, rs = d->r * d->s;
     if (is_full_extent(d)) {    // Y[n][k] = sum_j W[k][j] X[n][j]   (the FC forward product, layer.cu:677-685), then the bias
-        const int st = vdnn_sgemm(1, 0, d->k, d->n, crs, alpha, w, crs, x, crs, beta, y, d->k, algo_mode, workspace, workspace_bytes, stream);
+        const int st = sgemm(1, 0, d->k, d->n, crs, alpha, w, crs, x, crs, beta, y, d->k, algo_mode, workspace, workspace_bytes, as_stream(stream),
+                             full_extent_dense(d, VDNN_CONV_FWD));
         if (st != VDNN_OK || !bias) return st;
         return vdnn_add_bias(d->n, d->k, 1, 1.0f, bias, y, stream);
     }
     // few input channels, 3 x 3, stride 1 (the first layer of VGG16): 27 terms per output, an FFMA kernel of its own
-    if (g_engine != VDNN_ENGINE_FFMA && wgrad_small_c_shape(d, Q) && (reinterpret_cast<uintptr_t>(y) & 15u) == 0)
-        return fwd_small_c(d, P, Q, alpha, x, w, bias, beta, y, as_stream(stream));
+    if (g_engine != VDNN_ENGINE_FFMA && wgrad_small_c_shape(d, Q)) {
+        if ((reinterpret_cast<uintptr_t>(y) & 15u) == 0) return fwd_small_c(d, P, Q, alpha, x, w, bias, beta, y, as_stream(stream));
+        // y off the 16-byte boundaries: the workspace variant below needs what the size query does not report
+        if (!workspace || workspace_bytes < packed_weight_bytes(d, VDNN_CONV_FWD)) algo_mode = VDNN_ALGO_MEMORY_OPT;
+    }
     Epilogue e{};
     e.out = y; e.bias = bias; e.alpha = alpha; e.beta = beta;
     e.row_div = FastDiv(pq); e.row_hi = d->k * pq; e.row_lo = 1; e.col_stride = pq;
@@ -1038,43 +1120,16 @@ int vdnn_conv_bwd_data(const vdnn_conv_desc* d, int algo_mode, float alpha, cons
     if (!fits_int32(d, P, Q)) return VDNN_ERR_UNSUPPORTED;
     const int rs = d->r * d->s, hw = d->h * d->w, pq = P * Q;
     if (is_full_extent(d))      // dX[n][j] = sum_k W[k][j] dY[n][k]   (the FC data-gradient product, layer.cu:725-733)
-        return vdnn_sgemm(0, 0, d->c * rs, d->n, d->k, alpha, w, d->c * rs, dy, d->k, beta, dx, d->c * rs, algo_mode, workspace,
-                          workspace_bytes, stream);
-    if (d->c <= SMALL_C_MAX) {
-        const int st = window::launch(d, P, Q, alpha, beta, w, dy, dx, as_stream(stream));
-        if (st != VDNN_ERR_UNSUPPORTED) return st;
-    }
-    if (d->c <= SMALL_C_MAX && d->stride_h == d->stride_w && d->r <= 3 * d->stride_h && d->s <= 3 * d->stride_w) {
-        const bool narrow = (d->w - 1 + d->pad_w) / d->stride_w + 1 <= 64;      // class coordinates fit a 64-wide tile
-        cudaStream_t cs = as_stream(stream);
-        int st;
-        if (d->c == 3) st = narrow ? launch_dgrad_small_c_phase<64, 3>(d, P, Q, alpha, beta, w, dy, dx, cs)
-                                   : launch_dgrad_small_c_phase<128, 3>(d, P, Q, alpha, beta, w, dy, dx, cs);
-        else st = narrow ? launch_dgrad_small_c_phase<64, 4>(d, P, Q, alpha, beta, w, dy, dx, cs)
-                         : launch_dgrad_small_c_phase<128, 4>(d, P, Q, alpha, beta, w, dy, dx, cs);
-        if (st != VDNN_ERR_UNSUPPORTED) return st;
-    }
-    const size_t small_smem = static_cast<size_t>(d->k) * d->c * rs * sizeof(float);
-    if (d->c <= SMALL_C_MAX && small_smem <= SMALL_C_SMEM_MAX) {
-        int dev = 0;
-        VDNN_CUDA(cudaGetDevice(&dev));
-        if (VDNN_ONCE_PER_DEVICE(dev))
-            VDNN_CUDA(cudaFuncSetAttribute(dgrad_small_c_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SMALL_C_SMEM_MAX)));
-        const long long total = static_cast<long long>(d->n) * hw;
-        long long blocks = (total + 255) / 256;
-        const long long cap = static_cast<long long>(sm_count()) * (small_smem > 100 * 1024 ? 1 : 2) * 2;
-        if (blocks > cap) blocks = cap;
-        dgrad_small_c_kernel<<<static_cast<int>(blocks), 256, small_smem, as_stream(stream)>>>(
-            d->n, d->c, d->h, d->w, d->k, d->r, d->s, P, Q, d->pad_h, d->pad_w, d->stride_h, d->stride_w, alpha, beta, w, dy, dx);
-        VDNN_LAUNCHED();
-        return VDNN_OK;
-    }
+        return sgemm(0, 0, d->c * rs, d->n, d->k, alpha, w, d->c * rs, dy, d->k, beta, dx, d->c * rs, algo_mode, workspace,
+                     workspace_bytes, as_stream(stream), full_extent_dense(d, VDNN_CONV_BWD_DATA));
+    int st = dgrad_few_channels(d, P, Q, alpha, w, dy, beta, dx, as_stream(stream));
+    if (st != VDNN_ERR_UNSUPPORTED) return st;
     // Without workspace only: the gather-fed kernel with packed weights (PERF_OPT, channels or sizes that the TMA-fed kernels do
     // not take) is faster than the halo kernel on every shape measured -- 1.07 .. 2.0 times as fast at 3x3 (250 <- 500 channels,
     // 64 images of 28 x 28: 771 against 1565 us; 512 <- 256, 84 x 87: 121 against 209), 1.07 .. 2.5 at 5x5, 1.4 .. 3.0 at 7x7
     // and 9x9.
     if (algo_mode == VDNN_ALGO_MEMORY_OPT && g_engine != VDNN_ENGINE_FFMA && d->stride_h == 1 && d->stride_w == 1) {
-        const int st = dgrad_halo(d, P, Q, dy, w, alpha, beta, dx, as_stream(stream));
+        st = dgrad_halo(d, P, Q, dy, w, alpha, beta, dx, as_stream(stream));
         if (st != VDNN_ERR_UNSUPPORTED) return st;
     }
     DyGather A;
@@ -1101,7 +1156,7 @@ int vdnn_conv_bwd_data(const vdnn_conv_desc* d, int algo_mode, float alpha, cons
         char* tiles = (g_engine != VDNN_ENGINE_FFMA && (reinterpret_cast<uintptr_t>(workspace) & 127u) == 0) ? static_cast<char*>(workspace) : nullptr;
         if (tiles && tma_shape(d, VDNN_CONV_BWD_DATA) && !g_no_tma) {
             const tma::Problem q = tma_problem(d, VDNN_CONV_BWD_DATA, P, Q);
-            int st = tc::pack_b<SplitDense, false>(B, d->c, d->k * rs, s, tiles, tma_use_strips(q) ? tma::strip_tile_n(d->c) : 0);
+            st = tc::pack_b<SplitDense, false>(B, d->c, d->k * rs, s, tiles, tma_use_strips(q) ? tma::strip_tile_n(d->c) : 0);
             if (st != VDNN_OK) return st;
             return contract_tma(q, dy, tiles, e, static_cast<size_t>(M) * d->c, tiles + pack, workspace_bytes - pack, s);
         }
@@ -1121,7 +1176,8 @@ int vdnn_conv_bwd_filter(const vdnn_conv_desc* d, int algo_mode, float alpha, co
     if (!fits_int32(d, P, Q)) return VDNN_ERR_UNSUPPORTED;
     const int crs = d->c * d->r * d->s, pq = P * Q;
     if (is_full_extent(d))      // W[k][j] = alpha * sum_n X[n][j] dY[n][k] + beta * W[k][j]   (layer.cu:736-744)
-        return vdnn_sgemm(0, 1, crs, d->k, d->n, alpha, x, crs, dy, d->k, beta, dw, crs, algo_mode, workspace, workspace_bytes, stream);
+        return sgemm(0, 1, crs, d->k, d->n, alpha, x, crs, dy, d->k, beta, dw, crs, algo_mode, workspace, workspace_bytes, as_stream(stream),
+                     full_extent_dense(d, VDNN_CONV_BWD_FILTER));
     if (algo_mode == VDNN_ALGO_PERF_OPT && g_engine != VDNN_ENGINE_FFMA && wgrad_small_c_shape(d, Q) && workspace &&
         (reinterpret_cast<uintptr_t>(dy) & 15u) == 0 && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0)
         return wgrad_small_c(d, P, Q, x, dy, alpha, beta, dw, 0.0f, 0.0f, nullptr, static_cast<char*>(workspace), workspace_bytes, as_stream(stream));
@@ -1245,7 +1301,8 @@ int vdnn_conv_bwd_filter_static(const vdnn_conv_desc* d, float alpha, const floa
                                 float* dw, void* stream) {
     int P, Q;
     if (!x || !dy || !dw || !valid_desc(d, &P, &Q)) return VDNN_ERR_BAD_ARG;
-    const size_t need = vdnn_conv_workspace_bytes(VDNN_CONV_BWD_FILTER, VDNN_ALGO_PERF_OPT, d);
+    const size_t need = is_full_extent(d) ? vdnn_sgemm_workspace_bytes(VDNN_ALGO_PERF_OPT, d->c * d->r * d->s, d->k, d->n)
+                                          : vdnn_conv_workspace_bytes(VDNN_CONV_BWD_FILTER, VDNN_ALGO_PERF_OPT, d);
     if (need > VDNN_STATIC_SCRATCH_BYTES) return VDNN_ERR_SCRATCH_LIMIT;
     float* scratch = nullptr;
     const int st = static_scratch_address(&scratch);
@@ -1264,26 +1321,7 @@ size_t vdnn_sgemm_workspace_bytes(int algo_mode, int m, int n, int k) {
 int vdnn_sgemm(int transa, int transb, int m, int n, int k, float alpha, const float* A, int lda, const float* B,
                int ldb, float beta, float* C, int ldc, int algo_mode, void* workspace, size_t workspace_bytes,
                void* stream) {
-    if (!A || !B || !C || m <= 0 || n <= 0 || k <= 0 || ldc < m) return VDNN_ERR_BAD_ARG;
-    if (lda < (transa ? k : m) || ldb < (transb ? n : k)) return VDNN_ERR_BAD_ARG;
-    const long long lim = 0x7fffffffLL;
-    if (1LL * lda * (transa ? m : k) >= lim || 1LL * ldb * (transb ? k : n) >= lim || 1LL * ldc * n >= lim)
-        return VDNN_ERR_UNSUPPORTED;
-    // A'(i, kk) = op(A)[i][kk], B'(j, kk) = op(B)[kk][j]
-    SplitDense a = transa ? make_dense(A, m, k, lda, 1) : make_dense(A, m, k, 1, lda);
-    SplitDense b = transb ? make_dense(B, n, k, 1, ldb) : make_dense(B, n, k, ldb, 1);
-    Epilogue e{};
-    e.out = C; e.bias = nullptr; e.alpha = alpha; e.beta = beta;
-    e.row_div = FastDiv(1u << 30); e.row_hi = 0; e.row_lo = 1; e.col_stride = ldc;
-    const size_t dense = (ldc == m) ? static_cast<size_t>(m) * n : 0;
-    cudaStream_t s = as_stream(stream);
-    // operands that tensor copies can fetch run on the dense kernel, the others on the gather-fed one
-    if (g_engine != VDNN_ENGINE_FFMA && dense::supported(A, lda, B, ldb))
-        return sgemm_dense(transa, transb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, s);
-    if (transa && !transb) return contract<SplitDense, SplitDense, true, true>(a, b, e, m, n, k, dense, ldc, algo_mode, workspace, workspace_bytes, s);
-    if (!transa && !transb) return contract<SplitDense, SplitDense, false, true>(a, b, e, m, n, k, dense, ldc, algo_mode, workspace, workspace_bytes, s);
-    if (!transa && transb) return contract<SplitDense, SplitDense, false, false>(a, b, e, m, n, k, dense, ldc, algo_mode, workspace, workspace_bytes, s);
-    return contract<SplitDense, SplitDense, true, false>(a, b, e, m, n, k, dense, ldc, algo_mode, workspace, workspace_bytes, s);
+    return sgemm(transa, transb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, algo_mode, workspace, workspace_bytes, as_stream(stream), false);
 }
 
 }  // extern "C"

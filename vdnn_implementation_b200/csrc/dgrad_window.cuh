@@ -178,6 +178,7 @@ __global__ void __launch_bounds__(Shape<R, ST, TI, CC>::THREADS, Shape<R, ST, TI
         }
 }
 
+// Without tensors (dx null) it only answers whether it would launch.
 template <int R, int ST, int TI, int CC>
 int launch_shape(const vdnn_conv_desc* d, int P, int Q, float alpha, float beta, const float* w, const float* dy, float* dx, cudaStream_t stream) {
     typedef Shape<R, ST, TI, CC> Sh;
@@ -185,6 +186,7 @@ int launch_shape(const vdnn_conv_desc* d, int P, int Q, float alpha, float beta,
     const int hv = (d->h - 1 + d->pad_h) / ST + 1, wv = (d->w - 1 + d->pad_w) / ST + 1, ni = ceil_div(hv, TI);
     const long long total = static_cast<long long>(d->n) * ni * wv;
     if (total > 0x7ffffc00LL) return VDNN_ERR_UNSUPPORTED;
+    if (!dx) return VDNN_OK;
     constexpr int LIMIT = 200 * 1024, fit = LIMIT / (Sh::PER_K * 4);
     Params p;
     p.C = d->c; p.H = d->h; p.W = d->w; p.K = d->k; p.P = P; p.Q = Q; p.pad = d->pad_h;
