@@ -39,6 +39,13 @@ def test_sgemm_aligned(vdnn, oracle, size, trans, algo):
     assert ops.engine_status() == 0
 
 
+@pytest.mark.parametrize("n,k", [(320, 320), (320, 324), (321, 192), (321, 193), (324, 196), (64, 320), (32, 321), (1000, 256)])
+def test_sgemm_around_the_short_reductions(vdnn, oracle, n, k):
+    """Sizes at the lines between tiles whose C goes out through shared memory and the others."""
+    test_sgemm_aligned(vdnn, oracle, (260, n, k), (0, 1), 0)
+    test_sgemm_aligned(vdnn, oracle, (260, n, k), (1, 0), 0)
+
+
 @pytest.mark.parametrize("rows", [148 * 128, 148 * 128 + 1000])
 @pytest.mark.parametrize("n", [8, 64, 128])
 def test_sgemm_long_reduction(vdnn, n, rows):

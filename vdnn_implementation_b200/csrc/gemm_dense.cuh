@@ -445,9 +445,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 }
 
 // Columns of a tile.  A short reduction spends its time on C, not on the product: there 64-column tiles, which leave room
-// for two C tiles in shared memory, are the faster ones at any width.
-inline bool short_reduction(int K) { return K <= 256; }
-inline int tile_n(int N, int K) { return N <= 32 ? 32 : (N <= 64 || short_reduction(K) ? 64 : 128); }
+// for two C tiles in shared memory, are the faster ones.  Time with them over time without (B200, flushed L2): 25088 x 4096 and
+// 4096 x 4096 at K = 64 0.80 .. 0.83, 128 0.97, 192 0.97 .. 1.03, 256 1.06, 384 1.12, 768 1.23; 4096 x 1000 0.89, 1.00, 1.00, 1.07,
+// 1.16, 1.21.  Few columns leave SMs idle with wide tiles: 4096 x 200 and 9216 x 300 0.8 .. 0.9 up to K = 384, 1.00 at 1000;
+// 1024 x 128 1.00 at 320, 1.14 at 512; 4096 x 32 1.00 at 320, 1.17 at 384.
+inline bool short_reduction(int N, int K) { return K <= (N <= 320 ? 320 : 192); }
+inline int tile_n(int N, int K) { return N <= 32 ? 32 : (N <= 64 || short_reduction(N, K) ? 64 : 128); }
 
 constexpr int MAX_SPLITS = 8;                                        // CTAs of a portable cluster
 
@@ -539,7 +542,7 @@ int launch_bn(const float* A, int lda, const float* B, int ldb, Params p, int K,
 template <bool AK, bool BKM>
 int launch(const float* A, int lda, const float* B, int ldb, const Params& p, int K, cudaStream_t stream) {
     const int bn = tile_n(p.N, K);
-    const bool staged = short_reduction(K) && p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0;
+    const bool staged = short_reduction(p.N, K) && p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0;
     if (bn == 32) return staged ? launch_bn<AK, BKM, 32, true>(A, lda, B, ldb, p, K, stream) : launch_bn<AK, BKM, 32, false>(A, lda, B, ldb, p, K, stream);
     if (bn == 64) return staged ? launch_bn<AK, BKM, 64, true>(A, lda, B, ldb, p, K, stream) : launch_bn<AK, BKM, 64, false>(A, lda, B, ldb, p, K, stream);
     return launch_bn<AK, BKM, 128, false>(A, lda, B, ldb, p, K, stream);
