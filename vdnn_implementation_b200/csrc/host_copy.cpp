@@ -11,8 +11,15 @@ namespace vdnn {
 
 namespace {
 constexpr size_t kChunk = 2u << 20;         // a huge page of the host
-// Up to these sizes this thread alone is the faster way.  A write takes longer to be worth it: its source has been touched.
-constexpr size_t kDirectRead = 512u << 10, kDirectWrite = 2u << 20;
+// Up to these sizes one thread is the faster way.  Measured with the other way beside it (us, B200 host, fresh destinations):
+//   reads   64 KB 25 alone, 31 by threads; 512 KB 48 and 55; 1 MB 106 and 103; 2 MB 184 and 135
+//   writes  1 MB 61 by cudaMemcpy, 104 by threads; 2 MB 120 and 156; 4 MB 226 and 235; 6 MB 332 and 313; 8 MB 477 and 379
+// A write takes longer to be worth it: its source has been touched.
+constexpr size_t kDirectRead = 512u << 10, kDirectWrite = 4u << 20;
+// From this size on a thread takes whole huge pages.  Below, the page faults of the destination are what takes long, and smaller
+// pieces let more threads share them: 4 MB 179 us in quarters, 213 whole; 8 MB 308 and 331; 12 MB 452 and 424; 16 MB 613 and 530;
+// 32 MB 1520 and 1240.
+constexpr size_t kWholePages = 16u << 20;
 
 // Makes a device current for as long as it lives; the thread gets its own device back.
 struct OnDevice {
@@ -101,8 +108,7 @@ cudaError_t HostCopy::run(void* host, void* dev, size_t bytes, int device, bool 
     // chunk 0 ends at the first 2 MB boundary of the host address
     size_t head = kChunk - (reinterpret_cast<uintptr_t>(h) & (kChunk - 1));
     if (head > bytes) head = bytes;
-    // below a few chunks the page faults of the destination are what takes long: smaller pieces for more threads
-    const size_t piece = bytes >= 8 * kChunk ? kChunk : kChunk / 4;
+    const size_t piece = bytes >= kWholePages ? kChunk : kChunk / 4;
     if (piece < kChunk && head > piece) head = piece;
     const size_t chunks = 1 + (bytes - head + piece - 1) / piece;
     unsigned cores = std::thread::hardware_concurrency();
