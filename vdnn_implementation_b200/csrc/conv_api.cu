@@ -70,7 +70,8 @@ __global__ void __launch_bounds__(256) scale_matrix_kernel(int rows, int cols, i
 // out[i] = alpha * sum_s partial[s][i] + beta * out[i] in a fixed order.  A block takes 256 / lanes groups of VEC adjacent
 // sums; its lanes share a group's splits (lane l adds splits l, l + lanes, ... with four loads in flight) and their parts
 // are added in lane order.  With one thread per sum, a layer of few weights and many splits (an image's first filters: 864
-// sums of 150 parts) walked its splits one load after another on a handful of SMs: 10 us; now 3.
+// sums of 150 parts) walked its splits one load after another on a handful of SMs: 10 us in a single call; now 4.2, and 2.7
+// in a row of calls.
 template <int VEC>
 __global__ void __launch_bounds__(256) reduce_partials_kernel(size_t n, int splits, int lanes, float alpha, float beta,
                                                               const float* __restrict__ partial, float* __restrict__ out) {
@@ -365,8 +366,8 @@ bool tma_shape(const vdnn_conv_desc* d, int op) {
     if (op == VDNN_CONV_BWD_DATA && d->c <= SMALL_C_MAX) return false;          // the first layer has its own kernels
     if ((op == VDNN_CONV_FWD ? d->c : d->k) % 32 != 0) return false;
     // Only where the output has enough tiles to fill the GPU without splitting the reduction: the few-tile layers (14 x 14
-    // maps) stay on the gather kernel, which splits along k at a finer grain and needs no operand images.  With the
-    // engine forced to VDNN_ENGINE_TCGEN05 every eligible shape takes the TMA-fed path (small shapes in the tests).
+    // maps) stay on the gather kernel, which splits along k at a finer grain and needs no operand images (without workspace
+    // some of their data gradients run on the halo kernel, see dgrad_halo).  With the engine forced to VDNN_ENGINE_TCGEN05 every eligible shape takes the TMA-fed path (small shapes in the tests).
     if (g_engine == VDNN_ENGINE_TCGEN05) return true;
     const int P = (d->h + 2 * d->pad_h - d->r) / d->stride_h + 1, Q = (d->w + 2 * d->pad_w - d->s) / d->stride_w + 1;
     const long long pixels = static_cast<long long>(d->n) * (op == VDNN_CONV_FWD ? P * Q : d->h * d->w);

@@ -7,8 +7,9 @@
 // with all their phases and channels (TI * st * st * CC sums in registers) and, per filter, loads the (TI + U - 1) x U window
 // once (U = ceil(R / st); neighbouring threads share it through L1) against TI * R * R * CC multiply-adds; the weights of a
 // filter come as float4 broadcasts from shared memory, in the order they are used.
-// Walking one phase at a time, with dy staged through shared memory again for each of them, took 1243 us for 64 x 96 x 55 x 55
-// (11 x 11 / 4, C = 3: 10.9 TFLOP/s); this takes 410.  64 x 64 x 224 x 224 (3 x 3 / 1): 638, now 370.
+// Walking one phase at a time, with dy staged through shared memory again for each of them, took 1233 us for 64 x 96 x 55 x 55
+// (11 x 11 / 4, C = 3: 10.9 TFLOP/s); this takes 405 (calls one behind the other; 435 behind a flush of L2).  64 x 64 x 224 x 224
+// (3 x 3 / 1): 634, now 366.
 // What bounds it is the code of a filter, unrolled: 860 instructions for 11 x 11 / 4, and warps that wait for them.  One row
 // phase per block with more positions each reads fewer weights but measured slower (452 .. 558 us), as did a loop over the
 // columns of the window (624).

@@ -46,6 +46,10 @@ namespace {
 
 namespace cg = cooperative_groups;
 
+// Times in the comments of this file, before and after: B200, calls one behind the other in a graph, large tensors taken from
+// three sets that together pass L2, small ones resident in it (a launch of one value takes 1.1 us so).  A single call behind a
+// flush of L2 reads about 6 us more, the launch.
+
 constexpr int kThreads = 256;
 
 // Blocks for a streaming kernel in which every thread handles `per_thread` items per loop trip.
@@ -194,7 +198,7 @@ __global__ void __launch_bounds__(kThreads) fill_kernel(size_t n, float v, float
 //   BIAS_PLANE4  pq % 4 == 0: a float4 lies inside one channel's plane;   BIAS_ROW4  pq == 1, K % 4 == 0: a float4 takes
 //   four channels;   BIAS_SCALAR  everything else.
 // Bound by memory.  The form before this took a block per (image, channel) plane, which for a fully connected layer is one
-// block for every single value: 64 x 4096 cost 73 us; flat it costs 3 (2 MB in, 1 MB out, resident in L2).
+// block for every single value: 64 x 4096 cost 63 us; flat it costs 1.8 (1 MB in, 1 MB out).
 enum BiasForm { BIAS_SCALAR, BIAS_PLANE4, BIAS_ROW4 };
 template <BiasForm FORM>
 __global__ void __launch_bounds__(kThreads) add_bias_kernel(uint32_t items, FastDiv div_pq, FastDiv div_k, float alpha,
@@ -244,7 +248,8 @@ __device__ __forceinline__ float cluster_sum(float block_value, float* slot) {
 // db[ch] = alpha * sum over (n, pq) of dy[n][ch][pq] + beta * db[ch].  A cluster of up to eight blocks takes a channel and
 // adds its parts through distributed shared memory: one launch, no pre-scaling pass, no atomics, the same bits every time.
 // Bound by reading dy.  The flat index over (image, pixel) keeps all threads busy whatever the plane size; VEC = planes of
-// whole float4.  Measured (64 x 96 x 55 x 55, planes of odd size): 54.7 us with one strided plane after another, now 20.
+// whole float4.  Measured (64 x 96 x 55 x 55, planes of odd size): 58.6 us with one strided plane after another, now 26.5
+// (2.8 TB/s).
 template <int VEC>
 __global__ void __launch_bounds__(512) bwd_bias_kernel(uint32_t items, int k, FastDiv div_plane, float alpha, const float* __restrict__ dy,
                                                        float beta, float* __restrict__ db) {
@@ -284,8 +289,8 @@ __global__ void __launch_bounds__(512) bwd_bias_kernel(uint32_t items, int k, Fa
 
 // The same for planes of fewer than 32 values (a fully connected layer has planes of one): dy is then read along its rows,
 // a block taking 32 / pq whole channels = up to 32 adjacent columns, eight rows at a time; blocks of a cluster share the
-// rows.  Per-plane reading cost 145 us for 64 x 4096 (a block of 256 threads per channel, one value per row each); this
-// form 4.
+// rows.  Per-plane reading cost 90 us for 64 x 4096 (a block of 256 threads per channel, one value per row each); this
+// form 3.2.
 __global__ void __launch_bounds__(256) bwd_bias_narrow_kernel(int n, int k, int pq, float alpha, const float* __restrict__ dy, float beta,
                                                               float* __restrict__ db) {
     __shared__ float part[8][33];
@@ -330,7 +335,7 @@ __global__ void __launch_bounds__(256) bwd_bias_narrow_kernel(int n, int k, int 
 // ---------------------------------------------------------------- max pooling
 // One thread per output; the flat index is taken apart with multiplications (a 64-bit division per output was a third of the
 // time of this kernel).  WIN > 0: square window of that size, unrolled, so its loads are in flight together; 0: any window.
-// Bound by L1 (a stride-2 row touches every line twice): 64 x 96 x 55 x 55, 3 x 3 / 2: 44.3 us before, 17 now.
+// Bound by L1 (a stride-2 row touches every line twice): 64 x 96 x 55 x 55, 3 x 3 / 2: 42.0 us before, 22.2 now (4.2 TB/s).
 template <int WIN>
 __global__ void __launch_bounds__(kThreads) maxpool_fwd_generic(uint32_t total, int h, int w, FastDiv div_p, FastDiv div_q, int wh, int ww,
                                                                 int sh, int sw, const float* __restrict__ x,
@@ -384,8 +389,9 @@ __global__ void __launch_bounds__(kThreads) maxpool_fwd_2x2(size_t pairs, int w,
 // and hands place and dy to its right neighbour by shuffle, so that no shared memory and no barrier is involved and four
 // windows' loads are in flight.  The columns of all planes form one list: small planes share a warp; of a 3 x 3 warp's 32
 // columns the first is there for its neighbour only.  Sums are in scan order, the same every time.
-// With the windows in shared memory (two barriers, three times the instructions) 64 x 96 x 55 x 55, 3 x 3, took 78 us (now 49,
-// 3.4 TB/s), 128 x 256 x 13 x 13 57 (23), 64 x 512 x 14 x 14, 2 x 2, 57 (21).
+// With the windows in shared memory (two barriers, three times the instructions) 64 x 96 x 55 x 55, 3 x 3, took 78 us in a single
+// call behind a flush of L2 (now 49 so, and 41.6 at 4.0 TB/s one behind the other), 128 x 256 x 13 x 13 57 (23), 64 x 512 x 14 x
+// 14, 2 x 2, 57 (21).
 template <int WIN>
 __global__ void __launch_bounds__(kThreads, 4) maxpool_bwd_columns(int total, int h, int w, FastDiv div_items, int P, int Q, int band_rows, bool pairs,
                                                                    const float* __restrict__ dy, const float* __restrict__ x, float* __restrict__ dx) {
@@ -631,8 +637,8 @@ __device__ __forceinline__ double block_sum_f64(double v, double* part) {
 // correct bits.  The tensors stay fp32; the extra cost on N x 1000 elements is nil.
 //
 // A block per row, the row in registers (rows of up to 8 * 256 values; longer ones are read again in every pass).  These
-// calls are bound by latency: with one warp per row and a dependent loop per pass, 64 rows of 1000 took 7.1 us forward and
-// 6.5 backward; now 2.8 and 2.5.
+// calls are bound by latency: with one warp per row and a dependent loop per pass, 64 rows of 1000 took 7.2 us forward and
+// 5.2 backward; now 2.8 and 2.3.
 constexpr int ROW_VALUES = 8;
 __global__ void __launch_bounds__(256) softmax_fwd_kernel(int cols, const float* __restrict__ x, float* __restrict__ y) {
     __shared__ float part_m[8];
@@ -691,8 +697,8 @@ __global__ void __launch_bounds__(256) softmax_bwd_kernel(int cols, const float*
 
 // ---------------------------------------------------------------- loss (one cluster)
 // A warp per row, the rows dealt to the warps of up to eight blocks; the blocks' sums meet through distributed shared
-// memory in rank order.  One block of 32 warps took 11.9 us for 64 x 1000 (two rows after another per warp, 32 dependent
-// trips each); now 3.9.
+// memory in rank order.  One block of 32 warps took 11.1 us for 64 x 1000 (two rows after another per warp, 32 dependent
+// trips each); now 4.6.
 __global__ void __launch_bounds__(512) loss_kernel(int rows, int cols, const float* __restrict__ y,
                                                    const float* __restrict__ label, double* __restrict__ out2) {
     __shared__ double s_sq[16], s_ce[16];
@@ -818,8 +824,8 @@ __device__ __forceinline__ float lrn_pow(float s, float beta, float* inv_s) {
 // A thread takes LRN_CH channels of one position; their x (with two neighbours on either side, for backward four) is loaded
 // at once, so the loads of a thread are in flight together and there are c / LRN_CH times as many threads as positions;
 // adjacent chunks of a block of positions sit in one block, so the overlap is read from L1.  One thread per position,
-// walking all channels with one load in flight and a powf per channel, took 128.9 us forward and 272.5 backward for
-// 64 x 96 x 55 x 55 (1.15 and 1.09 TB/s); now 31 and 49.
+// walking all channels with one load in flight and a powf per channel, took 136.8 us forward and 242.7 backward for
+// 64 x 96 x 55 x 55 (1.09 and 0.92 TB/s); now 35.4 and 57.3 (4.2 and 3.9 TB/s).
 constexpr int LRN_CH = 16, LRN_POS = 64, LRN_CHUNKS = 4;
 template <bool BETA34>
 __global__ void __launch_bounds__(LRN_POS * LRN_CHUNKS) lrn_fwd_win5_kernel(int c, int hw, float alpha_over_n, float beta, float k,

@@ -4,12 +4,12 @@
 // of at most a few hundred rows, so the call is bound by streaming the weights -- if enough bytes are in flight and the
 // shared memory is not the bottleneck first.  The gather-fed kernel (gemm_tc.cuh) had one k block in flight per SM and moved
 // every operand element through registers and twice (hi, lo) through shared memory.  Here
-//   * one thread fetches raw fp32 tiles of both operands with tensor copies into a ring of 4 .. 7 stages (96 .. 170 KB in
+//   * one warp (its elected lane) fetches raw fp32 tiles of both operands with tensor copies into a ring of 4 .. 7 stages (96 .. 170 KB in
 //     flight per SM);
-//   * eight warps split them into tf32 hi / lo: the A tile goes from shared memory through registers into TENSOR MEMORY
+//   * two or three groups of four warps, taking stages in turn, split them into tf32 hi / lo: the A tile goes from shared memory through registers into TENSOR MEMORY
 //     (tcgen05.st; lane = row, column = k), where tcgen05.mma reads it without touching shared memory, whatever its
 //     orientation in memory was; the B tile is split in place (hi over the raw values, lo beside it);
-//   * one thread issues the 3xTF32 MMAs, eight warps add finished accumulators into fp32 registers and store.
+//   * one warp walks the stages and an elected lane of it issues the 3xTF32 MMAs, eight warps add finished accumulators into fp32 registers and store.
 // Shared-memory traffic per 128 x 64 x 32 block is 704 clocks' worth instead of 1344 with A staged as hi / lo tiles, just
 // under what HBM delivers (16 KB of weights in 712 clocks).
 // Measured (batch 64, 25088 -> 4096, flushed L2, B200; 411 MB of weights = 63 us at copy rate), gather-fed kernel before ->
@@ -280,7 +280,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         }
         if (STAGED && t == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     } else if (warp < TMA_WARP) {
-        // ------------------------------------------------------------------ split: group g takes every second stage
+        // ------------------------------------------------------------------ split: group g takes every GROUPS-th stage
         const int g = (warp - DRAIN_WARPS) >> 2, row = (warp & 3) * 32 + lane;
         const uint32_t tmem_lane = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + Cfg::A_COL;
         unsigned i = 0;
@@ -457,6 +457,9 @@ constexpr int MAX_SPLITS = 8;                                        // CTAs of 
 // Split of the reduction for the last, partly filled wave of tiles (`rest` of them), the `splits` CTAs of a tile in one
 // cluster.  A wave costs its k blocks plus about three for its start, three more for the sum over the cluster, and eight
 // (3 us) where it needs a launch of its own after the full waves.  resident(s): clusters of s CTAs that run at once.
+// Chosen against the best of 1 .. 8 on 15 shapes (1 .. 200 tiles, K = 512 .. 25088; B200, flushed L2): the same time on 14 of
+// them, 2 % more on one (25088 x 64, K = 4096: five parts 113.7 us, two 111.6, none 129).  4096 x 64, K = 25088: four parts 104
+// us, three 129, five 160; 9216 x 128, K = 4096: two 60, one 94, three 81; 12800 x 200, K = 640: none 41, two 42.
 template <class Resident> inline int plan_splits(long long rest, int kblocks, bool own_launch, Resident resident) {
     int best = 1;
     double best_cost = kblocks + 3.0;
