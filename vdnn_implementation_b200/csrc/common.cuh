@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "once.h"
 #include "vdnn_b200.h"
 
 namespace vdnn {
@@ -37,10 +38,13 @@ inline int cuda_fail(cudaError_t e) {
 // (queried once per device) so that every SM gets the same number of resident blocks.
 int sm_count();
 
-// True exactly once per device and call site (`seen` is the site's own table): kernels raise their dynamic shared
-// memory limit the first time they run on a device.  The table grows with the device ordinal.
-bool first_use_on_device(void** seen_table, int device);
-#define VDNN_ONCE_PER_DEVICE(dev) ([&]() { static void* _tbl = nullptr; return ::vdnn::first_use_on_device(&_tbl, (dev)); }())
+// Raises a kernel's limit of dynamic shared memory, once per device and kernel (each instance of a template is a place of its
+// own); no thread launches before it is raised.
+#define VDNN_ALLOW_SHARED(dev, kern, bytes)                                                                            \
+    do {                                                                                                               \
+        static ::vdnn::OncePerDevice _once;                                                                            \
+        VDNN_CUDA(_once.run((dev), [&]() { return cudaFuncSetAttribute((kern), cudaFuncAttributeMaxDynamicSharedMemorySize, (bytes)); })); \
+    } while (0)
 
 inline cudaStream_t as_stream(void* s) { return static_cast<cudaStream_t>(s); }
 

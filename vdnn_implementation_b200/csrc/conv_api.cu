@@ -294,8 +294,7 @@ int launch_dgrad_small_c_phase(const vdnn_conv_desc* d, int P, int Q, float alph
     auto kern = dgrad_small_c_phase_kernel<TW, CC>;
     int dev = 0;
     VDNN_CUDA(cudaGetDevice(&dev));
-    if (VDNN_ONCE_PER_DEVICE(dev))
-        VDNN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+    VDNN_ALLOW_SHARED(dev, kern, 96 * 1024);
     // class coordinates run over every i with 0 <= st*i + a - pad < H for some phase a: 0 .. (H - 1 + pad) / st
     const int hv = (d->h - 1 + d->pad_h) / st + 1, wv = (d->w - 1 + d->pad_w) / st + 1;
     dim3 grid(ceil_div(wv, TW), ceil_div(hv, S1_TH), static_cast<unsigned>(slices));
@@ -324,8 +323,7 @@ int dgrad_few_channels(const vdnn_conv_desc* d, int P, int Q, float alpha, const
     if (!dx) return VDNN_OK;
     int dev = 0;
     VDNN_CUDA(cudaGetDevice(&dev));
-    if (VDNN_ONCE_PER_DEVICE(dev))
-        VDNN_CUDA(cudaFuncSetAttribute(dgrad_small_c_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SMALL_C_SMEM_MAX)));
+    VDNN_ALLOW_SHARED(dev, dgrad_small_c_kernel, static_cast<int>(SMALL_C_SMEM_MAX));
     const long long total = static_cast<long long>(d->n) * d->h * d->w;
     long long blocks = (total + 255) / 256;
     const long long cap = static_cast<long long>(sm_count()) * (small_smem > 100 * 1024 ? 1 : 2) * 2;
@@ -690,7 +688,7 @@ int wgrad_small_c(const vdnn_conv_desc* d, int P, int Q, const float* x, const f
     VDNN_CUDA(cudaGetDevice(&dev));
 #define WSC_LAUNCH(CC)                                                                                                                   \
     {                                                                                                                                   \
-        if (VDNN_ONCE_PER_DEVICE(dev)) VDNN_CUDA(cudaFuncSetAttribute(wgrad_small_c_kernel<CC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024)); \
+        VDNN_ALLOW_SHARED(dev, wgrad_small_c_kernel<CC>, 80 * 1024); \
         wgrad_small_c_kernel<CC><<<grid, 256, smem, s>>>(x, dy, partial_w, partial_b, d->n, d->h, d->w, d->k, P, Q, d->pad_h, d->pad_w, tiles_y, tiles_x); \
     }
     switch (d->c) {
@@ -1003,8 +1001,7 @@ int vdnn_engine_mma_rate_probe(int iterations, double* flops, void* stream) {
     int dev = 0;
     VDNN_CUDA(cudaGetDevice(&dev));
     constexpr int smem = 200 * 1024;            // more than half an SM's shared memory: one CTA per SM
-    if (VDNN_ONCE_PER_DEVICE(dev))
-        VDNN_CUDA(cudaFuncSetAttribute(tc::mma_rate_probe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    VDNN_ALLOW_SHARED(dev, tc::mma_rate_probe_kernel, smem);
     const int ctas = sm_count();
     tc::mma_rate_probe_kernel<<<ctas, 128, smem, as_stream(stream)>>>(iterations);
     VDNN_LAUNCHED();

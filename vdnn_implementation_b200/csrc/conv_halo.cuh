@@ -475,7 +475,7 @@ int launch_bn(const Params& p, cudaStream_t stream) {
     int dev = 0;
     VDNN_CUDA(cudaGetDevice(&dev));
     auto kern = dgrad_kernel<BN>;
-    if (VDNN_ONCE_PER_DEVICE(dev)) VDNN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT));
+    VDNN_ALLOW_SHARED(dev, kern, SMEM_LIMIT);
     const int grid = static_cast<int>(p.units < sm_count() ? p.units : sm_count());
     kern<<<grid, THREADS, smem, stream>>>(p);
     VDNN_LAUNCHED();

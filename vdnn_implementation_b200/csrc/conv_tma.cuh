@@ -947,8 +947,7 @@ int launch_bn(const Problem& q, const float* src, char* images, const char* b_ti
     int dev = 0;
     VDNN_CUDA(cudaGetDevice(&dev));
     auto kern = conv_kernel<BN>;
-    if (VDNN_ONCE_PER_DEVICE(dev))
-        VDNN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
+    VDNN_ALLOW_SHARED(dev, kern, Cfg::SMEM_BYTES);
     const size_t elems = static_cast<size_t>(q.n) * q.cin * q.in_h * q.in_w;
     float* hi = reinterpret_cast<float*>(images);
     float* lo = hi + elems;
@@ -1049,8 +1048,7 @@ int strip_launch_bn(const Problem& q, const float* src, char* images, const char
     int dev = 0;
     VDNN_CUDA(cudaGetDevice(&dev));
     auto kern = strip_kernel<BN, MH>;
-    if (VDNN_ONCE_PER_DEVICE(dev))
-        VDNN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
+    VDNN_ALLOW_SHARED(dev, kern, Cfg::SMEM_BYTES);
     const StripGeom g = strip_geometry(q);
     if (!g.ok) return VDNN_ERR_UNSUPPORTED;
     const size_t elems = static_cast<size_t>(q.n) * g.lp * q.cin;
@@ -1226,8 +1224,7 @@ int wgrad_launch_bn(const WgradProblem& q, const float* x, const float* dy, char
     int dev = 0;
     VDNN_CUDA(cudaGetDevice(&dev));
     auto kern = wgrad_kernel<BN, MH>;
-    if (VDNN_ONCE_PER_DEVICE(dev))
-        VDNN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
+    VDNN_ALLOW_SHARED(dev, kern, Cfg::SMEM_BYTES);
     const size_t xe = static_cast<size_t>(q.n) * q.c * q.h * q.w, ye = static_cast<size_t>(q.n) * q.k * q.p * q.q;
     float* xh = reinterpret_cast<float*>(ws);
     float* xl = xh + xe;

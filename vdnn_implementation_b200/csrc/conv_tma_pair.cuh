@@ -278,8 +278,7 @@ int strip_pair_launch(const Problem& q, const float* src, char* images, const ch
     VDNN_CUDA(cudaGetDevice(&dev));
     typedef PairCfg<BNP> Cfg;
     auto kern = strip_pair_kernel<BNP>;
-    if (VDNN_ONCE_PER_DEVICE(dev))
-        VDNN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
+    VDNN_ALLOW_SHARED(dev, kern, Cfg::SMEM_BYTES);
     const StripGeom g = strip_geometry(q);
     if (!g.ok) return VDNN_ERR_UNSUPPORTED;
     const size_t elems = static_cast<size_t>(q.n) * g.lp * q.cin;
@@ -560,8 +559,7 @@ int wgrad_pair_launch(const CUtensorMap& mxh, const CUtensorMap& mxl, const CUte
     int dev = 0;
     VDNN_CUDA(cudaGetDevice(&dev));
     auto kern = wgrad_pair_kernel<BNP>;
-    if (VDNN_ONCE_PER_DEVICE(dev))
-        VDNN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WCfg::SMEM_BYTES));
+    VDNN_ALLOW_SHARED(dev, kern, WCfg::SMEM_BYTES);
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;

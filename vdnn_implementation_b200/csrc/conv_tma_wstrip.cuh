@@ -250,8 +250,7 @@ int wstrip_launch_bn(const Problem& fwd, int n_filters, const char* x_images, co
     int dev = 0;
     VDNN_CUDA(cudaGetDevice(&dev));
     auto kern = wgrad_strip_kernel<BN, RT>;
-    if (VDNN_ONCE_PER_DEVICE(dev))
-        VDNN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
+    VDNN_ALLOW_SHARED(dev, kern, Cfg::SMEM_BYTES);
     const StripGeom g = strip_geometry(fwd);
     WstripParams p;
     p.total_pos = static_cast<long long>(fwd.n) * g.lp;

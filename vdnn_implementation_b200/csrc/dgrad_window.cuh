@@ -197,7 +197,7 @@ int launch_shape(const vdnn_conv_desc* d, int P, int Q, float alpha, float beta,
     auto kern = dgrad_kernel<R, ST, TI, CC>;
     int dev = 0;
     VDNN_CUDA(cudaGetDevice(&dev));
-    if (VDNN_ONCE_PER_DEVICE(dev)) VDNN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LIMIT));
+    VDNN_ALLOW_SHARED(dev, kern, LIMIT);
     kern<<<static_cast<unsigned>(ceil_div<long long>(total, Sh::THREADS)), Sh::THREADS, p.k_chunk * Sh::PER_K * 4, stream>>>(p);
     VDNN_LAUNCHED();
     return VDNN_OK;

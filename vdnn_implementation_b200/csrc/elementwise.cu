@@ -30,18 +30,6 @@ int sm_count() {
     return cached[dev];
 }
 
-bool first_use_on_device(void** seen_table, int device) {
-    static std::mutex lock;
-    std::lock_guard<std::mutex> g(lock);
-    if (device < 0) return false;
-    std::vector<char>* seen = static_cast<std::vector<char>*>(*seen_table);
-    if (!seen) { seen = new std::vector<char>(); *seen_table = seen; }     // lives as long as the process
-    if (seen->size() <= static_cast<size_t>(device)) seen->resize(device + 1, 0);
-    if ((*seen)[device]) return false;
-    (*seen)[device] = 1;
-    return true;
-}
-
 namespace {
 
 namespace cg = cooperative_groups;

@@ -493,8 +493,7 @@ int launch_bn(const float* A, int lda, const float* B, int ldb, Params p, int K,
     int dev = 0;
     VDNN_CUDA(cudaGetDevice(&dev));
     auto kern = gemm_kernel<AK, BKM, BN, STAGED>;
-    if (VDNN_ONCE_PER_DEVICE(dev))
-        VDNN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
+    VDNN_ALLOW_SHARED(dev, kern, Cfg::SMEM_BYTES);
     CUtensorMap ma, mb;
     int st = AK ? tma::make_matrix_map(&ma, A, K, p.M, lda, BK, BM, CU_TENSOR_MAP_SWIZZLE_128B)
                 : tma::make_matrix_map(&ma, A, p.M, K, lda, BM, BK, CU_TENSOR_MAP_SWIZZLE_NONE);

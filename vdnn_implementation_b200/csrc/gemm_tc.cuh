@@ -488,8 +488,7 @@ int launch_bn(const OpA& a, const OpB& b, const Epilogue& epi, int M, int N, int
     int dev = 0;
     VDNN_CUDA(cudaGetDevice(&dev));
     auto kern = gemm_kernel<OpA, OpB, AKC, BKC, BN, BBULK>;
-    if (VDNN_ONCE_PER_DEVICE(dev))
-        VDNN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::ALONE_BYTES));
+    VDNN_ALLOW_SHARED(dev, kern, Cfg::ALONE_BYTES);
     dim3 grid(ceil_div(M, BM), ceil_div(N, BN), splits);
     if (grid.y > 65535u || grid.z > 65535u) return VDNN_ERR_UNSUPPORTED;
     const int kblocks = ceil_div(K, BK);
