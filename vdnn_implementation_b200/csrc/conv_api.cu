@@ -1199,7 +1199,9 @@ int vdnn_conv_bwd_filter(const vdnn_conv_desc* d, int algo_mode, float alpha, co
     if (algo_mode == VDNN_ALGO_PERF_OPT) {
         // workspace variant: dy, which every row tile of the gathered input needs again, is split into tf32 halves and
         // laid out as tile images once; the kernel's producers then gather x only
-        const size_t pack = packed_dy_bytes(d, P, Q);
+        // (tensors off the 16-byte boundaries of a layer whose workspace is sized for wgrad_small_c: its bytes hold the parts of the
+        // sums, two splits for each SM against that kernel's three blocks, but no images of dy)
+        const size_t pack = wgrad_small_c_shape(d, Q) && g_engine != VDNN_ENGINE_FFMA ? 0 : packed_dy_bytes(d, P, Q);
         if (pack && (!workspace || workspace_bytes < pack)) return VDNN_ERR_WORKSPACE;
         char* tiles = (pack && g_engine != VDNN_ENGINE_FFMA && (reinterpret_cast<uintptr_t>(workspace) & 127u) == 0)
                           ? static_cast<char*>(workspace) : nullptr;
