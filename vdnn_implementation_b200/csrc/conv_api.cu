@@ -13,7 +13,7 @@
 #include "gemm_ffma.cuh"
 #include "gemm_tc.cuh"
 #include "gemm_dense.cuh"
-#include "conv_tma.cuh"
+#include "conv_split16.cuh"
 #include "conv_halo.cuh"
 #include "dgrad_window.cuh"
 
@@ -23,9 +23,6 @@ namespace {
 int g_engine = VDNN_ENGINE_AUTO;
 // VDNN_NO_TMA=1 in the environment keeps PERF_OPT forward / data gradient on the gather-fed kernel (A/B measurements).
 const bool g_no_tma = []() { const char* v = getenv("VDNN_NO_TMA"); return v && *v && *v != '0'; }();
-// VDNN_TMA_BOXES=1: forward / data gradient fetch one box of pixels per tap (conv_kernel) instead of one strip of positions
-// per filter row (strip_kernel).
-const bool g_tma_boxes = []() { const char* v = getenv("VDNN_TMA_BOXES"); return v && *v && *v != '0'; }();
 // VDNN_TMA_WGRAD=0: the PERF_OPT filter gradient stays on the gather-fed kernel (default: TMA-fed where the shape allows).
 const bool g_tma_wgrad = []() { const char* v = getenv("VDNN_TMA_WGRAD"); return !(v && *v == '0'); }();
 
@@ -74,10 +71,11 @@ __global__ void __launch_bounds__(256) scale_matrix_kernel(int rows, int cols, i
 // in a row of calls.
 template <int VEC>
 __global__ void __launch_bounds__(256) reduce_partials_kernel(size_t n, int splits, int lanes, float alpha, float beta,
-                                                              const float* __restrict__ partial, float* __restrict__ out) {
+                                                              const float* __restrict__ partial, float* __restrict__ out, const int* skip) {
     __shared__ float part[256 * VEC];
     tc::follow_up();
     tc::after_predecessor();
+    if (skip && *skip) return;
     const int per_block = 256 / lanes, g = threadIdx.x % per_block, l = threadIdx.x / per_block;
     const size_t i = (static_cast<size_t>(blockIdx.x) * per_block + g) * VEC;
     float acc[VEC];
@@ -114,7 +112,8 @@ __global__ void __launch_bounds__(256) reduce_partials_kernel(size_t n, int spli
     }
 }
 
-int reduce_partials(size_t n, int splits, float alpha, float beta, const float* partial, float* out, cudaStream_t stream) {
+// skip (may be null): a word on the device that says that there are no partial results.
+int reduce_partials(size_t n, int splits, float alpha, float beta, const float* partial, float* out, cudaStream_t stream, const int* skip = nullptr) {
     const bool vec = n % 4 == 0 && ((reinterpret_cast<uintptr_t>(partial) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
     const size_t groups = vec ? n / 4 : n;
     // lanes per sum: as many as leave each one two splits, while the grid is below two blocks per SM
@@ -122,8 +121,8 @@ int reduce_partials(size_t n, int splits, float alpha, float beta, const float* 
     while (lanes < 32 && 4 * lanes <= splits && ceil_div<size_t>(groups * lanes, 256) < static_cast<size_t>(2 * sm_count())) lanes *= 2;
     const size_t blocks = ceil_div<size_t>(groups * lanes, 256);
     if (blocks > 0x7fffffffu) return VDNN_ERR_UNSUPPORTED;
-    if (vec) VDNN_CUDA(tc::launch_early(reduce_partials_kernel<4>, dim3(static_cast<unsigned>(blocks)), 256, 0, stream, n, splits, lanes, alpha, beta, partial, out));
-    else VDNN_CUDA(tc::launch_early(reduce_partials_kernel<1>, dim3(static_cast<unsigned>(blocks)), 256, 0, stream, n, splits, lanes, alpha, beta, partial, out));
+    if (vec) VDNN_CUDA(tc::launch_early(reduce_partials_kernel<4>, dim3(static_cast<unsigned>(blocks)), 256, 0, stream, n, splits, lanes, alpha, beta, partial, out, skip));
+    else VDNN_CUDA(tc::launch_early(reduce_partials_kernel<1>, dim3(static_cast<unsigned>(blocks)), 256, 0, stream, n, splits, lanes, alpha, beta, partial, out, skip));
     VDNN_LAUNCHED();
     return VDNN_OK;
 }
@@ -355,58 +354,145 @@ size_t packed_dy_bytes(const vdnn_conv_desc* d, int P, int Q) {
     return d->k >= 128 ? tc::bulk_bytes(d->k, d->n * P * Q) : 0;
 }
 
-// Forward and data gradient of a stride-1 convolution whose reduction channels (C for forward, K for the data
-// gradient) come in whole blocks of 32 run on the TMA-fed engine in PERF_OPT: the gathered tensor is rewritten once into
-// two channels-last images (tf32 hi / lo halves) in workspace and the kernel fetches its operand tiles by tensor copies.
-bool tma_shape(const vdnn_conv_desc* d, int op) {
-    if (op != VDNN_CONV_FWD && op != VDNN_CONV_BWD_DATA) return false;
-    if (d->stride_h != 1 || d->stride_w != 1 || is_full_extent(d)) return false;
-    if (op == VDNN_CONV_BWD_DATA && d->c <= SMALL_C_MAX) return false;          // the first layer has its own kernels
-    if ((op == VDNN_CONV_FWD ? d->c : d->k) % 32 != 0) return false;
-    // Only where the output has enough tiles to fill the GPU without splitting the reduction: the few-tile layers (14 x 14
-    // maps) stay on the gather kernel, which splits along k at a finer grain and needs no operand images (without workspace
-    // some of their data gradients run on the halo kernel, see dgrad_halo).  With the engine forced to VDNN_ENGINE_TCGEN05 every eligible shape takes the TMA-fed path (small shapes in the tests).
-    if (g_engine == VDNN_ENGINE_TCGEN05) return true;
-    const int P = (d->h + 2 * d->pad_h - d->r) / d->stride_h + 1, Q = (d->w + 2 * d->pad_w - d->s) / d->stride_w + 1;
-    const long long pixels = static_cast<long long>(d->n) * (op == VDNN_CONV_FWD ? P * Q : d->h * d->w);
-    const int cols = op == VDNN_CONV_FWD ? d->k : d->c;
-    return (pixels + 127) / 128 * ((cols + 255) / 256) >= sm_count();
+bool valid_desc(const vdnn_conv_desc* d, int* P, int* Q) {
+    if (!d || d->n <= 0 || d->c <= 0 || d->h <= 0 || d->w <= 0 || d->k <= 0 || d->r <= 0 || d->s <= 0 ||
+        d->pad_h < 0 || d->pad_w < 0 || d->stride_h <= 0 || d->stride_w <= 0)
+        return false;
+    if (d->h + 2 * d->pad_h < d->r || d->w + 2 * d->pad_w < d->s) return false;
+    *P = (d->h + 2 * d->pad_h - d->r) / d->stride_h + 1;
+    *Q = (d->w + 2 * d->pad_w - d->s) / d->stride_w + 1;
+    return true;
 }
 
-bool tma_wgrad_shape(const vdnn_conv_desc* d) {
-    return g_tma_wgrad && !g_no_tma && d->stride_h == 1 && d->stride_w == 1 && !is_full_extent(d) && d->c % 32 == 0 && d->k % 32 == 0;
+// Offsets are 32-bit inside the kernels: every tensor must stay below 2^31 elements.
+bool fits_int32(const vdnn_conv_desc* d, int P, int Q) {
+    const long long lim = 0x7fffffffLL;
+    return 1LL * d->n * d->c * d->h * d->w < lim && 1LL * d->n * d->k * P * Q < lim &&
+           1LL * d->k * d->c * d->r * d->s < lim;
 }
 
-tma::WgradProblem wgrad_problem(const vdnn_conv_desc* d, int P, int Q) {
-    return tma::WgradProblem{d->n, d->c, d->h, d->w, d->k, P, Q, d->r, d->s, d->pad_h, d->pad_w};
+// Stride-1 convolutions run on the TMA-fed kernels in PERF_OPT (conv_split16.cuh): the gathered tensors are rewritten once into
+// lists of positions in workspace and the kernels fetch their operand tiles by tensor copies.
+bool split16_layer(const vdnn_conv_desc* d) {
+    return g_engine != VDNN_ENGINE_FFMA && !g_no_tma && d->stride_h == 1 && d->stride_w == 1 && !is_full_extent(d);
 }
 
-// Operand images of at most this many bytes are kept in workspace at a time.
-constexpr size_t TMA_IMAGE_BUDGET = static_cast<size_t>(1) << 30;
-int tma_slab_images(int n, size_t bytes_per_image) {
-    if (bytes_per_image * n <= TMA_IMAGE_BUDGET) return n;
-    const size_t fit = TMA_IMAGE_BUDGET / bytes_per_image;
+// Lists of at most this many bytes are kept in workspace at a time; layers that need more are walked in slabs of whole images,
+// so the workspace stays at the budget whatever the batch size.
+constexpr size_t LIST_BUDGET = static_cast<size_t>(512) << 20;
+int slab_images(int n, size_t bytes_per_image) {
+    if (bytes_per_image * n <= LIST_BUDGET) return n;
+    const size_t fit = LIST_BUDGET / bytes_per_image;
     return fit > 1 ? static_cast<int>(fit) : 1;
 }
 
-tma::Problem tma_problem(const vdnn_conv_desc* d, int op, int P, int Q) {
-    if (op == VDNN_CONV_FWD) return tma::Problem{d->n, d->c, d->h, d->w, P, Q, d->k, d->r, d->s, 1, -d->pad_h, -d->pad_w};
+split16::Problem split16_problem(const vdnn_conv_desc* d, int op, int P, int Q) {
+    const split16::ListGeom g = split16::list_geometry(d->h, d->w, P, Q, d->pad_h, d->pad_w);
+    if (op == VDNN_CONV_FWD) return split16::Problem{d->n, d->c, d->h, d->w, P, Q, d->k, d->r, d->s, 1, -d->pad_h, -d->pad_w, g.wp, g.wp * g.hp};
     // dx[h][w] = sum over taps of dy[h + pad - r][w + pad - s] (stride 1)
-    return tma::Problem{d->n, d->k, P, Q, d->h, d->w, d->c, d->r, d->s, -1, d->pad_h, d->pad_w};
+    return split16::Problem{d->n, d->k, P, Q, d->h, d->w, d->c, d->r, d->s, -1, d->pad_h, d->pad_w, g.wp, g.wp * g.hp};
 }
 
-bool tma_use_strips(const tma::Problem& q) { return !g_tma_boxes && tma::strip_geometry(q).ok; }
-
-// Bytes of the two operand images of `images` images of the problem, in the layout the chosen kernel reads.
-size_t tma_operand_bytes(const tma::Problem& q, int images) {
-    tma::Problem part = q;
-    part.n = images;
-    return tma_use_strips(q) ? tma::strip_image_bytes(part) : tma::image_bytes(images, q.cin, q.in_h, q.in_w);
+split16::WgradProblem split16_wgrad_problem(const vdnn_conv_desc* d, int P, int Q) {
+    const split16::ListGeom g = split16::list_geometry(d->h, d->w, P, Q, d->pad_h, d->pad_w);
+    return split16::WgradProblem{d->n, d->c, d->h, d->w, d->k, P, Q, d->r, d->s, d->pad_h, d->pad_w, g.wp, g.wp * g.hp};
 }
 
-size_t tma_image_bytes(const vdnn_conv_desc* d, int op, int P, int Q) {
-    const tma::Problem q = tma_problem(d, op, P, Q);
-    return tma_operand_bytes(q, tma_slab_images(d->n, tma_operand_bytes(q, 1)));
+// What forward or the data gradient keeps in workspace: the scale record, the packed filters, the lists of a slab of images, the
+// parts of a split reduction.
+struct StripPlan { int slab, splits, group_chunk; size_t pack, lists, partial, total; };
+
+StripPlan strip_plan(const vdnn_conv_desc* d, int op, int P, int Q) {
+    const split16::Problem q = split16_problem(d, op, P, Q);
+    StripPlan plan;
+    plan.slab = slab_images(q.n, split16::list_bytes(1, q.cin, q.lp));
+    plan.pack = split16::packed_bytes(q.n_cols, q.cin, q.R * q.S);
+    plan.lists = split16::list_bytes(plan.slab, q.cin, q.lp);
+    // the reduction is split between groups where the tiles fill less than half of the GPU
+    const int groups = split16::strip_groups(q);
+    const long long tiles = split16::strip_tiles(q), slots = split16::strip_slots(q.n_cols);
+    int splits = 1;
+    if (plan.slab == q.n && 2 * tiles <= slots) splits = static_cast<int>(min(static_cast<long long>(groups), slots / tiles));
+    plan.group_chunk = ceil_div(groups, splits);
+    plan.splits = ceil_div(groups, plan.group_chunk);
+    plan.partial = plan.splits > 1 ? static_cast<size_t>(plan.splits) * q.n * q.n_cols * q.out_h * q.out_w * sizeof(float) : 0;
+    plan.total = split16::SCALE_BYTES + plan.pack + plan.lists + plan.partial;
+    return plan;
+}
+
+// The filter gradient's: the scale record, the lists of x and dy of a slab, the parts.
+struct WgradSpace { int slab; size_t x_lists, dy_lists, partial, total; };
+
+WgradSpace wgrad_space(const vdnn_conv_desc* d, int P, int Q, size_t limit = SIZE_MAX) {
+    split16::WgradProblem q = split16_wgrad_problem(d, P, Q);
+    WgradSpace w;
+    w.slab = slab_images(q.n, split16::list_bytes(1, q.c, q.lp) + split16::list_bytes(1, q.k, q.lp));
+    for (;; w.slab = (w.slab + 1) / 2) {
+        q.n = w.slab;
+        w.x_lists = split16::list_bytes(w.slab, q.c, q.lp);
+        w.dy_lists = split16::list_bytes(w.slab, q.k, q.lp);
+        w.partial = split16::wgrad_partial_bytes(q);
+        w.total = split16::SCALE_BYTES + w.x_lists + w.dy_lists + w.partial;
+        if (w.total <= limit || w.slab == 1) return w;
+    }
+}
+
+// Times in us of the two ways a product can take in PERF_OPT, fitted to 120 drawn layers of 32 .. 512 channels, 1x1 .. 5x5 (B200,
+// calls back to back; a tenth off on average, the gathered filter gradient a fifth).  On lists: launches, blocks of the
+// reduction in the waves of tiles, passes over the operands and the result (millions of elements), parts of a split
+// reduction.  Gathered: blocks and waves likewise.  Choosing by them costs 0.3 % (forward), 0.8 % (data gradient) and 2 % (filter
+// gradient) against the faster of the two for every layer, at worst 15, 28 and 48 %; lists everywhere or nowhere lose up to
+// 3.3 and 7 times.
+struct GatherRate { double block, wave; };
+double gathered_us(int M, int N, int K, bool may_split) {
+    const int bn = tc::tile_n(N), blocks = ceil_div(K, 32);
+    const long long tiles = static_cast<long long>(ceil_div(M, 128)) * ceil_div(N, bn);
+    int splits = 1;
+    if (may_split && tiles < sm_count()) splits = max(1, min(static_cast<int>(2 * sm_count() / tiles), K / 64));
+    const double waves = static_cast<double>(ceil_div<long long>(tiles * splits, bn == 64 ? 2 * sm_count() : sm_count()));
+    const GatherRate rate = bn == 64 ? GatherRate{1.4, 1.5} : (bn == 128 ? GatherRate{0.8, 4.9} : GatherRate{1.18, 7.7});
+    return (may_split ? 7.0 : 3.0) + waves * (rate.block * ceil_div(blocks, splits) + rate.wave);
+}
+
+// Forward and data gradient.  With the engine forced to VDNN_ENGINE_TCGEN05 every eligible shape runs on lists (small shapes in the
+// tests).
+bool split16_shape(const vdnn_conv_desc* d, int op) {
+    if (!split16_layer(d) || (op != VDNN_CONV_FWD && op != VDNN_CONV_BWD_DATA)) return false;
+    const bool fwd = op == VDNN_CONV_FWD;
+    if ((fwd ? d->c : d->k) < 8 || (!fwd && d->c <= SMALL_C_MAX)) return false;       // first layers have their own kernels
+    int P, Q;
+    if (!valid_desc(d, &P, &Q) || !fits_int32(d, P, Q)) return false;
+    const split16::Problem q = split16_problem(d, op, P, Q);
+    if (static_cast<long long>(q.n) * q.lp >= 0x7fffff00LL) return false;
+    if (g_engine == VDNN_ENGINE_TCGEN05) return true;
+    if (q.n * q.out_h * q.out_w < split16::BM) return false;         // less than a tile: nothing was fitted there
+    const StripPlan plan = strip_plan(d, op, P, Q);
+    const double src = 0.5e-6 * (static_cast<double>(q.n) * q.cin * q.in_h * q.in_w + static_cast<double>(q.n) * q.lp * split16::padded_channels(q.cin));
+    const double out = 1e-6 * q.n * q.n_cols * q.out_h * q.out_w, weights = 1e-6 * q.cin * q.n_cols * q.R * q.S;
+    const double waves = static_cast<double>(ceil_div<long long>(split16::strip_tiles(q) * plan.splits, split16::strip_slots(q.n_cols)));
+    const double lists = 20.0 + 0.8 * waves * plan.group_chunk * split16::taps_per_strip(q.S) + 1.8 * src + 1.1 * out * (plan.splits > 1 ? 1 + 2 * plan.splits : 1) + 7.7 * weights;
+    return lists < gathered_us(q.n * q.out_h * q.out_w, q.n_cols, q.cin * q.R * q.S, !fwd) + 0.5 * (src + out);
+}
+
+bool split16_wgrad_shape(const vdnn_conv_desc* d) {
+    if (!g_tma_wgrad || !split16_layer(d) || d->c < 8) return false;
+    int P, Q;
+    if (!valid_desc(d, &P, &Q) || !fits_int32(d, P, Q)) return false;
+    const split16::WgradProblem q = split16_wgrad_problem(d, P, Q);
+    if (static_cast<long long>(q.n) * q.lp >= 0x7fffff00LL) return false;
+    if (g_engine == VDNN_ENGINE_TCGEN05) return true;
+    if (d->n * P * Q < split16::BM) return false;
+    const split16::WgradPlan w = split16::wgrad_plan(q);
+    const double dw = 1e-6 * d->k * d->c * d->r * d->s, dy = 1e-6 * d->n * d->k * P * Q;
+    const double both = 0.5 * (1e-6 * d->n * d->c * d->h * d->w + dy + 1e-6 * q.n * q.lp * (split16::padded_channels(d->c) + split16::padded_channels(d->k)));
+    const double waves = static_cast<double>(ceil_div(ceil_div(w.groups, w.chunk) * w.ctas * ceil_div(d->k, w.bn) * w.splits, sm_count()));
+    const double lists = 27.0 + waves * ((w.bn == 64 ? 2.46 : (w.bn == 128 ? 1.32 : 1.23)) * w.kb_chunk + 3.9) + 2.0 * both + 4.5 * w.splits * dw;
+    const int M = d->c * d->r * d->s, bn = tc::tile_n(d->k);
+    const SplitPlan split = plan_split(M, d->k, d->n * P * Q);
+    const double gwaves = static_cast<double>(ceil_div(ceil_div(M, 128) * ceil_div(d->k, bn) * split.splits, sm_count()));
+    const double gathered = 10.0 + gwaves * ((bn == 64 ? 1.16 : (bn == 128 ? 1.2 : 1.5)) * (split.k_chunk / 32) + 3.3) + 1.4 * (split.splits > 1 ? split.splits : 0) * dw +
+                            (d->k >= 128 ? 3.25 : 0.0) * dy + 1.2 * dw;
+    return lists < 1.3 * gathered;          // the gather's time is the less certain one, and errs upwards
 }
 
 int stream_blocks(size_t n) {
@@ -513,71 +599,30 @@ int dgrad_halo(const vdnn_conv_desc* d, int P, int Q, const float* dy, const flo
     return halo::launch(bn, p, stream);
 }
 
-// The TMA-fed contraction with the split handling of contract(): `ws` holds the images, then the per-split partials.
-// Layers whose images would pass TMA_IMAGE_BUDGET are walked in slabs of whole images (transform a slab, contract it,
-// reuse the image buffer), so the workspace stays at the budget whatever the batch size.
-int contract_tma(const tma::Problem& q, const float* src, const char* b_tiles, Epilogue epi, size_t out_elems, char* ws,
-                 size_t ws_bytes, cudaStream_t stream) {
-    const bool strips = tma_use_strips(q);
-    const int slab = tma_slab_images(q.n, tma_operand_bytes(q, 1));
-    const size_t img = tma_operand_bytes(q, slab);
-    if (ws_bytes < img) return VDNN_ERR_WORKSPACE;
-    const int M = q.n * q.out_h * q.out_w, K = q.R * q.S * q.cin;
-    SplitPlan plan = plan_split(M, q.n_cols, K);
-    if (epi.bias || slab < q.n) { plan.splits = 1; plan.k_chunk = K; }
-    // the strip kernel splits the reduction between (filter row, channel block) groups of S k blocks
-    const int groups = q.R * (q.cin / 32);
-    int group_chunk = ceil_div(plan.k_chunk / 32, q.S);
-    if (group_chunk < 1) group_chunk = 1;
-    const int splits = strips ? ceil_div(groups, group_chunk) : plan.splits;
-    auto run = [&](const tma::Problem& part, const float* s, float* o, const float* bias, float alpha, float beta, int mode) {
-        return strips ? tma::strip_launch(part, s, ws, b_tiles, o, bias, alpha, beta, mode, out_elems, splits, group_chunk, stream)
-                      : tma::launch(part, s, ws, b_tiles, o, bias, alpha, beta, mode, out_elems, splits, plan.k_chunk, stream);
-    };
-    if (splits == 1) {
-        const size_t src_img = static_cast<size_t>(q.cin) * q.in_h * q.in_w, out_img = static_cast<size_t>(q.n_cols) * q.out_h * q.out_w;
-        for (int n0 = 0; n0 < q.n; n0 += slab) {
-            tma::Problem part = q;
-            part.n = min(slab, q.n - n0);
-            const int st = run(part, src + n0 * src_img, epi.out + n0 * out_img, epi.bias, epi.alpha, epi.beta, EPI_DIRECT);
-            if (st != VDNN_OK) return st;
-        }
-        return VDNN_OK;
-    }
-    const size_t need = static_cast<size_t>(splits) * out_elems * sizeof(float);
-    if (ws_bytes - img < need) return VDNN_ERR_WORKSPACE;
-    float* partial = reinterpret_cast<float*>(ws + img);
-    const int st = run(q, src, partial, nullptr, 1.0f, 0.0f, EPI_PARTIAL);
-    if (st != VDNN_OK) return st;
-    return reduce_partials(out_elems, splits, epi.alpha, epi.beta, partial, epi.out, stream);
+__global__ void __launch_bounds__(256) scale_gated_kernel(size_t n, float beta, float* out, const int* gate) {
+    tc::follow_up();
+    tc::after_predecessor();
+    if (*gate == 0) return;
+    const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
+    for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) out[i] = beta == 0.0f ? 0.0f : beta * out[i];
 }
 
-// Filter gradient on the TMA-fed engine, in slabs of whole images where the four operand images would pass the budget:
-// every slab adds its pixels' share, dw = alpha * (sum over slabs) + beta * dw.
-int wgrad_tma(const tma::WgradProblem& q, const float* x, const float* dy, char* ws, size_t ws_bytes, float* dw, float alpha,
-              float beta, cudaStream_t stream, float* bias_sums = nullptr, float bias_scale = 0.0f) {
-    tma::WgradProblem one = q;
-    one.n = 1;
-    const int slab = tma_slab_images(q.n, tma::wgrad_image_bytes(one));
-    tma::WgradProblem part = q;
-    part.n = slab;
-    if (ws_bytes < tma::wgrad_image_bytes(part) + tma::wgrad_partial_bytes(part)) return VDNN_ERR_WORKSPACE;
-    const size_t x_img = static_cast<size_t>(q.c) * q.h * q.w, dy_img = static_cast<size_t>(q.k) * q.p * q.q;
-    const size_t elems = static_cast<size_t>(q.k) * q.c * q.R * q.S;
-    for (int n0 = 0; n0 < q.n; n0 += slab) {
-        part.n = min(slab, q.n - n0);
-        int splits = 1;
-        float* partial = nullptr;
-        const float b = n0 == 0 ? beta : 1.0f;
-        int st = tma::wgrad_launch(part, x + n0 * x_img, dy + n0 * dy_img, ws, dw, alpha, b, stream, &splits, &partial,
-                                         bias_sums, bias_scale);
-        if (st != VDNN_OK) return st;
-        if (splits > 1) {
-            st = reduce_partials(elems, splits, alpha, b, partial, dw, stream);
-            if (st != VDNN_OK) return st;
+// The contraction without workspace on the gather-fed kernel, computed only where *gate is set when its turn comes: the call's
+// operands do not fit the form of split16.cuh.  The output is one dense block.
+template <class OpA, class OpB, bool AKC, bool BKC>
+int contract_gated(const OpA& a, const OpB& b, Epilogue epi, int M, int N, int K, const int* gate, cudaStream_t stream) {
+    SplitPlan plan = plan_split(M, N, K);
+    if (epi.bias) { plan.splits = 1; plan.k_chunk = ceil_div(K, 32) * 32; }
+    epi.mode = EPI_DIRECT;
+    if (plan.splits > 1) {
+        epi.mode = EPI_ATOMIC;
+        if (epi.beta != 1.0f) {
+            const size_t n = static_cast<size_t>(M) * N;
+            VDNN_CUDA(tc::launch_early(scale_gated_kernel, dim3(min(stream_blocks(n), 2 * sm_count())), 256, 0, stream, n, epi.beta, epi.out, gate));
+            VDNN_LAUNCHED();
         }
     }
-    return VDNN_OK;
+    return tc::launch_gated<OpA, OpB, AKC, BKC>(a, b, epi, M, N, K, plan.splits, plan.k_chunk, gate, stream);
 }
 
 // Filter gradient (and bias gradient) for layers with very few input channels and a 3 x 3 / stride-1 filter (VGG16's
@@ -799,42 +844,16 @@ int fwd_small_c(const vdnn_conv_desc* d, int P, int Q, float alpha, const float*
     return VDNN_OK;
 }
 
-// ---- one image pass over dy for both gradients --------------------------------------------------------------------
-// The data gradient's strip engine and the filter gradient both read dy as channels-last tf32 hi / lo images; the strip
-// layout (a padded position list) contains the plain image as a strided view, so where both gradients of a layer run on
-// the TMA-fed kernels one pass writes dy once (and forms the bias sums), and the two kernels run slab by slab from it.
-bool bwd_shared_shape(const vdnn_conv_desc* d, int P, int Q) {
-    if (g_no_tma || !tma_shape(d, VDNN_CONV_BWD_DATA) || !tma_wgrad_shape(d)) return false;
-    return tma_use_strips(tma_problem(d, VDNN_CONV_BWD_DATA, P, Q));
-}
-
-// The filter gradient of layers with at most 128 filters can run on the two position lists themselves
-// (conv_tma_wstrip.cuh: one strip of x per filter row instead of one box per tap).  VDNN_WGRAD_STRIPS=0 switches it off.
-bool g_wgrad_strips = []() { const char* e = getenv("VDNN_WGRAD_STRIPS"); return !e || e[0] != '0'; }();
-
-bool bwd_wstrip_shape(const vdnn_conv_desc* d, int P, int Q) {
-    return g_wgrad_strips && tma::wstrip_filters_ok(d->k, d->c) &&
-           tma::wstrip_ok(tma_problem(d, VDNN_CONV_FWD, P, Q), tma_problem(d, VDNN_CONV_BWD_DATA, P, Q));
-}
-
-struct BwdSharedPlan { int slab; bool wstrip; size_t pack, strips, ximg, partial, total; };
-
-BwdSharedPlan bwd_shared_plan(const vdnn_conv_desc* d, int P, int Q) {
-    BwdSharedPlan plan;
-    plan.wstrip = bwd_wstrip_shape(d, P, Q);
-    tma::Problem q = tma_problem(d, VDNN_CONV_BWD_DATA, P, Q), fq = tma_problem(d, VDNN_CONV_FWD, P, Q);
-    q.n = 1; fq.n = 1;
-    const size_t x_one = plan.wstrip ? tma::strip_image_bytes(fq) : tma::image_bytes(1, d->c, d->h, d->w);
-    plan.slab = tma_slab_images(d->n, tma::strip_image_bytes(q) + x_one);
-    q.n = plan.slab; fq.n = plan.slab;
-    plan.pack = packed_weight_bytes(d, VDNN_CONV_BWD_DATA);
-    plan.strips = tma::strip_image_bytes(q);
-    plan.ximg = plan.wstrip ? tma::strip_image_bytes(fq) : tma::image_bytes(plan.slab, d->c, d->h, d->w);
-    tma::WgradProblem wq = wgrad_problem(d, P, Q);
-    wq.n = plan.slab;
-    plan.partial = plan.wstrip ? tma::wstrip_partial_bytes(fq, d->k) : tma::wgrad_partial_bytes(wq);
-    plan.total = plan.pack + plan.strips + plan.ximg + plan.partial;
-    return plan;
+XGather make_xgather(const vdnn_conv_desc* d, const float* x, int P, int Q) {
+    XGather g;
+    g.x = x; g.C = d->c; g.H = d->h; g.W = d->w; g.R = d->r; g.S = d->s;
+    g.pad_h = d->pad_h; g.pad_w = d->pad_w; g.stride_h = d->stride_h; g.stride_w = d->stride_w;
+    g.n_pix = d->n * P * Q; g.n_filt = d->c * d->r * d->s;
+    g.Q = Q;
+    g.div_pq = FastDiv(P * Q); g.div_q = FastDiv(Q); g.div_rs = FastDiv(d->r * d->s); g.div_s = FastDiv(d->s);
+    g.div_c = FastDiv(d->c);
+    g.chw = d->c * d->h * d->w; g.hw = d->h * d->w;
+    return g;
 }
 
 // KCRS weights viewed as [c][(tap, ko)]: offset c*RS + tap + ko*C*RS (the B operand of the data gradient).
@@ -848,82 +867,201 @@ SplitDense dgrad_weight_view(const vdnn_conv_desc* d, const float* w) {
     return B;
 }
 
-int bwd_shared_tma(const vdnn_conv_desc* d, int P, int Q, float alpha_dx, const float* w, const float* x, const float* dy, float beta_dx,
-                   float* dx, float alpha_w, float beta_w, float* dw, float alpha_b, float beta_b, float* db, char* ws, size_t ws_bytes,
-                   cudaStream_t s) {
-    const BwdSharedPlan plan = bwd_shared_plan(d, P, Q);
+DyGather make_dygather(const vdnn_conv_desc* d, const float* dy, int P, int Q) {
+    DyGather A;
+    A.dy = dy; A.K = d->k; A.P = P; A.Q = Q; A.R = d->r; A.S = d->s;
+    A.pad_h = d->pad_h; A.pad_w = d->pad_w; A.stride_h = d->stride_h; A.stride_w = d->stride_w;
+    A.n_pix = d->n * d->h * d->w; A.n_cols = d->k * d->r * d->s;
+    A.div_hw = FastDiv(d->h * d->w); A.div_w = FastDiv(d->w); A.div_k = FastDiv(d->k); A.div_s = FastDiv(d->s);
+    A.div_sh = FastDiv(d->stride_h); A.div_sw = FastDiv(d->stride_w);
+    A.kpq = d->k * P * Q; A.pq = P * Q;
+    return A;
+}
+
+// dy viewed as [k][(n, pq)]: offset = k*PQ + n*K*PQ + pq
+SplitDense wgrad_dy_view(const vdnn_conv_desc* d, const float* dy, int pq) {
+    SplitDense B;
+    B.p = dy; B.rows = d->k; B.cols = d->n * pq;
+    B.row_div = FastDiv(1u << 30); B.row_hi = 0; B.row_lo = pq;
+    B.col_div = FastDiv(pq); B.col_hi = d->k * pq; B.col_lo = 1;
+    return B;
+}
+
+// Output addressing: rows are the pixels of `channels` planes of `plane` floats.
+Epilogue plane_epilogue(float* out, const float* bias, float alpha, float beta, int channels, int plane) {
+    Epilogue e{};
+    e.out = out; e.bias = bias; e.alpha = alpha; e.beta = beta;
+    e.row_div = FastDiv(plane); e.row_hi = channels * plane; e.row_lo = 1; e.col_stride = plane;
+    return e;
+}
+Epilogue filter_epilogue(float* dw, float alpha, float beta, int crs) {
+    Epilogue e{};
+    e.out = dw; e.bias = nullptr; e.alpha = alpha; e.beta = beta;
+    e.row_div = FastDiv(1u << 30); e.row_hi = 0; e.row_lo = 1; e.col_stride = crs;
+    return e;
+}
+
+// The three products on the gather-fed kernel without workspace, for operands that the TMA-fed kernels leave to it.
+int fwd_gated(const vdnn_conv_desc* d, int P, int Q, float alpha, const float* x, const float* w, const float* bias, float beta, float* y, const int* gate,
+              cudaStream_t s) {
+    const int crs = d->c * d->r * d->s;
+    XGatherPixRows A; A.g = make_xgather(d, x, P, Q);
+    return contract_gated<XGatherPixRows, SplitDense, false, true>(A, make_dense(w, d->k, crs, crs, 1), plane_epilogue(y, bias, alpha, beta, d->k, P * Q),
+                                                                   d->n * P * Q, d->k, crs, gate, s);
+}
+int dgrad_gated(const vdnn_conv_desc* d, int P, int Q, float alpha, const float* w, const float* dy, float beta, float* dx, const int* gate, cudaStream_t s) {
+    return contract_gated<DyGather, SplitDense, false, false>(make_dygather(d, dy, P, Q), dgrad_weight_view(d, w),
+                                                              plane_epilogue(dx, nullptr, alpha, beta, d->c, d->h * d->w), d->n * d->h * d->w, d->c,
+                                                              d->k * d->r * d->s, gate, s);
+}
+int wgrad_gated(const vdnn_conv_desc* d, int P, int Q, float alpha, const float* x, const float* dy, float beta, float* dw, const int* gate, cudaStream_t s) {
+    const int crs = d->c * d->r * d->s;
+    XGatherFiltRows A; A.g = make_xgather(d, x, P, Q);
+    return contract_gated<XGatherFiltRows, SplitDense, true, true>(A, wgrad_dy_view(d, dy, P * Q), filter_epilogue(dw, alpha, beta, crs), crs, d->k,
+                                                                   d->n * P * Q, gate, s);
+}
+
+bool aligned128(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 127u) == 0; }
+size_t x_elems(const vdnn_conv_desc* d) { return static_cast<size_t>(d->n) * d->c * d->h * d->w; }
+size_t w_elems(const vdnn_conv_desc* d) { return static_cast<size_t>(d->k) * d->c * d->r * d->s; }
+size_t y_elems(const vdnn_conv_desc* d, int P, int Q) { return static_cast<size_t>(d->n) * d->k * P * Q; }
+
+// Forward (src = x, out = y) or data gradient (src = dy, out = dx) on the TMA-fed kernels.
+int strips_split16(const vdnn_conv_desc* d, int op, int P, int Q, float alpha, const float* src, const float* w, const float* bias, float beta, float* out,
+                   char* ws, size_t ws_bytes, cudaStream_t s) {
+    const StripPlan plan = strip_plan(d, op, P, Q);
     if (ws_bytes < plan.total) return VDNN_ERR_WORKSPACE;
-    char* tiles = ws;
-    char* strips = tiles + plan.pack;
-    char* ximg = strips + plan.strips;
-    const tma::Problem q = tma_problem(d, VDNN_CONV_BWD_DATA, P, Q);
-    const tma::StripGeom g = tma::strip_geometry(q);
-    // the weights as they are now: the filter gradient below may update them in place (dw == w)
-    int st = tc::pack_b<SplitDense, false>(dgrad_weight_view(d, w), d->c, d->k * d->r * d->s, s, tiles, tma::strip_tile_n(d->c));
+    const bool fwd = op == VDNN_CONV_FWD;
+    const split16::Problem q = split16_problem(d, op, P, Q);
+    const int product = fwd ? split16::FWD : split16::DATA, operand = fwd ? split16::OP_X : split16::OP_DY;
+    const size_t src_elems = fwd ? x_elems(d) : y_elems(d, P, Q), out_elems = fwd ? y_elems(d, P, Q) : x_elems(d);
+    const split16::ScaleParts sp = split16::scale_parts(ws, fwd ? src_elems : 0, w_elems(d), fwd ? 0 : src_elems);
+    char* tiles = ws + split16::SCALE_BYTES;
+    char* lists = tiles + plan.pack;
+    int st = split16::find_magnitudes(sp, fwd ? src : nullptr, fwd ? src_elems : 0, w, w_elems(d), fwd ? nullptr : src, fwd ? 0 : src_elems, s);
     if (st != VDNN_OK) return st;
-    if (beta_b == 0.0f) VDNN_CUDA(cudaMemsetAsync(db, 0, sizeof(float) * d->k, s));
-    const size_t dy_img = static_cast<size_t>(d->k) * P * Q, x_img = static_cast<size_t>(d->c) * d->h * d->w;
-    const size_t dx_elems = static_cast<size_t>(d->n) * x_img, dw_elems = static_cast<size_t>(d->k) * d->c * d->r * d->s;
-    const int groups = q.R * (q.cin / 32);
-    tma::WgradProblem wq = wgrad_problem(d, P, Q);
-    for (int n0 = 0; n0 < d->n; n0 += plan.slab) {
-        tma::Problem part = q;
-        part.n = min(plan.slab, d->n - n0);
-        if ((st = tma::strip_prepare(part, dy + n0 * dy_img, strips, s, db, alpha_b)) != VDNN_OK) return st;
-        if ((st = tma::strip_launch(part, nullptr, strips, tiles, dx + n0 * x_img, nullptr, alpha_dx, beta_dx, EPI_DIRECT, dx_elems, 1, groups, s,
-                                    false)) != VDNN_OK)
-            return st;
-        wq.n = part.n;
-        const float* hi = reinterpret_cast<const float*>(strips);
-        const tma::SharedDy shared{hi, hi + static_cast<size_t>(part.n) * g.lp * q.cin, g.wp, g.lp};
-        int splits = 1;
-        float* partial = nullptr;
-        const float b = n0 == 0 ? beta_w : 1.0f;
-        if (plan.wstrip) {
-            // x as a position list of the same pitch; the filter gradient runs on the two lists
-            tma::Problem fpart = tma_problem(d, VDNN_CONV_FWD, P, Q);
-            fpart.n = part.n;
-            if ((st = tma::strip_prepare(fpart, x + n0 * x_img, ximg, s)) != VDNN_OK) return st;
-            partial = reinterpret_cast<float*>(ximg + tma::strip_image_bytes(fpart));
-            if ((st = tma::wstrip_launch(fpart, d->k, ximg, strips, partial, dw, alpha_w, b, s, &splits)) != VDNN_OK) return st;
-        } else if ((st = tma::wgrad_launch(wq, x + n0 * x_img, nullptr, ximg, dw, alpha_w, b, s, &splits, &partial, nullptr, 0.0f, &shared)) != VDNN_OK) {
-            return st;
-        }
-        if (splits > 1) {
-            st = reduce_partials(dw_elems, splits, alpha_w, b, partial, dw, s);
-            if (st != VDNN_OK) return st;
-        }
+    if ((st = split16::pack_filters(!fwd, w, d->k, d->c, d->r, d->s, tiles, sp, s)) != VDNN_OK) return st;
+    float* partial = plan.splits > 1 ? reinterpret_cast<float*>(lists + plan.lists) : nullptr;
+    const int* wide = &sp.scales->wide[product];
+    for (int n0 = 0; n0 < q.n; n0 += plan.slab) {
+        split16::Problem part = q;
+        part.n = min(plan.slab, q.n - n0);
+        const size_t src_at = src_elems / q.n * n0, out_at = out_elems / q.n * n0;
+        if ((st = split16::write_lists(src + src_at, lists, part.n, q.cin, q.in_h, q.in_w, q.wp, q.lp, sp, operand, false, s)) != VDNN_OK) return st;
+        if (partial) st = split16::strip_launch(part, lists, tiles, partial, nullptr, 1.0f, 0.0f, EPI_PARTIAL, out_elems, plan.splits, plan.group_chunk, sp.scales, product, s);
+        else st = split16::strip_launch(part, lists, tiles, out + out_at, bias, alpha, beta, EPI_DIRECT, out_elems, 1, plan.group_chunk, sp.scales, product, s);
+        if (st != VDNN_OK) return st;
     }
+    if (partial) {
+        if ((st = reduce_partials(out_elems, plan.splits, alpha, beta, partial, out, s, wide)) != VDNN_OK) return st;
+    }
+    st = fwd ? fwd_gated(d, P, Q, alpha, src, w, partial ? nullptr : bias, beta, out, wide, s) : dgrad_gated(d, P, Q, alpha, w, src, beta, out, wide, s);
+    if (st != VDNN_OK || !partial || !bias) return st;
+    return vdnn_add_bias(d->n, d->k, P * Q, 1.0f, bias, out, s);
+}
+
+// The bias gradient of a layer whose dy is rewritten as lists: that pass can form the sums (then *sums = db, scaled by beta_b here),
+// which spares a pass over dy, but adds them by atomics, a thousand or so to an address, one after the other.  Where dy fits L2
+// it is better read once more: 12 x 64 x 77 x 81 57 us with sums, 10 + 6 without.
+int bias_with_lists(const vdnn_conv_desc* d, int P, int Q, float alpha_b, const float* dy, float beta_b, float* db, float** sums, cudaStream_t s) {
+    if (y_elems(d, P, Q) * sizeof(float) <= (static_cast<size_t>(64) << 20) || (beta_b != 0.0f && beta_b != 1.0f))
+        return vdnn_conv_bwd_bias(d->n, d->k, P * Q, alpha_b, dy, beta_b, db, s);
+    *sums = db;
+    if (beta_b == 0.0f) VDNN_CUDA(cudaMemsetAsync(db, 0, sizeof(float) * d->k, s));
     return VDNN_OK;
 }
 
-bool valid_desc(const vdnn_conv_desc* d, int* P, int* Q) {
-    if (!d || d->n <= 0 || d->c <= 0 || d->h <= 0 || d->w <= 0 || d->k <= 0 || d->r <= 0 || d->s <= 0 ||
-        d->pad_h < 0 || d->pad_w < 0 || d->stride_h <= 0 || d->stride_w <= 0)
-        return false;
-    if (d->h + 2 * d->pad_h < d->r || d->w + 2 * d->pad_w < d->s) return false;
-    *P = (d->h + 2 * d->pad_h - d->r) / d->stride_h + 1;
-    *Q = (d->w + 2 * d->pad_w - d->s) / d->stride_w + 1;
-    return true;
+// Filter gradient on the TMA-fed kernels, and with `db` the bias gradient.  Every slab of images adds its share:
+// dw = alpha * (sum over slabs) + beta * dw.
+int wgrad_split16(const vdnn_conv_desc* d, int P, int Q, const float* x, const float* dy, char* ws, const WgradSpace& space, float* dw, float alpha, float beta,
+                  float* db, float alpha_b, float beta_b, cudaStream_t s) {
+    split16::WgradProblem q = split16_wgrad_problem(d, P, Q);
+    const split16::ScaleParts sp = split16::scale_parts(ws, x_elems(d), 0, y_elems(d, P, Q));
+    char* x_lists = ws + split16::SCALE_BYTES;
+    char* dy_lists = x_lists + space.x_lists;
+    float* partial = reinterpret_cast<float*>(dy_lists + space.dy_lists);
+    float* sums = nullptr;
+    int st = db ? bias_with_lists(d, P, Q, alpha_b, dy, beta_b, db, &sums, s) : VDNN_OK;
+    if (st != VDNN_OK) return st;
+    st = split16::find_magnitudes(sp, x, x_elems(d), nullptr, 0, dy, y_elems(d, P, Q), s);
+    if (st != VDNN_OK) return st;
+    bool fresh = split16::few_parts(sp);
+    if (!fresh) {
+        VDNN_CUDA(tc::launch_early(split16::scales_kernel, dim3(1), 256, 0, s, sp));
+        VDNN_LAUNCHED();
+    }
+    const int* wide = &sp.scales->wide[split16::FILTER];
+    const size_t x_img = x_elems(d) / d->n, dy_img = y_elems(d, P, Q) / d->n;
+    for (int n0 = 0; n0 < d->n; n0 += space.slab) {
+        q.n = min(space.slab, d->n - n0);
+        const float b = n0 == 0 ? beta : 1.0f;
+        if ((st = split16::write_lists(dy + n0 * dy_img, dy_lists, q.n, d->k, P, Q, q.wp, q.lp, sp, split16::OP_DY, fresh, s, sums, alpha_b)) != VDNN_OK) return st;
+        if ((st = split16::write_lists(x + n0 * x_img, x_lists, q.n, d->c, d->h, d->w, q.wp, q.lp, sp, split16::OP_X, false, s)) != VDNN_OK) return st;
+        fresh = false;
+        const split16::WgradPlan plan = split16::wgrad_plan(q);
+        if ((st = split16::wgrad_launch(q, plan, x_lists, dy_lists, partial, dw, alpha, b, sp.scales, s)) != VDNN_OK) return st;
+        if (plan.splits > 1 && (st = reduce_partials(w_elems(d), plan.splits, alpha, b, partial, dw, s, wide)) != VDNN_OK) return st;
+    }
+    return wgrad_gated(d, P, Q, alpha, x, dy, beta, dw, wide, s);
 }
 
-// Offsets are 32-bit inside the kernels: every tensor must stay below 2^31 elements.
-bool fits_int32(const vdnn_conv_desc* d, int P, int Q) {
-    const long long lim = 0x7fffffffLL;
-    return 1LL * d->n * d->c * d->h * d->w < lim && 1LL * d->n * d->k * P * Q < lim &&
-           1LL * d->k * d->c * d->r * d->s < lim;
+// ---- one pass over dy for both gradients ---------------------------------------------------------------------------
+// The data gradient and the filter gradient read the same lists of dy, so where both run on the TMA-fed kernels one pass writes
+// them once (and forms the bias sums), and the two kernels run slab by slab from them.
+bool bwd_shared_shape(const vdnn_conv_desc* d) { return split16_shape(d, VDNN_CONV_BWD_DATA) && split16_wgrad_shape(d); }
+
+struct BwdSharedPlan { int slab; size_t pack, dy_lists, x_lists, partial, total; };
+
+BwdSharedPlan bwd_shared_plan(const vdnn_conv_desc* d, int P, int Q) {
+    const split16::Problem q = split16_problem(d, VDNN_CONV_BWD_DATA, P, Q);
+    split16::WgradProblem wq = split16_wgrad_problem(d, P, Q);
+    BwdSharedPlan plan;
+    plan.slab = slab_images(d->n, split16::list_bytes(1, d->k, q.lp) + split16::list_bytes(1, d->c, q.lp));
+    plan.pack = split16::packed_bytes(q.n_cols, q.cin, q.R * q.S);
+    plan.dy_lists = split16::list_bytes(plan.slab, d->k, q.lp);
+    plan.x_lists = split16::list_bytes(plan.slab, d->c, q.lp);
+    wq.n = plan.slab;
+    plan.partial = split16::wgrad_partial_bytes(wq);
+    plan.total = split16::SCALE_BYTES + plan.pack + plan.dy_lists + plan.x_lists + plan.partial;
+    return plan;
 }
 
-XGather make_xgather(const vdnn_conv_desc* d, const float* x, int P, int Q) {
-    XGather g;
-    g.x = x; g.C = d->c; g.H = d->h; g.W = d->w; g.R = d->r; g.S = d->s;
-    g.pad_h = d->pad_h; g.pad_w = d->pad_w; g.stride_h = d->stride_h; g.stride_w = d->stride_w;
-    g.n_pix = d->n * P * Q; g.n_filt = d->c * d->r * d->s;
-    g.Q = Q;
-    g.div_pq = FastDiv(P * Q); g.div_q = FastDiv(Q); g.div_rs = FastDiv(d->r * d->s); g.div_s = FastDiv(d->s);
-    g.div_c = FastDiv(d->c);
-    g.chw = d->c * d->h * d->w; g.hw = d->h * d->w;
-    return g;
+int bwd_shared_split16(const vdnn_conv_desc* d, int P, int Q, float alpha_dx, const float* w, const float* x, const float* dy, float beta_dx, float* dx,
+                       float alpha_w, float beta_w, float* dw, float alpha_b, float beta_b, float* db, char* ws, size_t ws_bytes, cudaStream_t s) {
+    const BwdSharedPlan plan = bwd_shared_plan(d, P, Q);
+    if (ws_bytes < plan.total) return VDNN_ERR_WORKSPACE;
+    const split16::ScaleParts sp = split16::scale_parts(ws, x_elems(d), w_elems(d), y_elems(d, P, Q));
+    char* tiles = ws + split16::SCALE_BYTES;
+    char* dy_lists = tiles + plan.pack;
+    char* x_lists = dy_lists + plan.dy_lists;
+    float* partial = reinterpret_cast<float*>(x_lists + plan.x_lists);
+    const split16::Problem q = split16_problem(d, VDNN_CONV_BWD_DATA, P, Q);
+    split16::WgradProblem wq = split16_wgrad_problem(d, P, Q);
+    float* sums = nullptr;
+    int st = bias_with_lists(d, P, Q, alpha_b, dy, beta_b, db, &sums, s);
+    if (st != VDNN_OK) return st;
+    st = split16::find_magnitudes(sp, x, x_elems(d), w, w_elems(d), dy, y_elems(d, P, Q), s);
+    if (st != VDNN_OK) return st;
+    // the weights as they are now: the filter gradient below may update them in place (dw == w)
+    if ((st = split16::pack_filters(true, w, d->k, d->c, d->r, d->s, tiles, sp, s)) != VDNN_OK) return st;
+    if ((st = dgrad_gated(d, P, Q, alpha_dx, w, dy, beta_dx, dx, &sp.scales->wide[split16::DATA], s)) != VDNN_OK) return st;
+    const int* wide = &sp.scales->wide[split16::FILTER];
+    const size_t dy_img = y_elems(d, P, Q) / d->n, x_img = x_elems(d) / d->n;
+    const int groups = split16::strip_groups(q);
+    for (int n0 = 0; n0 < d->n; n0 += plan.slab) {
+        split16::Problem part = q;
+        part.n = wq.n = min(plan.slab, d->n - n0);
+        const float b = n0 == 0 ? beta_w : 1.0f;
+        if ((st = split16::write_lists(dy + n0 * dy_img, dy_lists, part.n, d->k, P, Q, q.wp, q.lp, sp, split16::OP_DY, false, s, sums, alpha_b)) != VDNN_OK) return st;
+        if ((st = split16::strip_launch(part, dy_lists, tiles, dx + n0 * x_img, nullptr, alpha_dx, beta_dx, EPI_DIRECT, x_elems(d), 1, groups, sp.scales,
+                                        split16::DATA, s)) != VDNN_OK)
+            return st;
+        if ((st = split16::write_lists(x + n0 * x_img, x_lists, part.n, d->c, d->h, d->w, q.wp, q.lp, sp, split16::OP_X, false, s)) != VDNN_OK) return st;
+        const split16::WgradPlan wplan = split16::wgrad_plan(wq);
+        if ((st = split16::wgrad_launch(wq, wplan, x_lists, dy_lists, partial, dw, alpha_w, b, sp.scales, s)) != VDNN_OK) return st;
+        if (wplan.splits > 1 && (st = reduce_partials(w_elems(d), wplan.splits, alpha_w, b, partial, dw, s, wide)) != VDNN_OK) return st;
+    }
+    return wgrad_gated(d, P, Q, alpha_w, x, dy, beta_w, dw, wide, s);
 }
 
 // vdnn_sgemm; parts_optional as in contract().
@@ -1023,20 +1161,18 @@ size_t vdnn_conv_workspace_bytes(int op, int algo_mode, const vdnn_conv_desc* d)
     size_t out;
     const int crs = d->c * d->r * d->s;
     if (op == VDNN_CONV_BWD_ALL) {
-        if (bwd_shared_shape(d, P, Q)) return bwd_shared_plan(d, P, Q).total;
+        if (bwd_shared_shape(d)) return bwd_shared_plan(d, P, Q).total;
         const size_t a = vdnn_conv_workspace_bytes(VDNN_CONV_BWD_DATA, algo_mode, d), b = vdnn_conv_workspace_bytes(VDNN_CONV_BWD_FILTER, algo_mode, d);
         return a > b ? a : b;
     }
-    if (op == VDNN_CONV_BWD_FILTER && tma_wgrad_shape(d)) {
-        tma::WgradProblem q = wgrad_problem(d, P, Q);
-        q.n = 1;
-        q.n = tma_slab_images(d->n, tma::wgrad_image_bytes(q));
-        size_t own = tma::wgrad_image_bytes(q) + tma::wgrad_partial_bytes(q);
+    if (op == VDNN_CONV_BWD_FILTER && split16_wgrad_shape(d)) {
+        size_t own = wgrad_space(d, P, Q).total;
         // a caller that sizes the filter gradient's workspace by this figure can also run all three gradients in it
         // (vdnn_conv_bwd_data_filter_bias)
-        if (bwd_shared_shape(d, P, Q)) { const size_t all = bwd_shared_plan(d, P, Q).total; if (all > own) own = all; }
+        if (bwd_shared_shape(d)) { const size_t all = bwd_shared_plan(d, P, Q).total; if (all > own) own = all; }
         return own;
     }
+    if (split16_shape(d, op)) return strip_plan(d, op, P, Q).total;
     if (is_full_extent(d)) {        // runs as the corresponding FC product
         if (full_extent_dense(d, op)) return 0;
         switch (op) {
@@ -1060,7 +1196,6 @@ size_t vdnn_conv_workspace_bytes(int op, int algo_mode, const vdnn_conv_desc* d)
     size_t bytes = plan.splits > 1 ? static_cast<size_t>(plan.splits) * out * sizeof(float) : 0;
     if (op == VDNN_CONV_FWD || op == VDNN_CONV_BWD_DATA) bytes += packed_weight_bytes(d, op);
     else bytes += packed_dy_bytes(d, P, Q);
-    if (tma_shape(d, op)) bytes += tma_image_bytes(d, op, P, Q);
     return bytes;
 }
 
@@ -1082,11 +1217,15 @@ int vdnn_conv_fwd(const vdnn_conv_desc* d, int algo_mode, float alpha, const flo
         // y off the 16-byte boundaries: the workspace variant below needs what the size query does not report
         if (!workspace || workspace_bytes < packed_weight_bytes(d, VDNN_CONV_FWD)) algo_mode = VDNN_ALGO_MEMORY_OPT;
     }
-    Epilogue e{};
-    e.out = y; e.bias = bias; e.alpha = alpha; e.beta = beta;
-    e.row_div = FastDiv(pq); e.row_hi = d->k * pq; e.row_lo = 1; e.col_stride = pq;
+    const Epilogue e = plane_epilogue(y, bias, alpha, beta, d->k, pq);
     const int M = d->n * pq;
     cudaStream_t s = as_stream(stream);
+    if (algo_mode == VDNN_ALGO_PERF_OPT && split16_shape(d, VDNN_CONV_FWD)) {
+        if (!workspace) return VDNN_ERR_WORKSPACE;
+        if (aligned128(workspace))
+            return strips_split16(d, VDNN_CONV_FWD, P, Q, alpha, x, w, bias, beta, y, static_cast<char*>(workspace), workspace_bytes, s);
+        algo_mode = VDNN_ALGO_MEMORY_OPT;       // workspace off the boundaries that tensor copies need
+    }
     if (algo_mode == VDNN_ALGO_PERF_OPT) {
         // workspace variant: reduce tap-major (k = tap*C + c: one bounds test per run of channels); the weights, read
         // through the matching view ko*CRS + c*RS + tap, are packed once into tile images that the kernel bulk-copies
@@ -1096,12 +1235,6 @@ int vdnn_conv_fwd(const vdnn_conv_desc* d, int algo_mode, float alpha, const flo
         SplitDense B = make_dense(w, d->k, crs, crs, 1);
         B.col_div = FastDiv(d->c); B.col_hi = 1; B.col_lo = rs;
         char* tiles = (g_engine != VDNN_ENGINE_FFMA && (reinterpret_cast<uintptr_t>(workspace) & 127u) == 0) ? static_cast<char*>(workspace) : nullptr;
-        if (tiles && tma_shape(d, VDNN_CONV_FWD) && !g_no_tma) {
-            const tma::Problem q = tma_problem(d, VDNN_CONV_FWD, P, Q);
-            int st = tc::pack_b<SplitDense, true>(B, d->k, crs, s, tiles, tma_use_strips(q) ? tma::strip_tile_n(d->k) : 0);
-            if (st != VDNN_OK) return st;
-            return contract_tma(q, x, tiles, e, static_cast<size_t>(M) * d->k, tiles + pack, workspace_bytes - pack, s);
-        }
         return contract<XGatherPixRowsTap, SplitDense, false, true>(A, B, e, M, d->k, crs, static_cast<size_t>(M) * d->k, 0, algo_mode,
                                                                     static_cast<char*>(workspace) + pack, workspace_bytes - pack, s, tiles);
     }
@@ -1116,7 +1249,7 @@ int vdnn_conv_bwd_data(const vdnn_conv_desc* d, int algo_mode, float alpha, cons
     int P, Q;
     if (!w || !dy || !dx || !valid_desc(d, &P, &Q)) return VDNN_ERR_BAD_ARG;
     if (!fits_int32(d, P, Q)) return VDNN_ERR_UNSUPPORTED;
-    const int rs = d->r * d->s, hw = d->h * d->w, pq = P * Q;
+    const int rs = d->r * d->s, hw = d->h * d->w;
     if (is_full_extent(d))      // dX[n][j] = sum_k W[k][j] dY[n][k]   (the FC data-gradient product, layer.cu:725-733)
         return sgemm(0, 0, d->c * rs, d->n, d->k, alpha, w, d->c * rs, dy, d->k, beta, dx, d->c * rs, algo_mode, workspace,
                      workspace_bytes, as_stream(stream), full_extent_dense(d, VDNN_CONV_BWD_DATA));
@@ -1130,34 +1263,22 @@ int vdnn_conv_bwd_data(const vdnn_conv_desc* d, int algo_mode, float alpha, cons
         st = dgrad_halo(d, P, Q, dy, w, alpha, beta, dx, as_stream(stream));
         if (st != VDNN_ERR_UNSUPPORTED) return st;
     }
-    DyGather A;
-    A.dy = dy; A.K = d->k; A.P = P; A.Q = Q; A.R = d->r; A.S = d->s;
-    A.pad_h = d->pad_h; A.pad_w = d->pad_w; A.stride_h = d->stride_h; A.stride_w = d->stride_w;
-    A.n_pix = d->n * hw; A.n_cols = d->k * rs;
-    A.div_hw = FastDiv(hw); A.div_w = FastDiv(d->w); A.div_k = FastDiv(d->k); A.div_s = FastDiv(d->s);
-    A.div_sh = FastDiv(d->stride_h); A.div_sw = FastDiv(d->stride_w);
-    A.kpq = d->k * pq; A.pq = pq;
-    Epilogue e{};
-    e.out = dx; e.bias = nullptr; e.alpha = alpha; e.beta = beta;
-    e.row_div = FastDiv(hw); e.row_hi = d->c * hw; e.row_lo = 1; e.col_stride = hw;
+    const DyGather A = make_dygather(d, dy, P, Q);
+    const Epilogue e = plane_epilogue(dx, nullptr, alpha, beta, d->c, hw);
     const int M = d->n * hw;
     cudaStream_t s = as_stream(stream);
-    SplitDense B;
-    B.p = w; B.rows = d->c; B.cols = d->k * rs;
-    B.row_div = FastDiv(1u << 30); B.row_hi = 0;
-    B.col_div = FastDiv(d->k);
-    B.row_lo = rs; B.col_hi = 1; B.col_lo = d->c * rs;      // KCRS weights viewed as [c][(tap, ko)]: offset c*RS + tap + ko*C*RS
+    const SplitDense B = dgrad_weight_view(d, w);
+    if (algo_mode == VDNN_ALGO_PERF_OPT && split16_shape(d, VDNN_CONV_BWD_DATA)) {
+        if (!workspace) return VDNN_ERR_WORKSPACE;
+        if (aligned128(workspace))
+            return strips_split16(d, VDNN_CONV_BWD_DATA, P, Q, alpha, dy, w, nullptr, beta, dx, static_cast<char*>(workspace), workspace_bytes, s);
+        algo_mode = VDNN_ALGO_MEMORY_OPT;
+    }
     if (algo_mode == VDNN_ALGO_PERF_OPT) {
         // workspace variant: that view is packed once into tile images that the kernel bulk-copies
         const size_t pack = packed_weight_bytes(d, VDNN_CONV_BWD_DATA);
         if (!workspace || workspace_bytes < pack) return VDNN_ERR_WORKSPACE;
         char* tiles = (g_engine != VDNN_ENGINE_FFMA && (reinterpret_cast<uintptr_t>(workspace) & 127u) == 0) ? static_cast<char*>(workspace) : nullptr;
-        if (tiles && tma_shape(d, VDNN_CONV_BWD_DATA) && !g_no_tma) {
-            const tma::Problem q = tma_problem(d, VDNN_CONV_BWD_DATA, P, Q);
-            st = tc::pack_b<SplitDense, false>(B, d->c, d->k * rs, s, tiles, tma_use_strips(q) ? tma::strip_tile_n(d->c) : 0);
-            if (st != VDNN_OK) return st;
-            return contract_tma(q, dy, tiles, e, static_cast<size_t>(M) * d->c, tiles + pack, workspace_bytes - pack, s);
-        }
         return contract<DyGather, SplitDense, false, false>(A, B, e, M, d->c, d->k * rs, static_cast<size_t>(M) * d->c, 0, algo_mode,
                                                             static_cast<char*>(workspace) + pack, workspace_bytes - pack, s, tiles);
     }
@@ -1183,18 +1304,16 @@ int vdnn_conv_bwd_filter(const vdnn_conv_desc* d, int algo_mode, float alpha, co
     // gathered input, supplies the 128 tile rows; dy supplies up to 256 columns, so every gathered element feeds up to
     // 256 multiply-adds and layers with few filters (K = 64) still fill the tile's rows.
     XGatherFiltRows A; A.g = make_xgather(d, x, P, Q);
-    // dy viewed as [k][(n, pq)]: offset = k*PQ + n*K*PQ + pq
-    SplitDense B;
-    B.p = dy; B.rows = d->k; B.cols = d->n * pq;
-    B.row_div = FastDiv(1u << 30); B.row_hi = 0; B.row_lo = pq;
-    B.col_div = FastDiv(pq); B.col_hi = d->k * pq; B.col_lo = 1;
-    Epilogue e{};
-    e.out = dw; e.bias = nullptr; e.alpha = alpha; e.beta = beta;
-    e.row_div = FastDiv(1u << 30); e.row_hi = 0; e.row_lo = 1; e.col_stride = crs;
-    if (algo_mode == VDNN_ALGO_PERF_OPT && tma_wgrad_shape(d) && g_engine != VDNN_ENGINE_FFMA && workspace &&
-        (reinterpret_cast<uintptr_t>(workspace) & 127u) == 0) {
-        // both operands as channels-last tf32 hi / lo images, fetched by tensor copies (conv_tma.cuh)
-        return wgrad_tma(wgrad_problem(d, P, Q), x, dy, static_cast<char*>(workspace), workspace_bytes, dw, alpha, beta, as_stream(stream));
+    const SplitDense B = wgrad_dy_view(d, dy, pq);
+    const Epilogue e = filter_epilogue(dw, alpha, beta, crs);
+    if (algo_mode == VDNN_ALGO_PERF_OPT && split16_wgrad_shape(d)) {
+        if (!workspace) return VDNN_ERR_WORKSPACE;
+        if (aligned128(workspace)) {
+            const WgradSpace space = wgrad_space(d, P, Q);
+            if (workspace_bytes < space.total) return VDNN_ERR_WORKSPACE;
+            return wgrad_split16(d, P, Q, x, dy, static_cast<char*>(workspace), space, dw, alpha, beta, nullptr, 0.0f, 0.0f, as_stream(stream));
+        }
+        algo_mode = VDNN_ALGO_MEMORY_OPT;
     }
     if (algo_mode == VDNN_ALGO_PERF_OPT) {
         // workspace variant: dy, which every row tile of the gathered input needs again, is split into tf32 halves and
@@ -1216,14 +1335,13 @@ int vdnn_conv_bwd_filter(const vdnn_conv_desc* d, int algo_mode, float alpha, co
 // Bias gradient and filter gradient of one convolution in one call (layer.cu:631-660: cudnnConvolutionBackwardBias, then
 // cudnnConvolutionBackwardFilter).  Where the filter gradient runs on the TMA-fed engine, the pass that rewrites dy into
 // operand images also forms the per-channel sums of dy, so dy is read once less and one kernel launch is saved; anywhere
-// else this is vdnn_conv_bwd_bias followed by vdnn_conv_bwd_filter.  beta_b must be 0 or 1 for the combined form.
+// else this is vdnn_conv_bwd_bias followed by vdnn_conv_bwd_filter.  
 int vdnn_conv_bwd_filter_bias(const vdnn_conv_desc* d, int algo_mode, float alpha, const float* x, const float* dy, float beta,
                               float* dw, float alpha_b, float beta_b, float* db, void* workspace, size_t workspace_bytes,
                               void* stream) {
     int P, Q;
     if (!x || !dy || !dw || !db || !valid_desc(d, &P, &Q)) return VDNN_ERR_BAD_ARG;
-    const bool combined = algo_mode == VDNN_ALGO_PERF_OPT && !is_full_extent(d) && tma_wgrad_shape(d) && g_engine != VDNN_ENGINE_FFMA && workspace &&
-                          (reinterpret_cast<uintptr_t>(workspace) & 127u) == 0 && (beta_b == 0.0f || beta_b == 1.0f) &&
+    const bool combined = algo_mode == VDNN_ALGO_PERF_OPT && split16_wgrad_shape(d) && workspace && aligned128(workspace) &&
                           fits_int32(d, P, Q);
     if (!combined && algo_mode == VDNN_ALGO_PERF_OPT && g_engine != VDNN_ENGINE_FFMA && wgrad_small_c_shape(d, Q) && workspace && fits_int32(d, P, Q) &&
         (reinterpret_cast<uintptr_t>(dy) & 15u) == 0 && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0)
@@ -1232,15 +1350,14 @@ int vdnn_conv_bwd_filter_bias(const vdnn_conv_desc* d, int algo_mode, float alph
         const int st = vdnn_conv_bwd_bias(d->n, d->k, P * Q, alpha_b, dy, beta_b, db, stream);
         return st != VDNN_OK ? st : vdnn_conv_bwd_filter(d, algo_mode, alpha, x, dy, beta, dw, workspace, workspace_bytes, stream);
     }
-    if (beta_b == 0.0f) VDNN_CUDA(cudaMemsetAsync(db, 0, sizeof(float) * d->k, as_stream(stream)));
-    return wgrad_tma(wgrad_problem(d, P, Q), x, dy, static_cast<char*>(workspace), workspace_bytes, dw, alpha, beta, as_stream(stream),
-                     db, alpha_b);
+    const WgradSpace space = wgrad_space(d, P, Q);
+    if (workspace_bytes < space.total) return VDNN_ERR_WORKSPACE;
+    return wgrad_split16(d, P, Q, x, dy, static_cast<char*>(workspace), space, dw, alpha, beta, db, alpha_b, beta_b, as_stream(stream));
 }
-
 
 // cudnnConvolutionBackwardData, BackwardBias and BackwardFilter of one layer (layer.cu:616-660) in one call and one
 // workspace (vdnn_conv_workspace_bytes(VDNN_CONV_BWD_ALL, ...), which the figure for VDNN_CONV_BWD_FILTER covers where the
-// gradients share an image pass).  The data
+// gradients share the lists of dy).  The data
 // gradient uses the weights as they are on entry, also when dw == w.  Where both gradients run on the TMA-fed engine, dy
 // is rewritten into operand images once for both; otherwise the three separate entry points run in the reference's order.
 int vdnn_conv_bwd_data_filter_bias(const vdnn_conv_desc* d, int algo_mode, float alpha_dx, const float* w, const float* x, const float* dy,
@@ -1248,12 +1365,11 @@ int vdnn_conv_bwd_data_filter_bias(const vdnn_conv_desc* d, int algo_mode, float
                                    void* workspace, size_t workspace_bytes, void* stream) {
     int P, Q;
     if (!w || !x || !dy || !dx || !dw || !db || !valid_desc(d, &P, &Q)) return VDNN_ERR_BAD_ARG;
-    const bool shared = algo_mode == VDNN_ALGO_PERF_OPT && g_engine != VDNN_ENGINE_FFMA && workspace &&
-                        (reinterpret_cast<uintptr_t>(workspace) & 127u) == 0 && (beta_b == 0.0f || beta_b == 1.0f) &&
-                        !is_full_extent(d) && fits_int32(d, P, Q) && bwd_shared_shape(d, P, Q);
+    const bool shared = algo_mode == VDNN_ALGO_PERF_OPT && workspace && aligned128(workspace) && fits_int32(d, P, Q) &&
+                        bwd_shared_shape(d);
     if (shared)
-        return bwd_shared_tma(d, P, Q, alpha_dx, w, x, dy, beta_dx, dx, alpha_w, beta_w, dw, alpha_b, beta_b, db, static_cast<char*>(workspace),
-                              workspace_bytes, as_stream(stream));
+        return bwd_shared_split16(d, P, Q, alpha_dx, w, x, dy, beta_dx, dx, alpha_w, beta_w, dw, alpha_b, beta_b, db, static_cast<char*>(workspace),
+                                  workspace_bytes, as_stream(stream));
     const int st = vdnn_conv_bwd_data(d, algo_mode, alpha_dx, w, dy, beta_dx, dx, workspace, workspace_bytes, stream);
     return st != VDNN_OK ? st
                          : vdnn_conv_bwd_filter_bias(d, algo_mode, alpha_w, x, dy, beta_w, dw, alpha_b, beta_b, db, workspace, workspace_bytes, stream);
@@ -1263,8 +1379,7 @@ int vdnn_conv_bwd_data_filter_bias(const vdnn_conv_desc* d, int algo_mode, float
 // apart loses nothing elsewhere).
 int vdnn_conv_bwd_shares_dy(const vdnn_conv_desc* d, int algo_mode) {
     int P, Q;
-    return (algo_mode == VDNN_ALGO_PERF_OPT && g_engine != VDNN_ENGINE_FFMA && valid_desc(d, &P, &Q) && !is_full_extent(d) &&
-            fits_int32(d, P, Q) && bwd_shared_shape(d, P, Q)) ? 1 : 0;
+    return (algo_mode == VDNN_ALGO_PERF_OPT && valid_desc(d, &P, &Q) && fits_int32(d, P, Q) && bwd_shared_shape(d)) ? 1 : 0;
 }
 
 }  // extern "C"
@@ -1301,12 +1416,21 @@ int vdnn_conv_bwd_filter_static(const vdnn_conv_desc* d, float alpha, const floa
                                 float* dw, void* stream) {
     int P, Q;
     if (!x || !dy || !dw || !valid_desc(d, &P, &Q)) return VDNN_ERR_BAD_ARG;
-    const size_t need = is_full_extent(d) ? vdnn_sgemm_workspace_bytes(VDNN_ALGO_PERF_OPT, d->c * d->r * d->s, d->k, d->n)
+    const bool lists = split16_wgrad_shape(d);
+    // layers that run on lists of operands: 8 bytes per element besides the parts, and as many images at a time as there is room for
+    const size_t need = lists ? 2 * sizeof(float) * (x_elems(d) + y_elems(d, P, Q)) + split16::wgrad_partial_bytes(split16_wgrad_problem(d, P, Q))
+                      : is_full_extent(d) ? vdnn_sgemm_workspace_bytes(VDNN_ALGO_PERF_OPT, d->c * d->r * d->s, d->k, d->n)
                                           : vdnn_conv_workspace_bytes(VDNN_CONV_BWD_FILTER, VDNN_ALGO_PERF_OPT, d);
     if (need > VDNN_STATIC_SCRATCH_BYTES) return VDNN_ERR_SCRATCH_LIMIT;
     float* scratch = nullptr;
     const int st = static_scratch_address(&scratch);
     if (st != VDNN_OK) return st;
+    if (lists) {
+        if (!fits_int32(d, P, Q)) return VDNN_ERR_UNSUPPORTED;
+        const WgradSpace space = wgrad_space(d, P, Q, VDNN_STATIC_SCRATCH_BYTES);
+        if (space.total > VDNN_STATIC_SCRATCH_BYTES) return VDNN_ERR_SCRATCH_LIMIT;
+        return wgrad_split16(d, P, Q, x, dy, reinterpret_cast<char*>(scratch), space, dw, alpha, beta, nullptr, 0.0f, 0.0f, as_stream(stream));
+    }
     // The partial sums of every split are written in full before the reduction reads them, so the
     // array's previous contents never matter.
     return vdnn_conv_bwd_filter(d, VDNN_ALGO_PERF_OPT, alpha, x, dy, beta, dw, scratch, VDNN_STATIC_SCRATCH_BYTES, stream);

@@ -260,10 +260,13 @@ inline cudaError_t launch_early(Kernel kern, dim3 grid, int threads, size_t smem
 // swizzled, zero-padded; see pack_b_tiles_kernel), one image per (n tile, k block).  A producer thread then
 // fetches a stage's B tiles with a single bulk asynchronous copy (the TMA engine, no tensor map needed for a
 // contiguous image) that reports its bytes to the stage's "full" barrier; the producers only gather A.
-template <class OpA, class OpB, bool AKC, bool BKC, int BN, bool BBULK>
+// GATED: the kernel does nothing unless *gate is set when its predecessors have finished (the call's other form could not take
+// the operands, see split16.cuh).  A grid of one CTA per tile would cost microseconds per wave just to leave, so at most one CTA
+// per SM is launched and walks the tiles, setting its barriers up anew for each.
+template <class OpA, class OpB, bool AKC, bool BKC, int BN, bool BBULK, bool GATED = false>
 __global__ void __launch_bounds__(THREADS, Config<BN, BN == 64 && !(AKC && BKC)>::CTAS_PER_SM)
 gemm_kernel(const OpA opa, const OpB opb, const Epilogue epi, int M, int N, int K, int k_chunk,
-            const char* __restrict__ b_tiles, int kblocks_total) {
+            const char* __restrict__ b_tiles, int kblocks_total, const int* gate) {
     typedef Config<BN, BN == 64 && !(AKC && BKC)> Cfg;
     constexpr int S = Cfg::STAGES;
     extern __shared__ char smem_raw[];
@@ -274,12 +277,11 @@ gemm_kernel(const OpA opa, const OpB opb, const Epilogue epi, int M, int N, int 
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S + 2);
 
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-    const int kbeg = blockIdx.z * k_chunk;
-    const int kend = min(K, kbeg + k_chunk);
-    const int nkb = kbeg < kend ? (kend - kbeg + BK - 1) / BK : 0;
-
-    if (t == 0) {
+    if constexpr (GATED) {
+        after_predecessor();
+        if (*gate == 0) return;
+    }
+    auto set_up = [&]() {
         for (int s = 0; s < S; ++s) {
             mbar_init(smem_u32(&bars[s]), PRODUCERS);
             mbar_init(smem_u32(&bars[S + s]), 1);
@@ -287,7 +289,8 @@ gemm_kernel(const OpA opa, const OpB opb, const Epilogue epi, int M, int N, int 
         mbar_init(smem_u32(&bars[2 * S]), 1);
         mbar_init(smem_u32(&bars[2 * S + 1]), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
+    };
+    if (t == 0) set_up();
     // Two accumulator buffers of BN columns each: the tensor core sums two 32-wide k blocks into a
     // buffer (a chain of 24 MMAs) while the previous pair's buffer is added into fp32 registers.
     // Keeping the in-TMEM chains short matters for accuracy: the tensor core truncates when it adds
@@ -299,9 +302,32 @@ gemm_kernel(const OpA opa, const OpB opb, const Epilogue epi, int M, int N, int 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // not before the tensor memory is allocated: a follower that took it first would wait for this kernel to finish
     follow_up();
-    after_predecessor();
+    if constexpr (!GATED) after_predecessor();
     const uint32_t tmem_base = *tmem_slot;
+
+    const int m_tiles = (M + BM - 1) / BM, n_tiles = (N + BN - 1) / BN;
+    const long long work = GATED ? static_cast<long long>(m_tiles) * n_tiles * ((K + k_chunk - 1) / k_chunk) : 1;
+    for (long long item = GATED ? blockIdx.x : 0; item < work; item += GATED ? gridDim.x : 1) {
+    int bx = blockIdx.x, by = blockIdx.y, bz = blockIdx.z;
+    if constexpr (GATED) {
+        if (item != blockIdx.x) {
+            if (t == 0) {
+                for (int b = 0; b < 2 * S + 2; ++b) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(&bars[b])) : "memory");
+                set_up();
+            }
+            __syncthreads();
+        }
+        const long long rest = item / m_tiles;
+        bx = static_cast<int>(item - rest * m_tiles);
+        bz = static_cast<int>(rest / n_tiles);
+        by = static_cast<int>(rest - static_cast<long long>(bz) * n_tiles);
+    }
+    const int m0 = bx * BM, n0 = by * BN;
+    const int kbeg = bz * k_chunk;
+    const int kend = min(K, kbeg + k_chunk);
+    const int nkb = kbeg < kend ? (kend - kbeg + BK - 1) / BK : 0;
 
     if (warp < PRODUCER_WARPS) {
         // ------------------------------------------------------------------ producers
@@ -309,8 +335,7 @@ gemm_kernel(const OpA opa, const OpB opb, const Epilogue epi, int M, int N, int 
         Gather<OpB, BKC, BN> gb;
         ga.init(opa, m0, t);
         if (!BBULK) gb.init(opb, n0, t);
-        const char* b_src = BBULK ? b_tiles + (static_cast<size_t>(blockIdx.y) * kblocks_total + kbeg / BK) * (2 * Cfg::B_TILE_BYTES)
-                                  : nullptr;
+        const char* b_src = BBULK ? b_tiles + (static_cast<size_t>(by) * kblocks_total + kbeg / BK) * (2 * Cfg::B_TILE_BYTES) : nullptr;
         // this thread owns row (warp & 3) * 32 + lane of the tile and a slice of its columns
         constexpr int NACC = BN / (PRODUCER_WARPS / 4);
         const int col_beg = (warp >> 2) * NACC;
@@ -379,7 +404,7 @@ gemm_kernel(const OpA opa, const OpB opb, const Epilogue epi, int M, int N, int 
 #pragma unroll
             for (int j = 0; j < NACC; ++j) {
                 const int n = n0 + col_beg + j;
-                if (n < N) epi.store(roff, n, acc[j], blockIdx.z);
+                if (n < N) epi.store(roff, n, acc[j], bz);
             }
         }
     } else {
@@ -405,10 +430,15 @@ gemm_kernel(const OpA opa, const OpB opb, const Epilogue epi, int M, int N, int 
             }
             __syncwarp();
         }
+        if constexpr (GATED)        // no arrival may be on its way when the barriers are set up for the next tile
+            for (int i = max(0, nkb - S); i < nkb; ++i)
+                if (!mbar_wait(smem_u32(&bars[S + i % S]), static_cast<uint32_t>(i / S) & 1u)) { atomicCAS(&g_tc_error, 0, 102); break; }
     }
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    }
     if (warp == PRODUCER_WARPS) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * BN) : "memory");
@@ -501,9 +531,32 @@ int launch_bn(const OpA& a, const OpB& b, const Epilogue& epi, int M, int N, int
         VDNN_LAUNCHED();
     }
     const bool alone = static_cast<long long>(grid.x) * grid.y * grid.z <= sm_count();
-    VDNN_CUDA(launch_early(kern, grid, THREADS, alone ? Cfg::ALONE_BYTES : Cfg::SMEM_BYTES, stream, a, b, epi, M, N, K, k_chunk, b_tiles, kblocks));
+    VDNN_CUDA(launch_early(kern, grid, THREADS, alone ? Cfg::ALONE_BYTES : Cfg::SMEM_BYTES, stream, a, b, epi, M, N, K, k_chunk, b_tiles, kblocks,
+                           static_cast<const int*>(nullptr)));
     VDNN_LAUNCHED();
     return VDNN_OK;
+}
+
+// The contraction without workspace, run only if *gate is set when its turn comes.
+template <class OpA, class OpB, bool AKC, bool BKC, int BN>
+int launch_gated_bn(const OpA& a, const OpB& b, const Epilogue& epi, int M, int N, int K, int splits, int k_chunk, const int* gate, cudaStream_t stream) {
+    typedef Config<BN, BN == 64 && !(AKC && BKC)> Cfg;
+    int dev = 0;
+    VDNN_CUDA(cudaGetDevice(&dev));
+    auto kern = gemm_kernel<OpA, OpB, AKC, BKC, BN, false, true>;
+    VDNN_ALLOW_SHARED(dev, kern, Cfg::ALONE_BYTES);
+    const long long tiles = static_cast<long long>(ceil_div(M, BM)) * ceil_div(N, BN) * splits;
+    const unsigned ctas = static_cast<unsigned>(tiles < sm_count() ? tiles : sm_count());
+    VDNN_CUDA(launch_early(kern, dim3(ctas), THREADS, Cfg::ALONE_BYTES, stream, a, b, epi, M, N, K, k_chunk, static_cast<const char*>(nullptr), 0, gate));
+    VDNN_LAUNCHED();
+    return VDNN_OK;
+}
+template <class OpA, class OpB, bool AKC, bool BKC>
+int launch_gated(const OpA& a, const OpB& b, const Epilogue& epi, int M, int N, int K, int splits, int k_chunk, const int* gate, cudaStream_t stream) {
+    const int bn = tile_n(N);
+    if (bn == 64) return launch_gated_bn<OpA, OpB, AKC, BKC, 64>(a, b, epi, M, N, K, splits, k_chunk, gate, stream);
+    if (bn == 128) return launch_gated_bn<OpA, OpB, AKC, BKC, 128>(a, b, epi, M, N, K, splits, k_chunk, gate, stream);
+    return launch_gated_bn<OpA, OpB, AKC, BKC, 256>(a, b, epi, M, N, K, splits, k_chunk, gate, stream);
 }
 
 // k_chunk must be a multiple of 32.  b_tiles: nullptr, or bulk_bytes(N, K) bytes of 128-byte-aligned scratch: B is then
