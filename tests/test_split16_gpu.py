@@ -21,9 +21,9 @@ def rel(got, want):
     return ((got.double() - want).norm() / want.norm().clamp_min(1e-300)).item()
 
 
-def make(ops, n, c, h, w, k, r, s, pad, offset=0, seed=0):
+def make(ops, n, c, h, w, k, r, s, pad, offset=0, seed=0, stride=1):
     gen = torch.Generator(device="cuda").manual_seed(seed + n + c + h + k)
-    d = ops.conv_desc(n, c, h, w, k, r, s, pad, (1, 1))
+    d = ops.conv_desc(n, c, h, w, k, r, s, pad, (stride, stride))
     P, Q = ops.conv_out_dims(d)
 
     def tensor(*shape):
@@ -46,9 +46,9 @@ def run(ops, d, t, **backward):
     assert ops.engine_status() == 0
 
 
-def exact(t, pad):
+def exact(t, pad, stride=1):
     x, w = t["x"].double().requires_grad_(), t["w"].double().requires_grad_()
-    y = torch.nn.functional.conv2d(x, w, t["b"].double(), padding=pad)
+    y = torch.nn.functional.conv2d(x, w, t["b"].double(), padding=pad, stride=stride)
     dx, dw = torch.autograd.grad(y, (x, w), t["dy"].double())
     return y.detach(), dx, dw, t["dy"].double().sum((0, 2, 3))
 
@@ -76,20 +76,33 @@ SHAPES = [  # n, c, h, w, k, r, s, pad
 ]
 
 
+STRIDED = [  # n, c, h, w, k, r, s, pad, stride: computed in folded form
+    (3, 3, 39, 47, 96, 11, 11, (0, 0), 4),    # a first layer; pixels that no tap reaches
+    (2, 3, 30, 31, 64, 7, 7, (3, 3), 2),
+    (2, 1, 23, 24, 32, 5, 5, (2, 1), 3),
+    (3, 32, 14, 15, 64, 3, 3, (1, 1), 2),
+    (2, 50, 9, 20, 130, 3, 3, (1, 1), 2),     # channels off every block
+    (4, 64, 13, 13, 256, 1, 1, (0, 0), 2),    # three pixels of four unused
+    (2, 19, 17, 70, 40, 2, 5, (0, 2), 3),     # the filter smaller than the stride in one direction
+    (1, 16, 150, 9, 64, 3, 3, (0, 0), 4),
+]
+
+
 @pytest.mark.parametrize("offset", [0, 1])
-@pytest.mark.parametrize("case", SHAPES, ids=str)
+@pytest.mark.parametrize("case", [shape + (1,) for shape in SHAPES] + STRIDED, ids=str)
 def test_against_float64(tensor_cores, case, offset):
     """offset 1: every tensor one float off the 16-byte boundaries."""
-    n, c, h, w, k, r, s, pad = case
-    d, t = make(tensor_cores, n, c, h, w, k, r, s, pad, offset)
+    n, c, h, w, k, r, s, pad, stride = case
+    d, t = make(tensor_cores, n, c, h, w, k, r, s, pad, offset, stride=stride)
     run(tensor_cores, d, t)
-    for got, want in zip((t["y"], t["dx"], t["dw"], t["db"]), exact(t, pad)):
+    for got, want in zip((t["y"], t["dx"], t["dw"], t["db"]), exact(t, pad, stride)):
         assert rel(got, want) < BOUND
 
 
-def test_scaling_and_update_in_place(tensor_cores):
-    d, t = make(tensor_cores, 4, 64, 12, 12, 128, 3, 3, (1, 1))
-    y, dx, dw, db = exact(t, (1, 1))
+@pytest.mark.parametrize("stride", [1, 2])
+def test_scaling_and_update_in_place(tensor_cores, stride):
+    d, t = make(tensor_cores, 4, 64, 12, 12, 128, 3, 3, (1, 1), stride=stride)
+    y, dx, dw, db = exact(t, (1, 1), stride)
     w0, b0, dx0 = t["w"].double(), t["b"].double(), t["dx"].double()
     want = w0 - 0.25 * dw, b0 - 0.5 * db, 2.0 * dx + 0.5 * dx0
     t["dw"], t["db"] = t["w"], t["b"]

@@ -6,6 +6,7 @@
 // workspace followed by a fixed-order reduction (PERF_OPT: deterministic).
 #include <cuda_pipeline.h>
 #include <math.h>
+#include <string.h>
 
 #include <type_traits>
 
@@ -373,8 +374,9 @@ bool fits_int32(const vdnn_conv_desc* d, int P, int Q) {
 
 // Stride-1 convolutions run on the TMA-fed kernels in PERF_OPT (conv_split16.cuh): the gathered tensors are rewritten once into
 // lists of positions in workspace and the kernels fetch their operand tiles by tensor copies.
+// Layers of stride 2 .. 4 do so in folded form (split16.cuh).
 bool split16_layer(const vdnn_conv_desc* d) {
-    return g_engine != VDNN_ENGINE_FFMA && !g_no_tma && d->stride_h == 1 && d->stride_w == 1 && !is_full_extent(d);
+    return g_engine != VDNN_ENGINE_FFMA && !g_no_tma && d->stride_h == d->stride_w && d->stride_h <= split16::FOLD_MAX && !is_full_extent(d);
 }
 
 // Lists of at most this many bytes are kept in workspace at a time; layers that need more are walked in slabs of whole images,
@@ -386,16 +388,44 @@ int slab_images(int n, size_t bytes_per_image) {
     return fit > 1 ? static_cast<int>(fit) : 1;
 }
 
+// A layer as the kernels see it: folded where it is strided, with the list geometry of its grid.
+struct ListLayer { int c, h, w, R, S, pad_h, pad_w, wp, lp; split16::Fold fold; };
+ListLayer list_layer(const vdnn_conv_desc* d, int P, int Q) {
+    const int s = d->stride_h;
+    ListLayer l{d->c, d->h, d->w, d->r, d->s, d->pad_h, d->pad_w, 0, 0, split16::Fold{s, d->c, d->h, d->w, d->pad_h, d->pad_w, d->r, d->s}};
+    if (s > 1) {
+        l.c = d->c * s * s; l.R = ceil_div(d->r, s); l.S = ceil_div(d->s, s); l.pad_h = l.pad_w = 0;
+        // all that the taps reach, and every pixel of x: the data gradient writes the ones that no tap reaches as well
+        l.h = max(P + l.R - 1, ceil_div(d->h + d->pad_h, s)); l.w = max(Q + l.S - 1, ceil_div(d->w + d->pad_w, s));
+    }
+    const split16::ListGeom g = split16::list_geometry(l.h, l.w, P, Q, l.pad_h, l.pad_w);
+    l.wp = g.wp; l.lp = g.wp * g.hp;
+    return l;
+}
+
 split16::Problem split16_problem(const vdnn_conv_desc* d, int op, int P, int Q) {
-    const split16::ListGeom g = split16::list_geometry(d->h, d->w, P, Q, d->pad_h, d->pad_w);
-    if (op == VDNN_CONV_FWD) return split16::Problem{d->n, d->c, d->h, d->w, P, Q, d->k, d->r, d->s, 1, -d->pad_h, -d->pad_w, g.wp, g.wp * g.hp};
+    const ListLayer l = list_layer(d, P, Q);
+    if (op == VDNN_CONV_FWD) return split16::Problem{d->n, l.c, l.h, l.w, P, Q, d->k, l.R, l.S, 1, -l.pad_h, -l.pad_w, l.wp, l.lp, l.fold};
     // dx[h][w] = sum over taps of dy[h + pad - r][w + pad - s] (stride 1)
-    return split16::Problem{d->n, d->k, P, Q, d->h, d->w, d->c, d->r, d->s, -1, d->pad_h, d->pad_w, g.wp, g.wp * g.hp};
+    return split16::Problem{d->n, d->k, P, Q, l.h, l.w, l.c, l.R, l.S, -1, l.pad_h, l.pad_w, l.wp, l.lp, l.fold};
 }
 
 split16::WgradProblem split16_wgrad_problem(const vdnn_conv_desc* d, int P, int Q) {
-    const split16::ListGeom g = split16::list_geometry(d->h, d->w, P, Q, d->pad_h, d->pad_w);
-    return split16::WgradProblem{d->n, d->c, d->h, d->w, d->k, P, Q, d->r, d->s, d->pad_h, d->pad_w, g.wp, g.wp * g.hp};
+    const ListLayer l = list_layer(d, P, Q);
+    return split16::WgradProblem{d->n, l.c, l.h, l.w, d->k, P, Q, l.R, l.S, l.pad_h, l.pad_w, l.wp, l.lp, l.fold};
+}
+
+// The lists of n images of x from image n0 on.
+int write_x_lists(const vdnn_conv_desc* d, int P, int Q, const float* x, int n0, int n, char* lists, const split16::ScaleParts& sp, bool fresh, cudaStream_t s) {
+    const ListLayer l = list_layer(d, P, Q);
+    const float* src = x + static_cast<size_t>(n0) * d->c * d->h * d->w;
+    if (l.fold.s > 1) return split16::write_folded_lists(src, lists, n, l.fold, l.h, l.w, sp, fresh, s);
+    return split16::write_lists(src, lists, n, d->c, d->h, d->w, l.wp, l.lp, sp, split16::OP_X, fresh, s);
+}
+int pack_layer(const vdnn_conv_desc* d, int P, int Q, bool data_gradient, const float* w, char* tiles, const split16::ScaleParts& sp, cudaStream_t s) {
+    const ListLayer l = list_layer(d, P, Q);
+    if (l.fold.s > 1) return split16::pack_folded(data_gradient, w, d->k, l.fold, l.R, l.S, tiles, sp, s);
+    return split16::pack_filters(data_gradient, w, d->k, d->c, d->r, d->s, tiles, sp, s);
 }
 
 // What forward or the data gradient keeps in workspace: the scale record, the packed filters, the lists of a slab of images, the
@@ -415,7 +445,7 @@ StripPlan strip_plan(const vdnn_conv_desc* d, int op, int P, int Q) {
     if (plan.slab == q.n && 2 * tiles <= slots) splits = static_cast<int>(min(static_cast<long long>(groups), slots / tiles));
     plan.group_chunk = ceil_div(groups, splits);
     plan.splits = ceil_div(groups, plan.group_chunk);
-    plan.partial = plan.splits > 1 ? static_cast<size_t>(plan.splits) * q.n * q.n_cols * q.out_h * q.out_w * sizeof(float) : 0;
+    plan.partial = plan.splits > 1 ? static_cast<size_t>(plan.splits) * d->n * (op == VDNN_CONV_FWD ? d->k * P * Q : d->c * d->h * d->w) * sizeof(float) : 0;
     plan.total = split16::SCALE_BYTES + plan.pack + plan.lists + plan.partial;
     return plan;
 }
@@ -444,23 +474,29 @@ WgradSpace wgrad_space(const vdnn_conv_desc* d, int P, int Q, size_t limit = SIZ
 // gradient) against the faster of the two for every layer, at worst 15, 28 and 48 %; lists everywhere or nowhere lose up to
 // 3.3 and 7 times.
 struct GatherRate { double block, wave; };
-double gathered_us(int M, int N, int K, bool may_split) {
-    const int bn = tc::tile_n(N), blocks = ceil_div(K, 32);
+double gathered_us(int M, int N, int K, bool may_split, bool strided) {
+    const int bn = tc::tile_n(N), blocks = ceil_div(K, 32), size = bn == 64 ? 0 : (bn == 128 ? 1 : 2);
     const long long tiles = static_cast<long long>(ceil_div(M, 128)) * ceil_div(N, bn);
     int splits = 1;
     if (may_split && tiles < sm_count()) splits = max(1, min(static_cast<int>(2 * sm_count() / tiles), K / 64));
     const double waves = static_cast<double>(ceil_div<long long>(tiles * splits, bn == 64 ? 2 * sm_count() : sm_count()));
-    const GatherRate rate = bn == 64 ? GatherRate{1.4, 1.5} : (bn == 128 ? GatherRate{0.8, 4.9} : GatherRate{1.18, 7.7});
-    return (may_split ? 7.0 : 3.0) + waves * (rate.block * ceil_div(blocks, splits) + rate.wave);
+    static const GatherRate plain[3] = {{1.4, 1.5}, {0.8, 4.9}, {1.18, 7.7}}, fwd[3] = {{2.4, 4.0}, {0.89, 7.8}, {1.33, 9.1}}, data[3] = {{1.2, 0.0}, {0.69, 0.0}, {1.24, 0.0}};
+    GatherRate rate = !strided ? plain[size] : (may_split ? data[size] : fwd[size]);
+    if (strided && !may_split && bn == 64 && tiles <= sm_count()) rate.block *= 0.5;      // a CTA has its SM to itself
+    return (strided && may_split ? 27.0 : (may_split ? 7.0 : 3.0)) + waves * (rate.block * ceil_div(blocks, splits) + rate.wave);
 }
 
 // Forward and data gradient.  With the engine forced to VDNN_ENGINE_TCGEN05 every eligible shape runs on lists (small shapes in the
 // tests).
-bool split16_shape(const vdnn_conv_desc* d, int op) {
+// Folded channels that fill most of their blocks of 64: a first layer of stride 4, or 16 channels and more.
+bool useful_channels(int c) { return 10 * c >= 7 * split16::padded_channels(c); }
+
+bool choose_strips(const vdnn_conv_desc* d, int op) {
     if (!split16_layer(d) || (op != VDNN_CONV_FWD && op != VDNN_CONV_BWD_DATA)) return false;
     const bool fwd = op == VDNN_CONV_FWD;
-    if ((fwd ? d->c : d->k) < 8 || (!fwd && d->c <= SMALL_C_MAX)) return false;       // first layers have their own kernels
     int P, Q;
+    const bool first = d->c <= SMALL_C_MAX;          // those of stride 1 have their own kernels
+    if ((first && d->stride_h == 1) || (fwd ? d->c * d->stride_h * d->stride_w : d->k) < 8) return false;
     if (!valid_desc(d, &P, &Q) || !fits_int32(d, P, Q)) return false;
     const split16::Problem q = split16_problem(d, op, P, Q);
     if (static_cast<long long>(q.n) * q.lp >= 0x7fffff00LL) return false;
@@ -470,12 +506,22 @@ bool split16_shape(const vdnn_conv_desc* d, int op) {
     const double src = 0.5e-6 * (static_cast<double>(q.n) * q.cin * q.in_h * q.in_w + static_cast<double>(q.n) * q.lp * split16::padded_channels(q.cin));
     const double out = 1e-6 * q.n * q.n_cols * q.out_h * q.out_w, weights = 1e-6 * q.cin * q.n_cols * q.R * q.S;
     const double waves = static_cast<double>(ceil_div<long long>(split16::strip_tiles(q) * plan.splits, split16::strip_slots(q.n_cols)));
-    const double lists = 20.0 + 0.8 * waves * plan.group_chunk * split16::taps_per_strip(q.S) + 1.8 * src + 1.1 * out * (plan.splits > 1 ? 1 + 2 * plan.splits : 1) + 7.7 * weights;
-    return lists < gathered_us(q.n * q.out_h * q.out_w, q.n_cols, q.cin * q.R * q.S, !fwd) + 0.5 * (src + out);
+    const double blocks = waves * plan.group_chunk * split16::taps_per_strip(q.S), parts = plan.splits > 1 ? 1 + 2 * plan.splits : 1;
+    const int M = fwd ? d->n * P * Q : d->n * d->h * d->w, N = fwd ? d->k : d->c, K = (fwd ? d->c : d->k) * d->r * d->s;
+    if (d->stride_h > 1) {
+        // Folded layers, fitted to 100 of stride 2 and 4.  The data gradient gains most (2.3 times as fast on average: the gather
+        // tests every tap of every pixel and multiplies zeros, the first layers' kernels do 33 TFLOP/s of multiply-adds); forward is
+        // bound by its passes, and taken where it is surely the faster.
+        if (fwd) return useful_channels(q.cin) && 1.15 * (14.5 + 5.5 * src + 3.2 * out * parts + 8.2 * weights) < gathered_us(M, N, K, false, true);
+        const double lists = 18.0 + 0.77 * blocks + 1.2 * src + 2.0 * out * parts + 5.1 * weights;
+        return 1.1 * lists < (first ? 10.0 + 78e-9 * d->n * P * Q * d->k * d->c * d->r * d->s : gathered_us(M, N, K, true, true));
+    }
+    const double lists = 20.0 + 0.8 * blocks + 1.8 * src + 1.1 * out * parts + 7.7 * weights;
+    return lists < gathered_us(M, N, K, !fwd, false) + 0.5 * (src + out);
 }
 
-bool split16_wgrad_shape(const vdnn_conv_desc* d) {
-    if (!g_tma_wgrad || !split16_layer(d) || d->c < 8) return false;
+bool choose_wgrad(const vdnn_conv_desc* d) {
+    if (!g_tma_wgrad || !split16_layer(d) || d->c * d->stride_h * d->stride_w < 8 || (d->c <= SMALL_C_MAX && d->stride_h == 1)) return false;
     int P, Q;
     if (!valid_desc(d, &P, &Q) || !fits_int32(d, P, Q)) return false;
     const split16::WgradProblem q = split16_wgrad_problem(d, P, Q);
@@ -484,16 +530,42 @@ bool split16_wgrad_shape(const vdnn_conv_desc* d) {
     if (d->n * P * Q < split16::BM) return false;
     const split16::WgradPlan w = split16::wgrad_plan(q);
     const double dw = 1e-6 * d->k * d->c * d->r * d->s, dy = 1e-6 * d->n * d->k * P * Q;
-    const double both = 0.5 * (1e-6 * d->n * d->c * d->h * d->w + dy + 1e-6 * q.n * q.lp * (split16::padded_channels(d->c) + split16::padded_channels(d->k)));
+    // where the data gradient runs on lists (in the same call: vdnn_conv_bwd_data_filter_bias), dy's are there already
+    const bool shared = choose_strips(d, VDNN_CONV_BWD_DATA);
+    const double spared = shared ? 0.3 * (dy + 1e-6 * q.n * q.lp * split16::padded_channels(d->k)) : 0.0, launches = shared ? 10.0 : 0.0;
+    const double both = 0.5 * (1e-6 * d->n * d->c * d->h * d->w + dy + 1e-6 * q.n * q.lp * (split16::padded_channels(q.c) + split16::padded_channels(d->k)));
     const double waves = static_cast<double>(ceil_div(ceil_div(w.groups, w.chunk) * w.ctas * ceil_div(d->k, w.bn) * w.splits, sm_count()));
-    const double lists = 27.0 + waves * ((w.bn == 64 ? 2.46 : (w.bn == 128 ? 1.32 : 1.23)) * w.kb_chunk + 3.9) + 2.0 * both + 4.5 * w.splits * dw;
+    double lists = 27.0 - launches + waves * ((w.bn == 64 ? 2.46 : (w.bn == 128 ? 1.32 : 1.23)) * w.kb_chunk + 3.9) + 2.0 * (both - spared) + 4.5 * w.splits * dw;
     const int M = d->c * d->r * d->s, bn = tc::tile_n(d->k);
     const SplitPlan split = plan_split(M, d->k, d->n * P * Q);
     const double gwaves = static_cast<double>(ceil_div(ceil_div(M, 128) * ceil_div(d->k, bn) * split.splits, sm_count()));
     const double gathered = 10.0 + gwaves * ((bn == 64 ? 1.16 : (bn == 128 ? 1.2 : 1.5)) * (split.k_chunk / 32) + 3.3) + 1.4 * (split.splits > 1 ? split.splits : 0) * dw +
                             (d->k >= 128 ? 3.25 : 0.0) * dy + 1.2 * dw;
+    if (d->stride_h > 1) {      // folded: bound by the passes over x; taken where surely faster
+        lists = 23.3 - launches + waves * ((w.bn == 64 ? 0.0 : 0.45) * w.kb_chunk + 6.2) + 4.4 * (both - spared) + 4.6 * w.splits * dw;
+        return useful_channels(q.c) && (shared ? 1.2 : 1.6) * lists < 1.3 * gathered;
+    }
     return lists < 1.3 * gathered;          // the gather's time is the less certain one, and errs upwards
 }
+
+// The choices of a layer are functions of its description (and of the engine), but take a microsecond or two, and a call asks
+// several times: each thread remembers those of the layers it met last.
+struct Choices { vdnn_conv_desc d; int engine; bool known, fwd, data, filter; };
+const Choices& choices(const vdnn_conv_desc* d) {
+    static thread_local Choices memo[64];
+    const unsigned h = ((d->n * 31u + d->c) * 31u + d->h) * 31u + d->k * 7u + d->r + d->stride_h;
+    Choices& m = memo[(h ^ (h >> 6) ^ (h >> 12)) & 63u];
+    if (!m.known || m.engine != g_engine || memcmp(&m.d, d, sizeof(*d)) != 0) {
+        m.known = false;
+        m.fwd = choose_strips(d, VDNN_CONV_FWD); m.data = choose_strips(d, VDNN_CONV_BWD_DATA); m.filter = choose_wgrad(d);
+        m.d = *d; m.engine = g_engine; m.known = true;
+    }
+    return m;
+}
+bool split16_shape(const vdnn_conv_desc* d, int op) {
+    return op == VDNN_CONV_FWD ? choices(d).fwd : (op == VDNN_CONV_BWD_DATA && choices(d).data);
+}
+bool split16_wgrad_shape(const vdnn_conv_desc* d) { return choices(d).filter; }
 
 int stream_blocks(size_t n) {
     size_t want = ceil_div<size_t>(n, 256);
@@ -933,21 +1005,23 @@ int strips_split16(const vdnn_conv_desc* d, int op, int P, int Q, float alpha, c
     if (ws_bytes < plan.total) return VDNN_ERR_WORKSPACE;
     const bool fwd = op == VDNN_CONV_FWD;
     const split16::Problem q = split16_problem(d, op, P, Q);
-    const int product = fwd ? split16::FWD : split16::DATA, operand = fwd ? split16::OP_X : split16::OP_DY;
+    const int product = fwd ? split16::FWD : split16::DATA;
     const size_t src_elems = fwd ? x_elems(d) : y_elems(d, P, Q), out_elems = fwd ? y_elems(d, P, Q) : x_elems(d);
     const split16::ScaleParts sp = split16::scale_parts(ws, fwd ? src_elems : 0, w_elems(d), fwd ? 0 : src_elems);
     char* tiles = ws + split16::SCALE_BYTES;
     char* lists = tiles + plan.pack;
     int st = split16::find_magnitudes(sp, fwd ? src : nullptr, fwd ? src_elems : 0, w, w_elems(d), fwd ? nullptr : src, fwd ? 0 : src_elems, s);
     if (st != VDNN_OK) return st;
-    if ((st = split16::pack_filters(!fwd, w, d->k, d->c, d->r, d->s, tiles, sp, s)) != VDNN_OK) return st;
+    if ((st = pack_layer(d, P, Q, !fwd, w, tiles, sp, s)) != VDNN_OK) return st;
     float* partial = plan.splits > 1 ? reinterpret_cast<float*>(lists + plan.lists) : nullptr;
     const int* wide = &sp.scales->wide[product];
     for (int n0 = 0; n0 < q.n; n0 += plan.slab) {
         split16::Problem part = q;
         part.n = min(plan.slab, q.n - n0);
         const size_t src_at = src_elems / q.n * n0, out_at = out_elems / q.n * n0;
-        if ((st = split16::write_lists(src + src_at, lists, part.n, q.cin, q.in_h, q.in_w, q.wp, q.lp, sp, operand, false, s)) != VDNN_OK) return st;
+        st = fwd ? write_x_lists(d, P, Q, src, n0, part.n, lists, sp, false, s)
+                 : split16::write_lists(src + src_at, lists, part.n, d->k, P, Q, q.wp, q.lp, sp, split16::OP_DY, false, s);
+        if (st != VDNN_OK) return st;
         if (partial) st = split16::strip_launch(part, lists, tiles, partial, nullptr, 1.0f, 0.0f, EPI_PARTIAL, out_elems, plan.splits, plan.group_chunk, sp.scales, product, s);
         else st = split16::strip_launch(part, lists, tiles, out + out_at, bias, alpha, beta, EPI_DIRECT, out_elems, 1, plan.group_chunk, sp.scales, product, s);
         if (st != VDNN_OK) return st;
@@ -996,7 +1070,7 @@ int wgrad_split16(const vdnn_conv_desc* d, int P, int Q, const float* x, const f
         q.n = min(space.slab, d->n - n0);
         const float b = n0 == 0 ? beta : 1.0f;
         if ((st = split16::write_lists(dy + n0 * dy_img, dy_lists, q.n, d->k, P, Q, q.wp, q.lp, sp, split16::OP_DY, fresh, s, sums, alpha_b)) != VDNN_OK) return st;
-        if ((st = split16::write_lists(x + n0 * x_img, x_lists, q.n, d->c, d->h, d->w, q.wp, q.lp, sp, split16::OP_X, false, s)) != VDNN_OK) return st;
+        if ((st = write_x_lists(d, P, Q, x, n0, q.n, x_lists, sp, false, s)) != VDNN_OK) return st;
         fresh = false;
         const split16::WgradPlan plan = split16::wgrad_plan(q);
         if ((st = split16::wgrad_launch(q, plan, x_lists, dy_lists, partial, dw, alpha, b, sp.scales, s)) != VDNN_OK) return st;
@@ -1016,10 +1090,10 @@ BwdSharedPlan bwd_shared_plan(const vdnn_conv_desc* d, int P, int Q) {
     const split16::Problem q = split16_problem(d, VDNN_CONV_BWD_DATA, P, Q);
     split16::WgradProblem wq = split16_wgrad_problem(d, P, Q);
     BwdSharedPlan plan;
-    plan.slab = slab_images(d->n, split16::list_bytes(1, d->k, q.lp) + split16::list_bytes(1, d->c, q.lp));
+    plan.slab = slab_images(d->n, split16::list_bytes(1, d->k, q.lp) + split16::list_bytes(1, wq.c, q.lp));
     plan.pack = split16::packed_bytes(q.n_cols, q.cin, q.R * q.S);
     plan.dy_lists = split16::list_bytes(plan.slab, d->k, q.lp);
-    plan.x_lists = split16::list_bytes(plan.slab, d->c, q.lp);
+    plan.x_lists = split16::list_bytes(plan.slab, wq.c, q.lp);
     wq.n = plan.slab;
     plan.partial = split16::wgrad_partial_bytes(wq);
     plan.total = split16::SCALE_BYTES + plan.pack + plan.dy_lists + plan.x_lists + plan.partial;
@@ -1043,7 +1117,7 @@ int bwd_shared_split16(const vdnn_conv_desc* d, int P, int Q, float alpha_dx, co
     st = split16::find_magnitudes(sp, x, x_elems(d), w, w_elems(d), dy, y_elems(d, P, Q), s);
     if (st != VDNN_OK) return st;
     // the weights as they are now: the filter gradient below may update them in place (dw == w)
-    if ((st = split16::pack_filters(true, w, d->k, d->c, d->r, d->s, tiles, sp, s)) != VDNN_OK) return st;
+    if ((st = pack_layer(d, P, Q, true, w, tiles, sp, s)) != VDNN_OK) return st;
     if ((st = dgrad_gated(d, P, Q, alpha_dx, w, dy, beta_dx, dx, &sp.scales->wide[split16::DATA], s)) != VDNN_OK) return st;
     const int* wide = &sp.scales->wide[split16::FILTER];
     const size_t dy_img = y_elems(d, P, Q) / d->n, x_img = x_elems(d) / d->n;
@@ -1056,7 +1130,7 @@ int bwd_shared_split16(const vdnn_conv_desc* d, int P, int Q, float alpha_dx, co
         if ((st = split16::strip_launch(part, dy_lists, tiles, dx + n0 * x_img, nullptr, alpha_dx, beta_dx, EPI_DIRECT, x_elems(d), 1, groups, sp.scales,
                                         split16::DATA, s)) != VDNN_OK)
             return st;
-        if ((st = split16::write_lists(x + n0 * x_img, x_lists, part.n, d->c, d->h, d->w, q.wp, q.lp, sp, split16::OP_X, false, s)) != VDNN_OK) return st;
+        if ((st = write_x_lists(d, P, Q, x, n0, part.n, x_lists, sp, false, s)) != VDNN_OK) return st;
         const split16::WgradPlan wplan = split16::wgrad_plan(wq);
         if ((st = split16::wgrad_launch(wq, wplan, x_lists, dy_lists, partial, dw, alpha_w, b, sp.scales, s)) != VDNN_OK) return st;
         if (wplan.splits > 1 && (st = reduce_partials(w_elems(d), wplan.splits, alpha_w, b, partial, dw, s, wide)) != VDNN_OK) return st;
@@ -1097,6 +1171,58 @@ int sgemm(int transa, int transb, int m, int n, int k, float alpha, const float*
 // the gather-fed kernel takes, run unsplit in that.
 bool full_extent_dense(const vdnn_conv_desc* d, int op) {
     return g_engine != VDNN_ENGINE_FFMA && d->c * d->r * d->s % 4 == 0 && (op == VDNN_CONV_FWD || d->k % 4 == 0);
+}
+
+// vdnn_conv_bwd_filter; lists: false keeps it on the gather-fed kernel.
+int bwd_filter(const vdnn_conv_desc* d, int algo_mode, float alpha, const float* x, const float* dy, float beta, float* dw, void* workspace,
+               size_t workspace_bytes, void* stream, bool lists) {
+    int P, Q;
+    if (!x || !dy || !dw || !valid_desc(d, &P, &Q)) return VDNN_ERR_BAD_ARG;
+    if (!fits_int32(d, P, Q)) return VDNN_ERR_UNSUPPORTED;
+    const int crs = d->c * d->r * d->s, pq = P * Q;
+    if (is_full_extent(d))      // W[k][j] = alpha * sum_n X[n][j] dY[n][k] + beta * W[k][j]   (layer.cu:736-744)
+        return sgemm(0, 1, crs, d->k, d->n, alpha, x, crs, dy, d->k, beta, dw, crs, algo_mode, workspace, workspace_bytes, as_stream(stream),
+                     full_extent_dense(d, VDNN_CONV_BWD_FILTER));
+    if (algo_mode == VDNN_ALGO_PERF_OPT && g_engine != VDNN_ENGINE_FFMA && wgrad_small_c_shape(d, Q) && workspace &&
+        (reinterpret_cast<uintptr_t>(dy) & 15u) == 0 && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0)
+        return wgrad_small_c(d, P, Q, x, dy, alpha, beta, dw, 0.0f, 0.0f, nullptr, static_cast<char*>(workspace), workspace_bytes, as_stream(stream));
+    // D[j][k] = sum over pixels of x(j; pixel) * dy(k; pixel), written to dw[k*CRS + j]: the expensive operand, the
+    // gathered input, supplies the 128 tile rows; dy supplies up to 256 columns, so every gathered element feeds up to
+    // 256 multiply-adds and layers with few filters (K = 64) still fill the tile's rows.
+    XGatherFiltRows A; A.g = make_xgather(d, x, P, Q);
+    const SplitDense B = wgrad_dy_view(d, dy, pq);
+    const Epilogue e = filter_epilogue(dw, alpha, beta, crs);
+    if (lists && algo_mode == VDNN_ALGO_PERF_OPT && split16_wgrad_shape(d)) {
+        if (!workspace) return VDNN_ERR_WORKSPACE;
+        if (aligned128(workspace)) {
+            const WgradSpace space = wgrad_space(d, P, Q);
+            if (workspace_bytes < space.total) return VDNN_ERR_WORKSPACE;
+            return wgrad_split16(d, P, Q, x, dy, static_cast<char*>(workspace), space, dw, alpha, beta, nullptr, 0.0f, 0.0f, as_stream(stream));
+        }
+        algo_mode = VDNN_ALGO_MEMORY_OPT;
+    }
+    if (algo_mode == VDNN_ALGO_PERF_OPT) {
+        // workspace variant: dy, which every row tile of the gathered input needs again, is split into tf32 halves and
+        // laid out as tile images once; the kernel's producers then gather x only
+        // (tensors off the 16-byte boundaries of a layer whose workspace is sized for wgrad_small_c: its bytes hold the parts of the
+        // sums, two splits for each SM against that kernel's three blocks, but no images of dy)
+        const size_t pack = wgrad_small_c_shape(d, Q) && g_engine != VDNN_ENGINE_FFMA ? 0 : packed_dy_bytes(d, P, Q);
+        if (pack && (!workspace || workspace_bytes < pack)) return VDNN_ERR_WORKSPACE;
+        char* tiles = (pack && g_engine != VDNN_ENGINE_FFMA && (reinterpret_cast<uintptr_t>(workspace) & 127u) == 0)
+                          ? static_cast<char*>(workspace) : nullptr;
+        return contract<XGatherFiltRows, SplitDense, true, true>(A, B, e, crs, d->k, d->n * pq, static_cast<size_t>(d->k) * crs, 0,
+                                                                 algo_mode, static_cast<char*>(workspace) + pack,
+                                                                 workspace_bytes - pack, as_stream(stream), tiles);
+    }
+    return contract<XGatherFiltRows, SplitDense, true, true>(A, B, e, crs, d->k, d->n * pq, static_cast<size_t>(d->k) * crs, 0,
+                                                             algo_mode, workspace, workspace_bytes, as_stream(stream));
+}
+
+// Workspace of the filter gradient on the gather-fed kernel.
+size_t gathered_filter_bytes(const vdnn_conv_desc* d, int P, int Q) {
+    const int crs = d->c * d->r * d->s;
+    const SplitPlan plan = plan_split(crs, d->k, d->n * P * Q);
+    return (plan.splits > 1 ? static_cast<size_t>(plan.splits) * crs * d->k * sizeof(float) : 0) + packed_dy_bytes(d, P, Q);
 }
 
 }  // namespace
@@ -1253,6 +1379,12 @@ int vdnn_conv_bwd_data(const vdnn_conv_desc* d, int algo_mode, float alpha, cons
     if (is_full_extent(d))      // dX[n][j] = sum_k W[k][j] dY[n][k]   (the FC data-gradient product, layer.cu:725-733)
         return sgemm(0, 0, d->c * rs, d->n, d->k, alpha, w, d->c * rs, dy, d->k, beta, dx, d->c * rs, algo_mode, workspace,
                      workspace_bytes, as_stream(stream), full_extent_dense(d, VDNN_CONV_BWD_DATA));
+    if (algo_mode == VDNN_ALGO_PERF_OPT && split16_shape(d, VDNN_CONV_BWD_DATA)) {
+        if (!workspace) return VDNN_ERR_WORKSPACE;
+        if (aligned128(workspace))
+            return strips_split16(d, VDNN_CONV_BWD_DATA, P, Q, alpha, dy, w, nullptr, beta, dx, static_cast<char*>(workspace), workspace_bytes, as_stream(stream));
+        algo_mode = VDNN_ALGO_MEMORY_OPT;       // workspace off the boundaries that tensor copies need
+    }
     int st = dgrad_few_channels(d, P, Q, alpha, w, dy, beta, dx, as_stream(stream));
     if (st != VDNN_ERR_UNSUPPORTED) return st;
     // Without workspace only: the gather-fed kernel with packed weights (PERF_OPT, channels or sizes that the TMA-fed kernels do
@@ -1268,12 +1400,6 @@ int vdnn_conv_bwd_data(const vdnn_conv_desc* d, int algo_mode, float alpha, cons
     const int M = d->n * hw;
     cudaStream_t s = as_stream(stream);
     const SplitDense B = dgrad_weight_view(d, w);
-    if (algo_mode == VDNN_ALGO_PERF_OPT && split16_shape(d, VDNN_CONV_BWD_DATA)) {
-        if (!workspace) return VDNN_ERR_WORKSPACE;
-        if (aligned128(workspace))
-            return strips_split16(d, VDNN_CONV_BWD_DATA, P, Q, alpha, dy, w, nullptr, beta, dx, static_cast<char*>(workspace), workspace_bytes, s);
-        algo_mode = VDNN_ALGO_MEMORY_OPT;
-    }
     if (algo_mode == VDNN_ALGO_PERF_OPT) {
         // workspace variant: that view is packed once into tile images that the kernel bulk-copies
         const size_t pack = packed_weight_bytes(d, VDNN_CONV_BWD_DATA);
@@ -1290,46 +1416,7 @@ int vdnn_conv_bwd_data(const vdnn_conv_desc* d, int algo_mode, float alpha, cons
 
 int vdnn_conv_bwd_filter(const vdnn_conv_desc* d, int algo_mode, float alpha, const float* x, const float* dy,
                          float beta, float* dw, void* workspace, size_t workspace_bytes, void* stream) {
-    int P, Q;
-    if (!x || !dy || !dw || !valid_desc(d, &P, &Q)) return VDNN_ERR_BAD_ARG;
-    if (!fits_int32(d, P, Q)) return VDNN_ERR_UNSUPPORTED;
-    const int crs = d->c * d->r * d->s, pq = P * Q;
-    if (is_full_extent(d))      // W[k][j] = alpha * sum_n X[n][j] dY[n][k] + beta * W[k][j]   (layer.cu:736-744)
-        return sgemm(0, 1, crs, d->k, d->n, alpha, x, crs, dy, d->k, beta, dw, crs, algo_mode, workspace, workspace_bytes, as_stream(stream),
-                     full_extent_dense(d, VDNN_CONV_BWD_FILTER));
-    if (algo_mode == VDNN_ALGO_PERF_OPT && g_engine != VDNN_ENGINE_FFMA && wgrad_small_c_shape(d, Q) && workspace &&
-        (reinterpret_cast<uintptr_t>(dy) & 15u) == 0 && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0)
-        return wgrad_small_c(d, P, Q, x, dy, alpha, beta, dw, 0.0f, 0.0f, nullptr, static_cast<char*>(workspace), workspace_bytes, as_stream(stream));
-    // D[j][k] = sum over pixels of x(j; pixel) * dy(k; pixel), written to dw[k*CRS + j]: the expensive operand, the
-    // gathered input, supplies the 128 tile rows; dy supplies up to 256 columns, so every gathered element feeds up to
-    // 256 multiply-adds and layers with few filters (K = 64) still fill the tile's rows.
-    XGatherFiltRows A; A.g = make_xgather(d, x, P, Q);
-    const SplitDense B = wgrad_dy_view(d, dy, pq);
-    const Epilogue e = filter_epilogue(dw, alpha, beta, crs);
-    if (algo_mode == VDNN_ALGO_PERF_OPT && split16_wgrad_shape(d)) {
-        if (!workspace) return VDNN_ERR_WORKSPACE;
-        if (aligned128(workspace)) {
-            const WgradSpace space = wgrad_space(d, P, Q);
-            if (workspace_bytes < space.total) return VDNN_ERR_WORKSPACE;
-            return wgrad_split16(d, P, Q, x, dy, static_cast<char*>(workspace), space, dw, alpha, beta, nullptr, 0.0f, 0.0f, as_stream(stream));
-        }
-        algo_mode = VDNN_ALGO_MEMORY_OPT;
-    }
-    if (algo_mode == VDNN_ALGO_PERF_OPT) {
-        // workspace variant: dy, which every row tile of the gathered input needs again, is split into tf32 halves and
-        // laid out as tile images once; the kernel's producers then gather x only
-        // (tensors off the 16-byte boundaries of a layer whose workspace is sized for wgrad_small_c: its bytes hold the parts of the
-        // sums, two splits for each SM against that kernel's three blocks, but no images of dy)
-        const size_t pack = wgrad_small_c_shape(d, Q) && g_engine != VDNN_ENGINE_FFMA ? 0 : packed_dy_bytes(d, P, Q);
-        if (pack && (!workspace || workspace_bytes < pack)) return VDNN_ERR_WORKSPACE;
-        char* tiles = (pack && g_engine != VDNN_ENGINE_FFMA && (reinterpret_cast<uintptr_t>(workspace) & 127u) == 0)
-                          ? static_cast<char*>(workspace) : nullptr;
-        return contract<XGatherFiltRows, SplitDense, true, true>(A, B, e, crs, d->k, d->n * pq, static_cast<size_t>(d->k) * crs, 0,
-                                                                 algo_mode, static_cast<char*>(workspace) + pack,
-                                                                 workspace_bytes - pack, as_stream(stream), tiles);
-    }
-    return contract<XGatherFiltRows, SplitDense, true, true>(A, B, e, crs, d->k, d->n * pq, static_cast<size_t>(d->k) * crs, 0,
-                                                             algo_mode, workspace, workspace_bytes, as_stream(stream));
+    return bwd_filter(d, algo_mode, alpha, x, dy, beta, dw, workspace, workspace_bytes, stream, true);
 }
 
 // Bias gradient and filter gradient of one convolution in one call (layer.cu:631-660: cudnnConvolutionBackwardBias, then
@@ -1416,24 +1503,26 @@ int vdnn_conv_bwd_filter_static(const vdnn_conv_desc* d, float alpha, const floa
                                 float* dw, void* stream) {
     int P, Q;
     if (!x || !dy || !dw || !valid_desc(d, &P, &Q)) return VDNN_ERR_BAD_ARG;
-    const bool lists = split16_wgrad_shape(d);
-    // layers that run on lists of operands: 8 bytes per element besides the parts, and as many images at a time as there is room for
-    const size_t need = lists ? 2 * sizeof(float) * (x_elems(d) + y_elems(d, P, Q)) + split16::wgrad_partial_bytes(split16_wgrad_problem(d, P, Q))
-                      : is_full_extent(d) ? vdnn_sgemm_workspace_bytes(VDNN_ALGO_PERF_OPT, d->c * d->r * d->s, d->k, d->n)
-                                          : vdnn_conv_workspace_bytes(VDNN_CONV_BWD_FILTER, VDNN_ALGO_PERF_OPT, d);
+    // what this call takes and refuses: layers of whole blocks of 32 channels by 8 bytes per element besides the parts, others by the
+    // figure of the gather-fed kernel
+    const bool blocks = g_tma_wgrad && !g_no_tma && d->stride_h == 1 && d->stride_w == 1 && !is_full_extent(d) && d->c % 32 == 0 && d->k % 32 == 0;
+    size_t need;
+    if (blocks) need = 2 * sizeof(float) * (x_elems(d) + y_elems(d, P, Q)) + split16::wgrad_partial_bytes(split16_wgrad_problem(d, P, Q));
+    else if (is_full_extent(d)) need = vdnn_sgemm_workspace_bytes(VDNN_ALGO_PERF_OPT, d->c * d->r * d->s, d->k, d->n);
+    else need = wgrad_small_c_shape(d, Q) ? wgrad_small_c_bytes(d) : gathered_filter_bytes(d, P, Q);
     if (need > VDNN_STATIC_SCRATCH_BYTES) return VDNN_ERR_SCRATCH_LIMIT;
     float* scratch = nullptr;
     const int st = static_scratch_address(&scratch);
     if (st != VDNN_OK) return st;
-    if (lists) {
-        if (!fits_int32(d, P, Q)) return VDNN_ERR_UNSUPPORTED;
+    if (split16_wgrad_shape(d)) {           // as many images at a time as there is room for
         const WgradSpace space = wgrad_space(d, P, Q, VDNN_STATIC_SCRATCH_BYTES);
-        if (space.total > VDNN_STATIC_SCRATCH_BYTES) return VDNN_ERR_SCRATCH_LIMIT;
-        return wgrad_split16(d, P, Q, x, dy, reinterpret_cast<char*>(scratch), space, dw, alpha, beta, nullptr, 0.0f, 0.0f, as_stream(stream));
+        if (space.total <= VDNN_STATIC_SCRATCH_BYTES)
+            return wgrad_split16(d, P, Q, x, dy, reinterpret_cast<char*>(scratch), space, dw, alpha, beta, nullptr, 0.0f, 0.0f, as_stream(stream));
     }
+    const bool gather_fits = is_full_extent(d) || wgrad_small_c_shape(d, Q) || gathered_filter_bytes(d, P, Q) <= VDNN_STATIC_SCRATCH_BYTES;
     // The partial sums of every split are written in full before the reduction reads them, so the
     // array's previous contents never matter.
-    return vdnn_conv_bwd_filter(d, VDNN_ALGO_PERF_OPT, alpha, x, dy, beta, dw, scratch, VDNN_STATIC_SCRATCH_BYTES, stream);
+    return bwd_filter(d, gather_fits ? VDNN_ALGO_PERF_OPT : VDNN_ALGO_MEMORY_OPT, alpha, x, dy, beta, dw, scratch, VDNN_STATIC_SCRATCH_BYTES, stream, false);
 }
 
 size_t vdnn_sgemm_workspace_bytes(int algo_mode, int m, int n, int k) {

@@ -54,6 +54,7 @@ struct Problem {
     int out_h, out_w, n_cols;      // output grid and channels
     int R, S, tap_sign, off_h, off_w;
     int wp, lp;                    // list geometry of the layer
+    Fold fold;                     // strided layers: the tensor x or dx, whose folded form the above describes
 };
 
 inline int padded_channels(int c) { return ceil_div(c, KB) * KB; }
@@ -135,6 +136,7 @@ struct StripParams {
     size_t partial_stride;
     const Scales* scales;
     int product;
+    Fold fold;                           // data gradient of a strided layer: where the columns lie in dx
 };
 
 constexpr int STRIP_HALF_BYTES = (BM + 8) * ROW_BYTES;             // 136 rows of 128 bytes, a multiple of the swizzle period
@@ -156,6 +158,26 @@ template <int BN, int MH, int CTAS> struct StripConfig {
     static constexpr uint32_t IDESC_WIDE = idesc(BM, 2 * BN <= 256 ? 2 * BN : 256, false);
     static_assert(TMEM_COLS <= 512 && SMEM_BYTES <= SMEM_LIMIT, "");
 };
+
+// Columns (c, a, b) of position (y, x) of a folded dx: pixel (s y + a - pad_h, s x + b - pad_w) of channel c.
+template <int N>
+__device__ __forceinline__ void store_folded(const StripParams& p, const uint64_t (&acc)[N], int col0, int n, int y, int x, const Unscale& value) {
+    const int s = p.fold.s;
+    int t = col0 / s, b = col0 - t * s, c = t / s, a = t - c * s;
+    float* out = p.out + static_cast<size_t>(n) * p.fold.c * p.fold.h * p.fold.w;
+    if (p.mode == EPI_PARTIAL) out += static_cast<size_t>(blockIdx.z) * p.partial_stride;
+#pragma unroll
+    for (int j = 0; j < 2 * N; ++j) {
+        const int h = s * y + a - p.fold.pad_h, w = s * x + b - p.fold.pad_w;
+        if (col0 + j < p.n_cols && static_cast<unsigned>(h) < static_cast<unsigned>(p.fold.h) && static_cast<unsigned>(w) < static_cast<unsigned>(p.fold.w)) {
+            float* dst = out + (static_cast<size_t>(c) * p.fold.h + h) * p.fold.w + w;
+            float v = value(sum_of(acc, j));
+            if (p.beta != 0.0f) v = fmaf(p.beta, *dst, v);
+            *dst = v;
+        }
+        if (++b == s) { b = 0; if (++a == s) { a = 0; ++c; } }
+    }
+}
 
 template <int BN, int MH, int CTAS>
 __global__ void __launch_bounds__(THREADS, 1)
@@ -246,6 +268,10 @@ strip_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__
                 p.div_wp.divmod(rem, y, x);
                 if (static_cast<int>(y) >= p.out_h || static_cast<int>(x) >= p.out_w) continue;
                 const int col0 = n0 + col_beg;
+                if (p.fold.s > 1) {
+                    store_folded(p, acc[h], col0, static_cast<int>(n), static_cast<int>(y), static_cast<int>(x), value);
+                    continue;
+                }
                 float* dst = p.out + (static_cast<size_t>(n) * p.n_cols + col0) * plane + static_cast<size_t>(y) * p.out_w + x;
                 if (p.mode == EPI_PARTIAL) dst += static_cast<size_t>(blockIdx.z) * p.partial_stride;
                 if (p.beta == 0.0f && col0 + NACC <= p.n_cols) {
@@ -416,6 +442,7 @@ struct WgradParams {
     int mode;
     size_t partial_stride;
     const Scales* scales;
+    Fold fold;                           // strided layers: the filters as they are
 };
 
 constexpr int WGRAD_MAX_STAGES = 6;
@@ -505,7 +532,7 @@ wgrad_kernel(const __grid_constant__ CUtensorMap x_hi, const __grid_constant__ C
         // this thread's rows: group 2 j + (row >> 6) of the CTA, channel row & 63 of its block
         const Unscale value = unscale(p.scales, FILTER, p.mode == EPI_PARTIAL ? 1.0f : p.alpha);
         const int taps = p.R * p.S, row = (warp & 3) * 32 + lane;
-        const size_t crs = static_cast<size_t>(p.C) * taps;
+        const size_t crs = p.fold.s > 1 ? static_cast<size_t>(p.fold.c) * p.fold.R * p.fold.S : static_cast<size_t>(p.C) * taps;
 #pragma unroll
         for (int j = 0; j < T; ++j) {
             const int group = g0 + 2 * j + (row >> 6);
@@ -514,6 +541,11 @@ wgrad_kernel(const __grid_constant__ CUtensorMap x_hi, const __grid_constant__ C
             const int ch = (u * CTAS + static_cast<int>(rank)) * KB + (row & 63);
             if (ch >= p.C) continue;
             float* o = p.out + static_cast<size_t>(ch) * taps + tap;
+            if (p.fold.s > 1) {
+                const int s = p.fold.s, v = ch / s, c = v / s, r = s * (tap / p.S) + v - c * s, q = s * (tap % p.S) + ch - v * s;
+                if (r >= p.fold.R || q >= p.fold.S) continue;
+                o = p.out + (static_cast<size_t>(c) * p.fold.R + r) * p.fold.S + q;
+            }
             if (p.mode == EPI_PARTIAL) o += static_cast<size_t>(blockIdx.z) * p.partial_stride;
 #pragma unroll
             for (int c = 0; c < NACC; ++c) {
@@ -657,6 +689,19 @@ inline int write_lists(const float* src, char* lists, int n, int c, int h, int w
     VDNN_LAUNCHED();
     return VDNN_OK;
 }
+// The lists of a folded x: n images of h2 x w2 positions.
+inline int write_folded_lists(const float* x, char* lists, int n, const Fold& f, int h2, int w2, const ScaleParts& sp, bool fresh, cudaStream_t stream) {
+    const int cp = padded_channels(f.c * f.s * f.s), cblocks = cp / KB;
+    __half* hi = reinterpret_cast<__half*>(lists);
+    __half* lo = hi + static_cast<size_t>(n) * h2 * w2 * cp;
+    const dim3 grid(ceil_div(w2, 64), h2, n * cblocks);
+    if (grid.y > 65535u || grid.z > 65535u) return VDNN_ERR_UNSUPPORTED;
+    auto kern = f.s == 2 ? fold_lists_kernel<2> : (f.s == 3 ? fold_lists_kernel<3> : fold_lists_kernel<4>);
+    VDNN_CUDA(tc::launch_early(kern, grid, 256, 0, stream, x, hi, lo, f, cp, h2, w2, cblocks, sp, fresh ? 1 : 0));
+    VDNN_LAUNCHED();
+    return VDNN_OK;
+}
+
 // Every block of lists_kernel may add the parts of the magnitudes up itself: a load for each thread.
 inline bool few_parts(const ScaleParts& sp) { return sp.blocks[0] <= 256 && sp.blocks[1] <= 256 && sp.blocks[2] <= 256; }
 
@@ -694,6 +739,18 @@ inline size_t packed_bytes(int n_cols, int reduction, int taps) {
 }
 
 // Packs the filters and writes the call's scale record (find_magnitudes() has been called).
+inline int pack_folded(bool data_gradient, const float* w, int K, const Fold& f, int R2, int S2, char* tiles, const ScaleParts& sp, cudaStream_t stream) {
+    const int channels = f.c * f.s * f.s, cols = data_gradient ? channels : K, bn = strip_columns(cols), n_tiles = ceil_div(cols, bn);
+    const int cblocks = padded_channels(data_gradient ? K : channels) / KB;
+    const size_t items = static_cast<size_t>(n_tiles) * R2 * S2 * cblocks * bn * 8, cap = static_cast<size_t>(sm_count()) * 8;
+    size_t blocks = ceil_div<size_t>(items, 256);
+    if (blocks > cap) blocks = cap;
+    const dim3 grid(static_cast<unsigned>(blocks));
+    if (data_gradient) VDNN_CUDA(tc::launch_early(pack_folded_kernel<true>, grid, 256, 0, stream, w, K, f, R2, S2, bn, n_tiles, cblocks, tiles, sp));
+    else VDNN_CUDA(tc::launch_early(pack_folded_kernel<false>, grid, 256, 0, stream, w, K, f, R2, S2, bn, n_tiles, cblocks, tiles, sp));
+    VDNN_LAUNCHED();
+    return VDNN_OK;
+}
 inline int pack_filters(bool data_gradient, const float* w, int K, int C, int R, int S, char* tiles, const ScaleParts& sp, cudaStream_t stream) {
     const int cols = data_gradient ? C : K, bn = strip_columns(cols), n_tiles = ceil_div(cols, bn), cblocks = padded_channels(data_gradient ? K : C) / KB;
     const size_t items = static_cast<size_t>(n_tiles) * R * cblocks * bn * 8, cap = static_cast<size_t>(sm_count()) * 8;
@@ -774,6 +831,8 @@ int strip_launch_as(const Problem& q, const char* lists, const char* b_tiles, fl
     p.kblocks_total = q.R * q.S * p.cblocks;
     p.out = out; p.bias = bias; p.alpha = alpha; p.beta = beta; p.mode = mode; p.partial_stride = partial_stride;
     p.scales = scales; p.product = product;
+    p.fold = q.fold;
+    if (product != DATA) p.fold.s = 1;
     const int ny = ceil_div(q.n_cols, BN);
     if (ny > 65535 || splits > 65535) return VDNN_ERR_UNSUPPORTED;
     CUtensorMap map_hi, map_lo, map_b;
@@ -827,6 +886,8 @@ struct WgradProblem {
     int k, p, q;             // dy: n x k x p x q
     int R, S, pad_h, pad_w;
     int wp, lp;
+    Fold fold;
+    size_t filter_elems() const { return static_cast<size_t>(k) * fold.c * fold.R * fold.S; }
 };
 
 // How a filter gradient is cut.
@@ -882,7 +943,7 @@ inline WgradPlan wgrad_plan(const WgradProblem& q) {
 
 inline size_t wgrad_partial_bytes(const WgradProblem& q) {
     const WgradPlan w = wgrad_plan(q);
-    return w.splits > 1 ? static_cast<size_t>(w.splits) * q.k * q.c * q.R * q.S * sizeof(float) : 0;
+    return w.splits > 1 ? static_cast<size_t>(w.splits) * q.filter_elems() * sizeof(float) : 0;
 }
 
 template <int BN, int T, int CTAS>
@@ -901,7 +962,8 @@ int wgrad_launch_as(const WgradProblem& q, const WgradPlan& w, const char* x_lis
     p.groups = w.groups; p.group_chunk = w.chunk; p.strips = w.strips; p.a_half = w.a_half; p.stages = w.stages;
     p.kb_total = w.kb_total; p.kb_chunk = w.kb_chunk;
     p.C = q.c; p.n_cols = q.k; p.cols_padded = padded_channels(q.k);
-    p.partial_stride = static_cast<size_t>(q.k) * q.c * q.R * q.S;
+    p.partial_stride = q.filter_elems();
+    p.fold = q.fold;
     if (w.splits > 1) { p.out = partial; p.alpha = 1.0f; p.beta = 0.0f; p.mode = EPI_PARTIAL; }
     else { p.out = dw; p.alpha = alpha; p.beta = beta; p.mode = EPI_DIRECT; }
     p.scales = scales;

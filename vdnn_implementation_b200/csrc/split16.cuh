@@ -353,6 +353,102 @@ __global__ void __launch_bounds__(256, SUMS && !VEC ? 3 : 5) lists_kernel(const 
     }
 }
 
+// ---- strided layers -----------------------------------------------------------------------------------------------
+//
+// A convolution of stride s in both directions is one of stride 1 over positions that hold s x s pixels:
+//     x'[(c, a, b)][i][j] = x[c][s i + a - pad_h][s j + b - pad_w],      w'[k][(c, a, b)][u][v] = w[k][c][s u + a][s v + b],
+// with ceil(R / s) x ceil(S / s) taps, no padding, and zeros outside x and past R and S.  The folded tensors exist as lists and
+// packed filters only.
+struct Fold { int s, c, h, w, pad_h, pad_w, R, S; };       // s = 1: not folded; the layer as it is
+
+// As lists_kernel for x' (every position of its h2 x w2 grid is written; there are no gaps).  A block takes 64 channels of x' x 64
+// positions of one row: it brings the rows of x that these need, each in one piece and all in flight at once (17 or 18 loads a
+// thread), into shared memory, and every thread puts chunks of eight channels together from there.
+constexpr int FOLD_MAX = 4;
+template <int S>
+__global__ void __launch_bounds__(256, 4) fold_lists_kernel(const float* x, __half* hi, __half* lo, const Fold f, int cp, int h2, int w2, int cblocks, const ScaleParts sp,
+                                                            int fresh) {
+    constexpr int ROWS = KB / S + 2, SPAN = S * 64, PITCH = SPAN + 1, LOADS = (ROWS * SPAN + 255) / 256;
+    __shared__ float tile[ROWS * PITCH];
+    tc::follow_up();
+    tc::after_predecessor();
+    int e;
+    if (fresh) {
+        int wide;
+        if (blockIdx.x + blockIdx.y + blockIdx.z == 0) write_scales(sp);
+        e = operand_exponent(sp, OP_X, &wide);
+    } else {
+        e = sp.scales->e[OP_X];
+    }
+    const float scale = pow2(e);
+    const int n = blockIdx.z / cblocks, c0 = (blockIdx.z - n * cblocks) * KB, i = blockIdx.y, j0 = blockIdx.x * 64;
+    const int channels = f.c * S * S, row0 = c0 / S, rows = f.c * S - row0;     // (channel, a) rows of x from row0 on
+    const int t = threadIdx.x, w0 = S * j0 - f.pad_w, h0 = S * i - f.pad_h;
+    const float* image = x + static_cast<size_t>(n) * f.c * f.h * f.w;
+    float v[LOADS];
+#pragma unroll
+    for (int k = 0; k < LOADS; ++k) {
+        const int at = t + 256 * k, q = at / SPAN, b = at - q * SPAN, c = (row0 + q) / S, h = h0 + (row0 + q - c * S), w = w0 + b;
+        const bool there = q < ROWS && q < rows && static_cast<unsigned>(h) < static_cast<unsigned>(f.h) && static_cast<unsigned>(w) < static_cast<unsigned>(f.w);
+        v[k] = there ? image[(static_cast<size_t>(c) * f.h + h) * f.w + w] : 0.0f;
+    }
+#pragma unroll
+    for (int k = 0; k < LOADS; ++k) {
+        const int at = t + 256 * k, q = at / SPAN;
+        if (q < ROWS) tile[q * PITCH + at - q * SPAN] = v[k];
+    }
+    __syncthreads();
+    const int oct = t & 7;
+#pragma unroll
+    for (int pass = 0; pass < 2; ++pass) {
+        const int j = pass * 32 + (t >> 3);
+        if (j0 + j >= w2) continue;
+        float u[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int c2 = c0 + oct * 8 + k, row = c2 / S;
+            u[k] = c2 < channels ? tile[(row - row0) * PITCH + S * j + (c2 - row * S)] : 0.0f;
+        }
+        uint4 h, l;
+        split8(u, scale, h, l);
+        const size_t q = ((static_cast<size_t>(n) * h2 + i) * w2 + j0 + j) * cp + c0 + oct * 8;
+        *reinterpret_cast<uint4*>(hi + q) = h;
+        *reinterpret_cast<uint4*>(lo + q) = l;
+    }
+}
+
+// As pack_filters_kernel for w'.
+template <bool DATA_GRADIENT>
+__global__ void __launch_bounds__(256) pack_folded_kernel(const float* w, int K, const Fold f, int R2, int S2, int bn, int n_tiles, int cblocks, char* out,
+                                                          const ScaleParts sp) {
+    tc::follow_up();
+    tc::after_predecessor();
+    if (blockIdx.x == 0) write_scales(sp);
+    int wide;
+    const float scale = pow2(operand_exponent(sp, OP_W, &wide));
+    const int s = f.s, channels = f.c * s * s, cols = DATA_GRADIENT ? channels : K, red = DATA_GRADIENT ? K : channels, kblocks = R2 * S2 * cblocks;
+    const size_t items = static_cast<size_t>(n_tiles) * kblocks * bn * 8, stride = static_cast<size_t>(gridDim.x) * 256;
+    for (size_t it = static_cast<size_t>(blockIdx.x) * 256 + threadIdx.x; it < items; it += stride) {
+        const int chunk = static_cast<int>(it & 7), row = static_cast<int>((it >> 3) % bn);
+        const size_t tile = (it >> 3) / bn;                                     // nt * kblocks + kb
+        const int kb = static_cast<int>(tile % kblocks), nt = static_cast<int>(tile / kblocks);
+        const int tap = kb / cblocks, u = tap / S2, v2 = tap - u * S2, c0 = (kb - tap * cblocks) * KB + chunk * 8, col = nt * bn + row;
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int k = DATA_GRADIENT ? c0 + j : col, c2 = DATA_GRADIENT ? col : c0 + j;
+            const int t = c2 / s, b = c2 - t * s, c = t / s, a = t - c * s, r = s * u + a, q = s * v2 + b;
+            const bool there = col < cols && c0 + j < red && r < f.R && q < f.S;
+            v[j] = there ? w[((static_cast<size_t>(k) * f.c + c) * f.R + r) * f.S + q] : 0.0f;
+        }
+        uint4 hi, lo;
+        split8(v, scale, hi, lo);
+        char* dst = out + tile * (2 * bn * ROW_BYTES) + tc::swz(row, chunk);
+        *reinterpret_cast<uint4*>(dst) = hi;
+        *reinterpret_cast<uint4*>(dst + bn * ROW_BYTES) = lo;
+    }
+}
+
 // ---- tensor-core side ---------------------------------------------------------------------------------------------
 
 // Instruction descriptor: D = F32, A = B = F16; MN = both operands MN-major.
