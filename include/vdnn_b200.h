@@ -51,10 +51,10 @@ const char* vdnn_build_info(void);
 typedef enum { VDNN_ALGO_MEMORY_OPT = 0, VDNN_ALGO_PERF_OPT = 1, VDNN_ALGO_DYNAMIC = 2 } vdnn_algo_mode;
 typedef enum { VDNN_CONV_FWD = 0, VDNN_CONV_BWD_DATA = 1, VDNN_CONV_BWD_FILTER = 2,
                VDNN_CONV_BWD_ALL = 3 /* the three gradients in one workspace: vdnn_conv_bwd_data_filter_bias */ } vdnn_conv_op;
-/* Which contraction engine runs CONV/FC.  AUTO picks TCGEN05 (3xTF32 on the 5th-generation
+/* Which contraction engine runs CONV/FC.  AUTO picks TCGEN05 (operands as pairs of tf32 or f16 values on the 5th-generation
  * tensor cores, fp32-accurate) when the shape is supported by it and FFMA otherwise.  In PERF_OPT the tensor-core
- * engine has a gather-fed and a TMA-fed kernel family; AUTO uses the TMA-fed one for stride-1 convolutions with
- * enough output tiles to fill the GPU, TCGEN05 for every shape it supports (workspace sizes follow the setting). */
+ * engine has a gather-fed and a TMA-fed kernel family; AUTO uses the one that is estimated the faster for the layer, TCGEN05
+ * the TMA-fed one for every shape it supports (workspace sizes follow the setting). */
 typedef enum { VDNN_ENGINE_AUTO = 0, VDNN_ENGINE_FFMA = 1, VDNN_ENGINE_TCGEN05 = 2 } vdnn_engine;
 int vdnn_set_engine(int engine);   /* process-wide; returns the previous value */
 int vdnn_get_engine(void);
@@ -94,7 +94,7 @@ int vdnn_pool_out_dims(int h, int w, int win_h, int win_w, int stride_h, int str
 /* cudnnGetConvolution{Forward,BackwardData,BackwardFilter}WorkspaceSize (layer.cu:268-294)
  * together with the algorithm choice of find{MemOpt,PerfOpt}*Algo (layer.cu:1013-1089):
  * 0 for VDNN_ALGO_MEMORY_OPT; otherwise what the PERF_OPT kernel that takes the shape reads or writes beside the tensors
- * (operand images, packed weights, split-K parts), 0 where it needs none. */
+ * (operand lists, packed weights, split-K parts), 0 where it needs none. */
 size_t vdnn_conv_workspace_bytes(int op, int algo_mode, const vdnn_conv_desc* d);
 
 /* cudnnConvolutionForward (layer.cu:560-569): y = alpha * (x corr w) + beta * y.
@@ -134,7 +134,7 @@ int vdnn_conv_bwd_filter_bias(const vdnn_conv_desc* d, int algo_mode, float alph
  * Workspace: vdnn_conv_workspace_bytes(VDNN_CONV_BWD_ALL, mode, d); where vdnn_conv_bwd_shares_dy is 1 the figure for
  * VDNN_CONV_BWD_FILTER is at least as large, elsewhere it is the larger of the two separate figures.
  * In PERF_OPT, where both gradients run on the TMA-fed kernels (vdnn_conv_bwd_shares_dy), dy is rewritten into operand
- * images once for both and the bias sums come from the same pass; elsewhere the separate entry points run in the
+ * lists once for both; elsewhere the separate entry points run in the
  * reference's order. */
 int vdnn_conv_bwd_data_filter_bias(const vdnn_conv_desc* d, int algo_mode, float alpha_dx, const float* w, const float* x,
                                    const float* dy, float beta_dx, float* dx, float alpha_w, float beta_w, float* dw,

@@ -378,7 +378,7 @@ int Layer::convolutionBackward(int _layer_id_to_prefetch, DATATYPE* _prefetchedS
     }
     // bias, then filter: gradient folded into the parameters (alpha = -lr, beta = 1), or written to
     // the staging buffer when gradients are all-reduced across ranks first.  One call: where the filter gradient
-    // prepares dy as operand images, that pass forms the bias sums as well.
+    // writes a large dy as operand lists, that pass forms the bias sums as well.
     if (workSpace != NULL) curWorkSpace = workSpace;
     else if (bwdFilterWorkSpaceSize > 0) {
         const int a = handle->alloc(&curWorkSpace, bwdFilterWorkSpaceSize, layerId, TAG_WS, isDynamic, {*stream_compute});

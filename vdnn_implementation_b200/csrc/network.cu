@@ -530,7 +530,7 @@ size_t Network::findMaxDxDySize() {
 }
 
 // network.cu:1025-1040 keeps this maximum in an int.  cuDNN's workspaces of a few GB then wrap and the shared block
-// comes out too small; this library's own workspaces (operand images of the large layers) pass 2^31 bytes as well,
+// comes out too small; this library's own workspaces (operand lists of the large layers) pass 2^31 bytes as well,
 // and a kernel writing them into a wrapped-size block would overrun it.  The maximum is therefore kept in 64 bits,
 // and BASELINE hands the shared block's true size to every call so that the size check of the C ABI is real.
 size_t Network::findMaxWorkSpaceSize() {
