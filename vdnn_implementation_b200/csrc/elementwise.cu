@@ -156,10 +156,21 @@ __global__ void __launch_bounds__(kThreads) act_bwd_kernel(size_t n4, size_t n, 
 }
 
 // ---------------------------------------------------------------- out = a - b, w += alpha g, fill
-__global__ void __launch_bounds__(kThreads) sub_kernel(size_t n, const float* __restrict__ a,
-                                                       const float* __restrict__ b, float* __restrict__ out) {
+// The loss's seed and the softmax kernels below end every step, a few microseconds each, and are launched early
+// (tc::launch_early): the four of 64 x 1000 called one behind the other take 12.7 us instead of 20.5.  Such a kernel starts beside its predecessor, so it reads what that one wrote by plain loads through
+// plain pointers: nothing may be fetched ahead, or through the read-only path, of the wait.
+__global__ void __launch_bounds__(kThreads) sub_kernel(size_t n4, size_t n, const float* a, const float* b, float* out) {
     const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
-    for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) out[i] = a[i] - b[i];
+    const size_t first = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    tc::follow_up();
+    tc::after_predecessor();
+    const float4* a4 = reinterpret_cast<const float4*>(a);
+    const float4* b4 = reinterpret_cast<const float4*>(b);
+    for (size_t i = first; i < n4; i += stride) {
+        const float4 u = a4[i], v = b4[i];
+        reinterpret_cast<float4*>(out)[i] = make_float4(u.x - v.x, u.y - v.y, u.z - v.z, u.w - v.w);
+    }
+    for (size_t j = n4 * 4 + first; j < n; j += stride) out[j] = a[j] - b[j];
 }
 
 __global__ void __launch_bounds__(kThreads) axpy_kernel(size_t n4, size_t n, float alpha, const float* __restrict__ g,
@@ -610,7 +621,7 @@ __device__ __forceinline__ double warp_sum_f64(double v) {
     return v;
 }
 
-// Sum over the block of one double per thread, in every thread; blocks of at most 8 warps.
+// Sum over the block of one double per thread, in every thread; `part` holds one per warp.
 __device__ __forceinline__ double block_sum_f64(double v, double* part) {
     v = warp_sum_f64(v);
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
@@ -624,13 +635,36 @@ __device__ __forceinline__ double block_sum_f64(double v, double* part) {
 // expression dy - sum(dy*y) cancels almost completely, and a float sum would leave only a few
 // correct bits.  The tensors stay fp32; the extra cost on N x 1000 elements is nil.
 //
-// A block per row, the row in registers (rows of up to 8 * 256 values; longer ones are read again in every pass).  These
-// calls are bound by latency: with one warp per row and a dependent loop per pass, 64 rows of 1000 took 7.2 us forward and
-// 5.2 backward; now 2.8 and 2.3.
-constexpr int ROW_VALUES = 8;
-__global__ void __launch_bounds__(256) softmax_fwd_kernel(int cols, const float* __restrict__ x, float* __restrict__ y) {
-    __shared__ float part_m[8];
-    __shared__ double part_s[8];
+// A block per row, the row in registers (rows of up to 8 * 1024 values; longer ones are read again in every pass: with
+// 256 threads at most, 256 rows of 4000 took 5.2 us forward and 4.2 backward; now 3.6 and 3.2).  These calls are bound by
+// latency: with one warp per row and a dependent loop per pass, 64 rows of 1000 took 7.2 us forward and 5.2 backward; now 2.1
+// and 1.8.  The followers are let in late, when the row is summed: let in at the start, their blocks
+// take slots beside rows that still load (256 x 4000: 7.5 us forward, so 3.6).
+constexpr int ROW_VALUES = 8, ROW_THREADS = 1024;
+
+// f(j, p[j], q[j]) for this thread's columns behind the register pass, ROW_VALUES loads in flight at a time: through plain
+// pointers the compiler would not fetch ahead of the stores that f may do.
+template <class F>
+__device__ __forceinline__ void beyond_registers(int cols, const float* p, const float* q, F f) {
+    const int t = threadIdx.x, nt = blockDim.x;
+    for (int j0 = t + ROW_VALUES * nt; j0 < cols; j0 += ROW_VALUES * nt) {
+        float a[ROW_VALUES], b[ROW_VALUES];
+#pragma unroll
+        for (int u = 0; u < ROW_VALUES; ++u) {
+            const int j = j0 + u * nt;
+            a[u] = j < cols ? p[j] : 0.0f;
+            b[u] = j < cols && q != p ? q[j] : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < ROW_VALUES; ++u)
+            if (j0 + u * nt < cols) f(j0 + u * nt, a[u], b[u]);
+    }
+}
+
+__global__ void __launch_bounds__(ROW_THREADS) softmax_fwd_kernel(int cols, const float* x, float* y) {
+    __shared__ float part_m[ROW_THREADS / 32];
+    __shared__ double part_s[ROW_THREADS / 32];
+    tc::after_predecessor();
     const float* xr = x + static_cast<size_t>(blockIdx.x) * cols;
     float* yr = y + static_cast<size_t>(blockIdx.x) * cols;
     const int t = threadIdx.x, nt = blockDim.x;
@@ -640,7 +674,7 @@ __global__ void __launch_bounds__(256) softmax_fwd_kernel(int cols, const float*
     for (int u = 0; u < ROW_VALUES; ++u) { v[u] = t + u * nt < cols ? xr[t + u * nt] : -INFINITY; }
 #pragma unroll
     for (int u = 0; u < ROW_VALUES; ++u) m = fmaxf(m, v[u]);
-    for (int j = t + ROW_VALUES * nt; j < cols; j += nt) m = fmaxf(m, xr[j]);
+    beyond_registers(cols, xr, xr, [&](int, float a, float) { m = fmaxf(m, a); });
     m = warp_max(m);
     if ((t & 31) == 0) part_m[t >> 5] = m;
     __syncthreads();
@@ -650,17 +684,18 @@ __global__ void __launch_bounds__(256) softmax_fwd_kernel(int cols, const float*
 #pragma unroll
     for (int u = 0; u < ROW_VALUES; ++u)
         if (t + u * nt < cols) { v[u] = expf(v[u] - m); s += static_cast<double>(v[u]); }
-    for (int j = t + ROW_VALUES * nt; j < cols; j += nt) s += static_cast<double>(expf(xr[j] - m));
+    beyond_registers(cols, xr, xr, [&](int, float a, float) { s += static_cast<double>(expf(a - m)); });
     const double inv = 1.0 / block_sum_f64(s, part_s);
+    tc::follow_up();
 #pragma unroll
     for (int u = 0; u < ROW_VALUES; ++u)
         if (t + u * nt < cols) yr[t + u * nt] = static_cast<float>(static_cast<double>(v[u]) * inv);
-    for (int j = t + ROW_VALUES * nt; j < cols; j += nt) yr[j] = static_cast<float>(static_cast<double>(expf(xr[j] - m)) * inv);
+    beyond_registers(cols, xr, xr, [&](int j, float a, float) { yr[j] = static_cast<float>(static_cast<double>(expf(a - m)) * inv); });
 }
 
-__global__ void __launch_bounds__(256) softmax_bwd_kernel(int cols, const float* __restrict__ y, const float* __restrict__ dy,
-                                                          float* __restrict__ dx) {
-    __shared__ double part_s[8];
+__global__ void __launch_bounds__(ROW_THREADS) softmax_bwd_kernel(int cols, const float* y, const float* dy, float* dx) {
+    __shared__ double part_s[ROW_THREADS / 32];
+    tc::after_predecessor();
     const size_t row = static_cast<size_t>(blockIdx.x) * cols;
     const int t = threadIdx.x, nt = blockDim.x;
     float a[ROW_VALUES], g[ROW_VALUES];
@@ -674,23 +709,27 @@ __global__ void __launch_bounds__(256) softmax_bwd_kernel(int cols, const float*
 #pragma unroll
     for (int u = 0; u < ROW_VALUES; ++u)
         if (t + u * nt < cols) dot += static_cast<double>(a[u]) * static_cast<double>(g[u]);
-    for (int j = t + ROW_VALUES * nt; j < cols; j += nt) dot += static_cast<double>(y[row + j]) * static_cast<double>(dy[row + j]);
+    beyond_registers(cols, y + row, dy + row, [&](int, float p, float q) { dot += static_cast<double>(p) * static_cast<double>(q); });
     dot = block_sum_f64(dot, part_s);
+    tc::follow_up();
 #pragma unroll
     for (int u = 0; u < ROW_VALUES; ++u)
         if (t + u * nt < cols) dx[row + t + u * nt] = static_cast<float>(static_cast<double>(a[u]) * (static_cast<double>(g[u]) - dot));
-    for (int j = t + ROW_VALUES * nt; j < cols; j += nt)
-        dx[row + j] = static_cast<float>(static_cast<double>(y[row + j]) * (static_cast<double>(dy[row + j]) - dot));
+    beyond_registers(cols, y + row, dy + row, [&](int j, float p, float q) {
+        dx[row + j] = static_cast<float>(static_cast<double>(p) * (static_cast<double>(q) - dot));
+    });
 }
 
 // ---------------------------------------------------------------- loss (one cluster)
 // A warp per row, the rows dealt to the warps of up to eight blocks; the blocks' sums meet through distributed shared
 // memory in rank order.  One block of 32 warps took 11.1 us for 64 x 1000 (two rows after another per warp, 32 dependent
-// trips each); now 4.6.
-__global__ void __launch_bounds__(512) loss_kernel(int rows, int cols, const float* __restrict__ y,
-                                                   const float* __restrict__ label, double* __restrict__ out2) {
-    __shared__ double s_sq[16], s_ce[16];
+// trips each), 8 x 512 threads 4.2.
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) loss_kernel(int rows, int cols, const float* y, const float* label, double* out2) {
+    __shared__ double s_sq[THREADS / 32], s_ce[THREADS / 32];
     __shared__ double block[2];
+    tc::follow_up();
+    tc::after_predecessor();
     cg::cluster_group cluster = cg::this_cluster();
     double sq = 0.0, ce = 0.0;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
@@ -925,7 +964,8 @@ int vdnn_activation_bwd(int mode, size_t count, const float* y, const float* dy,
 int vdnn_sub(size_t count, const float* a, const float* b, float* out, void* stream) {
     if (!a || !b || !out) return VDNN_ERR_BAD_ARG;
     if (count == 0) return VDNN_OK;
-    sub_kernel<<<stream_grid(count, 1), kThreads, 0, as_stream(stream)>>>(count, a, b, out);
+    const size_t n4 = (aligned16(a) && aligned16(b) && aligned16(out)) ? count / 4 : 0;
+    VDNN_CUDA(tc::launch_early(sub_kernel, dim3(stream_grid(n4 ? n4 : count, 1)), kThreads, 0, as_stream(stream), n4, count, a, b, out));
     VDNN_LAUNCHED();
     return VDNN_OK;
 }
@@ -1111,38 +1151,45 @@ int vdnn_maxpool_bwd(int n, int c, int h, int w, int win_h, int win_w, int strid
     return VDNN_OK;
 }
 
-// Threads of a softmax block: a register pass of ROW_VALUES values each covers the row, 32 .. 256.
+// Threads of a softmax block: four values each up to 256 threads, then up to ROW_VALUES each and more threads.
 static int softmax_threads(int cols) {
     int t = 32;
     while (t < 256 && t * 4 < cols) t *= 2;
+    while (t < ROW_THREADS && t * ROW_VALUES < cols) t *= 2;
     return t;
 }
 
 int vdnn_softmax_fwd(int rows, int cols, const float* x, float* y, void* stream) {
     if (!x || !y || rows <= 0 || cols <= 0) return VDNN_ERR_BAD_ARG;
-    softmax_fwd_kernel<<<rows, softmax_threads(cols), 0, as_stream(stream)>>>(cols, x, y);
+    VDNN_CUDA(tc::launch_early(softmax_fwd_kernel, dim3(rows), softmax_threads(cols), 0, as_stream(stream), cols, x, y));
     VDNN_LAUNCHED();
     return VDNN_OK;
 }
 
 int vdnn_softmax_bwd(int rows, int cols, const float* y, const float* dy, float* dx, void* stream) {
     if (!y || !dy || !dx || rows <= 0 || cols <= 0) return VDNN_ERR_BAD_ARG;
-    softmax_bwd_kernel<<<rows, softmax_threads(cols), 0, as_stream(stream)>>>(cols, y, dy, dx);
+    VDNN_CUDA(tc::launch_early(softmax_bwd_kernel, dim3(rows), softmax_threads(cols), 0, as_stream(stream), cols, y, dy, dx));
     VDNN_LAUNCHED();
     return VDNN_OK;
 }
 
 int vdnn_loss(int rows, int cols, const float* y, const float* label, double* out2, void* stream) {
     if (!y || !label || !out2 || rows <= 0 || cols <= 0) return VDNN_ERR_BAD_ARG;
+    // A warp per row up to 8 * 32 rows.  Fewer warps have more registers for loads in flight and meet sooner, so up to 8 * 16 rows
+    // take 512 threads (128 x 1000: 4.6 us, with 1024 5.0; 256 x 1000: 7.5 and 6.6).
+    const bool wide = rows > 8 * 16;
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = rows >= 8 ? 8 : 1;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr; cfg.numAttrs = 1;
-    cfg.gridDim = dim3(attr[0].val.clusterDim.x); cfg.blockDim = dim3(512);
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = 2;
+    cfg.gridDim = dim3(attr[0].val.clusterDim.x); cfg.blockDim = dim3(wide ? 1024 : 512);
     cfg.stream = as_stream(stream);
-    VDNN_CUDA(cudaLaunchKernelEx(&cfg, loss_kernel, rows, cols, y, label, out2));
+    if (wide) VDNN_CUDA(cudaLaunchKernelEx(&cfg, loss_kernel<1024>, rows, cols, y, label, out2));
+    else VDNN_CUDA(cudaLaunchKernelEx(&cfg, loss_kernel<512>, rows, cols, y, label, out2));
     VDNN_LAUNCHED();
     return VDNN_OK;
 }

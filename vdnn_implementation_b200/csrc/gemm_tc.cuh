@@ -239,23 +239,6 @@ struct Gather {
     }
 };
 
-// The kernels of one layer call follow each other within microseconds of work.  Launched like this a kernel may start while its
-// predecessor in the stream still runs (which says so by follow_up()) and sets itself up; its after_predecessor(), before the
-// first global access, waits until all of the predecessor's results are visible.  A kernel launched otherwise waits as always.
-// Measured: 5 x 48 x 27 x 31 -> 80, 3 x 3, forward and backward (nine kernels, 64 us of work): 78 -> 65 us.
-__device__ __forceinline__ void after_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void follow_up() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-template <class Kernel, class... Args>
-inline cudaError_t launch_early(Kernel kern, dim3 grid, int threads, size_t smem, cudaStream_t stream, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
-    cfg.attrs = attr; cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, args...);
-}
-
 // BBULK: the B operand was packed beforehand into images of its shared-memory tiles (hi and lo halves,
 // swizzled, zero-padded; see pack_b_tiles_kernel), one image per (n tile, k block).  A producer thread then
 // fetches a stage's B tiles with a single bulk asynchronous copy (the TMA engine, no tensor map needed for a
