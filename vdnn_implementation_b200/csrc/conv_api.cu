@@ -480,17 +480,19 @@ double gathered_us(int M, int N, int K, bool may_split, bool strided) {
     int splits = 1;
     if (may_split && tiles < sm_count()) splits = max(1, min(static_cast<int>(2 * sm_count() / tiles), K / 64));
     const double waves = static_cast<double>(ceil_div<long long>(tiles * splits, bn == 64 ? 2 * sm_count() : sm_count()));
-    static const GatherRate plain[3] = {{1.4, 1.5}, {0.8, 4.9}, {1.18, 7.7}}, fwd[3] = {{2.4, 4.0}, {0.89, 7.8}, {1.33, 9.1}}, data[3] = {{1.2, 0.0}, {0.69, 0.0}, {1.24, 0.0}};
+    static const GatherRate plain[3] = {{1.4, 1.5}, {0.8, 4.9}, {1.18, 7.7}}, fwd[3] = {{2.4, 4.0}, {0.89, 7.8}, {1.33, 9.1}}, data[3] = {{1.2, 0.0}, {0.69, 0.0}, {1.24, 0.0}};       // data gradients below 40 us start at 11
     GatherRate rate = !strided ? plain[size] : (may_split ? data[size] : fwd[size]);
     if (strided && !may_split && bn == 64 && tiles <= sm_count()) rate.block *= 0.5;      // a CTA has its SM to itself
-    return (strided && may_split ? 27.0 : (may_split ? 7.0 : 3.0)) + waves * (rate.block * ceil_div(blocks, splits) + rate.wave);
+    return (strided && may_split ? 14.0 : (may_split ? 7.0 : 3.0)) + waves * (rate.block * ceil_div(blocks, splits) + rate.wave);
 }
+
+// Folded channels that fill most of their blocks of 64: a first layer of stride 4, or 16 channels and more.
+// Small images cost the folding pass up to three times as much per element: its blocks take positions of one image.
+double small_images(const vdnn_conv_desc* d) { return 1.0 + 2.0 * min(1.0, 100.0 / (static_cast<double>(d->h) * d->w)); }
+bool useful_channels(int c) { return 10 * c >= 7 * split16::padded_channels(c); }
 
 // Forward and data gradient.  With the engine forced to VDNN_ENGINE_TCGEN05 every eligible shape runs on lists (small shapes in the
 // tests).
-// Folded channels that fill most of their blocks of 64: a first layer of stride 4, or 16 channels and more.
-bool useful_channels(int c) { return 10 * c >= 7 * split16::padded_channels(c); }
-
 bool choose_strips(const vdnn_conv_desc* d, int op) {
     if (!split16_layer(d) || (op != VDNN_CONV_FWD && op != VDNN_CONV_BWD_DATA)) return false;
     const bool fwd = op == VDNN_CONV_FWD;
@@ -509,14 +511,15 @@ bool choose_strips(const vdnn_conv_desc* d, int op) {
     const double blocks = waves * plan.group_chunk * split16::taps_per_strip(q.S), parts = plan.splits > 1 ? 1 + 2 * plan.splits : 1;
     const int M = fwd ? d->n * P * Q : d->n * d->h * d->w, N = fwd ? d->k : d->c, K = (fwd ? d->c : d->k) * d->r * d->s;
     if (d->stride_h > 1) {
-        // Folded layers, fitted to 100 of stride 2 and 4.  The data gradient gains most (2.3 times as fast on average: the gather
-        // tests every tap of every pixel and multiplies zeros, the first layers' kernels do 33 TFLOP/s of multiply-adds); forward is
-        // bound by its passes, and taken where it is surely the faster.
-        if (fwd) return useful_channels(q.cin) && 1.15 * (14.5 + 5.5 * src + 3.2 * out * parts + 8.2 * weights) < gathered_us(M, N, K, false, true);
-        const double lists = 18.0 + 0.77 * blocks + 1.2 * src + 2.0 * out * parts + 5.1 * weights;
-        return 1.1 * lists < (first ? 10.0 + 78e-9 * d->n * P * Q * d->k * d->c * d->r * d->s : gathered_us(M, N, K, true, true));
+        // Folded layers, fitted to 100 of stride 2 and 4 and corrected by 100 small ones (150 .. 30000 outputs), which lost up to
+        // 2.5 times as the data gradient and twice as forward before.  The data gradient gains most, 2 times and more from 1 GFLOP up: the
+        // gather tests every tap of every pixel and multiplies zeros, the first layers' kernels do 33 TFLOP/s of multiply-adds.
+        // Forward is bound by its passes, and taken where it is surely the faster.
+        if (fwd) return useful_channels(q.cin) && 1.1 * (25.0 + 0.4 * blocks + 5.5 * small_images(d) * src + 2.2 * out * parts + 5.0 * weights) < gathered_us(M, N, K, false, true);
+        const double lists = 26.0 + 0.77 * blocks + 1.2 * src + 2.0 * out * parts + 5.1 * weights;
+        return lists < (first ? 10.0 + 78e-9 * d->n * P * Q * d->k * d->c * d->r * d->s : gathered_us(M, N, K, true, true));
     }
-    const double lists = 20.0 + 0.8 * blocks + 1.8 * src + 1.1 * out * parts + 7.7 * weights;
+    const double lists = (fwd ? 25.0 : 20.0) + 0.8 * blocks + 1.8 * src + 1.1 * out * parts + 7.7 * weights;
     return lists < gathered_us(M, N, K, !fwd, false) + 0.5 * (src + out);
 }
 
@@ -542,8 +545,8 @@ bool choose_wgrad(const vdnn_conv_desc* d) {
     const double gathered = 10.0 + gwaves * ((bn == 64 ? 1.16 : (bn == 128 ? 1.2 : 1.5)) * (split.k_chunk / 32) + 3.3) + 1.4 * (split.splits > 1 ? split.splits : 0) * dw +
                             (d->k >= 128 ? 3.25 : 0.0) * dy + 1.2 * dw;
     if (d->stride_h > 1) {      // folded: bound by the passes over x; taken where surely faster
-        lists = 23.3 - launches + waves * ((w.bn == 64 ? 0.0 : 0.45) * w.kb_chunk + 6.2) + 4.4 * (both - spared) + 4.6 * w.splits * dw;
-        return useful_channels(q.c) && (shared ? 1.2 : 1.6) * lists < 1.3 * gathered;
+        lists = 23.3 - launches + waves * ((w.bn == 64 ? 0.0 : 0.45) * w.kb_chunk + 6.2) + 4.4 * small_images(d) * (both - spared) + 4.6 * w.splits * dw;
+        return useful_channels(q.c) && (shared ? 1.3 : 1.6) * lists < gathered;
     }
     return lists < 1.3 * gathered;          // the gather's time is the less certain one, and errs upwards
 }

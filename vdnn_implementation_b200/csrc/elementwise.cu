@@ -157,8 +157,9 @@ __global__ void __launch_bounds__(kThreads) act_bwd_kernel(size_t n4, size_t n, 
 
 // ---------------------------------------------------------------- out = a - b, w += alpha g, fill
 // The loss's seed and the softmax kernels below end every step, a few microseconds each, and are launched early
-// (tc::launch_early): the four of 64 x 1000 called one behind the other take 12.7 us instead of 20.5.  Such a kernel starts beside its predecessor, so it reads what that one wrote by plain loads through
-// plain pointers: nothing may be fetched ahead, or through the read-only path, of the wait.
+// (tc::launch_early): the four of 64 x 1000 called one behind the other take 12.7 us instead of 20.5.  Such a kernel starts
+// beside its predecessor, so it reads what that one wrote by plain loads through plain pointers: nothing may be fetched ahead,
+// or through the read-only path, of the wait.
 __global__ void __launch_bounds__(kThreads) sub_kernel(size_t n4, size_t n, const float* a, const float* b, float* out) {
     const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
     const size_t first = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -638,8 +639,8 @@ __device__ __forceinline__ double block_sum_f64(double v, double* part) {
 // A block per row, the row in registers (rows of up to 8 * 1024 values; longer ones are read again in every pass: with
 // 256 threads at most, 256 rows of 4000 took 5.2 us forward and 4.2 backward; now 3.6 and 3.2).  These calls are bound by
 // latency: with one warp per row and a dependent loop per pass, 64 rows of 1000 took 7.2 us forward and 5.2 backward; now 2.1
-// and 1.8.  The followers are let in late, when the row is summed: let in at the start, their blocks
-// take slots beside rows that still load (256 x 4000: 7.5 us forward, so 3.6).
+// and 1.8.  The followers are let in late, when the row is summed: let in at the start, their blocks take slots beside rows
+// that still load (256 x 4000 with 256 threads: 7.5 us forward instead of 5.2).
 constexpr int ROW_VALUES = 8, ROW_THREADS = 1024;
 
 // f(j, p[j], q[j]) for this thread's columns behind the register pass, ROW_VALUES loads in flight at a time: through plain
