@@ -545,8 +545,8 @@ bool choose_wgrad(const vdnn_conv_desc* d) {
     const double gathered = 10.0 + gwaves * ((bn == 64 ? 1.16 : (bn == 128 ? 1.2 : 1.5)) * (split.k_chunk / 32) + 3.3) + 1.4 * (split.splits > 1 ? split.splits : 0) * dw +
                             (d->k >= 128 ? 3.25 : 0.0) * dy + 1.2 * dw;
     if (d->stride_h > 1) {      // folded: bound by the passes over x; taken where surely faster
-        lists = 23.3 - launches + waves * ((w.bn == 64 ? 0.0 : 0.45) * w.kb_chunk + 6.2) + 4.4 * small_images(d) * (both - spared) + 4.6 * w.splits * dw;
-        return useful_channels(q.c) && (shared ? 1.3 : 1.6) * lists < gathered;
+        lists = 41.0 - launches + waves * ((w.bn == 64 ? 0.0 : 0.45) * w.kb_chunk + 6.2) + 4.4 * small_images(d) * (both - spared) + 4.6 * w.splits * dw;
+        return useful_channels(q.c) && (shared ? 1.2 : 1.6) * lists < 1.3 * gathered;
     }
     return lists < 1.3 * gathered;          // the gather's time is the less certain one, and errs upwards
 }
